@@ -58,7 +58,7 @@ struct asg_ctx {
     int n = 0;
     float left = 0.f, right = 0.f;
     bool loaded = false, knn_done = false, rk_checked = false, idx33_all = false;
-    int leaf = 32;  // tree bucket size scanned whole by the traversals (fastest on GB300)
+    int leaf = LEAF_DEFAULT;  // particles per tree leaf
     int dep_seg = 4096;  // pairs per deposit work item
     int knn_warps = 2;   // warps per block of the neighbour search (2 or 4)
     int dep_mma = deposit_default_mma();  // deposit engine: tensor cores (1, 2) or CUDA cores (0)
@@ -67,10 +67,9 @@ struct asg_ctx {
 
     Buf aos, pos_in, vel_in, igrp_in, rk_in, keys0, keys1, vals0, vals1, sort_tmp;
     Buf pos, vel, igrp, rk, t33, idx33;
-    Buf meta, parent, leaf_parent, flags, blo, bhi;
+    Buf boxes;       // boxes of the tree (TreeView::box)
     Buf dacc, dexp;  // dens: fixed-point sums and scale exponents
-    Buf blist;       // buckets each bundle's neighbour search scanned
-    Buf nrec;        // tree node records (TreeView::rec)
+    Buf blist;       // leaves each bundle's neighbour search scanned
     Buf dep_order;   // the deposit's tile processing order and its inverse
     std::vector<int> dep_order_key;  // the mesh sizes dep_order was made for
     bool dep_order_on = true;        // ASG_DEPOSIT_ORDER=tile: tile order
@@ -225,19 +224,14 @@ int finish(asg_ctx* ctx, const char* what)
 
 TreeView tree_view(asg_ctx* ctx)
 {
-    TreeView t;
-    t.n = ctx->n;
-    t.leaf = ctx->leaf;
-    t.meta = P<int4>(ctx->meta);
-    t.blo = P<float4>(ctx->blo);
-    t.bhi = P<float4>(ctx->bhi);
-    t.rec = P<float4>(ctx->nrec);
+    TreeView t = tree_shape(ctx->n, ctx->leaf);
+    t.box = P<float4>(ctx->boxes);
     return t;
 }
 
 int alloc_set(asg_ctx* ctx, int n)
 {
-    const size_t N = (size_t)n, M = (size_t)(n > 1 ? n - 1 : 1);
+    const size_t N = (size_t)n;
     int r = 0;
     r |= grow(ctx, ctx->pos_in, 16 * N);
     r |= grow(ctx, ctx->vel_in, 16 * N);
@@ -254,13 +248,7 @@ int alloc_set(asg_ctx* ctx, int n)
     r |= grow(ctx, ctx->rk, 4 * N);
     r |= grow(ctx, ctx->t33, 4 * N);
     r |= grow(ctx, ctx->idx33, 4 * N);
-    r |= grow(ctx, ctx->meta, 16 * M);
-    r |= grow(ctx, ctx->parent, 4 * M);
-    r |= grow(ctx, ctx->leaf_parent, 4 * N);
-    r |= grow(ctx, ctx->flags, 4 * M);
-    r |= grow(ctx, ctx->blo, 16 * M);
-    r |= grow(ctx, ctx->bhi, 16 * M);
-    r |= grow(ctx, ctx->nrec, 64 * M);
+    r |= grow(ctx, ctx->boxes, tree_box_bytes(n, ctx->leaf));
     r |= grow(ctx, ctx->dacc, 8 * N);
     r |= grow(ctx, ctx->dexp, 4 * N);
     r |= grow(ctx, ctx->blist, 4 * knn_list_words(n));
@@ -278,11 +266,7 @@ int build_index(asg_ctx* ctx)
     launch_gather_sorted(ctx->perm, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
                          P<int>(ctx->igrp_in), P<float>(ctx->rk_in), n, P<float4>(ctx->pos),
                          P<float4>(ctx->vel), P<int>(ctx->igrp), P<float>(ctx->rk), ctx->s);
-    launch_build_tree(ctx->keys, n, P<int4>(ctx->meta), P<int>(ctx->parent),
-                      P<int>(ctx->leaf_parent), ctx->s);
-    launch_tree_boxes(P<float4>(ctx->pos), nullptr, n, ctx->leaf, P<int4>(ctx->meta),
-                      P<int>(ctx->parent), P<int>(ctx->flags), P<float4>(ctx->blo),
-                      P<float4>(ctx->bhi), P<float4>(ctx->nrec), ctx->s);
+    launch_tree_boxes(P<float4>(ctx->pos), tree_view(ctx), ctx->s);
     phase_end(ctx);
     ctx->loaded = true;
     ctx->knn_done = false;
@@ -490,8 +474,8 @@ void asg_destroy(asg_ctx* ctx)
     Buf* bufs[] = {&ctx->aos, &ctx->pos_in, &ctx->vel_in, &ctx->igrp_in, &ctx->rk_in,
                    &ctx->keys0, &ctx->keys1, &ctx->vals0, &ctx->vals1, &ctx->sort_tmp,
                    &ctx->pos, &ctx->vel, &ctx->igrp, &ctx->rk, &ctx->t33, &ctx->idx33,
-                   &ctx->meta, &ctx->parent, &ctx->leaf_parent, &ctx->flags, &ctx->blo,
-                   &ctx->bhi, &ctx->dacc, &ctx->dexp, &ctx->blist, &ctx->nrec, &ctx->dep_order, &ctx->uf, &ctx->minin, &ctx->mark,
+                   &ctx->boxes, &ctx->dacc, &ctx->dexp, &ctx->blist, &ctx->dep_order, &ctx->uf,
+                   &ctx->minin, &ctx->mark,
                    &ctx->scan_tmp, &ctx->lab_cnt, &ctx->lab_scan, &ctx->halos, &ctx->hcount,
                    &ctx->hmass, &ctx->totals, &ctx->lohi, &ctx->dep_rec, &ctx->dep_pcount,
                    &ctx->dep_tiles, &ctx->dep_counter, &ctx->dep_pairs, &ctx->dep_sort,
@@ -914,7 +898,7 @@ static int run_knn(asg_ctx* ctx)
     phase_begin(ctx, ASG_PH_DENS);
     launch_dens(P<float4>(ctx->pos), t, P<float>(ctx->t33), P<int>(ctx->idx33), P<int>(ctx->blist),
                 P<float>(ctx->rk), P<int>(ctx->dexp), P<unsigned long long>(ctx->dacc),
-                P<float4>(ctx->vel), ctx->d_err, ctx->s);
+                P<float4>(ctx->vel), ctx->s);
     phase_end(ctx);
     ctx->knn_done = true;
     return 0;
@@ -960,7 +944,6 @@ static int collect_mark(asg_ctx* ctx, int nh, long* np_halo, double* m_halo)
         CK(cudaMemcpy(m8.data(), ctx->hmass.p, sizeof(double) * (size_t)nh,
                       cudaMemcpyDeviceToHost));
         for (int i = 0; i < nh; ++i) {  // halo order, as the reference's serial loop
-            if (cnt[(size_t)i] < 0) return fail(ctx, ASG_ERR_STACK, "mark_halos: stack overflow");
             tot += (long)cnt[(size_t)i];
             mh += m8[(size_t)i];
         }

@@ -13,12 +13,12 @@
 namespace asg {
 
 constexpr int K_NN = 33;        // KNeighbors::k (k_neighbors.h:47): 32 neighbours + self
-constexpr int LEAF_MAX = 32;    // largest bucket: a tree node with <= leaf particles (leaf <= 32) is scanned whole
-constexpr int STACK_MAX = 128;  // traversal stack entries per warp
+constexpr int LEAF_MAX = 32;    // largest tree leaf (consecutive particles scanned whole)
+constexpr int LEAF_DEFAULT = 16;
 constexpr int TIE_MAX = 16;     // exact d2 ties kept per pass of k_knn_ties at the 33rd neighbour
 
 // device error bits (ctx->d_err)
-constexpr int ERR_STACK = 1;       // traversal stack overflow
+constexpr int ERR_STACK = 1;       // a traversal ran out of its storage (no kernel sets it: the tree's depth is fixed)
 constexpr int ERR_FEW = 2;         // a query found fewer than 33 particles
 constexpr int ERR_ZERO_RK = 4;     // 33rd distance is zero (>= 33 coincident particles)
 constexpr int ERR_TIES = 8;        // tie selection ran out of passes (not reached for k = 33)
@@ -126,16 +126,6 @@ __device__ __forceinline__ float tent_integral_rn(float a, float b)
     return __fadd_rn(tent_pos_rn(b), tent_pos_rn(-a));  // a < 0 < b
 }
 
-// squared distance from a point to an AABB, rounded so that for every point p
-// inside the box norm2_rn(q, p) >= box_dist2_rn(q, box) (rounding is monotone)
-__device__ __forceinline__ float box_dist2_rn(float qx, float qy, float qz, float4 lo, float4 hi)
-{
-    const float dx = fmaxf(fmaxf(__fsub_rn(lo.x, qx), __fsub_rn(qx, hi.x)), 0.0f);
-    const float dy = fmaxf(fmaxf(__fsub_rn(lo.y, qy), __fsub_rn(qy, hi.y)), 0.0f);
-    const float dz = fmaxf(fmaxf(__fsub_rn(lo.z, qz), __fsub_rn(qz, hi.z)), 0.0f);
-    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-}
-
 // a / L rounded to nearest, given rL = 1/L rounded to nearest: q = RN(a rL) is
 // within one ulp of a/L, the residual a - q L is exact as one FMA, and
 // RN(q + residual * rL) is the correctly rounded quotient (Markstein's theorem:
@@ -181,53 +171,6 @@ __device__ __forceinline__ float box_dist2_fast(float qx, float qy, float qz, fl
 // norm2_rn: fl(t (1 + 2^-21)) >= t (1 + 6.9u) > t (1 + 6.1u), so a box holding
 // a point with norm2_rn <= t is never pruned (t = +inf stays +inf)
 __device__ __forceinline__ float prune_bound(float t) { return __fmul_rn(t, 1.0f + 0x1p-21f); }
-
-// A tree node record (TreeView::rec) holds in words 1-3 either a bucket's own
-// box, lo.xyz hi.x | hi.yz, or for a node with more than `leaf` particles the
-// boxes of both children as pairs, (lo0.x lo1.x lo0.y lo1.y | lo0.z lo1.z hi0.x
-// hi1.x | hi0.y hi1.y hi0.z hi1.z), so that both children are tested with
-// packed f32x2 operations.  A leaf child's box is its point, so its distance
-// equals norm2_rn to that point.
-
-// a bucket's own box in the fast form
-__device__ __forceinline__ float rec_fast0(float4 q, float4 r1, float4 r2)
-{
-    return box_dist2_fast(q.x, q.y, q.z, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y);
-}
-// a bucket's own box, rounded as box_dist2_rn
-__device__ __forceinline__ float rec_dist0(float4 q, float4 r1, float4 r2)
-{
-    return box_dist2_rn(q.x, q.y, q.z, make_float4(r1.x, r1.y, r1.z, 0.f),
-                        make_float4(r1.w, r2.x, r2.y, 0.f));
-}
-// both children of a node in the fast form (child 0 low, child 1 high):
-// box_dist2_fast's operations on each element; qx = (q.x, q.x) and so on
-__device__ __forceinline__ f32x2 node_fast2(f32x2 qx, f32x2 qy, f32x2 qz, float4 r1, float4 r2,
-                                            float4 r3)
-{
-    const f32x2 lx = sub2_rn(pack2(r1.x, r1.y), qx), hx = sub2_rn(qx, pack2(r2.z, r2.w));
-    const f32x2 ly = sub2_rn(pack2(r1.z, r1.w), qy), hy = sub2_rn(qy, pack2(r3.x, r3.y));
-    const f32x2 lz = sub2_rn(pack2(r2.x, r2.y), qz), hz = sub2_rn(qz, pack2(r3.z, r3.w));
-    const f32x2 dx = pack2(max3f(lo2(lx), lo2(hx), 0.0f), max3f(hi2(lx), hi2(hx), 0.0f));
-    const f32x2 dy = pack2(max3f(lo2(ly), lo2(hy), 0.0f), max3f(hi2(ly), hi2(hy), 0.0f));
-    const f32x2 dz = pack2(max3f(lo2(lz), lo2(hz), 0.0f), max3f(hi2(lz), hi2(hz), 0.0f));
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %1;\n\t"
-        "fma.rn.f32x2 %0, %2, %2, %0;\n\t"
-        "fma.rn.f32x2 %0, %3, %3, %0;" : "=&l"(r) : "l"(dx), "l"(dy), "l"(dz));
-    return r;
-}
-// child 0 / child 1 of a node, rounded as box_dist2_rn
-__device__ __forceinline__ float node_dist0(float4 q, float4 r1, float4 r2, float4 r3)
-{
-    return box_dist2_rn(q.x, q.y, q.z, make_float4(r1.x, r1.z, r2.x, 0.f),
-                        make_float4(r2.z, r3.x, r3.z, 0.f));
-}
-__device__ __forceinline__ float node_dist1(float4 q, float4 r1, float4 r2, float4 r3)
-{
-    return box_dist2_rn(q.x, q.y, q.z, make_float4(r1.y, r1.w, r2.y, 0.f),
-                        make_float4(r2.w, r3.y, r3.w, 0.f));
-}
 
 // double-float accumulation (Knuth two-sum): hi + lo carries ~48 bits
 // the same (hi, lo) as two_sum_acc for hi >= 0 and x >= 0: Fast2Sum on the

@@ -3,7 +3,7 @@
 // FOF (group_fof / link_friends_recursive1, fof.cpp:34-102; remove_small_groups,
 // fof.cpp:104-166): two particles are friends when norm2 <= ll*ll in float
 // (the reference's predicate, fof.cpp:85-91); groups are the connected
-// components.  GPU form: a warp-bundle range search over the radix tree links
+// components.  GPU form: a warp-bundle range search over the box tree links
 // every friend pair (i < j) in a lock-free union-find whose parent pointers
 // only ever decrease, so each component's root is its smallest sorted position
 // whatever the order of the unions.  Labels 1..ngroup are then assigned in
@@ -17,6 +17,7 @@
 
 #include "asg_common.cuh"
 #include "asg_internal.h"
+#include "asg_tree.cuh"
 
 namespace asg {
 
@@ -50,13 +51,10 @@ __device__ __forceinline__ bool uf_union(int* P, int a, int b)
     return false;
 }
 
-constexpr int NO_NODE = INT_MIN;  // no node: node ids are >= 0, a leaf i is ~i >= -n
-
 __global__ void __launch_bounds__(FOF_WARPS * 32)
-k_fof_link(const float4* __restrict__ pos, TreeView t, float ll2, int* P, int* err)
+k_fof_link(const float4* __restrict__ pos, const __grid_constant__ TreeView t, float ll2, int* P, int* err)
 {
-    __shared__ int stk[FOF_WARPS][STACK_MAX];
-    __shared__ float4 cand[FOF_WARPS][32];
+    __shared__ float4 cand[FOF_WARPS][LEAF_MAX];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = t.n;
     const int base = (blockIdx.x * FOF_WARPS + warp) * 32;
@@ -64,65 +62,31 @@ k_fof_link(const float4* __restrict__ pos, TreeView t, float ll2, int* P, int* e
     const int q = min(base + lane, n - 1);
     const bool active = base + lane < n;
     const float4 xq = pos[q];
+    const float bound = prune_bound(ll2);
     bool bad = false;
-
-    // child 0 is visited next directly; child 1 waits on the stack
-    int* st = stk[warp];
-    int sp = 0;
-    int next = tree_root(n);
-    bool overflow = false;
-    for (;;) {
-        int node = next;
-        next = NO_NODE;
-        if (node == NO_NODE) {
-            if (sp == 0) break;
-            node = st[--sp];
-            __syncwarp();  // every lane has read the slot before it is written again
-        }
-        int first, last;
-        if (node < 0) {
-            first = last = ~node;
-        } else {
-            // the node's record: meta and both children's boxes in one round trip
-            const float4* rp = t.rec + 4 * (size_t)node;
-            const float4 r0 = rp[0], r1 = rp[1], r2 = rp[2], r3 = rp[3];
-            const int4 m = make_int4(__float_as_int(r0.x), __float_as_int(r0.y),
-                                     __float_as_int(r0.z), __float_as_int(r0.w));
-            if (m.w - m.z + 1 > t.leaf) {
-                // child 0 holds [m.z, g] and child 1 [g + 1, m.w]: the radix tree
-                // names its children by the split g (node or leaf g, and g + 1)
-                const int g = m.x >= 0 ? m.x : ~m.x;
-                // only partners with a larger sorted position are linked from q
-                const bool n0 = m.x < 0 ? (active && ~m.x > q)
-                                        : (active && g > q && node_dist0(xq, r1, r2, r3) <= ll2);
-                const bool n1 = m.y < 0 ? (active && ~m.y > q)
-                                        : (active && m.w > q && node_dist1(xq, r1, r2, r3) <= ll2);
-                const bool v0 = __any_sync(FM, n0);
-                const bool v1 = __any_sync(FM, n1);
-                if (v1) {
-                    if (sp + 1 > STACK_MAX) { overflow = true; break; }
-                    if (lane == 0) st[sp] = m.y;
-                    ++sp;
-                    __syncwarp();
-                }
-                if (v0) next = m.x;
-                continue;
+    const TreeBox box = bundle_box(t, base / t.leaf, (min(base + 32, n) - 1) / t.leaf);
+    tree_walk(t,
+        [&](const TreeBox& c, int level, int id) {
+            // only partners with a larger sorted position are linked from q
+            const long long last = (((long long)id + 1) << (5 * level)) * t.leaf - 1;
+            return last > base && boxes_dist2_fast(box, c) <= bound;
+        },
+        [&](int id) {
+            const int first = id * t.leaf, cnt = leaf_count(t, id);
+            if (!__any_sync(FM, active && first + cnt - 1 > q &&
+                                    point_box_fast(xq, tree_box(t, 0, id)) <= bound))
+                return true;
+            __syncwarp();
+            if (lane < cnt) cand[warp][lane] = pos[first + lane];
+            __syncwarp();
+            for (int j = 0; j < cnt; ++j) {
+                const int s = first + j;
+                const float4 c = cand[warp][j];
+                if (active && s > q && norm2_rn(xq.x, xq.y, xq.z, c.x, c.y, c.z) <= ll2)
+                    bad |= !uf_union(P, q, s);
             }
-            first = m.z;
-            last = m.w;
-        }
-        const int cnt = last - first + 1;
-        if (lane < cnt) cand[warp][lane] = pos[first + lane];
-        __syncwarp();
-        for (int j = 0; j < cnt; ++j) {
-            const int s = first + j;
-            const float4 c = cand[warp][j];
-            if (active && s > q && norm2_rn(xq.x, xq.y, xq.z, c.x, c.y, c.z) <= ll2)
-                bad |= !uf_union(P, q, s);
-        }
-        __syncwarp();
-    }
-    if (overflow && lane == 0) atomicOr(err, ERR_STACK);
+            return true;
+        });
     if (bad) atomicOr(err, ERR_UF);
 }
 
@@ -231,11 +195,10 @@ void launch_relabel(int* igrp, int n, const uint32_t* scan, const uint32_t* keep
 constexpr int MH_WARPS = 4;
 
 __global__ void __launch_bounds__(MH_WARPS * 32)
-k_mark_halos(const float4* __restrict__ pos, TreeView t, const float* __restrict__ halos, int nh,
+k_mark_halos(const float4* __restrict__ pos, const __grid_constant__ TreeView t, const float* __restrict__ halos, int nh,
              float left, float right, int* __restrict__ igrp, long long* __restrict__ counts,
              double* __restrict__ mass8)
 {
-    __shared__ int stk[MH_WARPS][STACK_MAX];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = blockIdx.x * MH_WARPS + warp;
     if (h >= nh) return;
@@ -248,55 +211,24 @@ k_mark_halos(const float4* __restrict__ pos, TreeView t, const float* __restrict
         return;
     }
     const float r2 = __fmul_rn(r, r);
+    const float bound = prune_bound(r2);
+    const float4 c4 = make_float4(cx, cy, cz, 0.f);
     long long cnt = 0;
-    int* st = stk[warp];
-    if (lane == 0) st[0] = tree_root(t.n);
-    int sp = 1;
-    bool overflow = false;
-    __syncwarp();
-    while (sp > 0) {
-        const int node = st[--sp];
-        __syncwarp();
-        int first, last;
-        if (node < 0) {
-            first = last = ~node;
-        } else {
-            // the node's record: a node's children are tested by their boxes before
-            // they are pushed, a bucket (or a bucket root) by its own box
-            const float4* rp = t.rec + 4 * (size_t)node;
-            const float4 r0 = rp[0], r1 = rp[1], r2v = rp[2], r3 = rp[3];
-            const int4 m = make_int4(__float_as_int(r0.x), __float_as_int(r0.y),
-                                     __float_as_int(r0.z), __float_as_int(r0.w));
-            const float4 c4 = make_float4(cx, cy, cz, 0.f);
-            if (m.w - m.z + 1 > t.leaf) {
-                // a leaf child goes on as a one-particle bucket, tested by its norm2
-                const bool v0 = m.x < 0 || node_dist0(c4, r1, r2v, r3) < r2;
-                const bool v1 = m.y < 0 || node_dist1(c4, r1, r2v, r3) < r2;
-                if (sp + 2 > STACK_MAX) { overflow = true; break; }
-                if (lane == 0) {
-                    if (v1) st[sp] = m.y;
-                    if (v0) st[sp + (v1 ? 1 : 0)] = m.x;
-                }
-                sp += (v0 ? 1 : 0) + (v1 ? 1 : 0);
-                __syncwarp();
-                continue;
-            }
-            if (rec_dist0(c4, r1, r2v) >= r2) continue;
-            first = m.z;
-            last = m.w;
-        }
-        const int nb = last - first + 1;
-        bool hit = false;
-        if (lane < nb) {
-            const float4 p = pos[first + lane];
-            // norm2(x, particle[i].x) with x the halo centre (nbr_search.cpp:149)
-            hit = norm2_rn(cx, cy, cz, p.x, p.y, p.z) < r2;
-            if (hit) igrp[first + lane] = -1;
-        }
-        cnt += __popc(__ballot_sync(FM, hit));
-    }
+    tree_walk(t, [&](const TreeBox& c, int, int) { return point_box_fast(c4, c) <= bound; },
+              [&](int id) {
+                  const int first = id * t.leaf, nb = leaf_count(t, id);
+                  bool hit = false;
+                  if (lane < nb) {
+                      const float4 p = pos[first + lane];
+                      // norm2(x, particle[i].x) with x the halo centre (nbr_search.cpp:149)
+                      hit = norm2_rn(cx, cy, cz, p.x, p.y, p.z) < r2;
+                      if (hit) igrp[first + lane] = -1;
+                  }
+                  cnt += __popc(__ballot_sync(FM, hit));
+                  return true;
+              });
     if (lane == 0) {
-        counts[h] = overflow ? -1 : cnt;
+        counts[h] = cnt;
         mass8[h] = (double)__fdiv_rn(mass, 8.0f);  // h[i].mass/8.0f (:483)
     }
 }

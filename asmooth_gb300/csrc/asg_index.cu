@@ -3,8 +3,8 @@
 // (16 bits per axis; Morton order with ASG_SPACE_CURVE=morton) by a stable LSD
 // radix sort (each 8-bit digit pass is a counting sort: per-tile
 // digit histograms built with warp-aggregated shared-memory atomics, one
-// exclusive scan, a stable scatter), then a radix tree (Karras 2012) is built
-// over the sorted keys with AABBs computed bottom-up.
+// exclusive scan, a stable scatter), then the boxes of the blocked tree
+// (TreeView) are reduced level by level.
 //
 // Determinism: the sort is stable and starts from input order, so equal keys
 // stay in input-index order; the tree is a pure function of the sorted keys.
@@ -517,194 +517,91 @@ void launch_check_rk(const float* rk, int n, int* err, cudaStream_t s)
 }
 
 // ---------------------------------------------------------------------------
-// radix tree (Karras 2012, "Maximizing parallelism in the construction of
-// BVHs, octrees, and k-d trees"); duplicate keys are split by position
+// blocked box tree (TreeView)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int kdelta(const uint64_t* __restrict__ k, int n, int i, long long j)
+TreeView tree_shape(int n, int leaf)
 {
-    if (j < 0 || j >= n) return -1;
-    const uint64_t a = k[i], b = k[(int)j];
-    if (a == b) return 64 + __clz(i ^ (int)j);
-    return __clzll(a ^ b);
-}
-
-__global__ void k_build_tree(const uint64_t* __restrict__ keys, int n, int4* __restrict__ meta,
-                             int* __restrict__ parent, int* __restrict__ leaf_parent)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
-    const int d = (kdelta(keys, n, i, (long long)i + 1) - kdelta(keys, n, i, (long long)i - 1)) > 0 ? 1 : -1;
-    const int dmin = kdelta(keys, n, i, (long long)i - d);
-    long long lmax = 2;
-    while (kdelta(keys, n, i, (long long)i + lmax * d) > dmin) lmax <<= 1;
-    long long l = 0;
-    for (long long t = lmax >> 1; t >= 1; t >>= 1)
-        if (kdelta(keys, n, i, (long long)i + (l + t) * d) > dmin) l += t;
-    const long long j = (long long)i + l * d;
-    const int dnode = kdelta(keys, n, i, j);
-    long long s = 0;
-    long long t = l;
-    do {
-        t = (t + 1) >> 1;
-        if (kdelta(keys, n, i, (long long)i + (s + t) * d) > dnode) s += t;
-    } while (t > 1);
-    const int gamma = (int)((long long)i + s * d + (d < 0 ? d : 0));
-    const int lo = (int)(i < j ? i : j), hi = (int)(i < j ? j : i);
-    const int c0 = (lo == gamma) ? ~gamma : gamma;
-    const int c1 = (hi == gamma + 1) ? ~(gamma + 1) : gamma + 1;
-    meta[i] = make_int4(c0, c1, lo, hi);
-    if (c0 < 0) leaf_parent[~c0] = i; else parent[c0] = i;
-    if (c1 < 0) leaf_parent[~c1] = i; else parent[c1] = i;
-    if (i == 0) parent[0] = -1;
-}
-
-void launch_build_tree(const uint64_t* keys, int n, int4* meta, int* parent, int* leaf_parent,
-                       cudaStream_t s)
-{
-    if (n <= 1) {
-        if (n == 1) cudaMemsetAsync(leaf_parent, 0xff, sizeof(int), s);
-        return;
+    TreeView t{};
+    t.n = n;
+    t.leaf = leaf;
+    long long c = ((long long)n + leaf - 1) / leaf, off = 0;
+    for (;;) {
+        t.cnt[t.nlev] = (int)c;
+        t.off[t.nlev] = off;
+        off += c;
+        ++t.nlev;
+        if (c <= 32) break;
+        c = (c + 31) / 32;
     }
-    k_build_tree<<<(n - 1 + 255) / 256, 256, 0, s>>>(keys, n, meta, parent, leaf_parent);
-    count_launches(1);
+    return t;
 }
 
-// leaf box: the point itself, or [x-h', x+h'] with h' = rk*(1+1e-6) rounded up and
-// the bounds rounded outwards, so that a point outside it is farther than rk
-__device__ __forceinline__ void leaf_box(const float4* pos, const float* rk, int i, float4& lo,
-                                         float4& hi)
+size_t tree_box_bytes(int n, int leaf)
 {
-    const float4 p = pos[i];
-    if (rk) {
-        const float h = __fmul_ru(rk[i], 1.000001f);
-        lo = make_float4(__fsub_rd(p.x, h), __fsub_rd(p.y, h), __fsub_rd(p.z, h), 0.f);
-        hi = make_float4(__fadd_ru(p.x, h), __fadd_ru(p.y, h), __fadd_ru(p.z, h), 0.f);
-    } else {
-        lo = make_float4(p.x, p.y, p.z, 0.f);
-        hi = lo;
-    }
+    const TreeView t = tree_shape(n, leaf);
+    return 32 * (size_t)(t.off[t.nlev - 1] + t.cnt[t.nlev - 1]);
 }
 
-__device__ __forceinline__ void box_union(float4& l, float4& h, const float4& l1, const float4& h1)
+// union of the boxes of the lanes of each aligned group of G lanes
+template <int G>
+__device__ __forceinline__ void group_box(float (&r)[6])
 {
-    l = make_float4(fminf(l.x, l1.x), fminf(l.y, l1.y), fminf(l.z, l1.z), 0.f);
-    h = make_float4(fmaxf(h.x, h1.x), fmaxf(h.y, h1.y), fmaxf(h.z, h1.z), 0.f);
-}
-
-// the 64-byte record of node i (TreeView::rec): meta, then the boxes of both
-// children as coordinate pairs, or (bucket) the node's own box
-__device__ __forceinline__ void write_node_rec(float4* rec, int i, int4 m, float4 l0, float4 h0,
-                                               float4 l1, float4 h1)
-{
-    float4* r = rec + 4 * (size_t)i;
-    r[0] = make_float4(__int_as_float(m.x), __int_as_float(m.y), __int_as_float(m.z),
-                       __int_as_float(m.w));
-    r[1] = make_float4(l0.x, l1.x, l0.y, l1.y);
-    r[2] = make_float4(l0.z, l1.z, h0.x, h1.x);
-    r[3] = make_float4(h0.y, h1.y, h0.z, h1.z);
-}
-__device__ __forceinline__ void write_bucket_rec(float4* rec, int i, int4 m, float4 l, float4 h)
-{
-    float4* r = rec + 4 * (size_t)i;
-    r[0] = make_float4(__int_as_float(m.x), __int_as_float(m.y), __int_as_float(m.z),
-                       __int_as_float(m.w));
-    r[1] = make_float4(l.x, l.y, l.z, h.x);
-    r[2] = make_float4(h.y, h.z, 0.f, 0.f);
-    r[3] = make_float4(0.f, 0.f, 0.f, 0.f);
-}
-
-// Boxes of the nodes a traversal can read: the root and every child of a node
-// with more than `leaf` particles (the traversals scan smaller nodes whole and
-// never look below them).  A "top bucket" (<= leaf particles, parent larger)
-// reduces its contiguous particles directly, then climbs: a node with two
-// internal children is finished by the second arrival (atomic flag), a node
-// with one internal child by its only climber.  Unions of the same particle
-// boxes, so the boxes are the same bits as a climb from every particle.  With
-// rec, each finished node also gets its record (TreeView::rec): a top bucket
-// its own box, a larger node the boxes of its children, which its finisher
-// holds at that moment; a node inside a bucket is never visited and gets none.
-__global__ void k_tree_boxes(const float4* __restrict__ pos, const float* __restrict__ rk, int n,
-                             int leaf, const int4* __restrict__ meta, const int* __restrict__ parent,
-                             int* flags, float4* lo, float4* hi, float4* __restrict__ rec)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    const bool valid = i < n - 1;
-    const int4 m = valid ? meta[i] : make_int4(0, 0, 0, 0);
-    float4 l, h, l1, h1;
-    bool start = false;  // this thread finishes node i and climbs from it
-    bool top = false;    // node i is a top bucket
-    if (valid) {
-        if (m.w - m.z + 1 > leaf) {
-            start = m.x < 0 && m.y < 0;  // two particle children (leaf = 1 only)
-            if (start) {
-                leaf_box(pos, rk, ~m.x, l, h);
-                leaf_box(pos, rk, ~m.y, l1, h1);
-                if (rec) write_node_rec(rec, i, m, l, h, l1, h1);
-                box_union(l, h, l1, h1);
-            }
-        } else {
-            const int p = parent[i];
-            top = p < 0 || meta[p].w - meta[p].z + 1 > leaf;  // not inside a larger bucket
-            start = top;
-        }
-    }
-    // the warp reduces its top buckets one after another, lanes over the
-    // bucket's (at most 32) contiguous particles: one coalesced load each
-    unsigned tops = __ballot_sync(0xffffffffu, top);
-    while (tops) {
-        const int src = __ffs(tops) - 1;
-        tops &= tops - 1;
-        const int first = __shfl_sync(0xffffffffu, m.z, src);
-        const int last = __shfl_sync(0xffffffffu, m.w, src);
-        float4 bl, bh;
-        leaf_box(pos, rk, min(first + lane, last), bl, bh);
-        float r[6] = {bl.x, bl.y, bl.z, bh.x, bh.y, bh.z};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+    for (int o = G / 2; o > 0; o >>= 1)
 #pragma unroll
-            for (int a = 0; a < 6; ++a) {
-                const float v = __shfl_xor_sync(0xffffffffu, r[a], o);
-                r[a] = a < 3 ? fminf(r[a], v) : fmaxf(r[a], v);
-            }
-        if (lane == src) {
-            l = make_float4(r[0], r[1], r[2], 0.f);
-            h = make_float4(r[3], r[4], r[5], 0.f);
+        for (int a = 0; a < 6; ++a) {
+            const float v = __shfl_xor_sync(0xffffffffu, r[a], o);
+            r[a] = a < 3 ? fminf(r[a], v) : fmaxf(r[a], v);
         }
-    }
-    if (!start) return;
-    if (top && rec) write_bucket_rec(rec, i, m, l, h);
-    __stcg(&lo[i], l);
-    __stcg(&hi[i], h);
-    int node = parent[i];
-    while (node >= 0) {
-        const int4 mm = meta[node];
-        if (mm.x >= 0 && mm.y >= 0) {
-            __threadfence();
-            if (atomicAdd(&flags[node], 1) == 0) return;  // the sibling finishes this node
-            __threadfence();
-        }
-        if (mm.x < 0) leaf_box(pos, rk, ~mm.x, l, h);
-        else { l = __ldcg(&lo[mm.x]); h = __ldcg(&hi[mm.x]); }
-        if (mm.y < 0) leaf_box(pos, rk, ~mm.y, l1, h1);
-        else { l1 = __ldcg(&lo[mm.y]); h1 = __ldcg(&hi[mm.y]); }
-        if (rec) write_node_rec(rec, node, mm, l, h, l1, h1);
-        box_union(l, h, l1, h1);
-        __stcg(&lo[node], l);
-        __stcg(&hi[node], h);
-        node = parent[node];
-    }
+}
+__device__ __forceinline__ void store_box(float4* box, size_t id, const float (&r)[6])
+{
+    box[2 * id] = make_float4(r[0], r[1], r[2], r[3]);
+    box[2 * id + 1] = make_float4(r[4], r[5], 0.0f, 0.0f);
 }
 
-void launch_tree_boxes(const float4* pos, const float* rk, int n, int leaf, const int4* meta,
-                       const int* parent, int* flags, float4* lo, float4* hi, float4* rec,
-                       cudaStream_t s)
+// level 0: G lanes (16, or 32 for leaves of more particles) per leaf, one
+// coalesced load per lane
+template <int G>
+__global__ void k_leaf_boxes(const float4* __restrict__ pos, int n, int leaf, int nleaf,
+                             float4* __restrict__ box)
 {
-    if (n <= 1) return;
-    cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)(n - 1), s);
-    k_tree_boxes<<<(n - 1 + 255) / 256, 256, 0, s>>>(pos, rk, n, leaf, meta, parent, flags, lo, hi,
-                                                      rec);
-    count_launches(1);
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long id = t / G;
+    const int r = (int)(t % G);
+    const bool live = id < nleaf;
+    const long long i = min(id * leaf + min(r, leaf - 1), (long long)n - 1);
+    const float4 p = pos[live ? i : 0];
+    float b[6] = {p.x, p.y, p.z, p.x, p.y, p.z};
+    group_box<G>(b);
+    if (live && r == 0) store_box(box, (size_t)id, b);
+}
+
+// one level up: a warp per box, a child per lane
+__global__ void k_up_boxes(const float4* __restrict__ below, int nbelow, float4* __restrict__ box,
+                           int nbox)
+{
+    const long long id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    if (id >= nbox) return;
+    const long long c = min(id * 32 + (threadIdx.x & 31), (long long)nbelow - 1);
+    const float4 u = below[2 * c], v = below[2 * c + 1];
+    float b[6] = {u.x, u.y, u.z, u.w, v.x, v.y};
+    group_box<32>(b);
+    if ((threadIdx.x & 31) == 0) store_box(box, (size_t)id, b);
+}
+
+void launch_tree_boxes(const float4* pos, const TreeView& t, cudaStream_t s)
+{
+    if (t.n <= 0) return;
+    float4* box = const_cast<float4*>(t.box);
+    const int g = t.leaf <= 16 ? 16 : 32;
+    const unsigned nb = (unsigned)(((long long)t.cnt[0] * g + 255) / 256);
+    if (g == 16) k_leaf_boxes<16><<<nb, 256, 0, s>>>(pos, t.n, t.leaf, t.cnt[0], box);
+    else k_leaf_boxes<32><<<nb, 256, 0, s>>>(pos, t.n, t.leaf, t.cnt[0], box);
+    for (int l = 1; l < t.nlev; ++l)
+        k_up_boxes<<<(unsigned)(((long long)t.cnt[l] * 32 + 255) / 256), 256, 0, s>>>(
+            box + 2 * t.off[l - 1], t.cnt[l - 1], box + 2 * t.off[l], t.cnt[l]);
+    count_launches(t.nlev);
 }
 
 // ---------------------------------------------------------------------------

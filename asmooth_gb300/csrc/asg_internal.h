@@ -6,9 +6,8 @@
 //   vel   float4[N]  vx, vy, vz, dens                        -- Hilbert order
 //   igrp  int[N]                                             -- Hilbert order
 //   rk    float[N], t33 float[N], idx33 int[N]               -- Hilbert order
-// Radix tree over the N sorted space-filling-curve keys (Karras 2012), N-1 internal nodes:
-//   meta  int4[N-1]  child0, child1 (>=0 internal, <0 leaf ~i), first, last
-//   blo/bhi float4[N-1]  AABB of the node's particles
+// Blocked box tree over the sorted particles (TreeView): boxes of `leaf`
+// consecutive particles, then of 32 consecutive boxes, level by level.
 #pragma once
 
 #include <cstddef>
@@ -20,22 +19,19 @@ namespace asg {
 // process-wide count of kernel launches made by this library
 void count_launches(int k);
 
+// Levels of the box tree: leaf = 1 and n = 2^31 - 1 need 7.
+constexpr int TREE_LEVELS = 7;
 struct TreeView {
-    int n;                 // particles (leaves)
-    int leaf;              // bucket size: nodes with <= leaf particles are scanned whole (1..32)
-    const int4* meta;      // internal nodes 0..n-2 (root 0); empty when n == 1
-    const float4* blo;
-    const float4* bhi;
-    // 64 bytes per internal node, one load round trip per visit: word 0 the
-    // meta (c0, c1, first, last as int bits); words 1-3 the boxes of both
-    // children of a node with more than `leaf` particles (a leaf child as its
-    // point: lo0.xyz hi0.x | hi0.yz lo1.xy | lo1.z hi1.xyz), or the node's own
-    // box for a bucket (lo.xyz hi.x | hi.yz)
-    const float4* rec;
+    int n;                       // particles
+    int leaf;                    // particles per leaf (1..32), the last leaf may hold fewer
+    int nlev;                    // levels, level 0 = leaves; the top one has at most 32 boxes
+    int cnt[TREE_LEVELS];        // boxes of each level: ceil(n / leaf), then ceil(below / 32)
+    long long off[TREE_LEVELS];  // first box of each level in `box`
+    const float4* box;           // two float4 per box: lo.xyz hi.x | hi.yz 0 0
 };
-
-// root entry of a traversal: internal node 0, or leaf 0 when n == 1
-__host__ __device__ inline int tree_root(int n) { return n > 1 ? 0 : ~0; }
+// the tree's shape for n particles (box not set), and the bytes of its boxes
+TreeView tree_shape(int n, int leaf);
+size_t tree_box_bytes(int n, int leaf);
 
 // ---- index build (asg_index.cu) -------------------------------------------------
 // unpack reference Particle records (36 B), or SoA device arrays, into the
@@ -67,28 +63,21 @@ void launch_gather_sorted(const int* perm, const float4* pos_in, const float4* v
 void launch_iota(int* a, int n, cudaStream_t s);
 // err |= ERR_ZERO_RK when some rk is not a positive finite number
 void launch_check_rk(const float* rk, int n, int* err, cudaStream_t s);
-void launch_build_tree(const uint64_t* keys, int n, int4* meta, int* parent, int* leaf_parent,
-                       cudaStream_t s);
-// bottom-up AABBs of the nodes a traversal with bucket size `leaf` reads (the
-// root and the children of nodes with more than leaf particles); with
-// rk != nullptr the expanded boxes [x-h', x+h']; rec (or null) receives
-// TreeView::rec of those nodes (4 float4 per internal node)
-void launch_tree_boxes(const float4* pos, const float* rk, int n, int leaf, const int4* meta,
-                       const int* parent, int* flags, float4* lo, float4* hi, float4* rec,
-                       cudaStream_t s);
+// the boxes of every level of t from the sorted positions
+void launch_tree_boxes(const float4* pos, const TreeView& t, cudaStream_t s);
 // exclusive scan of uint32 counts (in place); temp from scan_temp_bytes
 size_t scan_temp_bytes(size_t n);
 void exclusive_scan_u32(uint32_t* data, size_t n, void* temp, cudaStream_t s);
 
 // ---- neighbour search (asg_knn.cu) -------------------------------------------
-// Buckets k_knn_t33 scanned, per 32-query bundle: word 0 = their count (-1 when
-// more than KNN_LIST), then the node ids (a bucket node, or ~i for one particle).
-// k_dens_scatter visits these instead of walking the tree again.
+// Leaves k_knn_t33 scanned, per 32-query bundle: word 0 = their count (-1 when
+// more than KNN_LIST), then the leaf numbers.  k_dens_scatter visits these
+// instead of walking the tree again.
 constexpr int KNN_LIST = 96;
 inline size_t knn_list_words(int n) { return (size_t)((n + 31) / 32) * (KNN_LIST + 1); }
 // t33, rk = sqrtf(t33), idx33 = -1 (no tie at the 33rd) or -2 (ties to resolve);
-// blist (knn_list_words ints, or null) receives the scanned buckets; warps: 2 or
-// 4 warps per block (tuning)
+// blist (knn_list_words ints, or null) receives the scanned leaves; warps: 2 or
+// 4 warps per block (tuning; leaves of 16 particles always run 1)
 void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk, int* idx33,
                     int* blist, int* err, cudaStream_t s, int warps = 2);
 // idx33 = input index of the 33rd key, for flagged queries (all = 0) or every query
@@ -98,7 +87,7 @@ void launch_knn_ties(const float4* pos, const TreeView& t, const float* t33, int
 // dexp (n ints) and acc (n uint64) are scratch; blist from launch_knn_t33 or null
 void launch_dens(const float4* pos, const TreeView& t, const float* t33, const int* idx33,
                  const int* blist, const float* rk, int* dexp, unsigned long long* acc,
-                 float4* vel, int* err, cudaStream_t s);
+                 float4* vel, cudaStream_t s);
 
 // ---- mesh deposit (asg_deposit.cu) ---------------------------------------------
 struct MeshJob {

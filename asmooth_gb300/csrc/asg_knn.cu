@@ -8,52 +8,110 @@
 // smallest keys (the 33rd excluded, self included) receive the tent weight
 // ker(p, q, 1/rk) in dens.
 //
-// Three warp-bundle kernels over the radix tree (its 64-byte node records); a
-// warp serves the 32 consecutive (Hilbert-ordered) particles of one bundle, one
-// lane per particle, and visits a node when any lane needs it:
+// Three warp-bundle kernels over the blocked box tree (asg_tree.cuh); a warp
+// serves the 32 consecutive (Hilbert-ordered) particles of one bundle, one
+// lane per particle, and scans a leaf when any lane's radius reaches its box:
 //   k_knn_t33   per-lane sorted top-33 of d2 in registers, candidates queued
 //               and merged by comparator networks (asg_knn_net.cuh)
 //               -> t33 = 33rd smallest d2 (exact, with multiplicity)
 //   k_knn_ties  exact-radius recount: L = #(d2 < t33), the tied indices
 //               -> idx33 = input index of the 33rd key, rk = sqrtf(t33)
 //   k_dens_scatter the bundle's queries are SOURCES q with their exact radii;
-//               in each bucket a lane holds a receiver j and adds ker(q, j)
+//               in each leaf a lane holds a receiver j and adds ker(q, j)
 //               for the queries q whose 32-set holds j, as 64-bit fixed point
 //               (per-receiver power-of-two scale, one integer atomic per
-//               receiver and bucket): exact integer sums, so deterministic in
-//               any order.  It visits the buckets k_knn_t33 recorded.
+//               receiver and leaf): exact integer sums, so deterministic in
+//               any order.  It visits the leaves k_knn_t33 recorded.
 #include <climits>
+#include <cstddef>
 #include <type_traits>
 
 #include "asg_common.cuh"
 #include "asg_internal.h"
 #include "asg_knn_net.cuh"
+#include "asg_tree.cuh"
 
 namespace asg {
 
 constexpr int KNN_WARPS = 4;
-// k_knn_t33 runs in blocks of W = 2 or 4 warps (32 warps per SM at 64
-// registers either way); in blocks of 2 a warp that finishes early frees its
-// slot sooner (23.07 against 23.25 ms on the 256^3 step in Morton order).  The
-// batched form's autotuner picks W.
+// k_dens_scatter: one warp per block and four queries per turn of its loop, 6.42
+// ms on the 256^3 step (4 warps and two queries 6.57)
+constexpr int DENS_WARPS = 1, DENS_UNROLL = 4;
+// k_knn_t33 runs 32 warps per SM at 64 registers, in blocks of 1 warp with the
+// default leaf size and of 2 or 4 with others (the batched form's autotuner
+// picks).
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int NO_NODE = INT_MIN;  // no node: node ids are >= 0, a leaf i is ~i >= -n
 
-// Merges a lane's queued candidates (KNN_QUEUE values in shared memory, column
-// `lane`, +inf where unused) into its ascending top-33 a[] and refills the
-// queue with +inf.  tie_out ("a particle outside a[] has d2 == a[32]") stays
+// A lane's queue holds up to KNN_SLOTS candidates; a flush merges the KNN_QUEUE
+// newest.  With room for twice as many values as a flush takes, the queues are
+// checked once per 16 candidates instead of once per 2, and a flush finds 8.4
+// values per lane instead of 6.3 (a CPU model on the 256^3 cube's clustering:
+// 12.6 flushes per bundle for 106 queued values per lane, against 14.0 for 89
+// with 16 slots and a check every 2).
+constexpr int KNN_SLOTS = 32;
+constexpr int KNN_CHUNK = 16;  // candidates between two checks
+static_assert(KNN_SLOTS >= KNN_QUEUE + KNN_CHUNK, "a chunk must fit behind a full flush");
+
+// A warp's shared memory in k_knn_t33, addressed with 32-bit shared addresses: a
+// lane's words lie at `column` (4 x lane into the struct) plus a constant.
+struct KnnWarp {
+    float queue[KNN_SLOTS][32];          // [slot][lane], +inf where unused
+    float cand[3][KNN_CHUNK];            // x, y, z of the candidates of a chunk
+    unsigned keys[TREE_LEVELS - 1][32];  // [level - 1][lane], pending children of the upper levels
+    TreeBox box;                         // the bundle's box
+};
+constexpr unsigned QUEUE_ROW = 32 * sizeof(float);
+
+template <unsigned OFF>
+__device__ __forceinline__ float lds_f32(unsigned a)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1 + %2];" : "=f"(v) : "r"(a), "n"(OFF) : "memory");
+    return v;
+}
+template <unsigned OFF>
+__device__ __forceinline__ void sts_f32(unsigned a, float v)
+{
+    asm volatile("st.shared.f32 [%0 + %1], %2;" : : "r"(a), "n"(OFF), "f"(v) : "memory");
+}
+template <unsigned OFF>
+__device__ __forceinline__ void lds_x2(unsigned a, f32x2& u, f32x2& v)
+{
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2 + %3];" : "=l"(u), "=l"(v) : "r"(a), "n"(OFF) : "memory");
+}
+// queues d when d <= limit: three predicated instructions, no branch
+__device__ __forceinline__ void knn_push(unsigned& slot, float d, float limit)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.le.f32 p, %1, %2;\n\t"
+        "@p st.shared.f32 [%0], %1;\n\t"
+        "@p add.u32 %0, %0, %3;\n\t}"
+        : "+r"(slot) : "f"(d), "f"(limit), "n"(QUEUE_ROW) : "memory");
+}
+
+template <int I>
+__device__ __forceinline__ void knn_take(float (&v)[KNN_QUEUE], unsigned q0)
+{
+    if constexpr (I < KNN_QUEUE) {
+        v[I] = lds_f32<I * QUEUE_ROW>(q0);
+        sts_f32<I * QUEUE_ROW>(q0, INFINITY);
+        knn_take<I + 1>(v, q0);
+    }
+}
+
+// Merges the up to KNN_QUEUE newest candidates of a lane's queue (at `column`;
+// `slot`: its next free slot) into its ascending top-33 a[] and refills their
+// slots with +inf.  tie_out ("a particle outside a[] has d2 == a[32]") stays
 // exact: the values dropped by the merge are all >= the 34th smallest t34, so
 // one of them ties the new a[32] exactly when t34 == a[32]; an earlier tie
 // survives only while a[32] is unchanged.
-__device__ __forceinline__ void knn_flush(float (&a)[K_NN], float* qb, float*& qp, bool& tie_out)
+__device__ __forceinline__ void knn_flush(float (&a)[K_NN], unsigned column, unsigned& slot,
+                                          bool& tie_out)
 {
+    slot = max(slot, column + QUEUE_ROW * KNN_QUEUE) - QUEUE_ROW * KNN_QUEUE;
     float v[KNN_QUEUE];
-#pragma unroll
-    for (int i = 0; i < KNN_QUEUE; ++i) {
-        v[i] = qb[32 * i];
-        qb[32 * i] = INFINITY;
-    }
-    qp = qb;
+    knn_take<0>(v, slot);
     knn_sort16(v);
     const float old = a[K_NN - 1];
     const float t34 = knn_merge33(a, v);
@@ -61,15 +119,26 @@ __device__ __forceinline__ void knn_flush(float (&a)[K_NN], float* qb, float*& q
     tie_out = (top == old && tie_out) || t34 == top;
 }
 
-// squared distance from the query to a child (point for a leaf child)
-__device__ __forceinline__ float child_dist2(const float4* __restrict__ pos, const TreeView& t,
-                                             int c, float4 q)
+// four candidates against the lane's query: the distances two at a time in
+// packed f32x2 operations (equal values queue too: the merge tracks ties)
+template <int J>
+__device__ __forceinline__ void knn_scan(unsigned warp_base, f32x2 qx, f32x2 qy, f32x2 qz,
+                                         float limit, unsigned& slot)
 {
-    if (c < 0) {
-        const float4 p = pos[~c];
-        return norm2_rn(q.x, q.y, q.z, p.x, p.y, p.z);
+    if constexpr (J < KNN_CHUNK) {
+        constexpr unsigned C = (unsigned)offsetof(KnnWarp, cand) + 4u * J, ROW = 4u * KNN_CHUNK;
+        f32x2 x0, x1, y0, y1, z0, z1;
+        lds_x2<C>(warp_base, x0, x1);
+        lds_x2<C + ROW>(warp_base, y0, y1);
+        lds_x2<C + 2 * ROW>(warp_base, z0, z1);
+        const f32x2 d01 = norm2_rn_x2(qx, qy, qz, x0, y0, z0);
+        const f32x2 d23 = norm2_rn_x2(qx, qy, qz, x1, y1, z1);
+        knn_push(slot, lo2(d01), limit);
+        knn_push(slot, hi2(d01), limit);
+        knn_push(slot, lo2(d23), limit);
+        knn_push(slot, hi2(d23), limit);
+        knn_scan<J + 4>(warp_base, qx, qy, qz, limit, slot);
     }
-    return box_dist2_rn(q.x, q.y, q.z, t.blo[c], t.bhi[c]);
 }
 
 // t33 = the 33rd smallest d2 (with multiplicity), rk = sqrtf(t33), and a tie
@@ -77,131 +146,165 @@ __device__ __forceinline__ float child_dist2(const float4* __restrict__ pos, con
 // 32-set is {d2 < t33} and needs no index), -2 when ties must be resolved.
 // Each lane keeps its 33 smallest d2 sorted in registers; a candidate with
 // d2 <= a[32] goes to the lane's queue in shared memory, and when any lane's
-// queue holds more than KNN_QUEUE - 2 values after a step of two candidates
-// the warp merges every queue with two comparator networks (sort the queue,
+// queue holds more than KNN_QUEUE values after a chunk of 16 candidates the
+// warp merges the newest of every queue with two comparator networks (sort,
 // odd-even merge with a[]), about a quarter of the min/max work of inserting
 // each candidate as it comes.  Thresholds are the merged a[32], an upper bound
-// of the true one while values wait in the queue.  The ids of the buckets
-// scanned go to blist for k_dens_scatter.
-template <int T33_WARPS>
+// of the true one while values wait in the queue.  The leaves scanned go to
+// blist for k_dens_scatter.
+//
+// Bound by instruction issue: 74% of issue slots busy, 18.3 K warp instructions
+// per bundle (a fifth of them the networks' min/max on the ALU pipe, 60% busy),
+// DRAM below 1%.  16.7 -> 11.0 ms on the 256^3 step (18.3 M particles) against
+// the binary radix tree with 27.7 K; 0.43 -> 0.27 ms at 377 k particles.
+//
+// The walk goes up from the bundle's own leaf: the siblings of its leaves
+// first, then at every level the siblings of its ancestor.  A node is opened by
+// all lanes together, a child per lane: the distance of the child's box to the
+// bundle's box, as an integer key with the lane in its low bits, so one warp
+// minimum gives the nearest child left, and a node is done when that one lies
+// beyond the largest radius of the bundle.  Keys of the levels above wait in
+// shared memory.  A leaf is scanned if some lane's own radius reaches its box.
+// LEAF16: leaves of 16 particles (the default), one chunk each.
+template <int T33_WARPS, bool LEAF16>
 __global__ void __launch_bounds__(T33_WARPS * 32, 32 / T33_WARPS)
-k_knn_t33(const float4* __restrict__ pos, TreeView t, float* __restrict__ t33,
-          float* __restrict__ rk, int* __restrict__ idx33, int* __restrict__ blist, int* err)
+k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
+          float* __restrict__ t33, float* __restrict__ rk, int* __restrict__ idx33,
+          int* __restrict__ blist, int* err)
 {
-    __shared__ int stk[T33_WARPS][STACK_MAX];
-    __shared__ __align__(16) float cand[T33_WARPS][3][32];  // x, y, z of the bucket's particles
-    __shared__ float queue[T33_WARPS][KNN_QUEUE][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ __align__(16) KnnWarp smem[T33_WARPS];
+    const int lane = threadIdx.x & 31;
     const int n = t.n;
-    const int base = (blockIdx.x * T33_WARPS + warp) * 32;
+    const int base = (blockIdx.x * T33_WARPS + (threadIdx.x >> 5)) * 32;
     if (base >= n) return;
-    const int q = min(base + lane, n - 1);
-    const float4 xq = pos[q];
-    const f32x2 qx = pack2(xq.x, xq.x), qy = pack2(xq.y, xq.y), qz = pack2(xq.z, xq.z);
+    KnnWarp& S = smem[threadIdx.x >> 5];
+    const unsigned warp_base = (unsigned)__cvta_generic_to_shared(&S);
+    const unsigned column = warp_base + 4u * (unsigned)lane;
+    const int leaf = LEAF16 ? 16 : t.leaf;
+#pragma unroll
+    for (int i = 0; i < KNN_SLOTS; ++i) S.queue[i][lane] = INFINITY;
+    f32x2 qx, qy, qz;
+    {
+        const float4 p = pos[min(base + lane, n - 1)];
+        qx = pack2(p.x, p.x);
+        qy = pack2(p.y, p.y);
+        qz = pack2(p.z, p.z);
+    }
     float a[K_NN];
 #pragma unroll
     for (int k = 0; k < K_NN; ++k) a[k] = INFINITY;
     bool tie_out = false;  // a particle outside a[] has d2 == a[32]
-    float* qb = &queue[warp][0][lane];
-    float* qp = qb;  // the lane's next free queue slot (qb + 32 x queued values)
-#pragma unroll
-    for (int i = 0; i < KNN_QUEUE; ++i) qb[32 * i] = INFINITY;
-    __shared__ int nlist[T33_WARPS];  // buckets scanned (kept in shared memory: registers are full)
-    if (lane == 0) nlist[warp] = 0;
+    unsigned slot = column;
+    int nlist = 0, entry = 0;  // leaves scanned; entry 32 k + lane of the list not yet written
 
-    // the nearer child is visited next without going through the stack; the
-    // farther one waits on it
-    int* st = stk[warp];
-    int sp = 0;
-    int next = tree_root(n);
-    bool overflow = false;
-    for (;;) {
-        int node = next;
-        next = NO_NODE;
-        const bool popped = node == NO_NODE;  // else its box passed the test just now
-        if (popped) {
-            if (sp == 0) break;
-            node = st[--sp];
-            __syncwarp();  // every lane has read the slot before it is written again
-        }
-        int first, last;
-        if (node < 0) {
-            first = last = ~node;
-        } else {
-            // the node's record in one round trip: meta and the child boxes (a
-            // leaf child's box is its point, so d equals the point's norm2)
-            const float4* rp = t.rec + 4 * (size_t)node;
-            const float4 r0 = rp[0], r1 = rp[1], r2 = rp[2], r3 = rp[3];
-            const int4 m = make_int4(__float_as_int(r0.x), __float_as_int(r0.y),
-                                     __float_as_int(r0.z), __float_as_int(r0.w));
-            if (m.w - m.z + 1 > t.leaf) {
-                const f32x2 d01 = node_fast2(qx, qy, qz, r1, r2, r3);
-                const float d0 = lo2(d01), d1 = hi2(d01);
-                const float bound = prune_bound(a[K_NN - 1]);
-                // a node whose distance equals a[32] can hold a tie: visit it
-                const bool v0 = __any_sync(FULL, d0 <= bound);
-                const bool v1 = __any_sync(FULL, d1 <= bound);
-                const bool c0_near = __popc(__ballot_sync(FULL, d0 <= d1)) >= 16;
-                const int nn = c0_near ? m.x : m.y, ff = c0_near ? m.y : m.x;
-                const bool vn = c0_near ? v0 : v1, vf = c0_near ? v1 : v0;
-                if (vf) {
-                    if (sp + 1 > STACK_MAX) { overflow = true; break; }
-                    if (lane == 0) st[sp] = ff;
-                    ++sp;
-                    __syncwarp();
-                }
-                if (vn) next = nn;
-                continue;
-            }
-            first = m.z;
-            last = m.w;
-            // thresholds may have shrunk since the push: re-test a popped bucket
-            if (popped && !__any_sync(FULL, rec_fast0(xq, r1, r2) <= prune_bound(a[K_NN - 1])))
-                continue;
-        }
-        if (blist && lane == 0) {
-            const int k = nlist[warp];
-            if (k < KNN_LIST) blist[(size_t)(base >> 5) * (KNN_LIST + 1) + 1 + k] = node;
-            nlist[warp] = k + 1;
-        }
-        const int cnt = last - first + 1;
-        // an odd bucket is padded with a NaN point, whose distance queues nowhere
-        if (lane < cnt) {
-            const float4 p = pos[first + lane];
-            cand[warp][0][lane] = p.x;
-            cand[warp][1][lane] = p.y;
-            cand[warp][2][lane] = p.z;
-        } else if (lane == cnt) {
-            cand[warp][0][lane] = __int_as_float(0x7fc00000);
-            cand[warp][1][lane] = 0.0f;
-            cand[warp][2][lane] = 0.0f;
-        }
+    // keys up to `bound` are within the bundle's largest radius.  The bundle's
+    // own leaves have keys below 32, all others at least 32, so they come first;
+    // a node at distance 0 (a key below 64) always passes.
+    unsigned bound = 0x7fffffffu;
+    int g;  // the open group of leaves, 32 g ... 32 g + 31
+    auto child_key = [&](int level, int id) {
+        return max(__float_as_uint(boxes_dist2_fast(S.box, tree_box(t, level, id))) & ~31u, 32u) |
+               (unsigned)lane;
+    };
+    unsigned key = ~0u;  // the lane's leaf of the group, ~0: none or visited
+    {
+        const int own0 = base / leaf, own1 = (min(base + 32, n) - 1) / leaf;
+        const TreeBox b = bundle_box(t, own0, own1);
+        if (lane == 0) S.box = b;
         __syncwarp();
-        // two candidates per step (their distances in packed f32x2 operations),
-        // then one check: every queue holds at most KNN_QUEUE - 2 values when a
-        // step begins (equal values queue too: the merge tracks ties)
-        const f32x2* cx = reinterpret_cast<const f32x2*>(cand[warp][0]);
-        const f32x2* cy = reinterpret_cast<const f32x2*>(cand[warp][1]);
-        const f32x2* cz = reinterpret_cast<const f32x2*>(cand[warp][2]);
-        for (int j = 0; j < cnt; j += 2) {
-            const f32x2 d2 = norm2_rn_x2(qx, qy, qz, cx[j >> 1], cy[j >> 1], cz[j >> 1]);
-            const float d0 = lo2(d2), d1 = hi2(d2);
-            const float top = a[K_NN - 1];
-            if (d0 <= top) { *qp = d0; qp += 32; }
-            if (d1 <= top) { *qp = d1; qp += 32; }
-            if (__any_sync(FULL, qp > qb + 32 * (KNN_QUEUE - 2))) knn_flush(a, qb, qp, tie_out);
-        }
-        __syncwarp();
+        g = own0 >> 5;
+        const int id = g * 32 + lane;
+        if (id < t.cnt[0]) key = id >= own0 && id <= own1 ? (unsigned)lane : child_key(0, id);
     }
-    if (__any_sync(FULL, qp > qb)) knn_flush(a, qb, qp, tie_out);
-    // every bucket any lane's final radius reaches was scanned, so the list is
-    // complete for k_dens_scatter unless it overflowed or the stack did
-    if (blist && lane == 0)
-        blist[(size_t)(base >> 5) * (KNN_LIST + 1)] =
-            (overflow || nlist[warp] > KNN_LIST) ? -1 : nlist[warp];
-    if (overflow) {
-        if (lane == 0) atomicOr(err, ERR_STACK);
-        return;
+    int top = 0;  // the highest level opened so far
+    for (;;) {
+        // ---- the leaves of group g, nearest first ----
+        for (;;) {
+            const unsigned m = __reduce_min_sync(FULL, key);
+            if (m > bound) break;
+            if (key == m) key = ~0u;
+            const int id = g * 32 + (int)(m & 31u);
+            const float4* bp = t.box + 2 * (size_t)id;
+            const TreeBox c = {bp[0], bp[1]};
+            if (!__any_sync(FULL, point_box_fast(make_float4(lo2(qx), lo2(qy), lo2(qz), 0.f), c) <=
+                                      prune_bound(a[K_NN - 1])))
+                continue;
+            if (lane == (nlist & 31)) entry = id;
+            ++nlist;
+            if (blist && (nlist & 31) == 0 && nlist <= KNN_LIST)
+                blist[(size_t)(base >> 5) * (KNN_LIST + 1) + 1 + nlist - 32 + lane] = entry;
+            const int cnt = LEAF16 ? 16 : leaf_count(t, id);
+            for (int c0 = 0; c0 < cnt; c0 += KNN_CHUNK) {
+                __syncwarp();  // every lane is done with the chunk before it
+                if (lane < KNN_CHUNK) {
+                    // missing candidates are NaN points, whose distances queue nowhere
+                    const int i = id * leaf + c0 + lane;
+                    const bool have = LEAF16 ? i < n : c0 + lane < cnt;
+                    const float4 p = pos[have ? i : 0];
+                    constexpr unsigned C = (unsigned)offsetof(KnnWarp, cand), ROW = 4u * KNN_CHUNK;
+                    sts_f32<C>(column, have ? p.x : __int_as_float(0x7fc00000));
+                    sts_f32<C + ROW>(column, p.y);
+                    sts_f32<C + 2 * ROW>(column, p.z);
+                }
+                __syncwarp();
+                knn_scan<0>(warp_base, qx, qy, qz, a[K_NN - 1], slot);
+                if (__any_sync(FULL, slot > column + QUEUE_ROW * KNN_QUEUE)) {
+                    knn_flush(a, column, slot, tie_out);
+                    bound = max(__reduce_max_sync(FULL, __float_as_uint(prune_bound(a[K_NN - 1]))) | 31u,
+                                63u);
+                }
+                if (LEAF16) break;
+            }
+        }
+        // ---- the next group: down the nearest pending child of the lowest level
+        // that has one, else the siblings of the bundle's ancestor ----
+        int L = 0, id = g;  // `id`: the group just done is node `id` of level L + 1
+        bool found = false;
+        for (;;) {
+            ++L;
+            int own = -1;
+            unsigned k;
+            if (L <= top) {
+                k = S.keys[L - 1][lane];
+            } else {
+                if (top == t.nlev - 1) break;
+                top = L;
+                own = id;
+                k = ~0u;
+            }
+            id >>= 5;  // the group of level L that node `id` was in
+            if (own >= 0) {
+                const int c = id * 32 + lane;
+                if (c < t.cnt[L] && c != own) k = child_key(L, c);
+            }
+            // descend as long as a child within reach is left
+            for (;;) {
+                const unsigned m = __reduce_min_sync(FULL, k);
+                if (m > bound) break;
+                S.keys[L - 1][lane] = k == m ? ~0u : k;
+                id = id * 32 + (int)(m & 31u);
+                --L;
+                const int c = id * 32 + lane;
+                k = c < t.cnt[L] ? child_key(L, c) : ~0u;
+                if (L == 0) {
+                    g = id;
+                    key = k;
+                    found = true;
+                    break;
+                }
+            }
+            if (found) break;
+            S.keys[L - 1][lane] = ~0u;  // nothing left here, now or later (radii only shrink)
+        }
+        if (!found) break;
+    }
+    if (__any_sync(FULL, slot > column)) knn_flush(a, column, slot, tie_out);
+    // every leaf any lane's final radius reaches was scanned, so the list is
+    // complete for k_dens_scatter unless it overflowed
+    if (blist) {
+        int* bl = blist + (size_t)(base >> 5) * (KNN_LIST + 1);
+        if (nlist <= KNN_LIST && lane < (nlist & 31)) bl[1 + (nlist & ~31) + lane] = entry;
+        if (lane == 0) bl[0] = nlist > KNN_LIST ? -1 : nlist;
     }
     if (base + lane < n) {
         const float v = a[K_NN - 1];
@@ -222,11 +325,10 @@ k_knn_t33(const float4* __restrict__ pos, TreeView t, float* __restrict__ t33,
 constexpr int TIE_PASSES = (K_NN + TIE_MAX - 1) / TIE_MAX;
 
 __global__ void __launch_bounds__(KNN_WARPS * 32)
-k_knn_ties(const float4* __restrict__ pos, TreeView t, const float* __restrict__ t33,
+k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, const float* __restrict__ t33,
            int* __restrict__ idx33, int all, int* err)
 {
-    __shared__ int stk[KNN_WARPS][STACK_MAX];
-    __shared__ float4 cand[KNN_WARPS][32];
+    __shared__ float4 cand[KNN_WARPS][LEAF_MAX];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = t.n;
     const int base = (blockIdx.x * KNN_WARPS + warp) * 32;
@@ -236,75 +338,62 @@ k_knn_ties(const float4* __restrict__ pos, TreeView t, const float* __restrict__
     const bool want = (base + lane < n) && (all || idx33[q] == -2);
     if (!__any_sync(FULL, want)) return;
     const float4 xq = pos[q];
-    const float T = t33[q];
+    const float T = t33[q], bound = prune_bound(T);
     int nless = 0, neq = 0;
     int need = 0;          // rank of the wanted index among the ties above floor
     int floor_idx = -1;    // this pass keeps tied indices > floor_idx
     bool open = want;      // this lane still looks for its index
     int result = -1;
     int tie[TIE_MAX];
-    int* st = stk[warp];
 
     for (int pass = 0; pass < TIE_PASSES; ++pass) {
         if (!__any_sync(FULL, open)) break;
 #pragma unroll
         for (int k = 0; k < TIE_MAX; ++k) tie[k] = INT_MAX;
-        if (lane == 0) st[0] = tree_root(n);
-        int sp = 1;
-        bool overflow = false;
-        __syncwarp();
-        while (sp > 0) {
-            const int node = st[--sp];
-            __syncwarp();
-            int first, last;
-            if (node < 0) {
-                first = last = ~node;
-            } else {
-                const float4* rp = t.rec + 4 * (size_t)node;
-                const float4 r0 = rp[0], r1 = rp[1], r2 = rp[2], r3 = rp[3];
-                const int4 m = make_int4(__float_as_int(r0.x), __float_as_int(r0.y),
-                                         __float_as_int(r0.z), __float_as_int(r0.w));
-                if (m.w - m.z + 1 > t.leaf) {
-                    const bool v0 = __any_sync(FULL, open && node_dist0(xq, r1, r2, r3) <= T);
-                    const bool v1 = __any_sync(FULL, open && node_dist1(xq, r1, r2, r3) <= T);
-                    if (sp + 2 > STACK_MAX) { overflow = true; break; }
-                    if (lane == 0) {
-                        if (v1) st[sp] = m.y;
-                        if (v0) st[sp + (v1 ? 1 : 0)] = m.x;
-                    }
-                    sp += (v0 ? 1 : 0) + (v1 ? 1 : 0);
-                    __syncwarp();
-                    continue;
-                }
-                first = m.z;
-                last = m.w;
-            }
-            const int cnt = last - first + 1;
-            if (lane < cnt) cand[warp][lane] = pos[first + lane];
-            __syncwarp();
-            for (int j = 0; j < cnt; ++j) {
-                const float4 c = cand[warp][j];
-                const float d2 = norm2_rn(xq.x, xq.y, xq.z, c.x, c.y, c.z);
-                if (pass == 0) nless += d2 < T ? 1 : 0;
-                const int ci = __float_as_int(c.w);
-                const bool eq = open && d2 == T && ci > floor_idx;
-                if (__any_sync(FULL, eq)) {
-                    if (pass == 0) neq += eq ? 1 : 0;
-                    int v = eq ? ci : INT_MAX;
+        // the box of the queries still open and their largest radius
+        TreeBox box;
+        box.a = open ? make_float4(xq.x, xq.y, xq.z, xq.x)
+                     : make_float4(INFINITY, INFINITY, INFINITY, -INFINITY);
+        box.b = open ? make_float4(xq.y, xq.z, 0.f, 0.f) : make_float4(-INFINITY, -INFINITY, 0.f, 0.f);
+        float reach = open ? bound : 0.0f;
 #pragma unroll
-                    for (int k = 0; k < TIE_MAX; ++k) {
-                        const int lo = min(tie[k], v);
-                        v = max(tie[k], v);
-                        tie[k] = lo;
+        for (int o = 16; o > 0; o >>= 1) {
+            TreeBox v;
+            v.a = make_float4(__shfl_xor_sync(FULL, box.a.x, o), __shfl_xor_sync(FULL, box.a.y, o),
+                              __shfl_xor_sync(FULL, box.a.z, o), __shfl_xor_sync(FULL, box.a.w, o));
+            v.b = make_float4(__shfl_xor_sync(FULL, box.b.x, o), __shfl_xor_sync(FULL, box.b.y, o),
+                              0.f, 0.f);
+            box_grow(box, v);
+            reach = fmaxf(reach, __shfl_xor_sync(FULL, reach, o));
+        }
+        tree_walk(t,
+            [&](const TreeBox& c, int, int) { return boxes_dist2_fast(box, c) <= reach; },
+            [&](int id) {
+                if (!__any_sync(FULL, open && point_box_fast(xq, tree_box(t, 0, id)) <= bound))
+                    return true;
+                const int first = id * t.leaf, cnt = leaf_count(t, id);
+                __syncwarp();
+                if (lane < cnt) cand[warp][lane] = pos[first + lane];
+                __syncwarp();
+                for (int j = 0; j < cnt; ++j) {
+                    const float4 c = cand[warp][j];
+                    const float d2 = norm2_rn(xq.x, xq.y, xq.z, c.x, c.y, c.z);
+                    if (pass == 0) nless += d2 < T ? 1 : 0;
+                    const int ci = __float_as_int(c.w);
+                    const bool eq = open && d2 == T && ci > floor_idx;
+                    if (__any_sync(FULL, eq)) {
+                        if (pass == 0) neq += eq ? 1 : 0;
+                        int v = eq ? ci : INT_MAX;
+#pragma unroll
+                        for (int k = 0; k < TIE_MAX; ++k) {
+                            const int lo = min(tie[k], v);
+                            v = max(tie[k], v);
+                            tie[k] = lo;
+                        }
                     }
                 }
-            }
-            __syncwarp();
-        }
-        if (overflow) {
-            if (lane == 0) atomicOr(err, ERR_STACK);
-            return;
-        }
+                return true;
+            });
         if (open) {
             if (pass == 0) {
                 need = K_NN - nless;  // position of the 33rd key among all the ties
@@ -333,9 +422,9 @@ k_knn_ties(const float4* __restrict__ pos, TreeView t, const float* __restrict__
 // w * 2^(FIX_BITS - e_j), where 2^e_j bounds hinv_j^3.  A query q that has j in
 // its 32-set has rk_j <= 2 rk_q (its 33 nearest lie within 2 rk_q of j), so
 // w <= hinv_q^3 <= 8 hinv_j^3 and every term stays below 2^(FIX_BITS + 3 + a
-// rounding margin).  A lane adds one bucket's terms (at most 32, in query
-// order) as a double-float and converts the sum to an integer once; the
-// integer atomics make the total independent of the order of the buckets.
+// rounding margin).  A lane adds the terms it takes in one leaf (at most 32, in
+// query order) as a double-float and converts the sum to an integer once; the
+// integer atomics make the total independent of the order of the leaves.
 constexpr int FIX_BITS = 40;
 
 // e_j with hinv_j^3 < 2^e_j (hinv^3 as the first factor of ker_rn); acc zeroed
@@ -352,27 +441,33 @@ __global__ void k_dens_prep(const float* __restrict__ rk, int n, int* __restrict
 }
 
 // The warp serves the 32 queries (sources) q of a bundle with their exact radii
-// and visits the buckets k_knn_t33 recorded for the bundle (each re-tested), or
-// walks the tree when the list overflowed or is absent.  In a bucket each lane
-// holds one candidate receiver j, and the warp loops over only the queries
-// whose radius reaches the bucket's box (a ballot; about 9 of 32 on the 256^3
-// cube): for each such q every lane tests whether its j is in q's 32-set
-// ((d2, index) below q's 33rd key) and adds ker(q, j) as 64-bit fixed point to
-// a register; one integer atomic per receiver and bucket adds the sum to
-// acc[j].  The sums are exact integers, so the order of the additions and
-// atomics does not matter.
-__global__ void __launch_bounds__(KNN_WARPS * 32)
-k_dens_scatter(const float4* __restrict__ pos, TreeView t, const float* __restrict__ t33,
+// and visits the leaves k_knn_t33 recorded for the bundle (each re-tested), or
+// walks the tree when the list overflowed or is absent.  In a leaf each lane
+// holds one candidate receiver j.  The queries whose radius reaches the leaf's
+// box (a ballot; about 10 of 32) put themselves into a list in shared memory,
+// and the warp loops over that list: for each such q every lane tests whether
+// its j is in q's 32-set ((d2, index) below q's 33rd key) and adds ker(q, j) as 64-bit fixed point to a register; one integer
+// atomic per receiver and leaf adds the sum to acc[j].  The sums are exact
+// integers, so the order of the additions and atomics does not matter.
+// HALVES (leaves of at most 16 particles): both half-warps hold the leaf's
+// receivers and take every second query, so no lane idles; their integer sums
+// are added by a shuffle before the atomic.
+// Bound by instruction issue (82% of slots busy, 11.3 K warp instructions per
+// bundle, of which the distances and weights are half): 7.10 -> 6.42 ms on the
+// 256^3 step against radix-tree buckets of 22 particles on average.
+template <bool HALVES>
+__global__ void __launch_bounds__(DENS_WARPS * 32)
+k_dens_scatter(const float4* __restrict__ pos, const __grid_constant__ TreeView t, const float* __restrict__ t33,
                const int* __restrict__ idx33, const int* __restrict__ blist,
                const float* __restrict__ rk, const int* __restrict__ dexp,
-               unsigned long long* __restrict__ acc, int* __restrict__ err)
+               unsigned long long* __restrict__ acc)
 {
-    __shared__ int stk[KNN_WARPS][STACK_MAX];
-    __shared__ float4 qpos[KNN_WARPS][32];  // x, y, z, t33 of the bundle's queries
-    __shared__ float4 qaux[KNN_WARPS][32];  // hinv, hinv^3, idx33 (int bits)
+    // the queries that reach the leaf at hand: x, y, z, t33 and hinv, hinv^3,
+    // idx33 (int bits), then entries that take nothing
+    __shared__ float4 qlist[DENS_WARPS][2][32 + 3];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = t.n;
-    const int base = (blockIdx.x * KNN_WARPS + warp) * 32;
+    const int base = (blockIdx.x * DENS_WARPS + warp) * 32;
     if (base >= n) return;
     const bool valid = base + lane < n;
     const int q = min(base + lane, n - 1);
@@ -380,29 +475,39 @@ k_dens_scatter(const float4* __restrict__ pos, TreeView t, const float* __restri
     const float T = valid ? t33[q] : -1.0f;  // a padding lane takes nothing
     const float hinv = __fdiv_rn(1.0f, rk[q]);
     const float bound = prune_bound(T);
-    qpos[warp][lane] = make_float4(xq.x, xq.y, xq.z, T);
-    qaux[warp][lane] = make_float4(hinv, __fmul_rn(__fmul_rn(hinv, hinv), hinv),
-                                   __int_as_float(idx33[q]), 0.0f);
-    __syncwarp();
-
-    // the bucket [first, last] (box from its node record, or a single particle)
-    // against the queries of mask M
+    const float4 qpos = make_float4(xq.x, xq.y, xq.z, T);
+    const float4 qaux = make_float4(hinv, __fmul_rn(__fmul_rn(hinv, hinv), hinv),
+                                    __int_as_float(idx33[q]), 0.0f);
     // the index rule of the 33rd key only matters in a bundle with a tied query
-    const bool any_tie = __any_sync(FULL, valid && idx33[q] >= 0);
-    auto scan = [&](int first, int last, unsigned M, auto ties) {
-        const int cnt = last - first + 1;
-        const bool have = lane < cnt;
-        const int j = first + (have ? lane : 0);
+    const bool any_tie = __any_sync(FULL, valid && __float_as_int(qaux.z) >= 0);
+    constexpr int STEP = HALVES ? 2 : 1;  // queries taken at a time
+    const bool upper = HALVES && lane >= 16;
+    // leaf `id` against the queries of mask M
+    auto scan = [&](int id, unsigned M, auto ties) {
+        const int first = id * t.leaf, cnt = leaf_count(t, id);
+        const int r = HALVES ? lane & 15 : lane;
+        const bool have = r < cnt;
+        const int j = first + (have ? r : 0);
         const float4 c = pos[j];
         const float sc = __int_as_float((127 + FIX_BITS - dexp[j]) << 23);  // 2^(FIX_BITS - e_j)
+        // the reaching queries, in lane order, padded to a multiple of the step
+        const int nq = __popc(M);
+        __syncwarp();  // the previous leaf's list is no longer read
+        if (M >> lane & 1u) {
+            const int k = __popc(M & lanemask_lt());
+            qlist[warp][0][k] = qpos;
+            qlist[warp][1][k] = qaux;
+        }
+        if (HALVES && lane == 0) qlist[warp][0][nq] = make_float4(0.f, 0.f, 0.f, -1.0f);
+        __syncwarp();
         const int cj = __float_as_int(c.w);
         const f32x2 cxy = pack2(c.x, c.y);
         float sh = 0.0f, sl = 0.0f;  // sum of the scaled weights, double-float
-        while (M) {
-            const int k = __ffs(M) - 1;
-            M &= M - 1;
-            const float4 Q = qpos[warp][k];
-            const float4 A = qaux[warp][k];
+        const float4* qp = &qlist[warp][0][upper ? 1 : 0];
+#pragma unroll DENS_UNROLL
+        for (int k = 0; k < nq; k += STEP) {
+            const float4 Q = qp[k];
+            const float4 A = qp[k + 35];
             // norm2 (nbr_search.cpp:20-25) and ker (:27-37) of (q, j), query first;
             // x and y as one packed pair (the same roundings)
             const f32x2 dxy = sub2_rn(pack2(Q.x, Q.y), cxy);
@@ -418,83 +523,40 @@ k_dens_scatter(const float4* __restrict__ pos, TreeView t, const float* __restri
             // w * 2^(FIX_BITS - e_j) is exact (a power-of-two scale)
             if (member) two_sum_acc_nonneg(sh, sl, __fmul_rn(w, sc));
         }
-        // one conversion per receiver and bucket: hi and lo rounded to integers
+        // one conversion per receiver and leaf: hi and lo rounded to integers
         // (lo may be negative; the sum is not)
-        const long long sum = __float2ll_rn(sh) + __float2ll_rn(sl);
-        if (have && sum) atomicAdd(&acc[j], (unsigned long long)sum);
+        long long sum = __float2ll_rn(sh) + __float2ll_rn(sl);
+        if constexpr (HALVES) sum += __shfl_down_sync(FULL, sum, 16);
+        if (have && !upper && sum) atomicAdd(&acc[j], (unsigned long long)sum);
     };
-    // the queries whose radius reaches a bucket node's box
-    auto reach = [&](int node) -> unsigned {
-        if (node < 0) return __ballot_sync(FULL, valid);
-        const float4* rp = t.rec + 4 * (size_t)node;
-        return __ballot_sync(FULL, rec_fast0(xq, rp[1], rp[2]) <= bound);
-    };
-    auto bucket_range = [&](int node, int& first, int& last) {
-        if (node < 0) {
-            first = last = ~node;
-        } else {
-            const float4 r0 = t.rec[4 * (size_t)node];
-            first = __float_as_int(r0.z);
-            last = __float_as_int(r0.w);
-        }
+    auto visit = [&](int id) {
+        // the queries whose radius reaches the leaf's box
+        const float4* bp = t.box + 2 * (size_t)id;
+        const unsigned M = __ballot_sync(FULL, point_box_fast(xq, TreeBox{bp[0], bp[1]}) <= bound);
+        if (!M) return;
+        if (any_tie) scan(id, M, std::true_type{});
+        else scan(id, M, std::false_type{});
     };
 
     const int* bl = blist ? blist + (size_t)(base >> 5) * (KNN_LIST + 1) : nullptr;
     const int nlist = bl ? bl[0] : -1;
     if (nlist >= 0) {
-        // the list in registers: entry i in lane i & 31 of word i >> 5
-        int e[(KNN_LIST + 31) / 32];
-#pragma unroll
-        for (int w = 0; w < (KNN_LIST + 31) / 32; ++w)
-            e[w] = 32 * w + lane < nlist ? bl[1 + 32 * w + lane] : 0;
-        for (int i = 0; i < nlist; ++i) {
-            int v = e[0];
-#pragma unroll
-            for (int w = 1; w < (KNN_LIST + 31) / 32; ++w)
-                if ((i >> 5) == w) v = e[w];
-            const int node = __shfl_sync(FULL, v, i & 31);
-            const unsigned M = reach(node);
-            if (!M) continue;
-            int first, last;
-            bucket_range(node, first, last);
-            if (any_tie) scan(first, last, M, std::true_type{});
-            else scan(first, last, M, std::false_type{});
+        for (int i0 = 0; i0 < nlist; i0 += 32) {
+            const int cnt = min(32, nlist - i0);
+            const int e = lane < cnt ? bl[1 + i0 + lane] : 0;
+            for (int i = 0; i < cnt; ++i) visit(__shfl_sync(FULL, e, i));
         }
         return;
     }
-
-    int* st = stk[warp];
-    if (lane == 0) st[0] = tree_root(n);
-    int sp = 1;
-    __syncwarp();
-    while (sp > 0) {
-        const int node = st[--sp];
-        __syncwarp();
-        if (node >= 0) {
-            const int4 m = t.meta[node];
-            if (m.w - m.z + 1 > t.leaf) {
-                const bool v0 = __any_sync(FULL, child_dist2(pos, t, m.x, xq) <= T);
-                const bool v1 = __any_sync(FULL, child_dist2(pos, t, m.y, xq) <= T);
-                if (sp + 2 > STACK_MAX) {
-                    if (lane == 0) atomicOr(err, ERR_STACK);
-                    break;
-                }
-                if (lane == 0) {
-                    if (v1) st[sp] = m.y;
-                    if (v0) st[sp + (v1 ? 1 : 0)] = m.x;
-                }
-                sp += (v0 ? 1 : 0) + (v1 ? 1 : 0);
-                __syncwarp();
-                continue;
-            }
-        }
-        const unsigned M = reach(node);
-        if (!M) continue;
-        int first, last;
-        bucket_range(node, first, last);
-        if (any_tie) scan(first, last, M, std::true_type{});
-        else scan(first, last, M, std::false_type{});
-    }
+    const TreeBox box = bundle_box(t, base / t.leaf, (min(base + 32, n) - 1) / t.leaf);
+    float reach = bound;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) reach = fmaxf(reach, __shfl_xor_sync(FULL, reach, o));
+    tree_walk(t, [&](const TreeBox& c, int, int) { return boxes_dist2_fast(box, c) <= reach; },
+              [&](int id) {
+                  visit(id);
+                  return true;
+              });
 }
 
 // dens_j += acc_j * 2^(e_j - FIX_BITS), one rounding to float
@@ -516,10 +578,16 @@ void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk,
                     int* blist, int* err, cudaStream_t s, int warps)
 {
     if (t.n <= 0) return;
-    if (warps == 4)
-        k_knn_t33<4><<<(t.n + 127) / 128, 128, 0, s>>>(pos, t, t33, rk, idx33, blist, err);
-    else
-        k_knn_t33<2><<<(t.n + 63) / 64, 64, 0, s>>>(pos, t, t33, rk, idx33, blist, err);
+    auto run = [&](auto kern, int w) {
+        kern<<<(unsigned)(((long long)t.n + 32 * w - 1) / (32 * w)), 32 * w, 0, s>>>(
+            pos, t, t33, rk, idx33, blist, err);
+    };
+    // Leaves of 16 run one warp per block, so that every warp that ends makes
+    // room at once: 11.02 against 11.44 ms in blocks of 2 on the 256^3 step
+    // (persistent warps that take bundles by ticket: 11.53).
+    if (t.leaf == 16) run(k_knn_t33<1, true>, 1);
+    else if (warps == 4) run(k_knn_t33<4, false>, 4);
+    else run(k_knn_t33<2, false>, 2);
     count_launches(1);
 }
 
@@ -533,13 +601,15 @@ void launch_knn_ties(const float4* pos, const TreeView& t, const float* t33, int
 
 void launch_dens(const float4* pos, const TreeView& t, const float* t33, const int* idx33,
                  const int* blist, const float* rk, int* dexp, unsigned long long* acc,
-                 float4* vel, int* err, cudaStream_t s)
+                 float4* vel, cudaStream_t s)
 {
     if (t.n <= 0) return;
-    const int nb = (t.n + 255) / 256;
+    const int nb = (t.n + 255) / 256, nw = (t.n + DENS_WARPS * 32 - 1) / (DENS_WARPS * 32);
     k_dens_prep<<<nb, 256, 0, s>>>(rk, t.n, dexp, acc);
-    k_dens_scatter<<<knn_blocks(t.n), KNN_WARPS * 32, 0, s>>>(pos, t, t33, idx33, blist, rk, dexp,
-                                                             acc, err);
+    if (t.leaf <= 16)
+        k_dens_scatter<true><<<nw, DENS_WARPS * 32, 0, s>>>(pos, t, t33, idx33, blist, rk, dexp, acc);
+    else
+        k_dens_scatter<false><<<nw, DENS_WARPS * 32, 0, s>>>(pos, t, t33, idx33, blist, rk, dexp, acc);
     k_dens_finish<<<nb, 256, 0, s>>>(acc, dexp, t.n, vel);
     count_launches(3);
 }

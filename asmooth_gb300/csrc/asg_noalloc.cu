@@ -42,8 +42,7 @@ constexpr int NOALLOC_MAX_DEVICES = 64;
 // byte offsets of the arrays carved out of the scratch for n particles
 struct NoallocLayout {
     size_t pos_in, vel_in, igrp_in, rk_in, keys0, keys1, vals0, vals1, sort_tmp;
-    size_t pos, vel, igrp, rk, t33, idx33, meta, parent, leaf_parent, flags;
-    size_t blo, bhi, rec, dacc, dexp, err, total;
+    size_t pos, vel, igrp, rk, t33, idx33, boxes, blist, dacc, dexp, err, total;
 };
 
 static constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
@@ -51,7 +50,6 @@ static constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 static NoallocLayout noalloc_layout(size_t n)
 {
     NoallocLayout L{};
-    const size_t m = n > 1 ? n - 1 : 1;
     size_t o = 0;
     auto take = [&](size_t bytes) {
         const size_t at = o;
@@ -73,13 +71,8 @@ static NoallocLayout noalloc_layout(size_t n)
     L.rk = take(4 * n);
     L.t33 = take(4 * n);
     L.idx33 = take(4 * n);
-    L.meta = take(16 * m);
-    L.parent = take(4 * m);
-    L.leaf_parent = take(4 * n);
-    L.flags = take(4 * m);
-    L.blo = take(16 * m);
-    L.bhi = take(16 * m);
-    L.rec = take(64 * m);
+    L.boxes = take(tree_box_bytes((int)n, LEAF_DEFAULT));
+    L.blist = take(4 * knn_list_words((int)n));
     L.dacc = take(8 * n);
     L.dexp = take(4 * n);
     L.err = take(16);
@@ -191,26 +184,17 @@ extern "C" int asg_neighbor_search_noalloc(const float* d_x, int np, float left,
     const int cur = radix_sort(reinterpret_cast<uint64_t*>(b + L.keys0), I(L.vals0),
                                reinterpret_cast<uint64_t*>(b + L.keys1), I(L.vals1), np, 48,
                                b + L.sort_tmp, s);
-    const uint64_t* keys = reinterpret_cast<const uint64_t*>(b + (cur ? L.keys1 : L.keys0));
     const int* perm = I(cur ? L.vals1 : L.vals0);
     launch_gather_sorted(perm, F4(L.pos_in), F4(L.vel_in), I(L.igrp_in), F(L.rk_in), np, F4(L.pos),
                          F4(L.vel), I(L.igrp), F(L.rk), s);
-    launch_build_tree(keys, np, reinterpret_cast<int4*>(b + L.meta), I(L.parent), I(L.leaf_parent),
-                      s);
-    launch_tree_boxes(F4(L.pos), nullptr, np, LEAF_MAX, reinterpret_cast<int4*>(b + L.meta),
-                      I(L.parent), I(L.flags), F4(L.blo), F4(L.bhi), F4(L.rec), s);
-    TreeView t;
-    t.n = np;
-    t.leaf = LEAF_MAX;
-    t.meta = reinterpret_cast<const int4*>(b + L.meta);
-    t.blo = F4(L.blo);
-    t.bhi = F4(L.bhi);
-    t.rec = F4(L.rec);
-    launch_knn_t33(F4(L.pos), t, F(L.t33), F(L.rk), I(L.idx33), nullptr, err, s);
+    TreeView t = tree_shape(np, LEAF_DEFAULT);
+    t.box = F4(L.boxes);
+    launch_tree_boxes(F4(L.pos), t, s);
+    launch_knn_t33(F4(L.pos), t, F(L.t33), F(L.rk), I(L.idx33), I(L.blist), err, s);
     launch_knn_ties(F4(L.pos), t, F(L.t33), I(L.idx33), 0, err, s);
     launch_check_rk(F(L.rk), np, err, s);
-    launch_dens(F4(L.pos), t, F(L.t33), I(L.idx33), nullptr, F(L.rk), I(L.dexp),
-                reinterpret_cast<unsigned long long*>(b + L.dacc), F4(L.vel), err, s);
+    launch_dens(F4(L.pos), t, F(L.t33), I(L.idx33), I(L.blist), F(L.rk), I(L.dexp),
+                reinterpret_cast<unsigned long long*>(b + L.dacc), F4(L.vel), s);
     k_noalloc_store<<<(np + 255) / 256, 256, 0, s>>>(perm, F(L.rk), F4(L.vel), np, d_rk, d_dens);
     count_launches(1);
 

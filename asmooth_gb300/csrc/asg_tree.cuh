@@ -1,0 +1,105 @@
+// asg_tree.cuh -- traversal of the blocked box tree (TreeView, asg_internal.h).
+//
+// Level 0 holds the boxes of `leaf` consecutive particles of the space-filling
+// curve, every level above the boxes of 32 consecutive boxes below, up to a top
+// level of at most 32 boxes.  The shape is implied by n and leaf, so a node is
+// its number and its children are 32 * number + lane: a warp opens a node with
+// one coalesced load, a child per lane.
+//
+// Why 32 children and a box test against the whole bundle: a binary radix tree
+// walked with one test per query and child took about 115 dependent visits of
+// some 60 instructions per 32-query bundle on the 256^3 cube; here a bundle
+// opens about 17 nodes of some 40 instructions, and only the leaves whose box
+// reaches the bundle's largest radius (about 110, of which 49 hold work) get a
+// test per query.
+#pragma once
+
+#include "asg_common.cuh"
+#include "asg_internal.h"
+
+namespace asg {
+
+// a box of the tree: two float4, lo.xyz hi.x | hi.yz - -
+struct TreeBox {
+    float4 a, b;
+};
+__device__ __forceinline__ TreeBox tree_box(const TreeView& t, int level, int id)
+{
+    const float4* p = t.box + 2 * ((size_t)t.off[level] + (size_t)id);
+    return {p[0], p[1]};
+}
+
+// Pruning-only squared distance between two boxes, compared against
+// prune_bound: per axis fl(lo - hi') is at most |fl(p - q)| for every p of one
+// box and q of the other (rounding is monotone), so box_dist2_fast's bound
+// holds for every pair of points.
+__device__ __forceinline__ float boxes_dist2_fast(const TreeBox& q, const TreeBox& c)
+{
+    const float dx = max3f(c.a.x - q.a.w, q.a.x - c.a.w, 0.0f);
+    const float dy = max3f(c.a.y - q.b.x, q.a.y - c.b.x, 0.0f);
+    const float dz = max3f(c.a.z - q.b.y, q.a.z - c.b.y, 0.0f);
+    return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+}
+// a point against a box, pruning only (box_dist2_fast)
+__device__ __forceinline__ float point_box_fast(float4 q, const TreeBox& c)
+{
+    return box_dist2_fast(q.x, q.y, q.z, c.a.x, c.a.y, c.a.z, c.a.w, c.b.x, c.b.y);
+}
+__device__ __forceinline__ void box_grow(TreeBox& q, const TreeBox& c)
+{
+    q.a = make_float4(fminf(q.a.x, c.a.x), fminf(q.a.y, c.a.y), fminf(q.a.z, c.a.z),
+                      fmaxf(q.a.w, c.a.w));
+    q.b = make_float4(fmaxf(q.b.x, c.b.x), fmaxf(q.b.y, c.b.y), 0.0f, 0.0f);
+}
+// the box of the leaves that hold particles [base, base + 31] (all of a bundle)
+__device__ __forceinline__ TreeBox bundle_box(const TreeView& t, int leaf0, int leaf1)
+{
+    TreeBox q = tree_box(t, 0, leaf0);
+    for (int i = leaf0 + 1; i <= leaf1; ++i) box_grow(q, tree_box(t, 0, i));
+    return q;
+}
+__device__ __forceinline__ int leaf_count(const TreeView& t, int id)
+{
+    return min(t.leaf, t.n - id * t.leaf);
+}
+
+// Visits, in a fixed order, every leaf all of whose ancestors pass: pass(box,
+// level, id) is asked by each lane for its own child, leaf(id) is called by the
+// whole warp (and may end the walk by returning false).  Lane l keeps the
+// pending children of the node open at level l.
+template <class Pass, class Leaf>
+__device__ __forceinline__ void tree_walk(const TreeView& t, Pass pass, Leaf leaf)
+{
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int L = t.nlev - 1, g = 0;
+    unsigned pending = 0;
+    auto open = [&]() {
+        const unsigned id = (unsigned)g * 32u + (unsigned)lane;
+        bool ok = id < (unsigned)t.cnt[L];
+        if (ok) ok = pass(tree_box(t, L, (int)id), L, (int)id);
+        const unsigned m = __ballot_sync(ALL, ok);
+        if (lane == L) pending = m;
+    };
+    open();
+    for (;;) {
+        const unsigned m = __shfl_sync(ALL, pending, L);
+        if (!m) {
+            if (L == t.nlev - 1) return;
+            ++L;
+            g >>= 5;
+            continue;
+        }
+        if (lane == L) pending = m & (m - 1);
+        const int id = g * 32 + __ffs(m) - 1;
+        if (L == 0) {
+            if (!leaf(id)) return;
+        } else {
+            --L;
+            g = id;
+            open();
+        }
+    }
+}
+
+}  // namespace asg
