@@ -4,11 +4,11 @@
 // write_mesh_separate, coarse_mesh.cpp:147-208; write_fof_halos).
 //
 // Catalogue: per label 1..nhalo, the float sums of x and v over the members in
-// the caller's array order (one thread per halo adds them sequentially, as the
-// reference's loop does, so the sums are the reference's bits), divided by the
-// member count; halos whose centre is strictly inside (0, boxsize)^3 are kept
-// in label order.  The members are grouped by a radix sort of
-// (label << 32 | input index).
+// the caller's array order (one lane per component adds them sequentially, as
+// the reference's loop does, so the sums are the reference's bits), divided by
+// the member count; halos whose centre is strictly inside (0, boxsize)^3 are
+// kept in label order.  The members are grouped by a stable radix sort of the
+// labels laid out in the caller's array order.
 #include <cstdio>
 #include <string>
 
@@ -36,8 +36,8 @@ static CatLayout cat_layout(int n, int nhalo)
         o = al256(o + b);
         return at;
     };
-    L.keys0 = take(8 * N);
-    L.keys1 = take(8 * N);
+    L.keys0 = take(4 * N);
+    L.keys1 = take(4 * N);
     L.vals0 = take(4 * N);
     L.vals1 = take(4 * N);
     L.sort_tmp = take(radix_sort_temp_bytes(n));
@@ -52,61 +52,127 @@ static CatLayout cat_layout(int n, int nhalo)
 
 size_t fof_catalogue_bytes(int n, int nhalo) { return cat_layout(n, nhalo).total; }
 
+// the label of the particle at position i of the caller's array, and its
+// position j in pos/vel (label 0: in no halo)
 __global__ void k_cat_keys(const float4* __restrict__ pos, const int* __restrict__ igrp, int n,
-                           int w_index, int nhalo, uint64_t* __restrict__ keys, int* __restrict__ vals)
+                           int w_index, int nhalo, uint32_t* __restrict__ keys, int* __restrict__ vals)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int lab = igrp[j];
-    const uint32_t idx = w_index ? (uint32_t)__float_as_int(pos[j].w) : (uint32_t)j;
-    const uint64_t hi = (lab >= 1 && lab <= nhalo) ? (uint64_t)lab : 0u;
-    keys[j] = (hi << 32) | idx;
-    vals[j] = j;
+    const int i = w_index ? __float_as_int(pos[j].w) : j;
+    keys[i] = (lab >= 1 && lab <= nhalo) ? (uint32_t)lab : 0u;
+    vals[i] = j;
 }
 
-__global__ void k_cat_bounds(const uint64_t* __restrict__ keys, int n, uint32_t* __restrict__ start,
+__global__ void k_cat_bounds(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ start,
                              uint32_t* __restrict__ end)
 {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n) return;
-    const uint32_t lab = (uint32_t)(keys[m] >> 32);
+    const uint32_t lab = keys[m];
     if (lab == 0) return;
-    if (m == 0 || (uint32_t)(keys[m - 1] >> 32) != lab) start[lab] = (uint32_t)m;
-    if (m == n - 1 || (uint32_t)(keys[m + 1] >> 32) != lab) end[lab] = (uint32_t)m + 1;
+    if (m == 0 || keys[m - 1] != lab) start[lab] = (uint32_t)m;
+    if (m == n - 1 || keys[m + 1] != lab) end[lab] = (uint32_t)m + 1;
 }
 
-// one thread per halo: sequential float sums in member (= caller array) order
-__global__ void k_cat_sums(const float4* __restrict__ pos, const float4* __restrict__ vel,
-                           const int* __restrict__ order, const uint32_t* __restrict__ start,
-                           const uint32_t* __restrict__ end, int nhalo, float boxsize,
-                           float* __restrict__ rec, uint32_t* __restrict__ flags)
+// The sums of a halo are six chains of dependent adds (four cycles each), so
+// the work around them is kept off the chains: T threads (a warp, or a block
+// for halos of more than CAT_BIG members) gather the next T members while
+// lanes 0-5 of the first warp add the previous T, one component each, from
+// shared memory.  On a 128^3 cube's catalogue (987 halos, the largest of 20,277
+// members) 7.5 -> 0.15 ms against one thread per halo, gathering as it added.
+// The blocks of large halos come first: they take longest.
+constexpr int CAT_THREADS = 256, CAT_BIG = 512;
+
+template <int T>
+struct CatRows {
+    float c[2][6][T + 4];  // [buffer][component][member of the chunk]
+};
+
+template <int T, class Sync>
+__device__ __forceinline__ float cat_sum(CatRows<T>& R, int tid, uint32_t s, uint32_t e,
+                                         const float4* __restrict__ pos,
+                                         const float4* __restrict__ vel,
+                                         const int* __restrict__ order, Sync sync)
 {
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= nhalo) return;
-    const uint32_t s = start[h + 1], e = end[h + 1];
-    float sx = 0.f, sy = 0.f, sz = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
-#pragma unroll 4
-    for (uint32_t m = s; m < e; ++m) {
-        const int j = order[m];
-        const float4 p = pos[j];
-        const float4 v = vel[j];
-        sx = __fadd_rn(sx, p.x);
-        sy = __fadd_rn(sy, p.y);
-        sz = __fadd_rn(sz, p.z);
-        ux = __fadd_rn(ux, v.x);
-        uy = __fadd_rn(uy, v.y);
-        uz = __fadd_rn(uz, v.z);
+    float sum = 0.f;
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), v = p;
+    // the member numbers are read one chunk before the members
+    int j = s + tid < e ? order[s + tid] : 0;
+    auto fetch = [&](uint32_t m) {
+        if (m + tid < e) {
+            p = pos[j];
+            v = vel[j];
+        }
+        if (m + T + tid < e) j = order[m + T + tid];
+    };
+    fetch(s);
+    int b = 0;
+    for (uint32_t m = s; m < e; m += T, b ^= 1) {
+        R.c[b][0][tid] = p.x;
+        R.c[b][1][tid] = p.y;
+        R.c[b][2][tid] = p.z;
+        R.c[b][3][tid] = v.x;
+        R.c[b][4][tid] = v.y;
+        R.c[b][5][tid] = v.z;
+        sync();  // the other buffer's chunk has been added by now, too
+        fetch(m + T);
+        if (tid < 6) {
+            const float* row = R.c[b][tid];
+            const int cnt = (int)min((uint32_t)T, e - m);
+            int i = 0;
+#pragma unroll 8
+            for (; i + 4 <= cnt; i += 4) {
+                const float4 x = *reinterpret_cast<const float4*>(row + i);
+                sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, x.x), x.y), x.z), x.w);
+            }
+            for (; i < cnt; ++i) sum = __fadd_rn(sum, row[i]);
+        }
     }
-    const int nf = (int)(e - s);
-    const float fn = __int2float_rn(nf);
-    float r[6] = {__fdiv_rn(sx, fn), __fdiv_rn(sy, fn), __fdiv_rn(sz, fn),
-                  __fdiv_rn(ux, fn), __fdiv_rn(uy, fn), __fdiv_rn(uz, fn)};
-    float* o = rec + (size_t)REC_WORDS * h;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) o[k] = r[k];
-    o[6] = __int_as_float(nf);
-    flags[h] = (0.0f < r[0] && r[0] < boxsize && 0.0f < r[1] && r[1] < boxsize && 0.0f < r[2] &&
-                r[2] < boxsize) ? 1u : 0u;
+    sync();  // the rows may be used again
+    return sum;
+}
+
+// lanes 0-5: the record's component sums divided by the member count
+__device__ __forceinline__ void cat_record(int lane, float sum, uint32_t members, float boxsize,
+                                           float* __restrict__ o, uint32_t* __restrict__ flag)
+{
+    const float r = __fdiv_rn(sum, __int2float_rn((int)members));
+    if (lane < 6) o[lane] = r;
+    if (lane == 6) o[6] = __int_as_float((int)members);
+    const bool in = lane >= 3 || (0.0f < r && r < boxsize);
+    const bool keep = __all_sync(0xffffffffu, in);
+    if (lane == 0) *flag = keep ? 1u : 0u;
+}
+
+__global__ void __launch_bounds__(CAT_THREADS)
+k_cat_sums(const float4* __restrict__ pos, const float4* __restrict__ vel,
+           const int* __restrict__ order, const uint32_t* __restrict__ start,
+           const uint32_t* __restrict__ end, int nhalo, int nbig, float boxsize,
+           float* __restrict__ rec, uint32_t* __restrict__ flags)
+{
+    constexpr int W = CAT_THREADS / 32;
+    __shared__ __align__(16) union Rows {
+        CatRows<CAT_THREADS> block;
+        CatRows<32> warp[W];
+    } R;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if ((int)blockIdx.x < nbig) {  // the large halos of every nbig-th label
+        for (int h = blockIdx.x; h < nhalo; h += nbig) {
+            const uint32_t s = start[h + 1], e = end[h + 1];
+            if (e - s <= CAT_BIG) continue;
+            const float sum = cat_sum<CAT_THREADS>(R.block, tid, s, e, pos, vel, order,
+                                                   [] { __syncthreads(); });
+            if (w == 0) cat_record(lane, sum, e - s, boxsize, rec + (size_t)REC_WORDS * h, flags + h);
+        }
+        return;
+    }
+    const int h = ((int)blockIdx.x - nbig) * W + w;  // a warp per halo
+    const uint32_t s = h < nhalo ? start[h + 1] : 0u, e = h < nhalo ? end[h + 1] : 0u;
+    if (h >= nhalo || e - s > CAT_BIG) return;
+    const float sum = cat_sum<32>(R.warp[w], lane, s, e, pos, vel, order, [] { __syncwarp(); });
+    cat_record(lane, sum, e - s, boxsize, rec + (size_t)REC_WORDS * h, flags + h);
 }
 
 // scan: exclusive scan of the keep flags over nhalo + 1 entries (the last flag
@@ -129,7 +195,6 @@ void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp,
 {
     const CatLayout L = cat_layout(n, nhalo);
     unsigned char* b = static_cast<unsigned char*>(scratch);
-    auto U64 = [&](size_t o) { return reinterpret_cast<uint64_t*>(b + o); };
     auto I = [&](size_t o) { return reinterpret_cast<int*>(b + o); };
     auto U = [&](size_t o) { return reinterpret_cast<uint32_t*>(b + o); };
     const size_t H = (size_t)nhalo + 1;
@@ -137,21 +202,21 @@ void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp,
     cudaMemsetAsync(b + L.end, 0, 4 * H, s);
     cudaMemsetAsync(b + L.flags, 0, 4 * H, s);
     if (n > 0) {
-        k_cat_keys<<<(n + 255) / 256, 256, 0, s>>>(pos, igrp, n, w_index, nhalo, U64(L.keys0),
+        k_cat_keys<<<(n + 255) / 256, 256, 0, s>>>(pos, igrp, n, w_index, nhalo, U(L.keys0),
                                                     I(L.vals0));
-        int bits = 32;
-        while (bits < 64 && ((uint64_t)nhalo >> (bits - 32)) != 0) ++bits;
-        const int cur = radix_sort(U64(L.keys0), I(L.vals0), U64(L.keys1), I(L.vals1), n, bits,
-                                   b + L.sort_tmp, s);
-        const uint64_t* keys = U64(cur ? L.keys1 : L.keys0);
+        int bits = 0;
+        while (bits < 31 && (nhalo >> bits) != 0) ++bits;
+        const int cur = radix_sort32(U(L.keys0), I(L.vals0), U(L.keys1), I(L.vals1), n, bits,
+                                     b + L.sort_tmp, s);
+        const uint32_t* keys = U(cur ? L.keys1 : L.keys0);
         const int* order = I(cur ? L.vals1 : L.vals0);
         k_cat_bounds<<<(n + 255) / 256, 256, 0, s>>>(keys, n, U(L.start), U(L.end));
         count_launches(2);
         if (nhalo > 0) {
-            k_cat_sums<<<(nhalo + 127) / 128, 128, 0, s>>>(pos, vel, order, U(L.start), U(L.end),
-                                                           nhalo, boxsize,
-                                                           reinterpret_cast<float*>(b + L.rec),
-                                                           U(L.flags));
+            const int nbig = nhalo < 8192 ? nhalo : 8192, per = CAT_THREADS / 32;
+            k_cat_sums<<<nbig + (nhalo + per - 1) / per, CAT_THREADS, 0, s>>>(
+                pos, vel, order, U(L.start), U(L.end), nhalo, nbig, boxsize,
+                reinterpret_cast<float*>(b + L.rec), U(L.flags));
             count_launches(1);
         }
     }
