@@ -59,9 +59,9 @@ struct asg_ctx {
     float left = 0.f, right = 0.f;
     bool loaded = false, knn_done = false, rk_checked = false, idx33_all = false;
     int leaf = LEAF_DEFAULT;  // particles per tree leaf
-    int dep_seg = 4096;  // pairs per deposit work item
+    int dep_seg = 4096;  // pairs per deposit work item, at most (small sets: deposit_seg)
     int knn_warps = 2;   // warps per block of the neighbour search (2 or 4)
-    int dep_mma = deposit_default_mma();  // deposit engine: tensor cores (1, 2) or CUDA cores (0)
+    int dep_mma = deposit_default_mma();  // deposit engine: tensor cores (1) or CUDA cores (0)
     int* perm = nullptr;       // sorted position -> input index
     uint64_t* keys = nullptr;  // sorted keys
 
@@ -70,19 +70,16 @@ struct asg_ctx {
     Buf boxes;       // boxes of the tree (TreeView::box)
     Buf dacc, dexp;  // dens: fixed-point sums and scale exponents
     Buf blist;       // leaves each bundle's neighbour search scanned
-    Buf dep_order;   // the deposit's tile processing order and its inverse
-    std::vector<int> dep_order_key;  // the mesh sizes dep_order was made for
-    bool dep_order_on = true;        // ASG_DEPOSIT_ORDER=tile: tile order
     Buf uf, minin, mark, scan_tmp, lab_cnt, lab_scan;
     Buf halos, hcount, hmass;
     Buf totals, lohi;
-    Buf dep_rec, dep_pcount, dep_tiles, dep_counter, dep_pairs, dep_sort, dep_partial;
+    Buf dep_rec, dep_pcount, dep_tiles, dep_items, dep_counter, dep_pairs, dep_sort, dep_partial;
     Buf cat, cat_out;  // FOF catalogue scratch and records
     Buf sh_in, sh_all; // periodic shell: interior input + bin sort, all copies + flags
     Buf dec_raw, dec_scan;  // file payloads on the device, zip count scans
     int dec_n = 0;          // particles of the last decode (in sh_in), 0 = none
-    uint32_t dep_npairs = 0;
-    int dep_tiles_n = 0;
+    uint32_t dep_npairs = 0, dep_nentries = 0;
+    int dep_tiles_n = 0, dep_cells = 0;  // tiles of the last deposit, cells of one
     uint32_t* h_u32 = nullptr;      // pinned, mapped
     uint32_t* h_u32_dev = nullptr;  // its device address
     float mesh_boxsize = 0.0f;
@@ -147,6 +144,7 @@ int device_status(int bits)
     if (bits & ERR_RANGE) return ASG_ERR_RANGE;
     if (bits & ERR_UF) return ASG_ERR_UNIONFIND;
     if (bits & ERR_BADCELL) return ASG_ERR_ARG;
+    if (bits & ERR_SORT) return ASG_ERR_CUDA;
     if (bits & ERR_CAP) return ASG_ERR_STATE;
     return ASG_OK;
 }
@@ -179,18 +177,20 @@ void phase_end(asg_ctx* ctx)
     ctx->open_phase = -1;
 }
 
-// Reads one or two device words into ctx->h_u32 and waits for them.  A kernel
+// Reads up to three device words into ctx->h_u32 and waits for them.  A kernel
 // stores them through the mapped host words: a copy would queue on the copy
 // engine behind any large device-to-host copy in flight on another stream.
-__global__ void k_read_words(const uint32_t* a, const uint32_t* b, uint32_t* out)
+__global__ void k_read_words(const uint32_t* a, const uint32_t* b, const uint32_t* c, uint32_t* out)
 {
     out[0] = *a;
     if (b) out[1] = *b;
+    if (c) out[2] = *c;
 }
 
-static int read_words(asg_ctx* ctx, const uint32_t* a, const uint32_t* b = nullptr)
+static int read_words(asg_ctx* ctx, const uint32_t* a, const uint32_t* b = nullptr,
+                      const uint32_t* c = nullptr)
 {
-    k_read_words<<<1, 1, 0, ctx->s>>>(a, b, ctx->h_u32_dev);
+    k_read_words<<<1, 1, 0, ctx->s>>>(a, b, c, ctx->h_u32_dev);
     count_launches(1);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(ctx->s));
@@ -260,7 +260,7 @@ int build_index(asg_ctx* ctx)
 {
     const int n = ctx->n;
     const int cur = radix_sort(P<uint64_t>(ctx->keys0), P<int>(ctx->vals0), P<uint64_t>(ctx->keys1),
-                               P<int>(ctx->vals1), n, 48, ctx->sort_tmp.p, ctx->s);
+                               P<int>(ctx->vals1), n, 48, true, ctx->sort_tmp.p, ctx->d_err, ctx->s);
     ctx->keys = cur ? P<uint64_t>(ctx->keys1) : P<uint64_t>(ctx->keys0);
     ctx->perm = cur ? P<int>(ctx->vals1) : P<int>(ctx->vals0);
     launch_gather_sorted(ctx->perm, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
@@ -302,8 +302,7 @@ void load_quant_device(asg_ctx* ctx, const int* d_cell, const uint16_t* d_off, c
     launch_unpack_quant(d_cell, d_off, d_v, np, grid, left, cell_size, P<float4>(ctx->pos_in),
                         P<float4>(ctx->vel_in), P<int>(ctx->igrp_in), P<float>(ctx->rk_in),
                         ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0),
-                  P<int>(ctx->vals0), ctx->s);
+    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0), ctx->s);
     build_index(ctx);
 }
 
@@ -442,7 +441,6 @@ int asg_create(asg_ctx** out, int device)
         const int v = std::atoi(e);
         if (v >= 1 && v <= LEAF_MAX) ctx->leaf = v;
     }
-    if (const char* e = std::getenv("ASG_DEPOSIT_ORDER")) ctx->dep_order_on = std::strcmp(e, "tile") != 0;
     if (const char* e = std::getenv("ASG_KNN_WARPS")) {  // tuning knob: 2 or 4 warps per block
         const int v = std::atoi(e);
         if (v == 2 || v == 4) ctx->knn_warps = v;
@@ -474,11 +472,11 @@ void asg_destroy(asg_ctx* ctx)
     Buf* bufs[] = {&ctx->aos, &ctx->pos_in, &ctx->vel_in, &ctx->igrp_in, &ctx->rk_in,
                    &ctx->keys0, &ctx->keys1, &ctx->vals0, &ctx->vals1, &ctx->sort_tmp,
                    &ctx->pos, &ctx->vel, &ctx->igrp, &ctx->rk, &ctx->t33, &ctx->idx33,
-                   &ctx->boxes, &ctx->dacc, &ctx->dexp, &ctx->blist, &ctx->dep_order, &ctx->uf,
+                   &ctx->boxes, &ctx->dacc, &ctx->dexp, &ctx->blist, &ctx->uf,
                    &ctx->minin, &ctx->mark,
                    &ctx->scan_tmp, &ctx->lab_cnt, &ctx->lab_scan, &ctx->halos, &ctx->hcount,
                    &ctx->hmass, &ctx->totals, &ctx->lohi, &ctx->dep_rec, &ctx->dep_pcount,
-                   &ctx->dep_tiles, &ctx->dep_counter, &ctx->dep_pairs, &ctx->dep_sort,
+                   &ctx->dep_tiles, &ctx->dep_items, &ctx->dep_counter, &ctx->dep_pairs, &ctx->dep_sort,
                    &ctx->dep_partial, &ctx->cat, &ctx->cat_out, &ctx->sh_in, &ctx->sh_all,
                    &ctx->dec_raw, &ctx->dec_scan};
     for (Buf* b : bufs)
@@ -554,11 +552,13 @@ static int load_shell(asg_ctx* ctx, int np, float boxsize, float bf, int* np_wit
     const uint32_t* keys = nullptr;
     const int* order = nullptr;
     launch_shell_bins(F4(L.pos), np, lt, rt, U(L.k0), I(L.v0), U(L.k1), I(L.v1), b + L.tmp,
-                      U(L.start), U(L.end), &keys, &order, ctx->s);
+                      U(L.start), U(L.end), &keys, &order, ctx->d_err, ctx->s);
     uint32_t se[54];
     CK(cudaMemcpyAsync(se, b + L.start, 27 * 4, cudaMemcpyDeviceToHost, ctx->s));
     CK(cudaMemcpyAsync(se + 27, b + L.end, 27 * 4, cudaMemcpyDeviceToHost, ctx->s));
+    CK(cudaMemcpyAsync(ctx->h_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->s));
     CK(cudaStreamSynchronize(ctx->s));
+    if (*ctx->h_err & ERR_SORT) return finish(ctx, "shell sort");
     // the reference's send loop order (exchange_buffer.cpp:120-150): source bin, then direction
     ShellPlan plan;
     size_t off = (size_t)np;
@@ -601,7 +601,7 @@ static int load_shell(asg_ctx* ctx, int np, float boxsize, float bf, int* np_wit
     ctx->right = boxsize + dx;
     phase_begin(ctx, ASG_PH_INDEX);
     launch_space_keys(P<float4>(ctx->pos_in), n, ctx->left, ctx->right, nullptr, 0,
-                  P<uint64_t>(ctx->keys0), P<int>(ctx->vals0), ctx->s);
+                  P<uint64_t>(ctx->keys0), ctx->s);
     build_index(ctx);
     int r = finish(ctx, "load_periodic_cube");
     if (r) ctx->loaded = false;
@@ -627,8 +627,7 @@ int asg_load_particles(asg_ctx* ctx, const asg_particle* p, int np, float left, 
     phase_begin(ctx, ASG_PH_INDEX);
     launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
                       P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0),
-                  P<int>(ctx->vals0), ctx->s);
+    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0), ctx->s);
     build_index(ctx);
     int r = finish(ctx, "load");
     if (r) ctx->loaded = false;
@@ -649,8 +648,7 @@ int asg_load_particles_device(asg_ctx* ctx, const float* d_x, const float* d_v,
     phase_begin(ctx, ASG_PH_INDEX);
     launch_unpack_soa(d_x, d_v, d_dens, d_igrp, np, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
                       P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0),
-                  P<int>(ctx->vals0), ctx->s);
+    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0), ctx->s);
     build_index(ctx);
     int r = finish(ctx, "load_device");
     if (r) ctx->loaded = false;
@@ -1030,10 +1028,16 @@ int asg_run_remove_small_groups(asg_ctx* ctx, int ngrp, int* nhalo)
     return 0;
 }
 
-// cap == 0: size the pair arrays from the pair count (one host synchronisation);
-// cap > 0: pair arrays of that capacity, no synchronisation (stream capture)
+// entries and pairs that a deposit's arrays hold
+struct DepositCap {
+    uint32_t entries = 0, pairs = 0;
+};
+
+// no cap: the arrays are sized from the counts (one host synchronisation); with a
+// cap: arrays of that capacity, no synchronisation (stream capture)
 static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, int sign,
-                         int periodic, const int* coords, int density_only, uint32_t cap = 0)
+                         int periodic, const int* coords, int density_only,
+                         const DepositCap* cap = nullptr, bool large_tiles = false)
 {
     if (!ncs || n_nc <= 0 || n_nc > MAX_MESHES) return fail(ctx, ASG_ERR_ARG, "1..8 meshes");
     if (!(boxsize > 0.0f) || !std::isfinite(boxsize)) return fail(ctx, ASG_ERR_ARG, "boxsize");
@@ -1050,90 +1054,98 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     p.sign = sign;
     p.periodic = periodic ? 1 : 0;
     p.density_only = density_only ? 1 : 0;
-    p.seg = ctx->dep_seg;
-    p.mma = ctx->dep_mma;
+    p.seg = deposit_seg(ctx->n, n_nc, ctx->dep_seg);
+    p.mma = large_tiles ? 0 : ctx->dep_mma;
     for (int d = 0; d < 3; ++d) p.offset[d] = periodic && coords ? boxsize * (float)coords[d] : 0.0f;
+    // the pair keys hold tile << 5 | image in 32 bits: meshes of more tiles than
+    // that allows take the engine with the larger tiles
+    auto count_tiles = [&]() {
+        deposit_tile_shape(p);
+        long long t = 0;
+        for (int k = 0; k < n_nc; ++k) {
+            long long m = 1;
+            for (int a = 0; a < 3; ++a) m *= (ncs[k] + (1 << p.shift[a]) - 1) >> p.shift[a];
+            t += m;
+        }
+        return t;
+    };
+    if (p.mma && count_tiles() >= (1LL << (periodic ? 27 : 31)) - 1) p.mma = 0;
+    count_tiles();
     int tiles = 0;
     for (int k = 0; k < n_nc; ++k) {
         MeshBuf& mb = ctx->meshes[(size_t)k];
         const int nc = ncs[k];
         const size_t nm = (size_t)nc * nc * nc * (density_only ? 1 : 6);
-        const int tpd = (nc + 7) / 8;
+        MeshJob& j = p.job[k];
+        int nt = 1;
+        for (int a = 0; a < 3; ++a) nt *= j.tiles[a] = (nc + (1 << p.shift[a]) - 1) >> p.shift[a];
         if (int r = grow(ctx, mb.mesh, 4 * nm)) return r;
-        if (int r = grow(ctx, mb.partial, 16 * (size_t)tpd * tpd * tpd)) return r;
+        if (int r = grow(ctx, mb.partial, 16 * (size_t)nt)) return r;
         mb.nc = nc;
         mb.words = nm;
-        MeshJob& j = p.job[k];
         j.nc = nc;
         j.dx = boxsize / nc;  // float / int, as coarse_mesh.cpp:58
         j.ncf = (float)nc;
-        j.tiles[0] = j.tiles[1] = j.tiles[2] = tpd;
         j.tile_begin = tiles;
         j.mesh = P<float>(mb.mesh);
         j.partial = P<double>(mb.partial);
-        tiles += tpd * tpd * tpd;
+        tiles += nt;
     }
-    if (int r = grow(ctx, ctx->totals, 16 * (size_t)n_nc)) return r;
-    // the tiles' processing order, cached while the meshes stay the same (a
-    // captured call without it takes the tiles in tile order: the same sums)
-    const std::vector<int> okey(ncs, ncs + n_nc);
-    if (ctx->dep_order_on && okey != ctx->dep_order_key && !cap) {
-        if (int r = grow(ctx, ctx->dep_order, 8 * (size_t)tiles)) return r;
-        std::vector<uint32_t> h(2 * (size_t)tiles);
-        deposit_tile_order(p, tiles, h.data());
-        CK(cudaMemcpyAsync(ctx->dep_order.p, h.data(), 8 * (size_t)tiles, cudaMemcpyHostToDevice,
-                           ctx->s));
-        CK(cudaStreamSynchronize(ctx->s));
-        ctx->dep_order_key = okey;
-    }
-    if (ctx->dep_order_on && okey == ctx->dep_order_key) {
-        p.order = P<uint32_t>(ctx->dep_order);
-        p.pos = p.order + tiles;
-    }
-    // particle records and pair counts, then size the pair arrays
+    if (int r = grow(ctx, ctx->totals, deposit_totals_bytes(n_nc))) return r;
+    // particle records and entry counts, then size the entry arrays
     const int n = ctx->n;
     const size_t T1 = (size_t)tiles + 1;
     if (int r = grow(ctx, ctx->dep_rec, deposit_prep_bytes(n))) return r;
-    if (int r = grow(ctx, ctx->dep_pcount, 4 * ((size_t)n + 1) + scan_temp_bytes((size_t)n + 1)))
-        return r;
+    const size_t B1 = ((size_t)n + 31) / 32 + 1;
+    if (int r = grow(ctx, ctx->dep_pcount, 4 * B1 + scan_temp_bytes(B1))) return r;
     if (int r = grow(ctx, ctx->dep_tiles, deposit_tile_bytes(tiles))) return r;
     if (int r = grow(ctx, ctx->dep_counter, 16)) return r;
     DepositScratch w;
     w.rec = P<float4>(ctx->dep_rec);
-    w.pcount = P<uint32_t>(ctx->dep_pcount);
-    w.scan_tmp_n = (void*)(w.pcount + n + 1);
-    w.tstart = P<uint32_t>(ctx->dep_tiles);
-    w.tcount = w.tstart + T1;
-    w.item_off = w.tcount + T1;
-    w.scan_tmp_t = (void*)(w.item_off + T1);
-    w.next_item = P<int>(ctx->dep_counter);
+    w.count = P<uint32_t>(ctx->dep_pcount);
+    w.scan_tmp_n = (void*)(w.count + B1);
+    w.tentry = P<uint32_t>(ctx->dep_tiles);
+    w.item_off = w.tentry + T1;
+    w.merge = w.item_off + T1;
+    w.scan_tmp_t = (void*)(w.merge + T1);
+    w.counters = P<int>(ctx->dep_counter);
     phase_begin(ctx, ASG_PH_DEPOSIT);
     launch_deposit_prep(P<float4>(ctx->pos), P<float4>(ctx->vel), P<int>(ctx->igrp),
                         P<float>(ctx->rk), n, p, w, ctx->d_err, ctx->s);
-    uint32_t npairs = cap;
-    if (!cap) {
-        if (int r = read_words(ctx, w.pcount + n)) return r;
-        npairs = ctx->h_u32[0];
+    DepositCap have;
+    if (cap) {
+        have = *cap;
+    } else {
+        const uint32_t* pairs = reinterpret_cast<uint32_t*>(w.counters + 2);
+        if (int r = read_words(ctx, w.count + (B1 - 1), pairs, pairs + 1)) return r;
+        have.entries = ctx->h_u32[0];
+        have.pairs = ctx->h_u32[1];
+        if (ctx->h_u32[2] || have.pairs > (uint32_t)INT_MAX) {  // past the 32-bit pair numbers
+            phase_end(ctx);
+            if (!p.mma) return fail(ctx, ASG_ERR_ARG, "more than 2^31 - 1 (particle, tile) pairs");
+            return queue_deposit(ctx, boxsize, ncs, n_nc, sign, periodic, coords, density_only, cap,
+                                 true);  // larger tiles, fewer pairs
+        }
     }
-    const size_t NP = (size_t)npairs + 1;
-    if (int r = grow(ctx, ctx->dep_pairs, 16 * NP)) return r;
-    if (int r = grow(ctx, ctx->dep_sort, radix_sort_temp_bytes((int)NP))) return r;
-    const uint32_t max_items = deposit_max_items(tiles, npairs, p.seg);
-    if (int r = grow(ctx, ctx->dep_partial, deposit_partial_bytes(max_items) + 16)) return r;
-    w.keys0 = P<uint32_t>(ctx->dep_pairs);
-    w.keys1 = w.keys0 + NP;
-    w.vals0 = reinterpret_cast<int*>(w.keys1 + NP);
-    w.vals1 = w.vals0 + NP;
+    if (int r = grow(ctx, ctx->dep_pairs, deposit_entry_bytes(have.entries))) return r;
+    if (int r = grow(ctx, ctx->dep_sort, radix_sort_temp_bytes((int)have.entries))) return r;
+    const uint32_t max_items = deposit_max_items(tiles, have.pairs, p.seg);
+    if (int r = grow(ctx, ctx->dep_partial,
+                     deposit_partial_bytes(max_items, 1 << (p.shift[0] + p.shift[1] + p.shift[2])) + 16))
+        return r;
+    if (int r = grow(ctx, ctx->dep_items, 4 * (size_t)max_items)) return r;
+    deposit_entry_layout(ctx->dep_pairs.p, have.entries, w);
+    w.item_tile = P<uint32_t>(ctx->dep_items);
     w.sort_tmp = ctx->dep_sort.p;
     w.partial = P<float>(ctx->dep_partial);
-    if (!cap) ctx->dep_npairs = npairs;
-    ctx->dep_tiles_n = tiles;
-    launch_deposit_run(n, p, tiles, npairs, cap != 0, w, ctx->d_err, ctx->s);
-    for (int k = 0; k < n_nc; ++k) {
-        const int tpd = (ncs[k] + 7) / 8;
-        launch_reduce_partials(P<double>(ctx->meshes[(size_t)k].partial), tpd * tpd * tpd,
-                               P<double>(ctx->totals) + 2 * k, ctx->s);
+    if (!cap) {
+        ctx->dep_npairs = have.pairs;
+        ctx->dep_nentries = have.entries;
     }
+    ctx->dep_tiles_n = tiles;
+    ctx->dep_cells = 1 << (p.shift[0] + p.shift[1] + p.shift[2]);
+    launch_deposit_run(n, p, tiles, have.entries, max_items, cap != nullptr, w, ctx->d_err, ctx->s);
+    launch_deposit_totals(p, tiles, P<double>(ctx->totals), ctx->s);
     phase_end(ctx);
     return 0;
 }
@@ -1290,7 +1302,7 @@ static int load_for_deposit(asg_ctx* ctx, const asg_particle* p, int np)
     launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
                       P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
     launch_space_keys(P<float4>(ctx->pos_in), np, 0.0f, 0.0f, P<int>(ctx->lohi), 0,
-                  P<uint64_t>(ctx->keys0), P<int>(ctx->vals0), ctx->s);
+                  P<uint64_t>(ctx->keys0), ctx->s);
     build_index(ctx);
     int r = finish(ctx, "load");
     if (r) ctx->loaded = false;
@@ -1376,7 +1388,8 @@ static int run_catalogue(asg_ctx* ctx, const float4* pos, const float4* vel, con
     unsigned char* ob = P<unsigned char>(ctx->cat_out);
     CK(cudaMemsetAsync(ob, 0, o_cnt + 16, ctx->s));
     launch_fof_catalogue(pos, vel, igrp, n, w_index, nhalo, boxsize, ctx->cat.p,
-                         reinterpret_cast<float*>(ob), reinterpret_cast<uint32_t*>(ob + o_cnt), ctx->s);
+                         reinterpret_cast<float*>(ob), reinterpret_cast<uint32_t*>(ob + o_cnt), ctx->d_err,
+                         ctx->s);
     if (nhalo > 0) CK(cudaMemcpyAsync(out, ob, sizeof(asg_fof_halo) * (size_t)nhalo,
                                       cudaMemcpyDeviceToHost, ctx->s));
     CK(cudaMemcpyAsync(ctx->h_u32, ob + o_cnt, 4, cudaMemcpyDeviceToHost, ctx->s));
@@ -1496,7 +1509,7 @@ int asg_deposit_stats(asg_ctx* ctx, long long* pairs, long long* tiles, long lon
     if (!ctx->dep_counter.p) return fail(ctx, ASG_ERR_STATE, "no deposit run yet");
     CK(cudaSetDevice(ctx->device));
     uint32_t it = 0;
-    const uint32_t* item_off = P<uint32_t>(ctx->dep_tiles) + 2 * ((size_t)ctx->dep_tiles_n + 1);
+    const uint32_t* item_off = P<uint32_t>(ctx->dep_tiles) + (size_t)ctx->dep_tiles_n + 1;
     CK(cudaMemcpy(&it, item_off + ctx->dep_tiles_n, 4, cudaMemcpyDeviceToHost));
     if (pairs) *pairs = ctx->dep_npairs;
     if (tiles) *tiles = ctx->dep_tiles_n;
@@ -1547,8 +1560,7 @@ int asg_smooth(asg_ctx* ctx, asg_particle* p, int np, float left, float right, f
     phase_begin(ctx, ASG_PH_INDEX);
     launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
                       P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0),
-                  P<int>(ctx->vals0), ctx->s);
+    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0), ctx->s);
     build_index(ctx);
     run_knn(ctx);
     if (int r = queue_mark(ctx, halos, nh)) return r;
@@ -1631,7 +1643,7 @@ struct asg_batch {
     Buf in_cell, in_off;
     std::vector<int> quant;
     std::vector<float> cell_size;
-    std::vector<uint32_t> cap;     // pair capacity per item (from the planning pass)
+    std::vector<DepositCap> cap;   // deposit capacity per item (from the planning pass)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     long long launches = 0;        // kernels per graph launch
@@ -1654,9 +1666,9 @@ void batch_drop_graph(asg_batch* b)
 }
 
 // one item's whole path on the stream of ctx (the batch's context or one of its
-// sub-contexts); cap = 0 sizes the deposit from its pair count (one
-// synchronisation), cap > 0 synchronises nowhere
-int batch_queue_item(asg_batch* b, asg_ctx* ctx, int i, uint32_t cap)
+// sub-contexts); without a cap the deposit is sized from its counts (one
+// synchronisation), with one nothing synchronises
+int batch_queue_item(asg_batch* b, asg_ctx* ctx, int i, const DepositCap* cap)
 {
     const int n = b->np[(size_t)i];
     const size_t o = b->off[(size_t)i];
@@ -1673,7 +1685,7 @@ int batch_queue_item(asg_batch* b, asg_ctx* ctx, int i, uint32_t cap)
                           n, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in), P<int>(ctx->igrp_in),
                           P<float>(ctx->rk_in), ctx->d_err, ctx->s);
     launch_space_keys(P<float4>(ctx->pos_in), n, ctx->left, ctx->right, nullptr, 0,
-                  P<uint64_t>(ctx->keys0), P<int>(ctx->vals0), ctx->s);
+                  P<uint64_t>(ctx->keys0), ctx->s);
     build_index(ctx);
     run_knn(ctx);
     if (int r = queue_deposit(ctx, b->box[(size_t)i], b->ncs.data(), b->n_nc, b->sign, 0, nullptr, 0,
@@ -1706,24 +1718,26 @@ int batch_plan(asg_batch* b)
         if (int r = alloc_set(c, b->max_n)) return fail(ctx, r, "batch: stream scratch");
         if (int r = grow(c, c->lab_scan, 4 * (size_t)b->max_n)) return fail(ctx, r, "batch: stream scratch");
     }
-    b->cap.assign((size_t)b->n_items, 0u);
-    uint32_t max_cap = 0;
+    b->cap.assign((size_t)b->n_items, DepositCap{});
+    uint32_t max_entries = 0, max_items = 0;
     for (int i = 0; i < b->n_items; ++i) {
         asg_ctx* c = b->sub[(size_t)i % S];
-        if (int r = batch_queue_item(b, c, i, 0)) return fail(ctx, r, c->last);
-        const uint32_t np = c->dep_npairs;
-        b->cap[(size_t)i] = np + np / 16 + 4096;  // headroom for inputs that change between runs
-        max_cap = std::max(max_cap, b->cap[(size_t)i]);
+        if (int r = batch_queue_item(b, c, i, nullptr)) return fail(ctx, r, c->last);
+        DepositCap& cap = b->cap[(size_t)i];  // headroom for inputs that change between runs
+        cap.entries = c->dep_nentries + c->dep_nentries / 16 + 4096;
+        cap.pairs = c->dep_npairs + c->dep_npairs / 16 + 4096;
+        max_entries = std::max(max_entries, cap.entries);
+        max_items = std::max(max_items, deposit_max_items(c->dep_tiles_n, cap.pairs,
+                                                          deposit_seg(c->n, b->n_nc, c->dep_seg)));
     }
     for (asg_ctx* c : b->sub)
         if (int r = finish(c, "batch plan")) return fail(ctx, r, c->last);
     // reserve the deposit arrays for the largest capacity, so that the capture allocates nothing
-    const size_t NP = (size_t)max_cap + 1;
     for (asg_ctx* c : b->sub) {
-        int r = grow(c, c->dep_pairs, 16 * NP);
-        if (!r) r = grow(c, c->dep_sort, radix_sort_temp_bytes((int)NP));
-        const uint32_t items = deposit_max_items(c->dep_tiles_n, max_cap, c->dep_seg);
-        if (!r) r = grow(c, c->dep_partial, deposit_partial_bytes(items) + 16);
+        int r = grow(c, c->dep_pairs, deposit_entry_bytes(max_entries));
+        if (!r) r = grow(c, c->dep_sort, radix_sort_temp_bytes((int)max_entries));
+        if (!r) r = grow(c, c->dep_partial, deposit_partial_bytes(max_items, c->dep_cells) + 16);
+        if (!r) r = grow(c, c->dep_items, 4 * (size_t)max_items);
         if (r) return fail(ctx, r, "batch: deposit reserve");
     }
     return 0;
@@ -1749,7 +1763,7 @@ int batch_capture(asg_batch* b)
                 r = fail(ctx, ASG_ERR_CUDA, "fork");
     }
     for (int i = 0; !r && i < b->n_items; ++i)
-        r = batch_queue_item(b, b->sub[(size_t)i % S], i, b->cap[(size_t)i]);
+        r = batch_queue_item(b, b->sub[(size_t)i % S], i, &b->cap[(size_t)i]);
     for (size_t s = 1; !r && s < S; ++s)  // join: the origin stream waits for every stream
         if (cudaEventRecord(b->join[s], b->sub[s]->s) != cudaSuccess ||
             cudaStreamWaitEvent(ctx->s, b->join[s], 0) != cudaSuccess)
@@ -1936,7 +1950,7 @@ int asg_batch_tune(asg_batch* b, int* leaf, int* seg)
         if (b->np[(size_t)i] > b->np[(size_t)item]) item = i;
     // tree bucket size x deposit work-item length x neighbour-search warps per
     // block x deposit engine (tensor cores or CUDA cores)
-    const int leaves[] = {16, 24, 32}, segs[] = {2048, 4096, 8192}, warps[] = {2, 4}, mmas[] = {1, 2, 0};
+    const int leaves[] = {16, 24, 32}, segs[] = {2048, 4096, 8192}, warps[] = {2, 4}, mmas[] = {1, 0};
     float best = INFINITY;
     int bl = ctx->leaf, bs = ctx->dep_seg, bw = ctx->knn_warps, bm = ctx->dep_mma;
     for (int l : leaves)
@@ -1950,7 +1964,7 @@ int asg_batch_tune(asg_batch* b, int* leaf, int* seg)
                     float ms = 0.0f;
                     for (int rep = 0; rep < 2; ++rep) {  // the first repetition warms up
                         CK(cudaEventRecord(b->e0, ctx->s));
-                        if (int r = batch_queue_item(b, ctx, item, 0)) return r;
+                        if (int r = batch_queue_item(b, ctx, item, nullptr)) return r;
                         CK(cudaEventRecord(b->e1, ctx->s));
                         CK(cudaEventSynchronize(b->e1));
                         CK(cudaEventElapsedTime(&ms, b->e0, b->e1));

@@ -26,6 +26,7 @@ constexpr int ERR_NONFINITE = 16;  // NaN / inf position
 constexpr int ERR_UF = 32;         // union-find retry limit hit
 constexpr int ERR_RANGE = 64;      // periodic deposit range wider than the mesh
 constexpr int ERR_BADCELL = 128;   // mixed-precision cell index outside the grid
+constexpr int ERR_SORT = 512;      // a radix sort's look-back gave up
 constexpr int ERR_CAP = 256;       // more deposit pairs than a pre-sized pair array holds
 
 // ---- exact float helpers (reference expression order) ----------------------

@@ -15,38 +15,49 @@
 // (a halo particle's sliver weight in a thin cell); these stay near 1e-6.
 //
 // Sort by target tile, then gather; deterministic, no atomics on the mesh.
-//  (1) k_dep_prep: one record per particle with x, hinv and the normalised
-//      edges (x -+ h)/boxsize, which do not depend on nc.
-//  (2) k_pair_count / k_pair_emit: every particle emits one (tile, image)
-//      pair per 8^3-cell tile its exact cell range touches, at an offset from
-//      an exclusive scan (so the emit order is the particle order).
-//  (3) a stable radix sort of the pairs by key = tile << 5 | image groups each
-//      tile's particles in particle order.
-//  (4) k_deposit_items: a persistent kernel whose warps take (tile, segment
-//      of seg pairs) work items; a warp accumulates its item in a private
-//      shared-memory tile and adds one pair after another, its lanes over the
-//      pair's 3-D cell box, so every cell sums its contributions in list
-//      order.  k_merge_tiles adds the partial tiles of multi-segment tiles in
-//      segment order.
-// n, c and halo are double-float (two-sum) sums, so the per-tile FP64 totals
-// reproduce the FP64 sum of the float weights.
+//  (1) k_dep_prep: one 32-byte record per particle (position, h, dens, v).  A
+//      particle makes one (tile, image) pair per tile its exact cell range
+//      touches; a bundle of 32 consecutive particles makes one entry (tile,
+//      image, lane mask) per tile that any of them touches, counted here.
+//  (2) k_entries: the entries, at offsets from an exclusive scan (so the emit
+//      order is the particle order).
+//  (3) a stable radix sort of the entries by key = tile << 5 | image (the tile
+//      alone without periodic images) groups each tile's particles in particle
+//      order; k_tile_items finds each tile's pairs and cuts them into work items.
+//  (4) k_deposit_mma: a persistent kernel whose warps take work items and sum
+//      the outer products of each item's pairs on the tensor cores
+//      (k_deposit_items on the CUDA cores with ASG_DEPOSIT=simt);
+//      k_merge_tiles adds the partial tiles of tiles with several items in item
+//      order.
+// n, c and halo are double-float (two-sum) sums; the FP64 totals are summed per
+// pair.
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
-#include <utility>
-#include <vector>
 
 #include "asg_common.cuh"
 #include "asg_internal.h"
 
 namespace asg {
 
-constexpr int TS = 8;             // tile edge in cells
-constexpr int TC = TS * TS * TS;   // cells per tile
-constexpr int DEP_THREADS = 256;   // threads of the tile-merge CTA
-constexpr int SEG_DEFAULT = 4096;  // pairs per work item unless DepositParams::seg says otherwise
+constexpr int TS = 8;             // tile edge in cells of the CUDA-core engine
+constexpr int TC = TS * TS * TS;   // cells of such a tile
+// Tiles of the tensor-core engine, cells in x, y, z.  A pair costs the dense tile
+// whatever it touches, so small tiles waste less on the narrow supports of halo
+// particles and of coarse meshes, and their sums fit a warp; wide supports then
+// reach more tiles.  All six channels: 8 x 4 x 4 (6.6 pairs per particle on the
+// 256^3 step's three meshes; 4.5 with 8 x 8 x 8, 8.2 with 4 x 4 x 4).  n alone: 8
+// x 8 x 8, whose one channel takes no more registers and whose meshes are the
+// finest (on 160^3 cells for 512 k particles 13 pairs per particle, 33 with 8 x 4 x 4).
+template <int NCH>
+struct TileShape {
+    static constexpr int X = 8, Y = NCH == 1 ? 8 : 4, Z = NCH == 1 ? 8 : 4;
+    static constexpr int CELLS = X * Y * Z;
+};
+constexpr int DEP_THREADS = 128;   // threads of the tile-merge CTA
 constexpr int PW = 9;              // partial words per cell
 constexpr int IMG_BITS = 5;        // periodic images per pair: up to 3 x 3 x 3
 // key bits of the image index: none without periodic images (every pair is
@@ -74,8 +85,8 @@ __device__ __forceinline__ TileGeo tile_geo(const DepositParams& P, int tile)
     const int tx = g.local % J.tiles[0];
     const int ty = (g.local / J.tiles[0]) % J.tiles[1];
     const int tz = g.local / (J.tiles[0] * J.tiles[1]);
-    g.O[0] = tx * TS; g.O[1] = ty * TS; g.O[2] = tz * TS;
-    for (int a = 0; a < 3; ++a) g.E[a] = min(TS, g.nc - g.O[a]);
+    g.O[0] = tx << P.shift[0]; g.O[1] = ty << P.shift[1]; g.O[2] = tz << P.shift[2];
+    for (int a = 0; a < 3; ++a) g.E[a] = min(1 << P.shift[a], g.nc - g.O[a]);
     return g;
 }
 
@@ -113,36 +124,6 @@ __device__ __forceinline__ AxisRange axis_range(float exlo, float exhi, const Me
 constexpr int FLAG_HALO = 1;  // sign*igrp > 0: deposit into the halo channel
 constexpr int FLAG_SKIP = 2;  // periodic particle outside [0, L) or a halo in an n-only mesh
 
-// One 32-byte record per particle: (x', y', z', h') and (dens, vx, vy, vz),
-// with x' the deposit position (plus the rank offset when periodic) and h' = h,
-// -h when the particle deposits into the halo channel, 0 when it deposits
-// nothing.  The cell-range edges (x' -+ h)/L and 1/h are recomputed from it
-// where they are needed (load_dep_rec), with the same rounded operations.
-__global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restrict__ vel,
-                           const int* __restrict__ igrp, const float* __restrict__ rk, int n,
-                           DepositParams P, float4* __restrict__ rec, int* err)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 p = pos[i];
-    const float4 v = vel[i];
-    const float h = rk[i];
-    if (!(h > 0.0f && h < INFINITY)) atomicOr(err, ERR_ZERO_RK);
-    const float L = P.boxsize;
-    const bool halo = (P.sign * igrp[i]) > 0;
-    bool skip = P.density_only && halo;
-    float x = p.x, y = p.y, z = p.z;
-    if (P.periodic) {  // global_mesh.cpp:52-61: skip outside the cube, then add the offset
-        if (x < 0.0f || x >= L || y < 0.0f || y >= L || z < 0.0f || z >= L) skip = true;
-        x = __fadd_rn(x, P.offset[0]);
-        y = __fadd_rn(y, P.offset[1]);
-        z = __fadd_rn(z, P.offset[2]);
-    }
-    if (!(h > 0.0f && h < INFINITY)) skip = true;
-    rec[2 * (size_t)i] = make_float4(x, y, z, skip ? 0.0f : (halo ? -h : h));
-    rec[2 * (size_t)i + 1] = make_float4(v.w, v.x, v.y, v.z);
-}
-
 // particle i's record as the deposit kernels use it: A = (x', 1/h), B = ((x'-h)/L,
 // dens), Cc = ((x'+h)/L, vx), D = (vy, vz, flags)
 __device__ __forceinline__ void load_dep_rec(const float4* __restrict__ rec, int i, float L,
@@ -159,117 +140,329 @@ __device__ __forceinline__ void load_dep_rec(const float4* __restrict__ rec, int
     D = make_float4(b.z, b.w, __int_as_float(flags), 0.0f);
 }
 
-// ---------------------------------------------------------------------------
-// (2) (tile, image) pairs
-// ---------------------------------------------------------------------------
 // tiles of one axis touched by image k: [t0, t1] (empty when t0 > t1)
-__device__ __forceinline__ void image_tiles(const AxisRange& r, int k, int nc, int& t0, int& t1)
+__device__ __forceinline__ void image_tiles(const AxisRange& r, int k, int nc, int shift, int& t0,
+                                            int& t1)
 {
     const int c0 = max(r.left - k * nc, 0), c1 = min(r.right - k * nc, nc);
-    t0 = c0 / TS;
-    t1 = c1 > c0 ? (c1 - 1) / TS : t0 - 1;
+    t0 = c0 >> shift;
+    t1 = c1 > c0 ? (c1 - 1) >> shift : t0 - 1;
 }
 
-// EMIT writes pair o only when o < cap (the pair arrays' capacity); a pair
-// beyond it sets ERR_CAP instead
-template <bool EMIT>
-__global__ void k_pairs(const float4* __restrict__ rec, int n, DepositParams P,
-                        uint32_t* __restrict__ counts, const uint32_t* __restrict__ offs,
-                        uint32_t* __restrict__ keys, int* __restrict__ vals, uint32_t cap, int* err)
+// Every entry (tile, image, mask) of the warp's 32 particles with cell-range edges
+// lo and hi (per axis, / boxsize; live: the lane deposits): f(tile, image, mask),
+// called by the whole warp, an entry's mask the lanes that touch the tile.  Per
+// mesh and image the warp goes through the tiles of the union of its lanes' tile
+// boxes; where that holds many more tiles than the lanes touch (particles far
+// apart), through each lane's own tiles, one lane after another.  Either way the
+// particles of a tile come in lane order.
+template <class F>
+__device__ __forceinline__ void for_entries(const DepositParams& P, const float (&lo)[3],
+                                            const float (&hi)[3], bool live, int* err, F f)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 a, b, c, d;
-    load_dep_rec(rec, i, P.boxsize, P.rbox, a, b, c, d);
-    const int flags = __float_as_int(d.z);
-    uint32_t cnt = 0;
-    uint32_t o = EMIT ? offs[i] : 0u;
     const bool periodic = P.periodic != 0;
-    if (!(flags & FLAG_SKIP)) {
-        for (int jb = 0; jb < P.n_jobs; ++jb) {
-            const MeshJob& J = P.job[jb];
-            const int nc = J.nc;
-            const AxisRange ax = axis_range(b.x, c.x, J, nc, periodic);
-            const AxisRange ay = axis_range(b.y, c.y, J, nc, periodic);
-            const AxisRange az = axis_range(b.z, c.z, J, nc, periodic);
-            if (ax.nk <= 0 || ay.nk <= 0 || az.nk <= 0) continue;
-            if (ax.nk > 3 || ay.nk > 3 || az.nk > 3) {  // support wider than two mesh periods
-                atomicOr(err, ERR_RANGE);
-                continue;
+    for (int jb = 0; jb < P.n_jobs; ++jb) {
+        const MeshJob& J = P.job[jb];
+        const int nc = J.nc;
+        AxisRange r[3];
+        bool on = live;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            r[a] = axis_range(lo[a], hi[a], J, nc, periodic);
+            on = on && r[a].nk > 0;
+        }
+        if (on && (r[0].nk > 3 || r[1].nk > 3 || r[2].nk > 3)) {  // wider than two mesh periods
+            atomicOr(err, ERR_RANGE);
+            on = false;
+        }
+        if (!__any_sync(FULLM, on)) continue;
+        int most[3] = {1, 1, 1};  // images per axis
+        if (periodic)
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                most[a] = (int)__reduce_max_sync(FULLM, (unsigned)(on ? r[a].nk : 0));
+        for (int image = 0; image < (periodic ? 27 : 1); ++image) {
+            const int dk[3] = {image % 3, (image / 3) % 3, image / 9};
+            if (dk[0] >= most[0] || dk[1] >= most[1] || dk[2] >= most[2]) continue;
+            int t0[3], t1[3];  // the lane's tiles, empty: t0 > t1
+            bool in = on;
+            int own = 1;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                image_tiles(r[a], r[a].k_lo + dk[a], nc, P.shift[a], t0[a], t1[a]);
+                in = in && dk[a] < r[a].nk && t0[a] <= t1[a];
+                own *= t1[a] - t0[a] + 1;
             }
-            for (int dz = 0; dz < az.nk; ++dz) {
-                int z0, z1;
-                image_tiles(az, az.k_lo + dz, nc, z0, z1);
-                for (int dy = 0; dy < ay.nk; ++dy) {
-                    int y0, y1;
-                    image_tiles(ay, ay.k_lo + dy, nc, y0, y1);
-                    for (int dx = 0; dx < ax.nk; ++dx) {
-                        int x0, x1;
-                        image_tiles(ax, ax.k_lo + dx, nc, x0, x1);
-                        if (x0 > x1 || y0 > y1 || z0 > z1) continue;
-                        const uint32_t combo = (uint32_t)(dz * 9 + dy * 3 + dx);
-                        if constexpr (!EMIT) {
-                            cnt += (uint32_t)((x1 - x0 + 1) * (y1 - y0 + 1) * (z1 - z0 + 1));
-                        } else {
-                            for (int tz = z0; tz <= z1; ++tz)
-                                for (int ty = y0; ty <= y1; ++ty)
-                                    for (int tx = x0; tx <= x1; ++tx) {
-                                        const uint32_t tile = (uint32_t)J.tile_begin +
-                                            (uint32_t)((tz * J.tiles[1] + ty) * J.tiles[0] + tx);
-                                        if (o < cap) {
-                                            keys[o] = (tile << img_bits(P)) | combo;
-                                            vals[o] = i;
-                                        } else {
-                                            atomicOr(err, ERR_CAP);
-                                        }
-                                        ++o;
-                                    }
+            unsigned lanes = __ballot_sync(FULLM, in);
+            if (!lanes) continue;
+            int u0[3], u1[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                if (!in) { t0[a] = INT_MAX; t1[a] = -1; }
+                u0[a] = (int)__reduce_min_sync(FULLM, (unsigned)t0[a]);
+                u1[a] = __reduce_max_sync(FULLM, t1[a]);
+            }
+            const long long box = (long long)(u1[0] - u0[0] + 1) * (u1[1] - u0[1] + 1) * (u1[2] - u0[2] + 1);
+            const unsigned touched = __reduce_add_sync(FULLM, in ? (unsigned)min(own, 1 << 24) : 0u);
+            if (box <= 2LL * touched + 64) {
+                for (int tz = u0[2]; tz <= u1[2]; ++tz) {
+                    const bool inz = t0[2] <= tz && tz <= t1[2];
+                    for (int ty = u0[1]; ty <= u1[1]; ++ty) {
+                        const bool iny = inz && t0[1] <= ty && ty <= t1[1];
+                        int tile = J.tile_begin + (tz * J.tiles[1] + ty) * J.tiles[0] + u0[0];
+                        for (int tx = u0[0]; tx <= u1[0]; ++tx, ++tile) {
+                            const unsigned m = __ballot_sync(FULLM, iny && t0[0] <= tx && tx <= t1[0]);
+                            if (m) f(tile, image, m);
                         }
                     }
+                }
+            } else {
+                while (lanes) {
+                    const int l = __ffs(lanes) - 1;
+                    lanes &= lanes - 1;
+                    const int x0 = __shfl_sync(FULLM, t0[0], l), x1 = __shfl_sync(FULLM, t1[0], l);
+                    const int y0 = __shfl_sync(FULLM, t0[1], l), y1 = __shfl_sync(FULLM, t1[1], l);
+                    const int z0 = __shfl_sync(FULLM, t0[2], l), z1 = __shfl_sync(FULLM, t1[2], l);
+                    for (int tz = z0; tz <= z1; ++tz)
+                        for (int ty = y0; ty <= y1; ++ty)
+                            for (int tx = x0; tx <= x1; ++tx)
+                                f(J.tile_begin + (tz * J.tiles[1] + ty) * J.tiles[0] + tx, image, 1u << l);
                 }
             }
         }
     }
-    if (!EMIT) counts[i] = cnt;
 }
 
-// pairs [*npairs, cap) of a pre-sized pair array: key of tile T (past the last
-// real tile), so they sort last and k_tile_bounds skips them
-__global__ void k_pad_pairs(uint32_t* __restrict__ keys, int* __restrict__ vals,
-                            const uint32_t* __restrict__ npairs, uint32_t cap, uint32_t pad_key)
-{
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= cap || j < *npairs) return;
-    keys[j] = pad_key;
-    vals[j] = 0;
-}
-
-// first pair and pair count of every tile (sorted keys; empty tiles stay 0;
-// tiles >= total_tiles are padding)
-__global__ void k_tile_bounds(const uint32_t* __restrict__ keys, int np, int total_tiles, int ib,
-                              uint32_t* __restrict__ tstart, uint32_t* __restrict__ tcount)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= np) return;
-    const uint32_t t = keys[j] >> ib;
-    if (t >= (uint32_t)total_tiles) return;
-    if (j == 0 || (keys[j - 1] >> ib) != t) tstart[t] = (uint32_t)j;
-    if (j == np - 1 || (keys[j + 1] >> ib) != t) tcount[t] = (uint32_t)j + 1;  // end for now
-}
-
-// tcount: end -> count; nitems: seg-pair work items per tile (at least one),
-// stored at the tile's slot of the processing order (DepositParams::pos)
-__global__ void k_tile_items(const uint32_t* __restrict__ tstart, uint32_t* __restrict__ tcount,
-                             int total_tiles, int seg, const uint32_t* __restrict__ pos,
-                             uint32_t* __restrict__ nitems)
+// One 32-byte record per particle: (x', y', z', h') and (dens, vx, vy, vz),
+// with x' the deposit position (plus the rank offset when periodic) and h' = h,
+// -h when the particle deposits into the halo channel, 0 when it deposits
+// nothing.  The cell-range edges (x' -+ h)/L and 1/h are recomputed from it
+// where they are needed (load_dep_rec), with the same rounded operations.
+// counts: the entries of each bundle, counts[bundles] = 0; *pairs += the pairs.
+__global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restrict__ vel,
+                           const int* __restrict__ igrp, const float* __restrict__ rk, int n,
+                           const __grid_constant__ DepositParams P, float4* __restrict__ rec,
+                           uint32_t* __restrict__ counts, unsigned long long* __restrict__ pairs,
+                           int* err)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < total_tiles) {
-        const uint32_t c = tcount[i] ? tcount[i] - tstart[i] : 0u;
-        tcount[i] = c;
-        nitems[pos ? pos[i] : (uint32_t)i] = max(1u, (c + (uint32_t)seg - 1) / (uint32_t)seg);
+    const int bundles = (n + 31) / 32;
+    if (i == 0) counts[bundles] = 0u;
+    if ((i & ~31) >= n) return;
+    bool live = i < n;
+    const int ii = live ? i : n - 1;
+    const float4 p = pos[ii];
+    const float4 v = vel[ii];
+    const float h = rk[ii];
+    const bool good = h > 0.0f && h < INFINITY;
+    if (live && !good) atomicOr(err, ERR_ZERO_RK);
+    const float L = P.boxsize;
+    const bool halo = (P.sign * igrp[ii]) > 0;
+    bool skip = !good || (P.density_only && halo);
+    float x[3] = {p.x, p.y, p.z};
+    if (P.periodic) {  // global_mesh.cpp:52-61: skip outside the cube, then add the offset
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (x[a] < 0.0f || x[a] >= L) skip = true;
+            x[a] = __fadd_rn(x[a], P.offset[a]);
+        }
     }
-    if (i == total_tiles) nitems[i] = 0u;
+    if (live) {
+        rec[2 * (size_t)i] = make_float4(x[0], x[1], x[2], skip ? 0.0f : (halo ? -h : h));
+        rec[2 * (size_t)i + 1] = make_float4(v.w, v.x, v.y, v.z);
+    }
+    live = live && !skip;
+    float lo[3], hi[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {  // as load_dep_rec
+        lo[a] = div_rn_by(__fsub_rn(x[a], h), L, P.rbox);
+        hi[a] = div_rn_by(__fadd_rn(x[a], h), L, P.rbox);
+    }
+    uint32_t cnt = 0, np = 0;
+    for_entries(P, lo, hi, live, err, [&](int, int, unsigned m) {
+        ++cnt;
+        np += (uint32_t)__popc(m);
+    });
+    if ((i & 31) == 0) {
+        counts[i >> 5] = cnt;
+        if (np) atomicAdd(pairs, (unsigned long long)np);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// (2) entries
+// ---------------------------------------------------------------------------
+// Entries instead of pairs: consecutive particles mostly touch the same tiles, so
+// an entry stands for about ten pairs, and what is sorted shrinks by as much: on
+// the 256^3 step pairs, their sort and the tiles' bounds took 4.2 ms, entries with
+// the same 2.0 ms.
+// entry o is written only when o < cap (the entry arrays' capacity); one beyond
+// it sets ERR_CAP instead
+__global__ void k_entries(const float4* __restrict__ rec, int n, const __grid_constant__ DepositParams P,
+                          const uint32_t* __restrict__ offs, uint32_t* __restrict__ keys,
+                          uint2* __restrict__ entry, uint32_t cap, int* err)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((i & ~31) >= n) return;
+    const int lane = threadIdx.x & 31;
+    float4 a, b, c, d;
+    load_dep_rec(rec, min(i, n - 1), P.boxsize, P.rbox, a, b, c, d);
+    const bool live = i < n && !(__float_as_int(d.z) & FLAG_SKIP);
+    const float lo[3] = {b.x, b.y, b.z}, hi[3] = {c.x, c.y, c.z};
+    uint32_t o = offs[i >> 5];  // the next group of up to 32 entries goes here
+    int held = 0;               // entries held by the lanes below it
+    uint32_t key = 0, mask = 0;
+    auto store = [&]() {
+        if (lane < held) {
+            if (o + lane < cap) {
+                keys[o + lane] = key;
+                entry[o + lane] = make_uint2((uint32_t)(i >> 5), mask);
+            } else {
+                atomicOr(err, ERR_CAP);
+            }
+        }
+        o += held;
+        held = 0;
+    };
+    for_entries(P, lo, hi, live, err, [&](int tile, int image, unsigned m) {
+        if (lane == held) {
+            key = ((uint32_t)tile << img_bits(P)) | (uint32_t)image;
+            mask = m;
+        }
+        if (++held == 32) store();
+    });
+    store();
+}
+
+// entries [*count, cap) of a pre-sized array: key of tile T (past the last real
+// tile), so they sort last and belong to no tile
+__global__ void k_pad_entries(uint32_t* __restrict__ keys, uint2* __restrict__ entry,
+                              const uint32_t* __restrict__ count, uint32_t cap, uint32_t pad_key)
+{
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= cap || j < *count) return;
+    keys[j] = pad_key;
+    entry[j] = make_uint2(0u, 0u);
+}
+
+// the entries in key order, and their pair counts (then scanned in place)
+__global__ void k_sorted_entries(const int* __restrict__ order, const uint2* __restrict__ entry,
+                                 uint32_t count, uint2* __restrict__ list, uint32_t* __restrict__ first,
+                                 const int* __restrict__ err)
+{
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j == count) first[j] = 0u;
+    if (j >= count) return;
+    // not in order when the sort gave up: no pairs at all
+    const uint2 e = (*err & ERR_SORT) ? make_uint2(0u, 0u) : entry[order[j]];
+    list[j] = e;
+    first[j] = (uint32_t)__popc(e.y);
+}
+
+// tentry[t]: the first entry of tile t (tentry[T]: past the last real tile), by
+// binary search over the sorted keys, in parallel over the tiles.  nitems:
+// seg-pair work items per tile (at least one), nitems[T] = 0.
+__device__ __forceinline__ uint32_t lower_bound(const uint32_t* __restrict__ keys, uint32_t n,
+                                                uint64_t key)
+{
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (keys[mid] < key) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+__global__ void k_tile_items(const uint32_t* __restrict__ keys, uint32_t count,
+                             const uint32_t* __restrict__ first, int total_tiles, int ib, int seg,
+                             uint32_t* __restrict__ tentry, uint32_t* __restrict__ nitems)
+{
+    __shared__ uint32_t e[257];
+    const int t = blockIdx.x * 256 + threadIdx.x;
+    const uint32_t b = lower_bound(keys, count, (uint64_t)min(t, total_tiles) << ib);
+    e[threadIdx.x] = b;
+    if (threadIdx.x == 255) e[256] = lower_bound(keys, count, (uint64_t)min(t + 1, total_tiles) << ib);
+    __syncthreads();
+    if (t > total_tiles) return;
+    tentry[t] = b;
+    if (t == total_tiles) {
+        nitems[t] = 0u;
+        return;
+    }
+    // e[t + 1] < b only when the keys are not in order (the sort gave up)
+    const uint32_t end = max(e[threadIdx.x + 1], b);
+    const uint32_t c = first[end] - first[b];
+    nitems[t] = max(1u, (c + (uint32_t)seg - 1) / (uint32_t)seg);
+}
+
+// item_tile[i]: the tile of item i; merge: the tiles with several items.  More
+// items than the arrays hold (a captured call whose pairs outgrew its capacity)
+// set ERR_CAP.
+__global__ void k_item_list(const uint32_t* __restrict__ item_off, int total_tiles,
+                            uint32_t max_items, uint32_t* __restrict__ item_tile,
+                            uint32_t* __restrict__ merge, int* __restrict__ counters, int* err)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total_tiles) return;
+    const uint32_t i0 = item_off[t], i1 = item_off[t + 1];
+    if (i1 > max_items) {
+        atomicOr(err, ERR_CAP);
+        return;
+    }
+    for (uint32_t i = i0; i < i1; ++i) item_tile[i] = (uint32_t)t;
+    if (i1 - i0 > 1) merge[atomicAdd(counters + 1, 1)] = (uint32_t)t;
+}
+
+// The pairs of one work item, 32 at a time: lane l of chunk c has pair 32 c + l.
+// A chunk spans at most 32 entries, which the lanes load together.
+struct PairCursor {
+    const uint2* list;
+    const uint32_t* first;
+    uint32_t at, end;  // the entry of the next chunk's first pair, the tile's last + 1
+
+    // particle and entry number of pair j (consecutive over the lanes, from the
+    // chunk's first pair on, all but the first chunk following the one before);
+    // lanes with j >= j1 get -1
+    __device__ __forceinline__ int take(uint32_t j, uint32_t j1, uint32_t& which)
+    {
+        const int lane = threadIdx.x & 31;
+        const uint32_t mine = at + lane;
+        const uint32_t f = mine < end ? first[mine] : 0xffffffffu;
+        const uint2 e = mine < end ? list[mine] : make_uint2(0u, 0u);
+        int l = 0;  // the last of the 32 entries that starts at or before pair j
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+            if (__shfl_sync(FULLM, f, l + s) <= j) l += s;
+        const uint32_t start = __shfl_sync(FULLM, f, l);
+        unsigned m = __shfl_sync(FULLM, e.y, l);
+        const uint32_t w = __shfl_sync(FULLM, e.x, l);
+        which = at + l;
+        // on to the entry of the pair after lane 31's
+        at += __shfl_sync(FULLM, l + (j - start + 1u == (uint32_t)__popc(m) ? 1 : 0), 31);
+        if (j >= j1) return -1;
+        // the (j - start)-th set bit of the mask
+        int k = (int)(j - start), bit = 0;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) {
+            const int c = __popc(m & ((1u << s) - 1u));
+            if (k >= c) {
+                k -= c;
+                m >>= s;
+                bit += s;
+            }
+        }
+        return (int)(w * 32u) + bit;
+    }
+};
+__device__ __forceinline__ PairCursor open_pairs(const uint2* __restrict__ list,
+                                                 const uint32_t* __restrict__ first, uint32_t e0,
+                                                 uint32_t e1, uint32_t j0)
+{
+    uint32_t lo = e0, hi = e1;  // the last entry in [e0, e1) that starts at or before pair j0
+    while (hi - lo > 1) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (first[mid] <= j0) lo = mid; else hi = mid;
+    }
+    return {list, first, lo, e1};
 }
 
 // ---------------------------------------------------------------------------
@@ -337,17 +530,6 @@ __device__ __forceinline__ void add_halo(WarpTile& S, int slot, float w3)
     S.hl[slot] = hl;
 }
 
-__device__ __forceinline__ int upper_index(const uint32_t* __restrict__ a, int n, uint32_t v)
-{
-    // largest i in [0, n) with a[i] <= v (a non-decreasing, a[0] = 0)
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (a[mid] <= v) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
 __device__ __forceinline__ void write_tile(const WarpTile& S, const DepositParams& P, const TileGeo& g,
                                            double& sn, double& sh, int lane)
 {
@@ -401,35 +583,34 @@ __device__ __forceinline__ void block_totals(double sn, double sh, double (*red)
 }
 
 __global__ void __launch_bounds__(32 * DEP_WARPS)
-k_deposit_items(const float4* __restrict__ rec, DepositParams P, int total_tiles,
-                const uint32_t* __restrict__ item_off, const uint32_t* __restrict__ tstart,
-                const uint32_t* __restrict__ tcount, const uint32_t* __restrict__ pkeys,
-                const int* __restrict__ pvals, float* __restrict__ partial,
-                int* __restrict__ next_item)
+k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositParams P,
+                int total_tiles, const uint32_t* __restrict__ item_off,
+                uint32_t max_items, const uint32_t* __restrict__ item_tile,
+                const uint32_t* __restrict__ tentry, const uint32_t* __restrict__ ekeys,
+                const uint2* __restrict__ list, const uint32_t* __restrict__ first,
+                float* __restrict__ partial, int* __restrict__ next_item)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     WarpTile& S = reinterpret_cast<WarpTile*>(smem_raw)[threadIdx.x >> 5];
     const bool periodic = P.periodic != 0;
-    const uint32_t total_items = item_off[total_tiles];
+    const uint32_t total_items = min(item_off[total_tiles], max_items);
 
     for (;;) {
-        int item = 0, tile = -1;
-        if (lane == 0) {
-            item = atomicAdd(next_item, 1);
-            if ((uint32_t)item < total_items) tile = upper_index(item_off, total_tiles + 1, (uint32_t)item);
-        }
+        int item = 0;
+        if (lane == 0) item = atomicAdd(next_item, 1);
         item = __shfl_sync(FULLM, item, 0);
-        const int slot = __shfl_sync(FULLM, tile, 0);  // items are numbered in slot order
         if ((uint32_t)item >= total_items) break;
-        tile = P.order ? (int)P.order[slot] : slot;
+        const int tile = (int)item_tile[item];
         const TileGeo g = tile_geo(P, tile);
         const MeshJob& J = P.job[g.job];
         const int nc = g.nc;
-        const int seg = item - (int)item_off[slot];
-        const int nseg = (int)(item_off[slot + 1] - item_off[slot]);
-        const int j0 = (int)tstart[tile] + seg * P.seg;
-        const int j1 = (int)tstart[tile] + min((int)tcount[tile], (seg + 1) * P.seg);
+        const int seg = item - (int)item_off[tile];
+        const int nseg = (int)(item_off[tile + 1] - item_off[tile]);
+        const uint32_t e0 = tentry[tile], e1 = max(tentry[tile + 1], e0);
+        const uint32_t j0 = first[e0] + (uint32_t)(seg * P.seg);
+        const uint32_t j1 = min(first[e1], j0 + (uint32_t)P.seg);
+        PairCursor pairs = open_pairs(list, first, e0, e1, j0);
 
         for (int e = lane; e < TC; e += 32) {
             S.a[e] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -438,17 +619,17 @@ k_deposit_items(const float4* __restrict__ rec, DepositParams P, int total_tiles
         }
         __syncwarp();
 
-        for (int c0 = j0; c0 < j1; c0 += 32) {
+        for (uint32_t c0 = j0; c0 < j1; c0 += 32) {
             // ---- setup: one pair per lane: exact ranges of its image, 1-D weights ----
             // rect packs tile-relative [x0,x1) [y0,y1) [z0,z1) in 4-bit fields and
             // the halo flag in bit 24; 0 means no cells
             uint32_t rect = 0;
             float4 val = make_float4(0.f, 0.f, 0.f, 0.f);
             {
-                const int j = c0 + lane;
-                if (j < j1) {
-                    const int i = pvals[j];
-                    const int combo = P.periodic ? (int)(pkeys[j] & ((1u << IMG_BITS) - 1u)) : 0;
+                uint32_t which;
+                const int i = pairs.take(c0 + lane, j1, which);
+                if (i >= 0) {
+                    const int combo = periodic ? (int)(ekeys[which] & ((1u << IMG_BITS) - 1u)) : 0;
                     const int dk[3] = {combo % 3, (combo / 3) % 3, combo / 9};
                     float4 A, B, Cc, D;
                     load_dep_rec(rec, i, P.boxsize, P.rbox, A, B, Cc, D);
@@ -485,7 +666,7 @@ k_deposit_items(const float4* __restrict__ rec, DepositParams P, int total_tiles
             }
             __syncwarp();
             // ---- the warp adds the chunk's pairs in order, lanes over each pair's cells ----
-            const int cnt = min(32, j1 - c0);
+            const int cnt = (int)min(32u, j1 - c0);
             for (int p = 0; p < cnt; ++p) {
                 const uint32_t rp = __shfl_sync(FULLM, rect, p);
                 const int x0 = rp & 15, nx = ((rp >> 4) & 15) - x0;
@@ -558,31 +739,38 @@ k_deposit_items(const float4* __restrict__ rec, DepositParams P, int total_tiles
 // A pair's contribution to its tile is separable: weight wx[x] wy[y] wz[z]
 // times the particle's value in each channel (n: 1, halo: 1, c: dens, v), so a
 // tile is a sum of outer products, C[(x, y)][(channel, z)] = sum over pairs of
-// A[(x, y)][p] B[p][(channel, z)] with A = wx wy (64 rows) and B = wz * value
-// (8 columns per channel): a GEMM with K = the item's pairs.  One warp runs it
-// with mma.sync m16n8k8 (TF32 in, FP32 accumulate), 8 pairs per K step, 4 x
-// NCH fragments of 16 x 8 held in registers.  TF32 keeps 11 significant bits,
-// so every operand is split into hi + lo TF32 parts and each K step issues
-// lo*hi, hi*lo and hi*hi (the lo*lo term is below 2^-22 relative), which
-// gives each product to about 2^-21.  Every 64 pairs the fragments are added
-// into per-lane double-float sums in shared memory and cleared, so the FP32
-// accumulation never carries more than 24 roundings.  Lane (g, t) owns the
-// cells x = g, z = 2t + {0, 1} and every y of the tile, both in the fragments
-// and in its sums, so the sums need no synchronisation.
+// A[(x, y)][p] B[p][(channel, z)] with A = wx wy (32 rows) and B = wz * value
+// (two channels x 4 z per block of 8 columns): a GEMM with K = the item's
+// pairs.  One warp runs it with mma.sync m16n8k8 (TF32 in, FP32 accumulate), 8
+// pairs per K step, on 2 row blocks x 3 column blocks of fragments.  TF32 keeps
+// 11 significant bits, so every operand is split into hi + lo TF32 parts and
+// each K step issues lo*hi, hi*lo and hi*hi (the lo*lo term is below 2^-22
+// relative), which gives each product to about 2^-21.  Every 64 pairs the
+// fragments are added into per-lane double-float sums in shared memory and
+// cleared, so the FP32 accumulation never carries more than 24 roundings.
+// Lane (g, t) owns the cells x = g, z = 2 (t mod 2) + {0, 1}, every y, of the
+// channels n, c, vy (t < 2) or halo, vx, vz (t >= 2), both in the fragments and
+// in its sums, so the sums need no synchronisation.
 // The FP64 mass totals do not come from the cells: each pair adds
 // (sum wx)(sum wy)(sum wz), formed in double-float arithmetic, to its lane's
-// double-float total.  A K step skips the row blocks (two y rows each) and the
-// channels that none of its 8 pairs touches: their products are exact zeros.
-constexpr int MMA_WARPS = 2;
+// double-float total.  A K step skips the row blocks (two y rows each) that none
+// of its 8 pairs touches, and the columns of c and v when all are halo
+// particles: their products are exact zeros.
+//
+// One warp per item and CTA: no barriers, and a warp that waits for its own
+// loads or its mma.sync chains leaves the SM to 23 others (8 KB of shared memory
+// each): 70% of issue slots busy against 48% with two warps per 8 x 8 x 8 item and
+// 16 warps per SM.  Bound by instruction issue, 44 warp instructions per pair, of
+// which the 1-D weights take two thirds.  9.22 -> 7.02 ms on the 256^3 step's
+// 120 M pairs; on 160^3 cells, n alone, 0.27 ms for 512 k particles.
 constexpr int MMA_FLUSH = 64;  // pairs between flushes of the fragments
-constexpr uint32_t INFO_MAIN = 1u << 8;  // a pair deposits into n, c and v
-constexpr uint32_t INFO_HALO = 1u << 9;  // a pair deposits into halo
 
 template <int NCH>
 struct MmaWarp {
-    float acc[NCH == 1 ? 2 : 9][16][32];  // [word][2 y + dz][lane]: n hi/lo, c hi/lo, halo hi/lo, v xyz
-    float w[32][WROW];                    // per pair of the chunk: wx[0..7] | wy[0..7] | wz[0..7]
-    float v[32][NCH == 1 ? 1 : 8];        // per pair: n, halo, c, vx, vy, vz values
+    // [word][lane]: 8 hi, 8 lo of n/halo; of c/vx; 8 of vy/vz (n alone: 16 hi, 16 lo)
+    float acc[NCH == 1 ? 32 : 40][32];
+    // per pair of the chunk: wx | wy | wz | dens, vx, vy, vz (n alone: padding)
+    float w[32][NCH == 1 ? 28 : 20];
 };
 
 __device__ __forceinline__ uint32_t tf32_rna(float x)
@@ -629,184 +817,230 @@ __device__ __forceinline__ void df_mul_df(float& hi, float& lo, float bh, float 
     hi = s;
 }
 
+// tent_integral_rn as selections, with the same operations where they matter and
+// so the same bits.  For a cell on one side of the centre with its nearer edge at
+// distance p and its farther one at q: (q - p)(1 - (p + q)/2), or (1 - p)^2/2 when
+// the support ends inside it, 0 when it lies beyond; q - p and p + q are |b - a| and
+// |a + b| to the bit (sign changes are exact), 1 - t/2 is one FMA because t/2 is
+// exact.  The cell around the centre (a < 0 < b) is tent_centre_rn.
+__device__ __forceinline__ float tent_side_rn(float a, float b)
+{
+    const float p = fminf(fabsf(a), fabsf(b)), q = fmaxf(fabsf(a), fabsf(b));
+    const float u = fmaxf(__fsub_rn(1.0f, p), 0.0f);
+    const float tail = __fmul_rn(__fmul_rn(0.5f, u), u);
+    const float mid = __fmul_rn(__fsub_rn(b, a), __fmaf_rn(-0.5f, fabsf(__fadd_rn(a, b)), 1.0f));
+    return q >= 1.0f ? tail : mid;
+}
+__device__ __forceinline__ float tent_centre_rn(float a, float b)
+{
+    const float t = fminf(b, 1.0f), s = fminf(-a, 1.0f);  // F(1) = 1/2 exactly
+    return __fadd_rn(__fmul_rn(t, __fmaf_rn(-0.5f, t, 1.0f)), __fmul_rn(s, __fmaf_rn(-0.5f, s, 1.0f)));
+}
+
 template <int NCH>
-__global__ void __launch_bounds__(32 * MMA_WARPS)
-k_deposit_mma(const float4* __restrict__ rec, DepositParams P, int total_tiles,
-              const uint32_t* __restrict__ item_off, const uint32_t* __restrict__ tstart,
-              const uint32_t* __restrict__ tcount, const uint32_t* __restrict__ pkeys,
-              const int* __restrict__ pvals, float* __restrict__ partial,
+__global__ void __launch_bounds__(32, 24)
+k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositParams P, int total_tiles,
+              const uint32_t* __restrict__ item_off, uint32_t max_items,
+              const uint32_t* __restrict__ item_tile, const uint32_t* __restrict__ tentry,
+              const uint32_t* __restrict__ ekeys, const uint2* __restrict__ list,
+              const uint32_t* __restrict__ first, float* __restrict__ partial,
               double* __restrict__ item_tot, int* __restrict__ next_item)
 {
+    constexpr int MX = TileShape<NCH>::X, MY = TileShape<NCH>::Y, MZ = TileShape<NCH>::Z;
+    constexpr int MC = TileShape<NCH>::CELLS;
+    constexpr int NB = NCH == 1 ? 1 : 3;  // column blocks: n (8 z) or n halo | c vx | vy vz (4 z each)
+    constexpr int RB = MY / 2;            // row blocks: 8 x and 2 y
+    constexpr int R = 4 * RB;             // cells per lane and column block
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int NW = NCH == 1 ? 2 : 9;
-    const int lane = threadIdx.x & 31;
+    MmaWarp<NCH>& S = *reinterpret_cast<MmaWarp<NCH>*>(smem_raw);
+    const int lane = threadIdx.x;
     const int g = lane >> 2, t = lane & 3;
-    MmaWarp<NCH>& S = reinterpret_cast<MmaWarp<NCH>*>(smem_raw)[threadIdx.x >> 5];
     const bool periodic = P.periodic != 0;
-    const uint32_t total_items = item_off[total_tiles];
+    const uint32_t total_items = min(item_off[total_tiles], max_items);
 
-    for (;;) {
-        int item = 0, tile = -1;
-        if (lane == 0) {
-            item = atomicAdd(next_item, 1);
-            if ((uint32_t)item < total_items) tile = upper_index(item_off, total_tiles + 1, (uint32_t)item);
-        }
-        item = __shfl_sync(FULLM, item, 0);
-        const int slot = __shfl_sync(FULLM, tile, 0);  // items are numbered in slot order
-        if ((uint32_t)item >= total_items) break;
-        tile = P.order ? (int)P.order[slot] : slot;
+    int item = 0;
+    if (lane == 0) item = atomicAdd(next_item, 1);
+    item = __shfl_sync(FULLM, item, 0);
+    while ((uint32_t)item < total_items) {
+        int next = 0;  // the next item's number arrives while this one runs
+        if (lane == 0) next = atomicAdd(next_item, 1);
+        const int tile = (int)item_tile[item];
         const TileGeo geo = tile_geo(P, tile);
         const MeshJob& J = P.job[geo.job];
         const int nc = geo.nc;
-        const int seg = item - (int)item_off[slot];
-        const int nseg = (int)(item_off[slot + 1] - item_off[slot]);
-        const int j0 = (int)tstart[tile] + seg * P.seg;
-        const int j1 = (int)tstart[tile] + min((int)tcount[tile], (seg + 1) * P.seg);
+        const int i0 = (int)item_off[tile], nseg = (int)item_off[tile + 1] - i0;
+        const uint32_t e0 = tentry[tile], e1 = max(tentry[tile + 1], e0);
+        const uint32_t j0 = first[e0] + (uint32_t)((item - i0) * P.seg);
+        const uint32_t j1 = min(first[e1], j0 + (uint32_t)P.seg);
+        PairCursor pairs = open_pairs(list, first, e0, e1, j0);
 
 #pragma unroll
-        for (int k = 0; k < NW; ++k)
+        for (int k = 0; k < (int)(sizeof(S.acc) / sizeof(S.acc[0])); ++k) S.acc[k][lane] = 0.f;
+        float C[RB][NB][4];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) S.acc[k][r][lane] = 0.f;
-        float C[4][NCH][4];
+        for (int m = 0; m < RB; ++m)
 #pragma unroll
-        for (int mb = 0; mb < 4; ++mb)
+            for (int b = 0; b < NB; ++b)
 #pragma unroll
-            for (int ch = 0; ch < NCH; ++ch)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) C[mb][ch][i] = 0.f;
+                for (int i = 0; i < 4; ++i) C[m][b][i] = 0.f;
         float tn_hi = 0.f, tn_lo = 0.f, th_hi = 0.f, th_lo = 0.f;  // this lane's pairs' totals
 
-        // adds the fragments into the lane's double-float sums and clears them
+        // adds the fragments into the lane's sums and clears them
         auto flush = [&]() {
 #pragma unroll
-            for (int mb = 0; mb < 4; ++mb)
+            for (int m = 0; m < RB; ++m)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int r = 2 * (2 * mb + (i >> 1)) + (i & 1);  // 2 y + dz
-                    float hi = S.acc[0][r][lane], lo = S.acc[1][r][lane];
-                    two_sum_acc(hi, lo, C[mb][0][i]);
-                    S.acc[0][r][lane] = hi;
-                    S.acc[1][r][lane] = lo;
-                    C[mb][0][i] = 0.f;
-                    if constexpr (NCH > 1) {
-                        hi = S.acc[4][r][lane]; lo = S.acc[5][r][lane];
-                        two_sum_acc(hi, lo, C[mb][1][i]);
-                        S.acc[4][r][lane] = hi; S.acc[5][r][lane] = lo;
-                        hi = S.acc[2][r][lane]; lo = S.acc[3][r][lane];
-                        two_sum_acc(hi, lo, C[mb][2][i]);
-                        S.acc[2][r][lane] = hi; S.acc[3][r][lane] = lo;
+                    const int r = 4 * m + i;
 #pragma unroll
-                        for (int d = 0; d < 3; ++d)
-                            S.acc[6 + d][r][lane] = __fadd_rn(S.acc[6 + d][r][lane], C[mb][3 + d][i]);
-#pragma unroll
-                        for (int ch = 1; ch < NCH; ++ch) C[mb][ch][i] = 0.f;
+                    for (int b = 0; b < (NB < 2 ? NB : 2); ++b) {
+                        float hi = S.acc[2 * R * b + r][lane], lo = S.acc[2 * R * b + R + r][lane];
+                        two_sum_acc(hi, lo, C[m][b][i]);
+                        S.acc[2 * R * b + r][lane] = hi;
+                        S.acc[2 * R * b + R + r][lane] = lo;
                     }
+                    if constexpr (NB > 2)
+                        S.acc[4 * R + r][lane] = __fadd_rn(S.acc[4 * R + r][lane], C[m][2][i]);
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) C[m][b][i] = 0.f;
                 }
         };
 
         int since_flush = 0;
-        for (int c0 = j0; c0 < j1; c0 += 32) {
+        for (uint32_t c0 = j0; c0 < j1; c0 += 32) {
             // ---- setup: one pair per lane: its image's cell range, 1-D weights
-            // (zero outside the range), channel values and FP64 mass; info =
-            // the y rows it touches (bits 0-7) and whether it deposits into the
-            // n, c, v channels (INFO_MAIN) or the halo channel (INFO_HALO) ----
-            uint32_t info = 0;
+            // (zero outside the range), channel values and FP64 mass.  The cells
+            // of an axis that some lane touches are taken by all lanes together ----
+            uint32_t rows = 0;  // the y rows the pair touches
+            bool halo = false;
             {
-                const int j = c0 + lane;
+                uint32_t which;
+                const int i = pairs.take(c0 + lane, j1, which);
                 float* wl = S.w[lane];
-                float vals[NCH == 1 ? 1 : 6];
+                float4* wz4 = reinterpret_cast<float4*>(wl);
 #pragma unroll
-                for (int k = 0; k < (NCH == 1 ? 1 : 6); ++k) vals[k] = 0.f;
-#pragma unroll
-                for (int k = 0; k < 3 * TS; ++k) wl[k] = 0.f;
-                if (j < j1) {
-                    const int i = pvals[j];
-                    const int combo = P.periodic ? (int)(pkeys[j] & ((1u << IMG_BITS) - 1u)) : 0;
-                    const int dk[3] = {combo % 3, (combo / 3) % 3, combo / 9};
-                    float4 A, B, Cc, D;
+                for (int k = 0; k < (MX + MY + MZ) / 4; ++k) wz4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A, Cc = A, D = A;
+                int combo = 0;
+                if (i >= 0) {
                     load_dep_rec(rec, i, P.boxsize, P.rbox, A, B, Cc, D);
-                    const float xs[3] = {A.x, A.y, A.z};
-                    const float lo[3] = {B.x, B.y, B.z};
-                    const float hi[3] = {Cc.x, Cc.y, Cc.z};
-                    const float hinv = A.w;
-                    float mh = 1.0f, ml = 0.0f;  // product of the three 1-D sums (double-float)
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const AxisRange ar = axis_range(lo[a], hi[a], J, nc, periodic);
-                        const int k = ar.k_lo + dk[a];
-                        const int sh = k * nc + geo.O[a];
-                        const int r0 = max(ar.left - sh, 0), r1 = min(ar.right - sh, geo.E[a]);
-                        // cell t covers [fi*dx, (fi+1)*dx] with fi = t + sh (see k_deposit_items)
-                        float fi = (float)(r0 + sh);
-                        float e0 = __fmul_rn(__fmaf_rn(fi, J.dx, -xs[a]), hinv);
-                        float sh_ = 0.f, sl_ = 0.f;
-                        for (int c = r0; c < r1; ++c) {
-                            fi = __fadd_rn(fi, 1.0f);
-                            const float e1 = __fmul_rn(__fmaf_rn(fi, J.dx, -xs[a]), hinv);
-                            const float wv = tent_integral_rn(e0, e1);
-                            wl[a * TS + c] = wv;
-                            two_sum_acc(sh_, sl_, wv);
-                            e0 = e1;
-                        }
-                        if (a == 0) { mh = sh_; ml = sl_; }
-                        else df_mul_df(mh, ml, sh_, sl_);
-                        if (a == 1 && r1 > r0) info = ((1u << r1) - 1u) & ~((1u << r0) - 1u);
-                    }
-                    const bool halo = (__float_as_int(D.z) & FLAG_HALO) != 0;
-                    if (info) info |= halo ? INFO_HALO : INFO_MAIN;
-                    if (!halo) {
-                        vals[0] = 1.0f;
-                        if constexpr (NCH > 1) {
-                            vals[2] = B.w;   // dens
-                            vals[3] = Cc.w;  // vx
-                            vals[4] = D.x;   // vy
-                            vals[5] = D.y;   // vz
-                        }
-                        two_sum_acc(tn_hi, tn_lo, mh);
-                        tn_lo = __fadd_rn(tn_lo, ml);
-                    } else {
-                        if constexpr (NCH > 1) vals[1] = 1.0f;
-                        two_sum_acc(th_hi, th_lo, mh);
-                        th_lo = __fadd_rn(th_lo, ml);
-                    }
+                    if (periodic) combo = (int)(ekeys[which] & ((1u << IMG_BITS) - 1u));
                 }
+                halo = (__float_as_int(D.z) & FLAG_HALO) != 0;
+                const int dk[3] = {combo % 3, (combo / 3) % 3, combo / 9};
+                const float xs[3] = {A.x, A.y, A.z};
+                const float lo[3] = {B.x, B.y, B.z};
+                const float hi[3] = {Cc.x, Cc.y, Cc.z};
+                const float hinv = A.w;
+                float mh = 0.0f, ml = 0.0f;  // product of the three 1-D sums (double-float)
 #pragma unroll
-                for (int k = 0; k < (NCH == 1 ? 1 : 6); ++k) S.v[lane][k] = vals[k];
+                for (int a = 0; a < 3; ++a) {
+                    constexpr int at[3] = {0, MX, MX + MY};
+                    const AxisRange ar = axis_range(lo[a], hi[a], J, nc, periodic);
+                    const int sh = (ar.k_lo + dk[a]) * nc + geo.O[a];
+                    int r0 = max(ar.left - sh, 0), r1 = min(ar.right - sh, geo.E[a]);
+                    if (i < 0 || r1 <= r0) r0 = r1 = 0;
+                    const int any0 = (int)__reduce_min_sync(FULLM, (unsigned)(r1 > r0 ? r0 : MX));
+                    const int any1 = (int)__reduce_max_sync(FULLM, (unsigned)r1);
+                    // cell c covers [fi*dx, (fi+1)*dx] with fi = c + sh (see k_deposit_items)
+                    float fi = (float)(any0 + sh);
+                    float e0 = __fmul_rn(__fmaf_rn(fi, J.dx, -xs[a]), hinv);
+                    float sh_ = 0.f, sl_ = 0.f;
+                    const unsigned mine = ((1u << r1) - 1u) & ~((1u << r0) - 1u);  // cells [r0, r1)
+                    for (int c = any0; c < any1; ++c) {
+                        fi = __fadd_rn(fi, 1.0f);
+                        const float e1 = __fmul_rn(__fmaf_rn(fi, J.dx, -xs[a]), hinv);
+                        float wv = tent_side_rn(e0, e1);
+                        const bool centre = e0 < 0.0f && e1 > 0.0f;
+                        if (__any_sync(FULLM, centre)) {
+                            const float wc = tent_centre_rn(e0, e1);
+                            wv = centre ? wc : wv;
+                        }
+                        wv = (mine >> c) & 1u ? wv : 0.0f;
+                        wl[at[a] + c] = wv;
+                        two_sum_acc_nonneg(sh_, sl_, wv);
+                        e0 = e1;
+                    }
+                    if (a == 0) { mh = sh_; ml = sl_; }
+                    else df_mul_df(mh, ml, sh_, sl_);
+                    if (a == 1) rows = mine;
+                }
+                // a halo particle counts in the halo channel only
+                if constexpr (NCH > 1)
+                    wz4[4] = halo ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(B.w, Cc.w, D.x, D.y);
+                if (!halo) {
+                    two_sum_acc(tn_hi, tn_lo, mh);
+                    tn_lo = __fadd_rn(tn_lo, ml);
+                } else {
+                    two_sum_acc(th_hi, th_lo, mh);
+                    th_lo = __fadd_rn(th_lo, ml);
+                }
             }
+            const unsigned halos = __ballot_sync(FULLM, halo);
             __syncwarp();
-            // ---- K steps of 8 pairs: pairs 8s + t (A) and 8s + t + 4 (B) for this lane ----
-            const int cnt = min(32, j1 - c0);
+            // ---- K steps of 8 pairs: pairs 8s + t and 8s + t + 4 for this lane ----
+            const int cnt = (int)min(32u, j1 - c0);
             for (int s8 = 0; s8 < cnt; s8 += 8) {
-                // the rows and channels the step's 8 pairs touch (warp-uniform);
-                // the products of the others are exact zeros and are skipped
-                const uint32_t kinfo =
-                    __reduce_or_sync(FULLM, (lane >= s8 && lane < s8 + 8) ? info : 0u);
+                const unsigned krows =
+                    __reduce_or_sync(FULLM, (unsigned)(lane - s8) < 8u ? rows : 0u);
                 const float* wa = S.w[s8 + t];
                 const float* wb = S.w[s8 + t + 4];
                 const float xa = wa[g], xb = wb[g];
-                const float za = wa[2 * TS + g], zb = wb[2 * TS + g];
-                uint32_t bh[NCH][2], bl[NCH][2];
+                const float za = wa[MX + MY + (NCH == 1 ? g : g & 3)];
+                const float zb = wb[MX + MY + (NCH == 1 ? g : g & 3)];
+                uint32_t bh[NB][2], bl[NB][2];
+                if constexpr (NCH == 1) {
+                    tf32_split(za, bh[0][0], bl[0][0]);
+                    tf32_split(zb, bh[0][1], bl[0][1]);
+                } else {
+                    const unsigned hs = halos >> (s8 + t);
+                    tf32_split((hs & 1u) == (unsigned)(g >> 2) ? za : 0.0f, bh[0][0], bl[0][0]);
+                    tf32_split(((hs >> 4) & 1u) == (unsigned)(g >> 2) ? zb : 0.0f, bh[0][1], bl[0][1]);
 #pragma unroll
-                for (int ch = 0; ch < NCH; ++ch) {
-                    if (!(kinfo & (ch == 1 && NCH > 1 ? INFO_HALO : INFO_MAIN))) continue;
-                    tf32_split(__fmul_rn(za, S.v[s8 + t][ch]), bh[ch][0], bl[ch][0]);
-                    tf32_split(__fmul_rn(zb, S.v[s8 + t + 4][ch]), bh[ch][1], bl[ch][1]);
-                }
-#pragma unroll
-                for (int mb = 0; mb < 4; ++mb) {
-                    if (!(kinfo & (3u << (2 * mb)))) continue;
-                    uint32_t ah[4], al[4];
-                    tf32_split(__fmul_rn(xa, wa[TS + 2 * mb]), ah[0], al[0]);
-                    tf32_split(__fmul_rn(xa, wa[TS + 2 * mb + 1]), ah[1], al[1]);
-                    tf32_split(__fmul_rn(xb, wb[TS + 2 * mb]), ah[2], al[2]);
-                    tf32_split(__fmul_rn(xb, wb[TS + 2 * mb + 1]), ah[3], al[3]);
-#pragma unroll
-                    for (int ch = 0; ch < NCH; ++ch) {
-                        if (!(kinfo & (ch == 1 && NCH > 1 ? INFO_HALO : INFO_MAIN))) continue;
-                        mma_tf32(C[mb][ch], al, bh[ch][0], bh[ch][1]);
-                        mma_tf32(C[mb][ch], ah, bl[ch][0], bl[ch][1]);
-                        mma_tf32(C[mb][ch], ah, bh[ch][0], bh[ch][1]);
+                    for (int b = 1; b < NB; ++b) {
+                        const int at = MX + MY + MZ + 2 * (b - 1) + (g >> 2);
+                        tf32_split(__fmul_rn(za, wa[at]), bh[b][0], bl[b][0]);
+                        tf32_split(__fmul_rn(zb, wb[at]), bh[b][1], bl[b][1]);
                     }
+                }
+                // two row blocks at a time, those this K step touches, both in one
+                // block of code when both do; the passes run over all live
+                // accumulators, so the independent accumulation chains interleave
+#pragma unroll
+                for (int h = 0; h < RB; h += 2) {
+                    const float4 ya = *reinterpret_cast<const float4*>(wa + MX + 2 * h);
+                    const float4 yb = *reinterpret_cast<const float4*>(wb + MX + 2 * h);
+                    auto blocks = [&](auto use0, auto use1) {
+                        constexpr bool U[2] = {decltype(use0)::value, decltype(use1)::value};
+                        uint32_t ah[2][4], al[2][4];
+#pragma unroll
+                        for (int m = 0; m < 2; ++m) {
+                            if (!U[m]) continue;
+                            tf32_split(__fmul_rn(xa, m ? ya.z : ya.x), ah[m][0], al[m][0]);
+                            tf32_split(__fmul_rn(xa, m ? ya.w : ya.y), ah[m][1], al[m][1]);
+                            tf32_split(__fmul_rn(xb, m ? yb.z : yb.x), ah[m][2], al[m][2]);
+                            tf32_split(__fmul_rn(xb, m ? yb.w : yb.y), ah[m][3], al[m][3]);
+                        }
+#pragma unroll
+                        for (int m = 0; m < 2; ++m)
+#pragma unroll
+                            for (int b = 0; b < NB; ++b)
+                                if (U[m]) mma_tf32(C[h + m][b], al[m], bh[b][0], bh[b][1]);
+#pragma unroll
+                        for (int m = 0; m < 2; ++m)
+#pragma unroll
+                            for (int b = 0; b < NB; ++b)
+                                if (U[m]) mma_tf32(C[h + m][b], ah[m], bl[b][0], bl[b][1]);
+#pragma unroll
+                        for (int m = 0; m < 2; ++m)
+#pragma unroll
+                            for (int b = 0; b < NB; ++b)
+                                if (U[m]) mma_tf32(C[h + m][b], ah[m], bh[b][0], bh[b][1]);
+                    };
+                    const bool r0 = (krows >> (2 * h) & 3u) != 0, r1 = (krows >> (2 * h) & 12u) != 0;
+                    if (r0 && r1) blocks(std::true_type{}, std::true_type{});
+                    else if (r0) blocks(std::true_type{}, std::false_type{});
+                    else if (r1) blocks(std::false_type{}, std::true_type{});
                 }
             }
             since_flush += 32;
@@ -814,7 +1048,7 @@ k_deposit_mma(const float4* __restrict__ rec, DepositParams P, int total_tiles,
                 flush();
                 since_flush = 0;
             }
-            __syncwarp();  // the next chunk's setup overwrites S.w and S.v
+            __syncwarp();  // the next chunk's setup overwrites S.w
         }
         if (since_flush > 0) flush();
 
@@ -825,353 +1059,49 @@ k_deposit_mma(const float4* __restrict__ rec, DepositParams P, int total_tiles,
             sn += __shfl_down_sync(FULLM, sn, o);
             shl += __shfl_down_sync(FULLM, shl, o);
         }
+        const bool low = NCH == 1 || t < 2;  // the lane's channels: n, c, vy, else halo, vx, vz
         if (nseg > 1) {
-            float* pt = partial + (size_t)item * TC * PW;
+            float* pt = partial + (size_t)item * MC * PW;
 #pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                const int y = r >> 1, z = 2 * t + (r & 1);
-                const int e = (z * TS + y) * TS + g;
-                pt[e] = S.acc[0][r][lane];
-                pt[TC + e] = S.acc[1][r][lane];
+            for (int r = 0; r < R; ++r) {
+                const int y = r >> 1, z = 2 * (NCH == 1 ? t : t & 1) + (r & 1);
+                const int e = (z * MY + y) * MX + g;
+                pt[(low ? 0 : 7) * MC + e] = S.acc[r][lane];
+                pt[(low ? 1 : 8) * MC + e] = S.acc[R + r][lane];
                 if constexpr (NCH > 1) {
-                    pt[2 * TC + e] = S.acc[2][r][lane];
-                    pt[3 * TC + e] = S.acc[3][r][lane];
-                    pt[4 * TC + e] = S.acc[6][r][lane];
-                    pt[5 * TC + e] = S.acc[7][r][lane];
-                    pt[6 * TC + e] = S.acc[8][r][lane];
-                    pt[7 * TC + e] = S.acc[4][r][lane];
-                    pt[8 * TC + e] = S.acc[5][r][lane];
-                }
-            }
-            if (lane == 0) {
-                item_tot[2 * item] = sn;
-                item_tot[2 * item + 1] = shl;
-            }
-        } else {
-            const size_t nmesh = (size_t)nc * nc * nc;
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                const int y = r >> 1, z = 2 * t + (r & 1);
-                if (g >= geo.E[0] || y >= geo.E[1] || z >= geo.E[2]) continue;
-                const size_t idx = ((size_t)(geo.O[2] + z) * nc + (geo.O[1] + y)) * nc + (geo.O[0] + g);
-                J.mesh[idx] = __fadd_rn(S.acc[0][r][lane], S.acc[1][r][lane]);
-                if constexpr (NCH > 1) {
-                    J.mesh[nmesh + idx] = __fadd_rn(S.acc[4][r][lane], S.acc[5][r][lane]);
-                    J.mesh[2 * nmesh + idx] = __fadd_rn(S.acc[2][r][lane], S.acc[3][r][lane]);
-                    J.mesh[3 * nmesh + 3 * idx] = S.acc[6][r][lane];
-                    J.mesh[3 * nmesh + 3 * idx + 1] = S.acc[7][r][lane];
-                    J.mesh[3 * nmesh + 3 * idx + 2] = S.acc[8][r][lane];
-                }
-            }
-            if (lane == 0) {
-                J.partial[2 * geo.local] = sn;
-                J.partial[2 * geo.local + 1] = shl;
-            }
-        }
-        __syncwarp();  // the next item clears the sums
-    }
-}
-
-// The same GEMM with the two warps of a CTA sharing one item: both warps set up
-// a chunk of 64 pairs (one pair per thread) in the CTA's staging, then each
-// warp runs the K steps for its own half of the tile's y rows (two row blocks,
-// 12 fragments) and keeps the double-float sums of its own 8 cells per lane.
-// Per CTA 27 KB of shared memory and per thread about half the fragments, so
-// about twice as many warps stay resident as with one warp per item.
-constexpr int MMA2_CHUNK = 64;  // pairs set up per chunk (one per thread)
-
-template <int NCH>
-struct Mma2Cta {
-    float acc[2][NCH == 1 ? 2 : 9][8][32];  // [warp][word][2 (y - 4 warp) + dz][lane]
-    float w[MMA2_CHUNK][WROW];
-    float v[MMA2_CHUNK][NCH == 1 ? 1 : 8];
-    uint32_t info[MMA2_CHUNK];
-    double tot[2][2];   // per warp: n and halo mass of the item
-    int item, tile;
-};
-
-template <int NCH>
-__global__ void __launch_bounds__(64)
-k_deposit_mma2(const float4* __restrict__ rec, DepositParams P, int total_tiles,
-               const uint32_t* __restrict__ item_off, const uint32_t* __restrict__ tstart,
-               const uint32_t* __restrict__ tcount, const uint32_t* __restrict__ pkeys,
-               const int* __restrict__ pvals, float* __restrict__ partial,
-               double* __restrict__ item_tot, int* __restrict__ next_item)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int NW = NCH == 1 ? 2 : 9;
-    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    Mma2Cta<NCH>& S = *reinterpret_cast<Mma2Cta<NCH>*>(smem_raw);
-    float(*acc)[8][32] = S.acc[wp];
-    const bool periodic = P.periodic != 0;
-    const uint32_t total_items = item_off[total_tiles];
-
-    for (;;) {
-        if (tid == 0) {
-            const int it = atomicAdd(next_item, 1);
-            S.item = it;
-            S.tile = (uint32_t)it < total_items ? upper_index(item_off, total_tiles + 1, (uint32_t)it) : -1;
-        }
-        __syncthreads();
-        const int item = S.item, slot = S.tile;  // items are numbered in slot order
-        if ((uint32_t)item >= total_items) break;
-        const int tile = P.order ? (int)P.order[slot] : slot;
-        const TileGeo geo = tile_geo(P, tile);
-        const MeshJob& J = P.job[geo.job];
-        const int nc = geo.nc;
-        const int seg = item - (int)item_off[slot];
-        const int nseg = (int)(item_off[slot + 1] - item_off[slot]);
-        const int j0 = (int)tstart[tile] + seg * P.seg;
-        const int j1 = (int)tstart[tile] + min((int)tcount[tile], (seg + 1) * P.seg);
-
-#pragma unroll
-        for (int k = 0; k < NW; ++k)
-#pragma unroll
-            for (int r = 0; r < 8; ++r) acc[k][r][lane] = 0.f;
-        float C[2][NCH][4];
-#pragma unroll
-        for (int mb = 0; mb < 2; ++mb)
-#pragma unroll
-            for (int ch = 0; ch < NCH; ++ch)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) C[mb][ch][i] = 0.f;
-        float tn_hi = 0.f, tn_lo = 0.f, th_hi = 0.f, th_lo = 0.f;
-
-        for (int c0 = j0; c0 < j1; c0 += MMA2_CHUNK) {
-            // ---- setup: one pair per thread (as in k_deposit_mma) ----
-            {
-                const int j = c0 + tid;
-                float* wl = S.w[tid];
-                float vals[NCH == 1 ? 1 : 6];
-#pragma unroll
-                for (int k = 0; k < (NCH == 1 ? 1 : 6); ++k) vals[k] = 0.f;
-#pragma unroll
-                for (int k = 0; k < 3 * TS; ++k) wl[k] = 0.f;
-                uint32_t info = 0;
-                if (j < j1) {
-                    const int i = pvals[j];
-                    const int combo = P.periodic ? (int)(pkeys[j] & ((1u << IMG_BITS) - 1u)) : 0;
-                    const int dk[3] = {combo % 3, (combo / 3) % 3, combo / 9};
-                    float4 A, B, Cc, D;
-                    load_dep_rec(rec, i, P.boxsize, P.rbox, A, B, Cc, D);
-                    const float xs[3] = {A.x, A.y, A.z};
-                    const float lo[3] = {B.x, B.y, B.z};
-                    const float hi[3] = {Cc.x, Cc.y, Cc.z};
-                    const float hinv = A.w;
-                    float mh = 1.0f, ml = 0.0f;
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const AxisRange ar = axis_range(lo[a], hi[a], J, nc, periodic);
-                        const int k = ar.k_lo + dk[a];
-                        const int sh = k * nc + geo.O[a];
-                        const int r0 = max(ar.left - sh, 0), r1 = min(ar.right - sh, geo.E[a]);
-                        float fi = (float)(r0 + sh);
-                        float e0 = __fmul_rn(__fmaf_rn(fi, J.dx, -xs[a]), hinv);
-                        float sh_ = 0.f, sl_ = 0.f;
-                        for (int c = r0; c < r1; ++c) {
-                            fi = __fadd_rn(fi, 1.0f);
-                            const float e1 = __fmul_rn(__fmaf_rn(fi, J.dx, -xs[a]), hinv);
-                            const float wv = tent_integral_rn(e0, e1);
-                            wl[a * TS + c] = wv;
-                            two_sum_acc(sh_, sl_, wv);
-                            e0 = e1;
-                        }
-                        if (a == 0) { mh = sh_; ml = sl_; }
-                        else df_mul_df(mh, ml, sh_, sl_);
-                        if (a == 1 && r1 > r0) info = ((1u << r1) - 1u) & ~((1u << r0) - 1u);
-                    }
-                    const bool halo = (__float_as_int(D.z) & FLAG_HALO) != 0;
-                    if (info) info |= halo ? INFO_HALO : INFO_MAIN;
-                    if (!halo) {
-                        vals[0] = 1.0f;
-                        if constexpr (NCH > 1) {
-                            vals[2] = B.w;
-                            vals[3] = Cc.w;
-                            vals[4] = D.x;
-                            vals[5] = D.y;
-                        }
-                        two_sum_acc(tn_hi, tn_lo, mh);
-                        tn_lo = __fadd_rn(tn_lo, ml);
+                    if (low) {
+                        pt[2 * MC + e] = S.acc[2 * R + r][lane];
+                        pt[3 * MC + e] = S.acc[3 * R + r][lane];
                     } else {
-                        if constexpr (NCH > 1) vals[1] = 1.0f;
-                        two_sum_acc(th_hi, th_lo, mh);
-                        th_lo = __fadd_rn(th_lo, ml);
+                        pt[4 * MC + e] = __fadd_rn(S.acc[2 * R + r][lane], S.acc[3 * R + r][lane]);
                     }
+                    pt[(low ? 5 : 6) * MC + e] = S.acc[4 * R + r][lane];
                 }
-#pragma unroll
-                for (int k = 0; k < (NCH == 1 ? 1 : 6); ++k) S.v[tid][k] = vals[k];
-                S.info[tid] = info;
             }
-            __syncthreads();
-            // ---- K steps over the chunk, this warp's row blocks 2 wp and 2 wp + 1 ----
-            const int cnt = min(MMA2_CHUNK, j1 - c0);
-            for (int s8 = 0; s8 < cnt; s8 += 8) {
-                const uint32_t kinfo = __reduce_or_sync(FULLM, S.info[s8 + (lane & 7)]);
-                const uint32_t rows = 0xfu << (4 * wp);  // the y rows of this warp
-                if (!(kinfo & rows)) continue;
-                const float* wa = S.w[s8 + t];
-                const float* wb = S.w[s8 + t + 4];
-                const float xa = wa[g], xb = wb[g];
-                const float za = wa[2 * TS + g], zb = wb[2 * TS + g];
-                // the channels fed by main particles (n, c, v) and by halo
-                // particles (halo) are tested once each, and within a group the
-                // three passes run pass by pass over its channels, so the
-                // independent accumulation chains interleave
-                const bool k_main = (kinfo & INFO_MAIN) != 0;
-                const bool k_halo = NCH > 1 && (kinfo & INFO_HALO) != 0;
-                uint32_t bh[NCH][2], bl[NCH][2];
-                if (k_main) {
-#pragma unroll
-                    for (int ch = 0; ch < NCH; ++ch) {
-                        if (NCH > 1 && ch == 1) continue;
-                        tf32_split(__fmul_rn(za, S.v[s8 + t][ch]), bh[ch][0], bl[ch][0]);
-                        tf32_split(__fmul_rn(zb, S.v[s8 + t + 4][ch]), bh[ch][1], bl[ch][1]);
-                    }
-                }
-                if (k_halo) {
-                    tf32_split(__fmul_rn(za, S.v[s8 + t][1]), bh[1][0], bl[1][0]);
-                    tf32_split(__fmul_rn(zb, S.v[s8 + t + 4][1]), bh[1][1], bl[1][1]);
-                }
-                // the warp's row blocks this K step touches, both in one block
-                // of code when both do (twice the independent chains)
-                auto blocks = [&](auto use0, auto use1) {
-                    constexpr bool U[2] = {decltype(use0)::value, decltype(use1)::value};
-                    uint32_t ah[2][4], al[2][4];
-#pragma unroll
-                    for (int m = 0; m < 2; ++m) {
-                        if (!U[m]) continue;
-                        const int mb = 2 * wp + m;
-                        tf32_split(__fmul_rn(xa, wa[TS + 2 * mb]), ah[m][0], al[m][0]);
-                        tf32_split(__fmul_rn(xa, wa[TS + 2 * mb + 1]), ah[m][1], al[m][1]);
-                        tf32_split(__fmul_rn(xb, wb[TS + 2 * mb]), ah[m][2], al[m][2]);
-                        tf32_split(__fmul_rn(xb, wb[TS + 2 * mb + 1]), ah[m][3], al[m][3]);
-                    }
-                    if (k_main) {
-#pragma unroll
-                        for (int m = 0; m < 2; ++m)
-#pragma unroll
-                            for (int ch = 0; ch < NCH; ++ch)
-                                if (U[m] && !(NCH > 1 && ch == 1))
-                                    mma_tf32(C[m][ch], al[m], bh[ch][0], bh[ch][1]);
-#pragma unroll
-                        for (int m = 0; m < 2; ++m)
-#pragma unroll
-                            for (int ch = 0; ch < NCH; ++ch)
-                                if (U[m] && !(NCH > 1 && ch == 1))
-                                    mma_tf32(C[m][ch], ah[m], bl[ch][0], bl[ch][1]);
-#pragma unroll
-                        for (int m = 0; m < 2; ++m)
-#pragma unroll
-                            for (int ch = 0; ch < NCH; ++ch)
-                                if (U[m] && !(NCH > 1 && ch == 1))
-                                    mma_tf32(C[m][ch], ah[m], bh[ch][0], bh[ch][1]);
-                    }
-                    if (k_halo) {
-#pragma unroll
-                        for (int m = 0; m < 2; ++m)
-                            if (U[m]) mma_tf32(C[m][1], al[m], bh[1][0], bh[1][1]);
-#pragma unroll
-                        for (int m = 0; m < 2; ++m)
-                            if (U[m]) mma_tf32(C[m][1], ah[m], bl[1][0], bl[1][1]);
-#pragma unroll
-                        for (int m = 0; m < 2; ++m)
-                            if (U[m]) mma_tf32(C[m][1], ah[m], bh[1][0], bh[1][1]);
-                    }
-                };
-                const bool r0 = (kinfo & (3u << (4 * wp))) != 0;
-                const bool r1 = (kinfo & (3u << (4 * wp + 2))) != 0;
-                if (r0 && r1) blocks(std::true_type{}, std::true_type{});
-                else if (r0) blocks(std::true_type{}, std::false_type{});
-                else blocks(std::false_type{}, std::true_type{});
-            }
-            // ---- flush the fragments into the lane's sums (every chunk of 64 pairs) ----
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = 2 * (2 * m + (i >> 1)) + (i & 1);  // 2 (y - 4 wp) + dz
-                    float hi = acc[0][r][lane], lo = acc[1][r][lane];
-                    two_sum_acc(hi, lo, C[m][0][i]);
-                    acc[0][r][lane] = hi;
-                    acc[1][r][lane] = lo;
-                    C[m][0][i] = 0.f;
-                    if constexpr (NCH > 1) {
-                        hi = acc[4][r][lane]; lo = acc[5][r][lane];
-                        two_sum_acc(hi, lo, C[m][1][i]);
-                        acc[4][r][lane] = hi; acc[5][r][lane] = lo;
-                        hi = acc[2][r][lane]; lo = acc[3][r][lane];
-                        two_sum_acc(hi, lo, C[m][2][i]);
-                        acc[2][r][lane] = hi; acc[3][r][lane] = lo;
-#pragma unroll
-                        for (int d = 0; d < 3; ++d)
-                            acc[6 + d][r][lane] = __fadd_rn(acc[6 + d][r][lane], C[m][3 + d][i]);
-#pragma unroll
-                        for (int ch = 1; ch < NCH; ++ch) C[m][ch][i] = 0.f;
-                    }
-                }
-            __syncthreads();  // the next chunk's setup overwrites the staging
-        }
-
-        // ---- the item's FP64 mass (both warps' setup lanes), then the cells ----
-        double sn = (double)tn_hi + (double)tn_lo, shl = (double)th_hi + (double)th_lo;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            sn += __shfl_down_sync(FULLM, sn, o);
-            shl += __shfl_down_sync(FULLM, shl, o);
-        }
-        if (lane == 0) {
-            S.tot[wp][0] = sn;
-            S.tot[wp][1] = shl;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            sn = S.tot[0][0] + S.tot[1][0];
-            shl = S.tot[0][1] + S.tot[1][1];
-            if (nseg > 1) {
-                item_tot[2 * item] = sn;
-                item_tot[2 * item + 1] = shl;
-            } else {
-                J.partial[2 * geo.local] = sn;
-                J.partial[2 * geo.local + 1] = shl;
-            }
-        }
-        if (nseg > 1) {
-            float* pt = partial + (size_t)item * TC * PW;
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int y = 4 * wp + (r >> 1), z = 2 * t + (r & 1);
-                const int e = (z * TS + y) * TS + g;
-                pt[e] = acc[0][r][lane];
-                pt[TC + e] = acc[1][r][lane];
-                if constexpr (NCH > 1) {
-                    pt[2 * TC + e] = acc[2][r][lane];
-                    pt[3 * TC + e] = acc[3][r][lane];
-                    pt[4 * TC + e] = acc[6][r][lane];
-                    pt[5 * TC + e] = acc[7][r][lane];
-                    pt[6 * TC + e] = acc[8][r][lane];
-                    pt[7 * TC + e] = acc[4][r][lane];
-                    pt[8 * TC + e] = acc[5][r][lane];
-                }
+            if (lane == 0) {
+                item_tot[2 * (size_t)item] = sn;
+                item_tot[2 * (size_t)item + 1] = shl;
             }
         } else {
             const size_t nmesh = (size_t)nc * nc * nc;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int y = 4 * wp + (r >> 1), z = 2 * t + (r & 1);
+            for (int r = 0; r < R; ++r) {
+                const int y = r >> 1, z = 2 * (NCH == 1 ? t : t & 1) + (r & 1);
                 if (g >= geo.E[0] || y >= geo.E[1] || z >= geo.E[2]) continue;
                 const size_t idx = ((size_t)(geo.O[2] + z) * nc + (geo.O[1] + y)) * nc + (geo.O[0] + g);
-                J.mesh[idx] = __fadd_rn(acc[0][r][lane], acc[1][r][lane]);
+                J.mesh[(low ? 0 : nmesh) + idx] = __fadd_rn(S.acc[r][lane], S.acc[R + r][lane]);
                 if constexpr (NCH > 1) {
-                    J.mesh[nmesh + idx] = __fadd_rn(acc[4][r][lane], acc[5][r][lane]);
-                    J.mesh[2 * nmesh + idx] = __fadd_rn(acc[2][r][lane], acc[3][r][lane]);
-                    J.mesh[3 * nmesh + 3 * idx] = acc[6][r][lane];
-                    J.mesh[3 * nmesh + 3 * idx + 1] = acc[7][r][lane];
-                    J.mesh[3 * nmesh + 3 * idx + 2] = acc[8][r][lane];
+                    J.mesh[low ? 2 * nmesh + idx : 3 * nmesh + 3 * idx] =
+                        __fadd_rn(S.acc[2 * R + r][lane], S.acc[3 * R + r][lane]);
+                    J.mesh[3 * nmesh + 3 * idx + (low ? 1 : 2)] = S.acc[4 * R + r][lane];
                 }
             }
+            if (lane == 0) {
+                J.partial[2 * (size_t)geo.local] = sn;
+                J.partial[2 * (size_t)geo.local + 1] = shl;
+            }
         }
-        __syncthreads();  // the next item's fetch overwrites S.item, S.tot
+        item = __shfl_sync(FULLM, next, 0);
     }
 }
 
@@ -1179,64 +1109,70 @@ k_deposit_mma2(const float4* __restrict__ rec, DepositParams P, int total_tiles,
 // (5) merge the partial tiles of multi-segment tiles, in segment order
 // ---------------------------------------------------------------------------
 // item_tot (the tensor-core deposit): the FP64 mass of every item, summed in
-// item order; null: the mass is summed from the merged cells
+// item order; null: the mass is summed from the merged cells.  A CTA takes every
+// gridDim.x-th tile of the list `merge` (counters[1] tiles with several items).
 __global__ void __launch_bounds__(DEP_THREADS)
-k_merge_tiles(DepositParams P, int total_tiles, const uint32_t* __restrict__ item_off,
+k_merge_tiles(const __grid_constant__ DepositParams P, const uint32_t* __restrict__ item_off,
+              const uint32_t* __restrict__ merge, const int* __restrict__ counters,
               const float* __restrict__ partial, const double* __restrict__ item_tot)
 {
     __shared__ double red[2][DEP_THREADS / 32];
-    const int tile = blockIdx.x;
-    const int slot = P.pos ? (int)P.pos[tile] : tile;
-    const int i0 = (int)item_off[slot], i1 = (int)item_off[slot + 1];
-    if (i1 - i0 <= 1) return;
-    const TileGeo g = tile_geo(P, tile);
-    const MeshJob& J = P.job[g.job];
-    const int nc = g.nc;
-    const size_t nmesh = (size_t)nc * nc * nc;
+    const int cells = 1 << (P.shift[0] + P.shift[1] + P.shift[2]);
     const int tid = threadIdx.x;
-    double sn = 0.0, sh = 0.0;
-    for (int e = tid; e < TC; e += DEP_THREADS) {
-        float nh = 0.f, nl = 0.f, ch = 0.f, cl = 0.f, vx = 0.f, vy = 0.f, vz = 0.f, hh = 0.f, hl = 0.f;
-        for (int it = i0; it < i1; ++it) {
-            const float* pt = partial + (size_t)it * TC * PW;
-            two_sum_acc(nh, nl, pt[e]);
-            nl = __fadd_rn(nl, pt[TC + e]);
-            two_sum_acc(ch, cl, pt[2 * TC + e]);
-            cl = __fadd_rn(cl, pt[3 * TC + e]);
-            vx = __fadd_rn(vx, pt[4 * TC + e]);
-            vy = __fadd_rn(vy, pt[5 * TC + e]);
-            vz = __fadd_rn(vz, pt[6 * TC + e]);
-            two_sum_acc(hh, hl, pt[7 * TC + e]);
-            hl = __fadd_rn(hl, pt[8 * TC + e]);
+    const int listed = counters[1];
+    for (int k = blockIdx.x; k < listed; k += gridDim.x) {
+        const int tile = (int)merge[k];
+        const int i0 = (int)item_off[tile], i1 = (int)item_off[tile + 1];
+        const TileGeo g = tile_geo(P, tile);
+        const MeshJob& J = P.job[g.job];
+        const int nc = g.nc;
+        const size_t nmesh = (size_t)nc * nc * nc;
+        double sn = 0.0, sh = 0.0;
+        for (int e = tid; e < cells; e += DEP_THREADS) {
+            float nh = 0.f, nl = 0.f, ch = 0.f, cl = 0.f, vx = 0.f, vy = 0.f, vz = 0.f, hh = 0.f, hl = 0.f;
+#pragma unroll 4
+            for (int it = i0; it < i1; ++it) {
+                const float* pt = partial + (size_t)it * cells * PW;
+                two_sum_acc(nh, nl, pt[e]);
+                nl = __fadd_rn(nl, pt[cells + e]);
+                if (!P.density_only) {
+                    two_sum_acc(ch, cl, pt[2 * cells + e]);
+                    cl = __fadd_rn(cl, pt[3 * cells + e]);
+                    vx = __fadd_rn(vx, pt[4 * cells + e]);
+                    vy = __fadd_rn(vy, pt[5 * cells + e]);
+                    vz = __fadd_rn(vz, pt[6 * cells + e]);
+                    two_sum_acc(hh, hl, pt[7 * cells + e]);
+                    hl = __fadd_rn(hl, pt[8 * cells + e]);
+                }
+            }
+            const int lx = e & ((1 << P.shift[0]) - 1), ly = (e >> P.shift[0]) & ((1 << P.shift[1]) - 1);
+            const int lz = e >> (P.shift[0] + P.shift[1]);
+            if (lx >= g.E[0] || ly >= g.E[1] || lz >= g.E[2]) continue;
+            const size_t idx = ((size_t)(g.O[2] + lz) * nc + (g.O[1] + ly)) * nc + (g.O[0] + lx);
+            sn += (double)nh + (double)nl;
+            sh += (double)hh + (double)hl;
+            J.mesh[idx] = __fadd_rn(nh, nl);
+            if (!P.density_only) {
+                J.mesh[nmesh + idx] = __fadd_rn(hh, hl);
+                J.mesh[2 * nmesh + idx] = __fadd_rn(ch, cl);
+                J.mesh[3 * nmesh + 3 * idx] = vx;
+                J.mesh[3 * nmesh + 3 * idx + 1] = vy;
+                J.mesh[3 * nmesh + 3 * idx + 2] = vz;
+            }
         }
-        const int lz = e / (TS * TS), c = e % (TS * TS);
-        const int lx = c % TS, ly = c / TS;
-        if (lx >= g.E[0] || ly >= g.E[1] || lz >= g.E[2]) continue;
-        const size_t idx = ((size_t)(g.O[2] + lz) * nc + (g.O[1] + ly)) * nc + (g.O[0] + lx);
-        sn += (double)nh + (double)nl;
-        sh += (double)hh + (double)hl;
-        J.mesh[idx] = __fadd_rn(nh, nl);
-        if (!P.density_only) {
-            J.mesh[nmesh + idx] = __fadd_rn(hh, hl);
-            J.mesh[2 * nmesh + idx] = __fadd_rn(ch, cl);
-            J.mesh[3 * nmesh + 3 * idx] = vx;
-            J.mesh[3 * nmesh + 3 * idx + 1] = vy;
-            J.mesh[3 * nmesh + 3 * idx + 2] = vz;
-        }
-    }
-    if (item_tot) {
-        if (tid == 0) {
+        if (!item_tot) {
+            block_totals(sn, sh, red, J, g.local, tid);
+            __syncthreads();  // red is written again
+        } else if (tid == 0) {
             double a = 0.0, b = 0.0;
             for (int it = i0; it < i1; ++it) {
-                a += item_tot[2 * it];
-                b += item_tot[2 * it + 1];
+                a += item_tot[2 * (size_t)it];
+                b += item_tot[2 * (size_t)it + 1];
             }
-            J.partial[2 * g.local] = a;
-            J.partial[2 * g.local + 1] = b;
+            J.partial[2 * (size_t)g.local] = a;
+            J.partial[2 * (size_t)g.local + 1] = b;
         }
-        return;
     }
-    block_totals(sn, sh, red, J, g.local, tid);
 }
 
 // ---------------------------------------------------------------------------
@@ -1244,49 +1180,38 @@ k_merge_tiles(DepositParams P, int total_tiles, const uint32_t* __restrict__ ite
 // ---------------------------------------------------------------------------
 size_t deposit_prep_bytes(int n) { return 32 * (size_t)n; }
 
-// bits 0-10 of v spread to every third bit
-static uint64_t spread3_11(uint32_t v)
+void deposit_tile_shape(DepositParams& p)
 {
-    uint64_t r = 0;
-    for (int b = 0; b < 11; ++b) r |= (uint64_t)((v >> b) & 1u) << (3 * b);
-    return r;
-}
-
-void deposit_tile_order(const DepositParams& p, int total_tiles, uint32_t* out)
-{
-    int ncmax = 1;
-    for (int k = 0; k < p.n_jobs; ++k) ncmax = std::max(ncmax, p.job[k].nc);
-    std::vector<std::pair<uint64_t, uint32_t>> key((size_t)total_tiles);
-    for (int k = 0; k < p.n_jobs; ++k) {
-        const MeshJob& J = p.job[k];
-        int rank = 0;  // coarser meshes first at the same place
-        for (int j = 0; j < p.n_jobs; ++j)
-            rank += p.job[j].nc < J.nc || (p.job[j].nc == J.nc && j < k);
-        // a tile's lower corner, in tiles of the finest mesh (plus half of one)
-        const double ratio = (double)ncmax / (double)J.nc;
-        const int nt = J.tiles[0] * J.tiles[1] * J.tiles[2];
-        for (int t = 0; t < nt; ++t) {
-            const int c[3] = {t % J.tiles[0], (t / J.tiles[0]) % J.tiles[1],
-                              t / (J.tiles[0] * J.tiles[1])};
-            uint64_t m = 0;
-            for (int a = 0; a < 3; ++a)
-                m |= spread3_11(std::min(2047u, (uint32_t)(c[a] * ratio + 0.5))) << a;
-            key[(size_t)(J.tile_begin + t)] = {(m << 4) | (uint64_t)rank,
-                                               (uint32_t)(J.tile_begin + t)};
-        }
-    }
-    std::sort(key.begin(), key.end());
-    for (int slot = 0; slot < total_tiles; ++slot) {
-        out[slot] = key[(size_t)slot].second;
-        out[(size_t)total_tiles + key[(size_t)slot].second] = (uint32_t)slot;
-    }
+    p.shift[0] = 3;
+    p.shift[1] = p.shift[2] = p.mma && !p.density_only ? 2 : 3;
 }
 
 size_t deposit_tile_bytes(int total_tiles)
 {
-    // tstart, tcount, item_off (+1 each) and their scan scratch
+    // tentry, item_off, merge (+1 each) and their scan scratch
     const size_t T1 = (size_t)total_tiles + 1;
     return 4 * T1 * 3 + scan_temp_bytes(T1) + 256;
+}
+
+// keys and values of the sort (ping-pong), entries as emitted and in key order, and
+// the first pair of each with its scan scratch
+size_t deposit_entry_bytes(uint32_t entries)
+{
+    const size_t E = (size_t)entries + 2;
+    return (4 + 4 + 8) * 2 * E + 4 * E + scan_temp_bytes(E) + 256;
+}
+
+void deposit_entry_layout(void* base, uint32_t entries, DepositScratch& w)
+{
+    const size_t E = ((size_t)entries + 2) & ~size_t(1);  // entry and list stay 8-byte aligned
+    w.entry = static_cast<uint2*>(base);
+    w.list = w.entry + E;
+    w.keys0 = reinterpret_cast<uint32_t*>(w.list + E);
+    w.keys1 = w.keys0 + E;
+    w.vals0 = reinterpret_cast<int*>(w.keys1 + E);
+    w.vals1 = w.vals0 + E;
+    w.first = reinterpret_cast<uint32_t*>(w.vals1 + E);
+    w.scan_tmp_e = w.first + E;
 }
 
 static int key_bits(int total_tiles, int ib)
@@ -1296,24 +1221,22 @@ static int key_bits(int total_tiles, int ib)
     return b + ib;
 }
 
-// the default deposit engine: 2 the tensor cores with the two warps of a CTA
-// per item, 1 with one warp per item, 0 the CUDA cores; ASG_DEPOSIT=mma2, mma
-// or simt selects one (a comparison knob; a context's tuner may choose)
+// the default deposit engine: 1 the tensor cores, 0 the CUDA cores
+// (ASG_DEPOSIT=simt, a comparison knob; a context's tuner may choose)
 int deposit_default_mma()
 {
     static const int m = [] {
         const char* e = std::getenv("ASG_DEPOSIT");
-        if (e && std::strcmp(e, "simt") == 0) return 0;
-        if (e && std::strcmp(e, "mma") == 0) return 1;
-        return 2;  // 15.3 against 15.6 ms (one warp per item) on the 256^3 step
+        return e && std::strcmp(e, "simt") == 0 ? 0 : 1;
     }();
     return m;
 }
 
 // per-item FP64 masses after the partial tiles of deposit_max_items items
-static double* deposit_item_totals(float* partial, uint32_t items)
+static double* deposit_item_totals(float* partial, uint32_t items, const DepositParams& p)
 {
-    const size_t off = ((size_t)items * TC * PW * sizeof(float) + 15) & ~size_t(15);
+    const size_t cells = (size_t)1 << (p.shift[0] + p.shift[1] + p.shift[2]);
+    const size_t off = ((size_t)items * cells * PW * sizeof(float) + 15) & ~size_t(15);
     return reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(partial) + off);
 }
 
@@ -1339,114 +1262,132 @@ void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, 
                          int n, const DepositParams& p, DepositScratch& w, int* err,
                          cudaStream_t s)
 {
-    const int nb = (n + 255) / 256;
-    k_dep_prep<<<nb, 256, 0, s>>>(pos, vel, igrp, rk, n, p, w.rec, err);
-    k_pairs<false><<<nb, 256, 0, s>>>(w.rec, n, p, w.pcount, nullptr, nullptr, nullptr, 0u, err);
-    cudaMemsetAsync(w.pcount + n, 0, 4, s);
-    exclusive_scan_u32(w.pcount, (size_t)n + 1, w.scan_tmp_n, s);
-    count_launches(2);
+    const int bundles = (n + 31) / 32;
+    cudaMemsetAsync(w.counters, 0, 16, s);
+    k_dep_prep<<<(bundles + 7) / 8, 256, 0, s>>>(pos, vel, igrp, rk, n, p, w.rec, w.count,
+                                                 reinterpret_cast<unsigned long long*>(w.counters + 2),
+                                                 err);
+    exclusive_scan_u32(w.count, (size_t)bundles + 1, w.scan_tmp_n, s);
+    count_launches(1);
 }
 
-void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t npairs, bool padded,
-                        DepositScratch& w, int* err, cudaStream_t s)
+void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t entries,
+                        uint32_t max_items, bool padded, DepositScratch& w, int* err, cudaStream_t s)
 {
-    const int T = total_tiles;
-    const int nb = (n + 255) / 256;
-    k_pairs<true><<<nb, 256, 0, s>>>(w.rec, n, p, nullptr, w.pcount, w.keys0, w.vals0, npairs, err);
+    const int T = total_tiles, bundles = (n + 31) / 32;
+    k_entries<<<(bundles + 7) / 8, 256, 0, s>>>(w.rec, n, p, w.count, w.keys0, w.entry, entries, err);
     count_launches(1);
-    if (padded && npairs > 0) {  // npairs is the capacity; the count itself is pcount[n]
-        k_pad_pairs<<<(npairs + 255) / 256, 256, 0, s>>>(w.keys0, w.vals0, w.pcount + n, npairs,
-                                                          (uint32_t)T << img_bits(p));
+    if (padded && entries > 0) {  // `entries` is the capacity; the count itself is count[bundles]
+        k_pad_entries<<<(entries + 255) / 256, 256, 0, s>>>(w.keys0, w.entry, w.count + bundles, entries,
+                                                            (uint32_t)T << img_bits(p));
         count_launches(1);
     }
-    const int cur = radix_sort32(w.keys0, w.vals0, w.keys1, w.vals1, (int)npairs,
-                                 key_bits(padded ? T + 1 : T, img_bits(p)), w.sort_tmp, s);
+    const int cur = radix_sort32(w.keys0, w.vals0, w.keys1, w.vals1, (int)entries,
+                                 key_bits(padded ? T + 1 : T, img_bits(p)), true, w.sort_tmp, err, s);
     const uint32_t* keys = cur ? w.keys1 : w.keys0;
-    const int* vals = cur ? w.vals1 : w.vals0;
-    cudaMemsetAsync(w.tstart, 0, 4 * (size_t)T, s);
-    cudaMemsetAsync(w.tcount, 0, 4 * (size_t)T, s);
-    if (npairs > 0) {
-        k_tile_bounds<<<(npairs + 255) / 256, 256, 0, s>>>(keys, (int)npairs, T, img_bits(p), w.tstart,
-                                                           w.tcount);
-        count_launches(1);
-    }
-    k_tile_items<<<(T + 1 + 255) / 256, 256, 0, s>>>(w.tstart, w.tcount, T, p.seg, p.pos, w.item_off);
+    k_sorted_entries<<<entries / 256 + 1, 256, 0, s>>>(cur ? w.vals1 : w.vals0, w.entry, entries, w.list,
+                                                       w.first, err);
+    exclusive_scan_u32(w.first, (size_t)entries + 1, w.scan_tmp_e, s);
+    k_tile_items<<<T / 256 + 1, 256, 0, s>>>(keys, entries, w.first, T, img_bits(p), p.seg, w.tentry,
+                                             w.item_off);
     exclusive_scan_u32(w.item_off, (size_t)T + 1, w.scan_tmp_t, s);
-    cudaMemsetAsync(w.next_item, 0, sizeof(int), s);
+    k_item_list<<<(T + 255) / 256, 256, 0, s>>>(w.item_off, T, max_items, w.item_tile, w.merge,
+                                                w.counters, err);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     double* item_tot = nullptr;
-    if (p.mma == 2) {
-        item_tot = deposit_item_totals(w.partial, deposit_max_items(T, npairs, p.seg));
+    if (p.mma) {
+        item_tot = deposit_item_totals(w.partial, max_items, p);
         if (p.density_only)
-            launch_persistent(k_deposit_mma2<1>, dev, sms, 64, sizeof(Mma2Cta<1>), s, w.rec, p, T,
-                              w.item_off, w.tstart, w.tcount, keys, vals, w.partial, item_tot,
-                              w.next_item);
+            launch_persistent(k_deposit_mma<1>, dev, sms, 32, sizeof(MmaWarp<1>), s, w.rec, p, T,
+                              w.item_off, max_items, w.item_tile, w.tentry, keys, w.list, w.first,
+                              w.partial, item_tot, w.counters);
         else
-            launch_persistent(k_deposit_mma2<6>, dev, sms, 64, sizeof(Mma2Cta<6>), s, w.rec, p, T,
-                              w.item_off, w.tstart, w.tcount, keys, vals, w.partial, item_tot,
-                              w.next_item);
-    } else if (p.mma) {
-        item_tot = deposit_item_totals(w.partial, deposit_max_items(T, npairs, p.seg));
-        if (p.density_only)
-            launch_persistent(k_deposit_mma<1>, dev, sms, 32 * MMA_WARPS,
-                              MMA_WARPS * sizeof(MmaWarp<1>), s, w.rec, p, T, w.item_off, w.tstart,
-                              w.tcount, keys, vals, w.partial, item_tot, w.next_item);
-        else
-            launch_persistent(k_deposit_mma<6>, dev, sms, 32 * MMA_WARPS,
-                              MMA_WARPS * sizeof(MmaWarp<6>), s, w.rec, p, T, w.item_off, w.tstart,
-                              w.tcount, keys, vals, w.partial, item_tot, w.next_item);
+            launch_persistent(k_deposit_mma<6>, dev, sms, 32, sizeof(MmaWarp<6>), s, w.rec, p, T,
+                              w.item_off, max_items, w.item_tile, w.tentry, keys, w.list, w.first,
+                              w.partial, item_tot, w.counters);
     } else {
         launch_persistent(k_deposit_items, dev, sms, 32 * DEP_WARPS, DEP_WARPS * sizeof(WarpTile), s,
-                          w.rec, p, T, w.item_off, w.tstart, w.tcount, keys, vals, w.partial,
-                          w.next_item);
+                          w.rec, p, T, w.item_off, max_items, w.item_tile, w.tentry, keys, w.list,
+                          w.first, w.partial, w.counters);
     }
-    k_merge_tiles<<<T, DEP_THREADS, 0, s>>>(p, T, w.item_off, w.partial, item_tot);
-    count_launches(3);
+    k_merge_tiles<<<std::min(T, 8 * sms), DEP_THREADS, 0, s>>>(p, w.item_off, w.merge, w.counters,
+                                                               w.partial, item_tot);
+    count_launches(5);
 }
 
 uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int seg)
 {
-    return (uint32_t)total_tiles + npairs / (uint32_t)(seg > 0 ? seg : SEG_DEFAULT) + 1;
+    return (uint32_t)total_tiles + npairs / (uint32_t)seg + 1;
 }
 
-int deposit_default_seg() { return SEG_DEFAULT; }
+// An item is a serial chain for its warp, so a small set takes short items and
+// all warps: a quarter of the pairs a warp would get if the items were dealt out
+// evenly (about 2 n per mesh over 24 warps on 152 SMs), in steps of the 64 pairs
+// between two flushes.  One item length of 4096 pairs left a set of 13,840
+// particles to 20 warps: 354 us against 18.
+int deposit_seg(int n, int n_nc, int most)
+{
+    const long long fair = 2LL * n * n_nc / (4 * 24 * 152);
+    const long long seg = (fair + 63) / 64 * 64;
+    return (int)std::max(64LL, std::min(seg, (long long)most));
+}
 
 // partial tiles of multi-item tiles, then each item's FP64 mass (2 doubles)
-size_t deposit_partial_bytes(uint32_t items)
+size_t deposit_partial_bytes(uint32_t items, int cells)
 {
-    return (((size_t)items * TC * PW * sizeof(float) + 15) & ~size_t(15)) + 16 * (size_t)items;
+    return (((size_t)items * cells * PW * sizeof(float) + 15) & ~size_t(15)) +
+           16 * (size_t)items;
 }
 
-__global__ void k_reduce_partials(const double* __restrict__ partial, int ntiles, double* out2)
+// FP64 totals of every mesh from its tiles' partial sums: block (b, mesh) adds a
+// fixed slice of the tiles; with one block per mesh into out, else into scratch
+// for the second launch (one block per mesh over the REDUCE_BLOCKS sums), which
+// takes 12 us for the 150 k tiles of the 256^3 step (one block per mesh: 85 us for
+// a quarter as many).
+constexpr int REDUCE_BLOCKS = 64, REDUCE_MIN = 8192;
+__global__ void __launch_bounds__(256)
+k_reduce_partials(const __grid_constant__ DepositParams P, const double* __restrict__ in,
+                  double* __restrict__ out)
 {
     __shared__ double r[2][256];
+    const int k = blockIdx.y, B = gridDim.x;
+    const MeshJob& J = P.job[k];
+    const double* src = in ? in + 2 * (size_t)k * REDUCE_BLOCKS : J.partial;
+    const int count = in ? REDUCE_BLOCKS : J.tiles[0] * J.tiles[1] * J.tiles[2];
     double a = 0.0, b = 0.0;
-    for (int i = threadIdx.x; i < ntiles; i += blockDim.x) {
-        a += partial[2 * i];
-        b += partial[2 * i + 1];
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < count; i += B * 256) {
+        a += src[2 * (size_t)i];
+        b += src[2 * (size_t)i + 1];
     }
     r[0][threadIdx.x] = a;
     r[1][threadIdx.x] = b;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+    for (int o = 128; o > 0; o >>= 1) {
         if ((int)threadIdx.x < o) {
             r[0][threadIdx.x] += r[0][threadIdx.x + o];
             r[1][threadIdx.x] += r[1][threadIdx.x + o];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        out2[0] = r[0][0];
-        out2[1] = r[1][0];
-    }
+    if (threadIdx.x < 2) out[2 * ((size_t)k * B + blockIdx.x) + threadIdx.x] = r[threadIdx.x][0];
 }
 
-void launch_reduce_partials(const double* partial, int ntiles, double* out2, cudaStream_t s)
+size_t deposit_totals_bytes(int n_nc) { return 16 * (size_t)n_nc * (1 + REDUCE_BLOCKS); }
+
+void launch_deposit_totals(const DepositParams& p, int total_tiles, double* totals, cudaStream_t s)
 {
-    k_reduce_partials<<<1, 256, 0, s>>>(partial, ntiles, out2);
-    count_launches(1);
+    const unsigned k = (unsigned)p.n_jobs;
+    if (total_tiles <= REDUCE_MIN) {
+        k_reduce_partials<<<dim3(1, k), 256, 0, s>>>(p, nullptr, totals);
+        count_launches(1);
+        return;
+    }
+    double* part = totals + 2 * p.n_jobs;
+    k_reduce_partials<<<dim3(REDUCE_BLOCKS, k), 256, 0, s>>>(p, nullptr, part);
+    k_reduce_partials<<<dim3(1, k), 256, 0, s>>>(p, part, totals);
+    count_launches(2);
 }
 
 // write_mesh_separate normalisation (coarse_mesh.cpp:158-171), in place

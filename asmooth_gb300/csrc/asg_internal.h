@@ -49,15 +49,16 @@ void launch_unpack_quant(const int* cell, const uint16_t* off, const float* v, i
 // over [left, right)^3, or over the particles' own bounding cube when d_lohi
 // (2 ints of scratch) is given; key_prefix lands in bits 48+ (batched cubes)
 void launch_space_keys(const float4* pos_in, int n, float left, float right, int* d_lohi,
-                       uint64_t key_prefix, uint64_t* keys, int* vals, cudaStream_t s);
-// stable LSD radix sort of (keys, vals) on the low `bits` bits; ping-pong buffers;
-// returns which buffer (0/1) holds the result
+                       uint64_t key_prefix, uint64_t* keys, cudaStream_t s);
+// stable LSD radix sort of (keys, vals) on the low `bits` bits; iota: vals0 is not
+// read, the values are the input positions; ping-pong buffers; returns which
+// buffer (0/1) holds the result.  err |= ERR_SORT if a tile's look-back gives up.
 size_t radix_sort_temp_bytes(int n);
-int radix_sort32(uint32_t* keys0, int* vals0, uint32_t* keys1, int* vals1, int n, int bits,
-                 void* temp, cudaStream_t s);
-int radix_sort(uint64_t* keys0, int* vals0, uint64_t* keys1, int* vals1, int n, int bits,
-               void* temp, cudaStream_t s);
-void launch_gather_sorted(const int* perm, const float4* pos_in, const float4* vel_in,
+int radix_sort32(uint32_t* keys0, int* vals0, uint32_t* keys1, int* vals1, int n, int bits, bool iota,
+                 void* temp, int* err, cudaStream_t s);
+int radix_sort(uint64_t* keys0, int* vals0, uint64_t* keys1, int* vals1, int n, int bits, bool iota,
+               void* temp, int* err, cudaStream_t s);
+void launch_gather_sorted(int* perm, const float4* pos_in, const float4* vel_in,
                           const int* igrp_in, const float* rk_in, int n, float4* pos, float4* vel,
                           int* igrp, float* rk, cudaStream_t s);
 void launch_iota(int* a, int n, cudaStream_t s);
@@ -94,7 +95,7 @@ struct MeshJob {
     int nc;           // cells per dimension
     float dx;         // boxsize / nc (host float division, as the reference)
     float ncf;        // (float)nc
-    int tiles[3];     // tiles per dimension
+    int tiles[3];     // tiles per dimension (x, y, z)
     int tile_begin;   // first global tile id of this mesh
     float* mesh;      // 6*nc^3 floats (reference layout) or nc^3 (density only)
     double* partial;  // per-tile FP64 partial sums, 2 per tile (n, halo)
@@ -110,53 +111,60 @@ struct DepositParams {
     float offset[3];  // periodic: rank cube offset
     int density_only;
     int seg;          // pairs per work item of the persistent deposit (tuning, > 0)
-    int mma;          // the deposit engine: 1 or 2 tensor cores (one or two warps per
-                      // item), 0 the CUDA cores (tuning)
-    // the order in which the persistent deposit takes the tiles (slot -> tile)
-    // and its inverse (tile -> slot), or null for tile order: tiles of every
-    // mesh sorted by position along a Morton curve, coarse before fine at the
-    // same place, so that the tiles of all meshes that read the same particle
-    // records run close together in time and find them in L2
-    const uint32_t* order;
-    const uint32_t* pos;
+    int mma;          // the deposit engine: 1 the tensor cores, 0 the CUDA cores
+    int shift[3];     // log2 of the tile edges in cells (deposit_tile_shape)
 };
-// the processing order above for the meshes of p (host; 2 * total tiles words:
-// order, then pos)
-void deposit_tile_order(const DepositParams& p, int total_tiles, uint32_t* out);
-// scratch of one deposit: particle records, (tile, image) pairs, work items
+// the tile shape of the engine p.mma
+void deposit_tile_shape(DepositParams& p);
+// scratch of one deposit: particle records, entries (a bundle of 32 particles and
+// those of them that touch a tile), work items
 struct DepositScratch {
     float4* rec;          // [2n] x', y', z', h (-h: halo channel, 0: skipped) | dens, v
-    uint32_t* pcount;     // [n+1] pairs per particle, then their exclusive scan
-    void* scan_tmp_n;     // scan scratch for n+1 entries
-    uint32_t* keys0;      // [npairs] tile << 5 | image (periodic), else tile; ping-pong with keys1
+    uint32_t* count;      // [bundles+1] entries per bundle, then their exclusive scan
+    void* scan_tmp_n;     // scan scratch for bundles+1 entries
+    uint2* entry;         // [entries] bundle, lane mask, as emitted
+    uint2* list;          // [entries] the same in key order
+    uint32_t* keys0;      // [entries] tile << 5 | image (periodic), else tile; ping-pong with keys1
     uint32_t* keys1;
-    int* vals0;           // [npairs] particle (sorted position), ping-pong with vals1
+    int* vals0;           // [entries] emission number, ping-pong with vals1
     int* vals1;
-    void* sort_tmp;       // radix sort scratch for npairs
-    uint32_t* tstart;     // [T] first pair of each tile
-    uint32_t* tcount;     // [T] pairs of each tile
+    uint32_t* first;      // [entries+1] first pair of each sorted entry
+    void* scan_tmp_e;     // scan scratch for entries+1
+    void* sort_tmp;       // radix sort scratch for the entries
+    uint32_t* tentry;     // [T+1] first entry of each tile
     uint32_t* item_off;   // [T+1] exclusive scan of work items per tile
+    uint32_t* merge;      // [T] tiles with several items
+    uint32_t* item_tile;  // [items] tile of each work item
     void* scan_tmp_t;     // scan scratch for T+1 entries
     float* partial;       // [items] partial tiles of multi-segment tiles
-    int* next_item;       // work counter of the persistent kernel
+    int* counters;        // work counter of the persistent kernel, length of merge, then
+                          // the number of pairs (64 bits)
 };
 size_t deposit_prep_bytes(int n);
 size_t deposit_tile_bytes(int total_tiles);
+size_t deposit_entry_bytes(uint32_t entries);
+// the per-entry arrays of w inside one block of deposit_entry_bytes
+void deposit_entry_layout(void* base, uint32_t entries, DepositScratch& w);
 uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int seg);
-int deposit_default_seg();
+// pairs per work item for n particles on n_nc meshes, at most `most`
+int deposit_seg(int n, int n_nc, int most);
 int deposit_default_mma();
-size_t deposit_partial_bytes(uint32_t items);
-// pass 1: particle records and pair counts; pcount[n] then holds the number of pairs
+size_t deposit_partial_bytes(uint32_t items, int cells);  // of tiles of that many cells
+// pass 1: particle records and entry counts; count[bundles] then holds the number
+// of entries, counters[2..3] the number of pairs
 void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, const float* rk,
                          int n, const DepositParams& p, DepositScratch& w, int* err,
                          cudaStream_t s);
-// pass 2: emit and sort the pairs, deposit every (tile, segment), merge multi-segment tiles.
-// padded = false: npairs is the exact pair count (read back from pcount[n]);
-// padded = true: npairs is the arrays' capacity, the count stays on the device
-// (no host synchronisation, e.g. under stream capture) and a larger count sets ERR_CAP
-void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t npairs, bool padded,
-                        DepositScratch& w, int* err, cudaStream_t s);
-void launch_reduce_partials(const double* partial, int ntiles, double* out2, cudaStream_t s);
+// pass 2: emit and sort the entries, deposit every (tile, segment), merge multi-segment tiles.
+// padded = false: `entries` is the exact number (read back from count[bundles]);
+// padded = true: it is the arrays' capacity, the number stays on the device
+// (no host synchronisation, e.g. under stream capture) and a larger one sets ERR_CAP,
+// as do more than max_items work items
+void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t entries,
+                        uint32_t max_items, bool padded, DepositScratch& w, int* err, cudaStream_t s);
+// totals: 2 doubles per mesh (n, halo), then scratch: deposit_totals_bytes
+size_t deposit_totals_bytes(int n_nc);
+void launch_deposit_totals(const DepositParams& p, int total_tiles, double* totals, cudaStream_t s);
 void launch_normalise(float* mesh, int nc, float vol, cudaStream_t s);
 
 // ---- FOF and SO halos (asg_fof.cu) -----------------------------------------------
@@ -180,7 +188,7 @@ struct ShellPlan {
 };
 void launch_shell_bins(const float4* pos, int n, float lt, float rt, uint32_t* keys0, int* vals0,
                        uint32_t* keys1, int* vals1, void* sort_tmp, uint32_t* start, uint32_t* end,
-                       const uint32_t** keys, const int** order, cudaStream_t s);
+                       const uint32_t** keys, const int** order, int* err, cudaStream_t s);
 void launch_shell_emit(const float4* pos, const float4* vel, const int* igrp, const float* rk,
                        const uint32_t* keys, const int* order, const uint32_t* start, int n,
                        const ShellPlan& plan, float L, float4* apos, float4* avel, int* aigrp,
@@ -208,7 +216,7 @@ void launch_zip_particles(const uint8_t* off, const int16_t* vq, const uint32_t*
 size_t fof_catalogue_bytes(int n, int nhalo);
 void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp, int n, int w_index,
                           int nhalo, float boxsize, void* scratch, float* out, uint32_t* nlocal,
-                          cudaStream_t s);
+                          int* err, cudaStream_t s);
 int write_mesh_files(const char* base, int inode, const float* mesh, int nc);
 int write_fof_file(const char* filename, const float* rec, int nlocal);
 

@@ -34,9 +34,9 @@
 namespace asg {
 
 constexpr int KNN_WARPS = 4;
-// k_dens_scatter: one warp per block and four queries per turn of its loop, 6.42
-// ms on the 256^3 step (4 warps and two queries 6.57)
-constexpr int DENS_WARPS = 1, DENS_UNROLL = 4;
+// k_dens_scatter: four warps per block and four queries per turn of its loop, 6.47
+// ms on the 256^3 step (two queries 6.57, one warp per block 6.81)
+constexpr int DENS_WARPS = 4, DENS_UNROLL = 4;
 // k_knn_t33 runs 32 warps per SM at 64 registers, in blocks of 1 warp with the
 // default leaf size and of 2 or 4 with others (the batched form's autotuner
 // picks).
@@ -453,7 +453,7 @@ __global__ void k_dens_prep(const float* __restrict__ rk, int n, int* __restrict
 // receivers and take every second query, so no lane idles; their integer sums
 // are added by a shuffle before the atomic.
 // Bound by instruction issue (82% of slots busy, 11.3 K warp instructions per
-// bundle, of which the distances and weights are half): 7.10 -> 6.42 ms on the
+// bundle, of which the distances and weights are half): 7.10 -> 6.47 ms on the
 // 256^3 step against radix-tree buckets of 22 particles on average.
 template <bool HALVES>
 __global__ void __launch_bounds__(DENS_WARPS * 32)

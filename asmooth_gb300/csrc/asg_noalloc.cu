@@ -128,6 +128,7 @@ static int noalloc_status(int bits)
     if (bits & ERR_FEW) return ASG_ERR_FEW;
     if (bits & ERR_ZERO_RK) return ASG_ERR_ZERO_RK;
     if (bits & ERR_TIES) return ASG_ERR_TIES;
+    if (bits & ERR_SORT) return ASG_ERR_CUDA;
     return ASG_OK;
 }
 
@@ -180,11 +181,11 @@ extern "C" int asg_neighbor_search_noalloc(const float* d_x, int np, float left,
     launch_unpack_soa(d_x, nullptr, d_dens, nullptr, np, F4(L.pos_in), F4(L.vel_in), I(L.igrp_in),
                       F(L.rk_in), err, s);
     launch_space_keys(F4(L.pos_in), np, left, right, nullptr, 0,
-                  reinterpret_cast<uint64_t*>(b + L.keys0), I(L.vals0), s);
+                  reinterpret_cast<uint64_t*>(b + L.keys0), s);
     const int cur = radix_sort(reinterpret_cast<uint64_t*>(b + L.keys0), I(L.vals0),
                                reinterpret_cast<uint64_t*>(b + L.keys1), I(L.vals1), np, 48,
-                               b + L.sort_tmp, s);
-    const int* perm = I(cur ? L.vals1 : L.vals0);
+                               true, b + L.sort_tmp, err, s);
+    int* perm = I(cur ? L.vals1 : L.vals0);
     launch_gather_sorted(perm, F4(L.pos_in), F4(L.vel_in), I(L.igrp_in), F(L.rk_in), np, F4(L.pos),
                          F4(L.vel), I(L.igrp), F(L.rk), s);
     TreeView t = tree_shape(np, LEAF_DEFAULT);

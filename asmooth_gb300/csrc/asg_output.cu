@@ -65,11 +65,12 @@ __global__ void k_cat_keys(const float4* __restrict__ pos, const int* __restrict
     vals[i] = j;
 }
 
+// (no members when the sort gave up)
 __global__ void k_cat_bounds(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ start,
-                             uint32_t* __restrict__ end)
+                             uint32_t* __restrict__ end, const int* __restrict__ err)
 {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= n) return;
+    if (m >= n || (*err & ERR_SORT)) return;
     const uint32_t lab = keys[m];
     if (lab == 0) return;
     if (m == 0 || keys[m - 1] != lab) start[lab] = (uint32_t)m;
@@ -191,7 +192,7 @@ __global__ void k_cat_compact(const float* __restrict__ rec, const uint32_t* __r
 
 void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp, int n, int w_index,
                           int nhalo, float boxsize, void* scratch, float* out, uint32_t* nlocal,
-                          cudaStream_t s)
+                          int* err, cudaStream_t s)
 {
     const CatLayout L = cat_layout(n, nhalo);
     unsigned char* b = static_cast<unsigned char*>(scratch);
@@ -207,10 +208,10 @@ void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp,
         int bits = 0;
         while (bits < 31 && (nhalo >> bits) != 0) ++bits;
         const int cur = radix_sort32(U(L.keys0), I(L.vals0), U(L.keys1), I(L.vals1), n, bits,
-                                     b + L.sort_tmp, s);
+                                     false, b + L.sort_tmp, err, s);
         const uint32_t* keys = U(cur ? L.keys1 : L.keys0);
         const int* order = I(cur ? L.vals1 : L.vals0);
-        k_cat_bounds<<<(n + 255) / 256, 256, 0, s>>>(keys, n, U(L.start), U(L.end));
+        k_cat_bounds<<<(n + 255) / 256, 256, 0, s>>>(keys, n, U(L.start), U(L.end), err);
         count_launches(2);
         if (nhalo > 0) {
             const int nbig = nhalo < 8192 ? nhalo : 8192, per = CAT_THREADS / 32;

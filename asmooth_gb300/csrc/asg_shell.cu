@@ -19,7 +19,7 @@
 namespace asg {
 
 __global__ void k_shell_bins(const float4* __restrict__ pos, int n, float lt, float rt,
-                             uint32_t* __restrict__ keys, int* __restrict__ vals)
+                             uint32_t* __restrict__ keys)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -28,7 +28,6 @@ __global__ void k_shell_bins(const float4* __restrict__ pos, int n, float lt, fl
     const int by = (p.y >= lt) + (p.y > rt);
     const int bz = (p.z >= lt) + (p.z > rt);
     keys[i] = (uint32_t)(bx + 3 * by + 9 * bz);
-    vals[i] = i;
 }
 
 __global__ void k_shell_bounds(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ start,
@@ -115,12 +114,12 @@ __global__ void k_shell_compact(const float4* __restrict__ apos, const float4* _
 
 void launch_shell_bins(const float4* pos, int n, float lt, float rt, uint32_t* keys0, int* vals0,
                        uint32_t* keys1, int* vals1, void* sort_tmp, uint32_t* start, uint32_t* end,
-                       const uint32_t** keys, const int** order, cudaStream_t s)
+                       const uint32_t** keys, const int** order, int* err, cudaStream_t s)
 {
     cudaMemsetAsync(start, 0, 27 * sizeof(uint32_t), s);
     cudaMemsetAsync(end, 0, 27 * sizeof(uint32_t), s);
-    k_shell_bins<<<(n + 255) / 256, 256, 0, s>>>(pos, n, lt, rt, keys0, vals0);
-    const int cur = radix_sort32(keys0, vals0, keys1, vals1, n, 5, sort_tmp, s);
+    k_shell_bins<<<(n + 255) / 256, 256, 0, s>>>(pos, n, lt, rt, keys0);
+    const int cur = radix_sort32(keys0, vals0, keys1, vals1, n, 5, true, sort_tmp, err, s);
     *keys = cur ? keys1 : keys0;
     *order = cur ? vals1 : vals0;
     k_shell_bounds<<<(n + 255) / 256, 256, 0, s>>>(*keys, n, start, end);

@@ -319,7 +319,7 @@ int asg_batch_set_streams(asg_batch* batch, int streams);
 int asg_batch_tune(asg_batch* batch, int* leaf, int* seg);
 /* The batch's configuration (tuned or default): tree bucket size, deposit
  * work-item length, neighbour-search warps per block and the deposit engine
- * (1 or 2: tensor cores with one or two warps per tile item; 0: CUDA cores).
+ * (1: tensor cores, one warp per work item; 0: CUDA cores).
  * Any pointer may be NULL. */
 int asg_batch_config(asg_batch* batch, int* leaf, int* seg, int* knn_warps, int* deposit_engine);
 int asg_batch_run(asg_batch* batch);
@@ -353,8 +353,9 @@ const char* asg_phase_name(int phase);
 /* Measured FP32 FMA throughput of this GPU (TFLOP/s, 2 flops per FMA) from a
  * register-resident FMA-chain kernel over all SMs: the FP32 roofline ceiling. */
 int asg_measure_fp32_peak(asg_ctx* ctx, double* tflops);
-/* Work statistics of the last deposit: (particle, 8^3-cell tile) pairs
- * deposited, mesh tiles, work items run. */
+/* Work statistics of the last deposit: (particle, mesh tile) pairs deposited,
+ * mesh tiles (8x4x4 cells; 8^3 for density-only meshes and on the CUDA cores),
+ * work items run. */
 int asg_deposit_stats(asg_ctx* ctx, long long* pairs, long long* tiles, long long* items);
 
 /* ---- allocation-free neighbour search -------------------------------------------- */

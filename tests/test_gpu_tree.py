@@ -1,6 +1,7 @@
 """GPU tests of the blocked box tree at the sizes where its shape changes (a
-partial last leaf, one and two boxes above 32, a second level) and for leaf
-sizes on both sides of 16: 33rd keys and FOF groups equal the oracle's exactly,
+partial last leaf, one and two boxes above 32, a second level) and where the
+index sort takes one tile more (multiples of 3072), for leaf sizes on both
+sides of 16: 33rd keys and FOF groups equal the oracle's exactly,
 dens is within 1e-5 of the FP64 sum over the oracle's lists."""
 import os
 
@@ -25,7 +26,7 @@ def points(n, seed):
 
 
 @pytest.mark.parametrize("leaf", ["", "5", "17", "32"])
-@pytest.mark.parametrize("n", [33, 47, 511, 513, 1056, 16385, 17000])
+@pytest.mark.parametrize("n", [33, 47, 511, 513, 1056, 3072, 3073, 16385, 17000])
 def test_tree_shapes(oracle, monkeypatch, leaf, n):
     if leaf:
         monkeypatch.setenv("ASG_LEAF_SIZE", leaf)
