@@ -57,15 +57,14 @@ struct asg_ctx {
     // loaded particle set
     int n = 0;
     float left = 0.f, right = 0.f;
-    bool loaded = false, knn_done = false, rk_checked = false, idx33_all = false;
+    bool loaded = false, knn_done = false, idx33_all = false;
     int leaf = LEAF_DEFAULT;  // particles per tree leaf
-    int dep_seg = 4096;  // pairs per deposit work item, at most (small sets: deposit_seg)
+    int dep_seg = 4096;  // pairs per deposit work item, at most
     int knn_warps = 2;   // warps per block of the neighbour search (2 or 4)
     int dep_mma = deposit_default_mma();  // deposit engine: tensor cores (1) or CUDA cores (0)
     int* perm = nullptr;       // sorted position -> input index
-    uint64_t* keys = nullptr;  // sorted keys
 
-    Buf aos, pos_in, vel_in, igrp_in, rk_in, keys0, keys1, vals0, vals1, sort_tmp;
+    Buf aos, rec_in, rk_in, keys0, keys1, vals0, vals1, sort_tmp;  // rec_in: staged particles
     Buf pos, vel, igrp, rk, t33, idx33;
     Buf boxes;       // boxes of the tree (TreeView::box)
     Buf dacc, dexp;  // dens: fixed-point sums and scale exponents
@@ -78,6 +77,7 @@ struct asg_ctx {
     Buf sh_in, sh_all; // periodic shell: interior input + bin sort, all copies + flags
     Buf dec_raw, dec_scan;  // file payloads on the device, zip count scans
     int dec_n = 0;          // particles of the last decode (in sh_in), 0 = none
+    bool dec_rk = false;    // they have smoothing lengths
     uint32_t dep_npairs = 0, dep_nentries = 0;
     int dep_tiles_n = 0, dep_cells = 0;  // tiles of the last deposit, cells of one
     uint32_t* h_u32 = nullptr;      // pinned, mapped
@@ -233,9 +233,7 @@ int alloc_set(asg_ctx* ctx, int n)
 {
     const size_t N = (size_t)n;
     int r = 0;
-    r |= grow(ctx, ctx->pos_in, 16 * N);
-    r |= grow(ctx, ctx->vel_in, 16 * N);
-    r |= grow(ctx, ctx->igrp_in, 4 * N);
+    r |= grow(ctx, ctx->rec_in, 32 * N);
     r |= grow(ctx, ctx->rk_in, 4 * N);
     r |= grow(ctx, ctx->keys0, 8 * N);
     r |= grow(ctx, ctx->keys1, 8 * N);
@@ -255,22 +253,20 @@ int alloc_set(asg_ctx* ctx, int n)
     return r ? ASG_ERR_NOMEM : 0;
 }
 
-// sort the staged SoA (pos_in/vel_in/igrp_in/rk_in + keys0/vals0) and build the tree
-int build_index(asg_ctx* ctx)
+// put the staged particles (rec_in, keys0, and rk_in when they have smoothing
+// lengths) in key order and build the tree
+int build_index(asg_ctx* ctx, bool with_rk)
 {
     const int n = ctx->n;
     const int cur = radix_sort(P<uint64_t>(ctx->keys0), P<int>(ctx->vals0), P<uint64_t>(ctx->keys1),
                                P<int>(ctx->vals1), n, 48, true, ctx->sort_tmp.p, ctx->d_err, ctx->s);
-    ctx->keys = cur ? P<uint64_t>(ctx->keys1) : P<uint64_t>(ctx->keys0);
     ctx->perm = cur ? P<int>(ctx->vals1) : P<int>(ctx->vals0);
-    launch_gather_sorted(ctx->perm, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
-                         P<int>(ctx->igrp_in), P<float>(ctx->rk_in), n, P<float4>(ctx->pos),
-                         P<float4>(ctx->vel), P<int>(ctx->igrp), P<float>(ctx->rk), ctx->s);
-    launch_tree_boxes(P<float4>(ctx->pos), tree_view(ctx), ctx->s);
+    launch_gather(ctx->perm, P<float4>(ctx->rec_in), with_rk ? P<float>(ctx->rk_in) : nullptr,
+                  tree_view(ctx), P<float4>(ctx->pos), P<float4>(ctx->vel), P<int>(ctx->igrp),
+                  P<float>(ctx->rk), ctx->s);
     phase_end(ctx);
     ctx->loaded = true;
     ctx->knn_done = false;
-    ctx->rk_checked = false;
     return 0;
 }
 
@@ -299,11 +295,9 @@ void load_quant_device(asg_ctx* ctx, const int* d_cell, const uint16_t* d_off, c
     ctx->left = left;
     ctx->right = right;
     phase_begin(ctx, ASG_PH_INDEX);
-    launch_unpack_quant(d_cell, d_off, d_v, np, grid, left, cell_size, P<float4>(ctx->pos_in),
-                        P<float4>(ctx->vel_in), P<int>(ctx->igrp_in), P<float>(ctx->rk_in),
-                        ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0), ctx->s);
-    build_index(ctx);
+    launch_unpack_quant(d_cell, d_off, d_v, np, grid, left, cell_size, P<float4>(ctx->rec_in),
+                        key_grid(left, right), P<uint64_t>(ctx->keys0), ctx->d_err, ctx->s);
+    build_index(ctx, false);
 }
 
 // host mixed-precision arrays -> one staging buffer [cell | off (16-B padded) | v]
@@ -321,17 +315,6 @@ int stage_quant(asg_ctx* ctx, const int* cell, const uint16_t* off, const float*
     *d_cell = reinterpret_cast<const int*>(b);
     *d_off = reinterpret_cast<const uint16_t*>(b + o_off);
     *d_v = v ? reinterpret_cast<const float*>(b + o_v) : nullptr;
-    return 0;
-}
-
-// the smoothing lengths are checked once per neighbour search
-int ensure_rk_checked(asg_ctx* ctx)
-{
-    if (ctx->rk_checked) return 0;
-    phase_begin(ctx, ASG_PH_CHECK);
-    launch_check_rk(P<float>(ctx->rk), ctx->n, ctx->d_err, ctx->s);
-    phase_end(ctx);
-    ctx->rk_checked = true;
     return 0;
 }
 
@@ -469,7 +452,7 @@ void asg_destroy(asg_ctx* ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->s) cudaStreamSynchronize(ctx->s);
-    Buf* bufs[] = {&ctx->aos, &ctx->pos_in, &ctx->vel_in, &ctx->igrp_in, &ctx->rk_in,
+    Buf* bufs[] = {&ctx->aos, &ctx->rec_in, &ctx->rk_in,
                    &ctx->keys0, &ctx->keys1, &ctx->vals0, &ctx->vals1, &ctx->sort_tmp,
                    &ctx->pos, &ctx->vel, &ctx->igrp, &ctx->rk, &ctx->t33, &ctx->idx33,
                    &ctx->boxes, &ctx->dacc, &ctx->dexp, &ctx->blist, &ctx->uf,
@@ -503,8 +486,8 @@ long long asg_kernel_launches(asg_ctx*) { return g_launches.load(); }
 
 // ---- periodic shell of a single-cube run ----------------------------------------------
 
-struct ShellIn {  // interior particles + bin sort scratch inside ctx->sh_in
-    size_t pos, vel, igrp, rk, k0, k1, v0, v1, tmp, start, end, total;
+struct ShellIn {  // interior particles (staged) + bin sort scratch inside ctx->sh_in
+    size_t rec, rk, k0, k1, v0, v1, tmp, start, end, total;
 };
 
 static ShellIn shell_in_layout(int n)
@@ -517,9 +500,7 @@ static ShellIn shell_in_layout(int n)
         o = (o + b + 255) & ~size_t(255);
         return at;
     };
-    L.pos = take(16 * N);
-    L.vel = take(16 * N);
-    L.igrp = take(4 * N);
+    L.rec = take(32 * N);
     L.rk = take(4 * N);
     L.k0 = take(4 * N);
     L.k1 = take(4 * N);
@@ -540,7 +521,8 @@ static int check_shell(asg_ctx* ctx, int np, float boxsize, float bf)
     return 0;
 }
 
-// sh_in holds the interior particles (unpacked); build the shell and load the set
+// sh_in holds the interior particles (staged, with smoothing lengths if dec_rk);
+// build the shell and load the set
 static int load_shell(asg_ctx* ctx, int np, float boxsize, float bf, int* np_with, int* np_local)
 {
     const ShellIn L = shell_in_layout(np);
@@ -551,7 +533,7 @@ static int load_shell(asg_ctx* ctx, int np, float boxsize, float bf, int* np_wit
     const float lt = bf * boxsize, rt = (1.0f - bf) * boxsize;  // exchange_buffer.cpp:23-24
     const uint32_t* keys = nullptr;
     const int* order = nullptr;
-    launch_shell_bins(F4(L.pos), np, lt, rt, U(L.k0), I(L.v0), U(L.k1), I(L.v1), b + L.tmp,
+    launch_shell_bins(F4(L.rec), np, lt, rt, U(L.k0), I(L.v0), U(L.k1), I(L.v1), b + L.tmp,
                       U(L.start), U(L.end), &keys, &order, ctx->d_err, ctx->s);
     uint32_t se[54];
     CK(cudaMemcpyAsync(se, b + L.start, 27 * 4, cudaMemcpyDeviceToHost, ctx->s));
@@ -576,21 +558,22 @@ static int load_shell(asg_ctx* ctx, int np, float boxsize, float bf, int* np_wit
     if (off > (size_t)INT_MAX) return fail(ctx, ASG_ERR_ARG, "shell too large for int indices");
     const int n_all = (int)off;
     const size_t A = (size_t)n_all;
-    const size_t o_vel = 16 * A, o_igrp = 32 * A, o_rk = 36 * A, o_flags = 40 * A;
+    const size_t o_rk = 32 * A, o_flags = 36 * A;
     const size_t o_scan = (o_flags + 4 * (A + 1) + 255) & ~size_t(255);
     if (int r = grow(ctx, ctx->sh_all, o_scan + scan_temp_bytes(A + 1))) return r;
     if (int r = alloc_set(ctx, n_all)) return r;  // the kept set is at most n_all
     unsigned char* a = P<unsigned char>(ctx->sh_all);
-    launch_shell_emit(F4(L.pos), F4(L.vel), I(L.igrp), reinterpret_cast<float*>(b + L.rk), keys,
-                      order, U(L.start), np, plan, boxsize, reinterpret_cast<float4*>(a),
-                      reinterpret_cast<float4*>(a + o_vel), reinterpret_cast<int*>(a + o_igrp),
-                      reinterpret_cast<float*>(a + o_rk), ctx->s);
+    float* rk = ctx->dec_rk ? reinterpret_cast<float*>(b + L.rk) : nullptr;
+    float* ark = rk ? reinterpret_cast<float*>(a + o_rk) : nullptr;
+    launch_shell_emit(F4(L.rec), rk, keys, order, U(L.start), np, plan, boxsize,
+                      reinterpret_cast<float4*>(a), ark, ctx->s);
     const float dx = bf * boxsize;  // clumping_tree_main.cpp:556-558
     uint32_t* flags = reinterpret_cast<uint32_t*>(a + o_flags);
-    launch_shell_filter(reinterpret_cast<float4*>(a), reinterpret_cast<float4*>(a + o_vel),
-                        reinterpret_cast<int*>(a + o_igrp), reinterpret_cast<float*>(a + o_rk),
-                        n_all, -dx, boxsize + dx, flags, a + o_scan, P<float4>(ctx->pos_in),
-                        P<float4>(ctx->vel_in), P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->s);
+    phase_begin(ctx, ASG_PH_INDEX);
+    launch_shell_filter(reinterpret_cast<float4*>(a), ark, n_all, -dx, boxsize + dx, flags, a + o_scan,
+                        P<float4>(ctx->rec_in), rk ? P<float>(ctx->rk_in) : nullptr,
+                        key_grid(-dx, boxsize + dx), P<uint64_t>(ctx->keys0), ctx->s);
+    phase_end(ctx);
     if (int r = read_words(ctx, flags + n_all, flags + np)) return r;
     const int n = (int)ctx->h_u32[0];
     if (np_with) *np_with = n;
@@ -600,9 +583,7 @@ static int load_shell(asg_ctx* ctx, int np, float boxsize, float bf, int* np_wit
     ctx->left = -dx;
     ctx->right = boxsize + dx;
     phase_begin(ctx, ASG_PH_INDEX);
-    launch_space_keys(P<float4>(ctx->pos_in), n, ctx->left, ctx->right, nullptr, 0,
-                  P<uint64_t>(ctx->keys0), ctx->s);
-    build_index(ctx);
+    build_index(ctx, rk != nullptr);
     int r = finish(ctx, "load_periodic_cube");
     if (r) ctx->loaded = false;
     return r;
@@ -625,10 +606,9 @@ int asg_load_particles(asg_ctx* ctx, const asg_particle* p, int np, float left, 
                        ctx->s));
     phase_end(ctx);
     phase_begin(ctx, ASG_PH_INDEX);
-    launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
-                      P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0), ctx->s);
-    build_index(ctx);
+    launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->rec_in), P<float>(ctx->rk_in),
+                      key_grid(left, right), P<uint64_t>(ctx->keys0), ctx->d_err, ctx->s);
+    build_index(ctx, true);
     int r = finish(ctx, "load");
     if (r) ctx->loaded = false;
     return r;
@@ -646,10 +626,9 @@ int asg_load_particles_device(asg_ctx* ctx, const float* d_x, const float* d_v,
     ctx->left = left;
     ctx->right = right;
     phase_begin(ctx, ASG_PH_INDEX);
-    launch_unpack_soa(d_x, d_v, d_dens, d_igrp, np, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
-                      P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0), ctx->s);
-    build_index(ctx);
+    launch_unpack_soa(d_x, d_v, d_dens, d_igrp, np, P<float4>(ctx->rec_in), key_grid(left, right),
+                      P<uint64_t>(ctx->keys0), ctx->d_err, ctx->s);
+    build_index(ctx, false);
     int r = finish(ctx, "load_device");
     if (r) ctx->loaded = false;
     return r;
@@ -702,10 +681,10 @@ int asg_load_periodic_cube(asg_ctx* ctx, const asg_particle* p, int np_local, fl
     CK(cudaMemcpyAsync(ctx->aos.p, p, sizeof(asg_particle) * (size_t)np_local,
                        cudaMemcpyHostToDevice, ctx->s));
     unsigned char* b = P<unsigned char>(ctx->sh_in);
-    launch_unpack_aos(ctx->aos.p, np_local, reinterpret_cast<float4*>(b + L.pos),
-                      reinterpret_cast<float4*>(b + L.vel), reinterpret_cast<int*>(b + L.igrp),
-                      reinterpret_cast<float*>(b + L.rk), ctx->d_err, ctx->s);
+    launch_unpack_aos(ctx->aos.p, np_local, reinterpret_cast<float4*>(b + L.rec),
+                      reinterpret_cast<float*>(b + L.rk), KeyGrid{}, nullptr, ctx->d_err, ctx->s);
     ctx->dec_n = np_local;  // sh_in now holds these interior particles
+    ctx->dec_rk = true;
     return load_shell(ctx, np_local, boxsize, buffer_factor, np_with_buffers, np_local_kept);
 }
 
@@ -720,10 +699,10 @@ int asg_load_periodic_cube_device(asg_ctx* ctx, const float* d_x, const float* d
     const ShellIn L = shell_in_layout(np_local);
     if (int r = grow(ctx, ctx->sh_in, L.total)) return r;
     unsigned char* b = P<unsigned char>(ctx->sh_in);
-    launch_unpack_soa(d_x, d_v, nullptr, nullptr, np_local, reinterpret_cast<float4*>(b + L.pos),
-                      reinterpret_cast<float4*>(b + L.vel), reinterpret_cast<int*>(b + L.igrp),
-                      reinterpret_cast<float*>(b + L.rk), ctx->d_err, ctx->s);
+    launch_unpack_soa(d_x, d_v, nullptr, nullptr, np_local, reinterpret_cast<float4*>(b + L.rec),
+                      KeyGrid{}, nullptr, ctx->d_err, ctx->s);
     ctx->dec_n = np_local;  // sh_in now holds these interior particles
+    ctx->dec_rk = false;
     return load_shell(ctx, np_local, boxsize, buffer_factor, np_with_buffers, np_local_kept);
 }
 
@@ -741,11 +720,11 @@ int asg_decode_xv(asg_ctx* ctx, const float* xv, int np, const float* shift)
     if (int r = grow(ctx, ctx->dec_raw, 24 * (size_t)np)) return r;
     CK(cudaMemcpyAsync(ctx->dec_raw.p, xv, 24 * (size_t)np, cudaMemcpyHostToDevice, ctx->s));
     unsigned char* b = P<unsigned char>(ctx->sh_in);
-    launch_decode_xv(P<float>(ctx->dec_raw), np, shift, reinterpret_cast<float4*>(b + L.pos),
-                     reinterpret_cast<float4*>(b + L.vel), reinterpret_cast<int*>(b + L.igrp),
-                     reinterpret_cast<float*>(b + L.rk), ctx->d_err, ctx->s);
+    launch_decode_xv(P<float>(ctx->dec_raw), np, shift, reinterpret_cast<float4*>(b + L.rec),
+                     ctx->d_err, ctx->s);
     if (int r = finish(ctx, "decode_xv")) return r;
     ctx->dec_n = np;
+    ctx->dec_rk = false;
     return ASG_OK;
 }
 
@@ -783,11 +762,11 @@ int asg_decode_zip(asg_ctx* ctx, const uint8_t* zip0, const int16_t* zip1, const
                                           ", the header says " + std::to_string(np_local));
     unsigned char* b = P<unsigned char>(ctx->sh_in);
     launch_zip_particles(raw + o0, reinterpret_cast<const int16_t*>(raw + o1), start, ncell, nc,
-                         np_local, mesh_scale, v_r2i, shift, reinterpret_cast<float4*>(b + L.pos),
-                         reinterpret_cast<float4*>(b + L.vel), reinterpret_cast<int*>(b + L.igrp),
-                         reinterpret_cast<float*>(b + L.rk), ctx->s);
+                         np_local, mesh_scale, v_r2i, shift, reinterpret_cast<float4*>(b + L.rec),
+                         ctx->s);
     if (int r = finish(ctx, "decode_zip")) return r;
     ctx->dec_n = np_local;
+    ctx->dec_rk = false;
     return ASG_OK;
 }
 
@@ -860,9 +839,8 @@ int asg_copy_decoded(asg_ctx* ctx, asg_particle* out)
     const ShellIn L = shell_in_layout(n);
     if (int r = grow(ctx, ctx->aos, sizeof(asg_particle) * (size_t)n)) return r;
     unsigned char* b = P<unsigned char>(ctx->sh_in);
-    launch_pack_aos(nullptr, reinterpret_cast<float4*>(b + L.pos), reinterpret_cast<float4*>(b + L.vel),
-                    reinterpret_cast<float*>(b + L.rk), nullptr, reinterpret_cast<int*>(b + L.igrp), n,
-                    ctx->aos.p, ctx->s);
+    launch_pack_staged(reinterpret_cast<float4*>(b + L.rec),
+                       ctx->dec_rk ? reinterpret_cast<float*>(b + L.rk) : nullptr, n, ctx->aos.p, ctx->s);
     CK(cudaMemcpyAsync(out, ctx->aos.p, sizeof(asg_particle) * (size_t)n, cudaMemcpyDeviceToHost,
                        ctx->s));
     return finish(ctx, "copy_decoded");
@@ -888,11 +866,10 @@ static int run_knn(asg_ctx* ctx)
     phase_end(ctx);
     phase_begin(ctx, ASG_PH_TIES);  // only bundles with an exact tie at the 33rd distance
     launch_knn_ties(P<float4>(ctx->pos), t, P<float>(ctx->t33), P<int>(ctx->idx33), 0,
+                    P<float>(ctx->rk), P<int>(ctx->dexp), P<unsigned long long>(ctx->dacc),
                     ctx->d_err, ctx->s);
     phase_end(ctx);
     ctx->idx33_all = false;
-    ctx->rk_checked = false;
-    ensure_rk_checked(ctx);
     phase_begin(ctx, ASG_PH_DENS);
     launch_dens(P<float4>(ctx->pos), t, P<float>(ctx->t33), P<int>(ctx->idx33), P<int>(ctx->blist),
                 P<float>(ctx->rk), P<int>(ctx->dexp), P<unsigned long long>(ctx->dacc),
@@ -1043,7 +1020,6 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     if (!(boxsize > 0.0f) || !std::isfinite(boxsize)) return fail(ctx, ASG_ERR_ARG, "boxsize");
     for (int k = 0; k < n_nc; ++k)
         if (ncs[k] <= 0 || ncs[k] > 1290) return fail(ctx, ASG_ERR_ARG, "nc out of range");
-    ensure_rk_checked(ctx);
     if ((int)ctx->meshes.size() < n_nc) ctx->meshes.resize((size_t)n_nc);
     ctx->mesh_boxsize = boxsize;
     DepositParams p;
@@ -1054,7 +1030,7 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     p.sign = sign;
     p.periodic = periodic ? 1 : 0;
     p.density_only = density_only ? 1 : 0;
-    p.seg = deposit_seg(ctx->n, n_nc, ctx->dep_seg);
+    p.seg = ctx->dep_seg;
     p.mma = large_tiles ? 0 : ctx->dep_mma;
     for (int d = 0; d < 3; ++d) p.offset[d] = periodic && coords ? boxsize * (float)coords[d] : 0.0f;
     // the pair keys hold tile << 5 | image in 32 bits: meshes of more tiles than
@@ -1099,7 +1075,7 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     const size_t B1 = ((size_t)n + 31) / 32 + 1;
     if (int r = grow(ctx, ctx->dep_pcount, 4 * B1 + scan_temp_bytes(B1))) return r;
     if (int r = grow(ctx, ctx->dep_tiles, deposit_tile_bytes(tiles))) return r;
-    if (int r = grow(ctx, ctx->dep_counter, 16)) return r;
+    if (int r = grow(ctx, ctx->dep_counter, 32)) return r;
     DepositScratch w;
     w.rec = P<float4>(ctx->dep_rec);
     w.count = P<uint32_t>(ctx->dep_pcount);
@@ -1221,17 +1197,11 @@ int asg_store_particles(asg_ctx* ctx, asg_particle* p)
     if (!ctx->loaded) return fail(ctx, ASG_ERR_STATE, "no particle set loaded");
     CK(cudaSetDevice(ctx->device));
     if (int r = grow(ctx, ctx->aos, sizeof(asg_particle) * (size_t)ctx->n)) return r;
-    launch_pack_aos(ctx->perm, P<float4>(ctx->pos), P<float4>(ctx->vel), P<float>(ctx->rk), nullptr,
+    launch_pack_aos(ctx->perm, P<float4>(ctx->pos), P<float4>(ctx->vel), P<float>(ctx->rk),
                     P<int>(ctx->igrp), ctx->n, ctx->aos.p, ctx->s);
     CK(cudaMemcpyAsync(p, ctx->aos.p, sizeof(asg_particle) * (size_t)ctx->n, cudaMemcpyDeviceToHost,
                        ctx->s));
     return finish(ctx, "store");
-}
-
-__global__ static void k_dens_of(const float4* vel, int n, float* dens)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dens[i] = vel[i].w;
 }
 
 int asg_store_fields_device(asg_ctx* ctx, float* d_rk, float* d_dens, int* d_igrp)
@@ -1239,15 +1209,8 @@ int asg_store_fields_device(asg_ctx* ctx, float* d_rk, float* d_dens, int* d_igr
     if (!ctx) return ASG_ERR_ARG;
     if (!ctx->loaded) return fail(ctx, ASG_ERR_STATE, "no particle set loaded");
     CK(cudaSetDevice(ctx->device));
-    float* dens_s = nullptr;
-    if (d_dens) {  // sorted dens lives in vel.w: stage it in a scratch array
-        if (int r = grow(ctx, ctx->lab_scan, 4 * (size_t)ctx->n)) return r;
-        dens_s = P<float>(ctx->lab_scan);
-        k_dens_of<<<(ctx->n + 255) / 256, 256, 0, ctx->s>>>(P<float4>(ctx->vel), ctx->n, dens_s);
-        count_launches(1);
-    }
-    launch_scatter_fields(ctx->perm, P<float>(ctx->rk), dens_s, P<int>(ctx->igrp), ctx->n, d_rk,
-                          d_dens, d_igrp, ctx->s);
+    launch_scatter_fields(ctx->perm, P<float>(ctx->rk), P<float4>(ctx->vel), P<int>(ctx->igrp), ctx->n,
+                          d_rk, d_dens, d_igrp, ctx->s);
     return finish(ctx, "store_fields");
 }
 
@@ -1261,7 +1224,7 @@ int asg_get_knn(asg_ctx* ctx, float* t33, int* idx33)
     if (int r = grow(ctx, ctx->minin, 4 * n)) return r;
     if (!ctx->idx33_all) {  // the hot path resolves idx33 only where the 33rd value is tied
         launch_knn_ties(P<float4>(ctx->pos), tree_view(ctx), P<float>(ctx->t33),
-                        P<int>(ctx->idx33), 1, ctx->d_err, ctx->s);
+                        P<int>(ctx->idx33), 1, nullptr, nullptr, nullptr, ctx->d_err, ctx->s);
         ctx->idx33_all = true;
     }
     launch_scatter_fields(ctx->perm, P<float>(ctx->t33), nullptr, P<int>(ctx->idx33), ctx->n,
@@ -1299,11 +1262,10 @@ static int load_for_deposit(asg_ctx* ctx, const asg_particle* p, int np)
                        ctx->s));
     phase_end(ctx);
     phase_begin(ctx, ASG_PH_INDEX);
-    launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
-                      P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), np, 0.0f, 0.0f, P<int>(ctx->lohi), 0,
-                  P<uint64_t>(ctx->keys0), ctx->s);
-    build_index(ctx);
+    launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->rec_in), P<float>(ctx->rk_in), KeyGrid{}, nullptr,
+                      ctx->d_err, ctx->s);
+    launch_own_keys(P<float4>(ctx->rec_in), np, P<int>(ctx->lohi), P<uint64_t>(ctx->keys0), ctx->s);
+    build_index(ctx, true);
     int r = finish(ctx, "load");
     if (r) ctx->loaded = false;
     return r;
@@ -1377,9 +1339,10 @@ int asg_mark_halo_particles(asg_ctx* ctx, asg_particle* p, int np, const asg_hal
 
 // ---- outputs ----------------------------------------------------------------------
 
-// FOF catalogue on device arrays indexed by j; records and count back to the host
+// FOF catalogue of sorted arrays or (igrp null) staged records; records and count
+// back to the host
 static int run_catalogue(asg_ctx* ctx, const float4* pos, const float4* vel, const int* igrp, int n,
-                         int w_index, int nhalo, float boxsize, asg_fof_halo* out, int* nlocal)
+                         int nhalo, float boxsize, asg_fof_halo* out, int* nlocal)
 {
     const size_t rec_bytes = sizeof(asg_fof_halo) * (size_t)(nhalo > 0 ? nhalo : 1);
     const size_t o_cnt = (rec_bytes + 15) & ~size_t(15);
@@ -1387,7 +1350,7 @@ static int run_catalogue(asg_ctx* ctx, const float4* pos, const float4* vel, con
     if (int r = grow(ctx, ctx->cat_out, o_cnt + 16)) return r;
     unsigned char* ob = P<unsigned char>(ctx->cat_out);
     CK(cudaMemsetAsync(ob, 0, o_cnt + 16, ctx->s));
-    launch_fof_catalogue(pos, vel, igrp, n, w_index, nhalo, boxsize, ctx->cat.p,
+    launch_fof_catalogue(pos, vel, igrp, n, nhalo, boxsize, ctx->cat.p,
                          reinterpret_cast<float*>(ob), reinterpret_cast<uint32_t*>(ob + o_cnt), ctx->d_err,
                          ctx->s);
     if (nhalo > 0) CK(cudaMemcpyAsync(out, ob, sizeof(asg_fof_halo) * (size_t)nhalo,
@@ -1407,16 +1370,14 @@ int asg_fof_halos(asg_ctx* ctx, const asg_particle* p, int np, int nhalo, float 
     const size_t n = (size_t)np;
     // staging buffers only: a loaded particle set stays valid
     int r = grow(ctx, ctx->aos, sizeof(asg_particle) * n);
-    if (!r) r = grow(ctx, ctx->pos_in, 16 * n);
-    if (!r) r = grow(ctx, ctx->vel_in, 16 * n);
-    if (!r) r = grow(ctx, ctx->igrp_in, 4 * n);
+    if (!r) r = grow(ctx, ctx->rec_in, 32 * n);
     if (!r) r = grow(ctx, ctx->rk_in, 4 * n);
     if (r) return r;
     CK(cudaMemcpyAsync(ctx->aos.p, p, sizeof(asg_particle) * n, cudaMemcpyHostToDevice, ctx->s));
-    launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
-                      P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
-    return run_catalogue(ctx, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in), P<int>(ctx->igrp_in),
-                         np, 0, nhalo, boxsize, out, nlocal);
+    launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->rec_in), P<float>(ctx->rk_in), KeyGrid{}, nullptr,
+                      ctx->d_err, ctx->s);
+    return run_catalogue(ctx, P<float4>(ctx->rec_in), P<float4>(ctx->rec_in) + 1, nullptr, np, nhalo,
+                         boxsize, out, nlocal);
 }
 
 int asg_run_fof_halos(asg_ctx* ctx, int nhalo, float boxsize, asg_fof_halo* out, int* nlocal)
@@ -1425,8 +1386,8 @@ int asg_run_fof_halos(asg_ctx* ctx, int nhalo, float boxsize, asg_fof_halo* out,
     if (!ctx->loaded) return fail(ctx, ASG_ERR_STATE, "no particle set loaded");
     if (nhalo > ctx->n) return fail(ctx, ASG_ERR_ARG, "nhalo larger than the particle count");
     CK(cudaSetDevice(ctx->device));
-    return run_catalogue(ctx, P<float4>(ctx->pos), P<float4>(ctx->vel), P<int>(ctx->igrp), ctx->n, 1,
-                         nhalo, boxsize, out, nlocal);
+    return run_catalogue(ctx, P<float4>(ctx->pos), P<float4>(ctx->vel), P<int>(ctx->igrp), ctx->n, nhalo,
+                         boxsize, out, nlocal);
 }
 
 int asg_write_fof_halos(asg_ctx* ctx, const char* filename, const asg_particle* p, int np,
@@ -1558,16 +1519,15 @@ int asg_smooth(asg_ctx* ctx, asg_particle* p, int np, float left, float right, f
                        ctx->s));
     phase_end(ctx);
     phase_begin(ctx, ASG_PH_INDEX);
-    launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
-                      P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), np, left, right, nullptr, 0, P<uint64_t>(ctx->keys0), ctx->s);
-    build_index(ctx);
+    launch_unpack_aos(ctx->aos.p, np, P<float4>(ctx->rec_in), P<float>(ctx->rk_in),
+                      key_grid(left, right), P<uint64_t>(ctx->keys0), ctx->d_err, ctx->s);
+    build_index(ctx, true);
     run_knn(ctx);
     if (int r = queue_mark(ctx, halos, nh)) return r;
     // rk, dens and igrp are final: copy the records out while the deposit runs
     CK(cudaEventRecord(ctx->fields_ready, ctx->s));
     CK(cudaStreamWaitEvent(ctx->s_out, ctx->fields_ready, 0));
-    launch_pack_aos(ctx->perm, P<float4>(ctx->pos), P<float4>(ctx->vel), P<float>(ctx->rk), nullptr,
+    launch_pack_aos(ctx->perm, P<float4>(ctx->pos), P<float4>(ctx->vel), P<float>(ctx->rk),
                     P<int>(ctx->igrp), np, ctx->aos.p, ctx->s_out);
     CK(cudaMemcpyAsync(p, ctx->aos.p, sizeof(asg_particle) * (size_t)np, cudaMemcpyDeviceToHost,
                        ctx->s_out));
@@ -1595,7 +1555,6 @@ int asg_smooth_quantised(asg_ctx* ctx, const int* cell, const uint16_t* off, con
     const size_t n = (size_t)np;
     if (int r = grow(ctx, ctx->uf, 4 * n)) return r;
     if (int r = grow(ctx, ctx->minin, 4 * n)) return r;
-    if (int r = grow(ctx, ctx->lab_scan, 4 * n)) return r;
     const int* dc = nullptr;
     const uint16_t* doff = nullptr;
     const float* dv = nullptr;
@@ -1607,10 +1566,7 @@ int asg_smooth_quantised(asg_ctx* ctx, const int* cell, const uint16_t* off, con
     // rk and dens are final: back to input order and out while the deposit runs
     CK(cudaEventRecord(ctx->fields_ready, ctx->s));
     CK(cudaStreamWaitEvent(ctx->s_out, ctx->fields_ready, 0));
-    k_dens_of<<<(np + 255) / 256, 256, 0, ctx->s_out>>>(P<float4>(ctx->vel), np,
-                                                         P<float>(ctx->lab_scan));
-    count_launches(1);
-    launch_scatter_fields(ctx->perm, P<float>(ctx->rk), P<float>(ctx->lab_scan), nullptr, np,
+    launch_scatter_fields(ctx->perm, P<float>(ctx->rk), P<float4>(ctx->vel), nullptr, np,
                           P<float>(ctx->uf), P<float>(ctx->minin), nullptr, ctx->s_out);
     if (rk) CK(cudaMemcpyAsync(rk, ctx->uf.p, 4 * n, cudaMemcpyDeviceToHost, ctx->s_out));
     if (dens) CK(cudaMemcpyAsync(dens, ctx->minin.p, 4 * n, cudaMemcpyDeviceToHost, ctx->s_out));
@@ -1678,22 +1634,18 @@ int batch_queue_item(asg_batch* b, asg_ctx* ctx, int i, const DepositCap* cap)
     if (b->quant[(size_t)i] > 0)
         launch_unpack_quant(P<int>(b->in_cell) + o, P<uint16_t>(b->in_off) + 3 * o,
                             P<float>(b->in_v) + 3 * o, n, b->quant[(size_t)i], ctx->left,
-                            b->cell_size[(size_t)i], P<float4>(ctx->pos_in), P<float4>(ctx->vel_in),
-                            P<int>(ctx->igrp_in), P<float>(ctx->rk_in), ctx->d_err, ctx->s);
+                            b->cell_size[(size_t)i], P<float4>(ctx->rec_in),
+                            key_grid(ctx->left, ctx->right), P<uint64_t>(ctx->keys0), ctx->d_err, ctx->s);
     else
         launch_unpack_soa(P<float>(b->in_x) + 3 * o, P<float>(b->in_v) + 3 * o, nullptr, nullptr,
-                          n, P<float4>(ctx->pos_in), P<float4>(ctx->vel_in), P<int>(ctx->igrp_in),
-                          P<float>(ctx->rk_in), ctx->d_err, ctx->s);
-    launch_space_keys(P<float4>(ctx->pos_in), n, ctx->left, ctx->right, nullptr, 0,
-                  P<uint64_t>(ctx->keys0), ctx->s);
-    build_index(ctx);
+                          n, P<float4>(ctx->rec_in), key_grid(ctx->left, ctx->right),
+                          P<uint64_t>(ctx->keys0), ctx->d_err, ctx->s);
+    build_index(ctx, false);
     run_knn(ctx);
     if (int r = queue_deposit(ctx, b->box[(size_t)i], b->ncs.data(), b->n_nc, b->sign, 0, nullptr, 0,
                               cap))
         return r;
-    k_dens_of<<<(n + 255) / 256, 256, 0, ctx->s>>>(P<float4>(ctx->vel), n, P<float>(ctx->lab_scan));
-    count_launches(1);
-    launch_scatter_fields(ctx->perm, P<float>(ctx->rk), P<float>(ctx->lab_scan), nullptr, n,
+    launch_scatter_fields(ctx->perm, P<float>(ctx->rk), P<float4>(ctx->vel), nullptr, n,
                           P<float>(b->out_rk) + o, P<float>(b->out_dens) + o, nullptr, ctx->s);
     for (int k = 0; k < b->n_nc; ++k) {
         const MeshBuf& mb = ctx->meshes[(size_t)k];
@@ -1716,7 +1668,6 @@ int batch_plan(asg_batch* b)
         c->knn_warps = ctx->knn_warps;
         c->dep_mma = ctx->dep_mma;
         if (int r = alloc_set(c, b->max_n)) return fail(ctx, r, "batch: stream scratch");
-        if (int r = grow(c, c->lab_scan, 4 * (size_t)b->max_n)) return fail(ctx, r, "batch: stream scratch");
     }
     b->cap.assign((size_t)b->n_items, DepositCap{});
     uint32_t max_entries = 0, max_items = 0;
@@ -1727,8 +1678,7 @@ int batch_plan(asg_batch* b)
         cap.entries = c->dep_nentries + c->dep_nentries / 16 + 4096;
         cap.pairs = c->dep_npairs + c->dep_npairs / 16 + 4096;
         max_entries = std::max(max_entries, cap.entries);
-        max_items = std::max(max_items, deposit_max_items(c->dep_tiles_n, cap.pairs,
-                                                          deposit_seg(c->n, b->n_nc, c->dep_seg)));
+        max_items = std::max(max_items, deposit_max_items(c->dep_tiles_n, cap.pairs, c->dep_seg));
     }
     for (asg_ctx* c : b->sub)
         if (int r = finish(c, "batch plan")) return fail(ctx, r, c->last);
@@ -1944,7 +1894,6 @@ int asg_batch_tune(asg_batch* b, int* leaf, int* seg)
     asg_ctx* ctx = b->ctx;
     CK(cudaSetDevice(ctx->device));
     if (int r = alloc_set(ctx, b->max_n)) return r;
-    if (int r = grow(ctx, ctx->lab_scan, 4 * (size_t)b->max_n)) return r;
     int item = 0;  // the largest item
     for (int i = 1; i < b->n_items; ++i)
         if (b->np[(size_t)i] > b->np[(size_t)item]) item = i;

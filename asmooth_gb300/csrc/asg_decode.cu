@@ -15,18 +15,15 @@
 namespace asg {
 
 __global__ void k_decode_xv(const float* __restrict__ xv, int n, float s0, float s1, float s2,
-                            float4* __restrict__ pos, float4* __restrict__ vel,
-                            int* __restrict__ igrp, float* __restrict__ rk, int* err)
+                            float4* __restrict__ rec, int* err)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float* r = xv + 6 * (size_t)i;
     const float x = __fsub_rn(r[0], s0), y = __fsub_rn(r[1], s1), z = __fsub_rn(r[2], s2);
     if (!(isfinite(x) && isfinite(y) && isfinite(z))) atomicOr(err, ERR_NONFINITE);
-    pos[i] = make_float4(x, y, z, __int_as_float(i));
-    vel[i] = make_float4(r[3], r[4], r[5], 0.0f);
-    igrp[i] = 0;
-    rk[i] = 0.0f;
+    rec[2 * (size_t)i] = make_float4(x, y, z, __int_as_float(0));
+    rec[2 * (size_t)i + 1] = make_float4(r[3], r[4], r[5], 0.0f);
 }
 
 __global__ void k_zip_big(const uint8_t* __restrict__ c8, int ncell, uint32_t* __restrict__ flag)
@@ -63,8 +60,7 @@ __global__ void k_zip_counts(const uint8_t* __restrict__ c8, const uint32_t* __r
 __global__ void k_zip_particles(const uint8_t* __restrict__ off, const int16_t* __restrict__ vq,
                                 const uint32_t* __restrict__ start, int ncell, int nc, int n,
                                 float scale, float v_r2i, float s0, float s1, float s2,
-                                float4* __restrict__ pos, float4* __restrict__ vel,
-                                int* __restrict__ igrp, float* __restrict__ rk)
+                                float4* __restrict__ rec)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
@@ -85,18 +81,14 @@ __global__ void k_zip_particles(const uint8_t* __restrict__ off, const int16_t* 
         x[d] = __fsub_rn(__fmul_rn(scale, __fsub_rn(t, 1.0f)), sh[d]);
         v[d] = __fdiv_rn((float)vq[3 * (size_t)p + d], v_r2i);
     }
-    pos[p] = make_float4(x[0], x[1], x[2], __int_as_float(p));
-    vel[p] = make_float4(v[0], v[1], v[2], 0.0f);
-    igrp[p] = 0;
-    rk[p] = 0.0f;
+    rec[2 * (size_t)p] = make_float4(x[0], x[1], x[2], __int_as_float(0));
+    rec[2 * (size_t)p + 1] = make_float4(v[0], v[1], v[2], 0.0f);
 }
 
-void launch_decode_xv(const float* xv, int n, const float* shift, float4* pos, float4* vel,
-                      int* igrp, float* rk, int* err, cudaStream_t s)
+void launch_decode_xv(const float* xv, int n, const float* shift, float4* rec, int* err, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_decode_xv<<<(n + 255) / 256, 256, 0, s>>>(xv, n, shift[0], shift[1], shift[2], pos, vel, igrp,
-                                                 rk, err);
+    k_decode_xv<<<(n + 255) / 256, 256, 0, s>>>(xv, n, shift[0], shift[1], shift[2], rec, err);
     count_launches(1);
 }
 
@@ -125,12 +117,11 @@ void launch_zip_counts(const uint8_t* c8, const int* c32, int n32, int ncell, vo
 
 void launch_zip_particles(const uint8_t* off, const int16_t* vq, const uint32_t* start, int ncell,
                           int nc, int n, int mesh_scale, float v_r2i, const float* shift,
-                          float4* pos, float4* vel, int* igrp, float* rk, cudaStream_t s)
+                          float4* rec, cudaStream_t s)
 {
     if (n <= 0) return;
     k_zip_particles<<<(n + 255) / 256, 256, 0, s>>>(off, vq, start, ncell, nc, n, (float)mesh_scale,
-                                                     v_r2i, shift[0], shift[1], shift[2], pos, vel,
-                                                     igrp, rk);
+                                                     v_r2i, shift[0], shift[1], shift[2], rec);
     count_launches(1);
 }
 

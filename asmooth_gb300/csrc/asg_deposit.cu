@@ -57,7 +57,6 @@ struct TileShape {
     static constexpr int X = 8, Y = NCH == 1 ? 8 : 4, Z = NCH == 1 ? 8 : 4;
     static constexpr int CELLS = X * Y * Z;
 };
-constexpr int DEP_THREADS = 128;   // threads of the tile-merge CTA
 constexpr int PW = 9;              // partial words per cell
 constexpr int IMG_BITS = 5;        // periodic images per pair: up to 3 x 3 x 3
 // key bits of the image index: none without periodic images (every pair is
@@ -156,11 +155,10 @@ __device__ __forceinline__ void image_tiles(const AxisRange& r, int k, int nc, i
 // boxes; where that holds many more tiles than the lanes touch (particles far
 // apart), through each lane's own tiles, one lane after another.  Either way the
 // particles of a tile come in lane order.
-template <class F>
+template <bool PERIODIC, class F>
 __device__ __forceinline__ void for_entries(const DepositParams& P, const float (&lo)[3],
                                             const float (&hi)[3], bool live, int* err, F f)
 {
-    const bool periodic = P.periodic != 0;
     for (int jb = 0; jb < P.n_jobs; ++jb) {
         const MeshJob& J = P.job[jb];
         const int nc = J.nc;
@@ -168,43 +166,39 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
         bool on = live;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            r[a] = axis_range(lo[a], hi[a], J, nc, periodic);
+            r[a] = axis_range(lo[a], hi[a], J, nc, PERIODIC);
             on = on && r[a].nk > 0;
         }
-        if (on && (r[0].nk > 3 || r[1].nk > 3 || r[2].nk > 3)) {  // wider than two mesh periods
+        if (PERIODIC && on && (r[0].nk > 3 || r[1].nk > 3 || r[2].nk > 3)) {  // wider than two mesh periods
             atomicOr(err, ERR_RANGE);
             on = false;
         }
         if (!__any_sync(FULLM, on)) continue;
-        int most[3] = {1, 1, 1};  // images per axis
-        if (periodic)
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-                most[a] = (int)__reduce_max_sync(FULLM, (unsigned)(on ? r[a].nk : 0));
-        for (int image = 0; image < (periodic ? 27 : 1); ++image) {
-            const int dk[3] = {image % 3, (image / 3) % 3, image / 9};
-            if (dk[0] >= most[0] || dk[1] >= most[1] || dk[2] >= most[2]) continue;
-            int t0[3], t1[3];  // the lane's tiles, empty: t0 > t1
+        // one image of the mesh per axis (nx, ny, nz: the lane's 0th, 1st or 2nd)
+        auto one_image = [&](int nx, int ny, int nz) {
+            const int dk[3] = {nx, ny, nz};
+            const int image = nz * 9 + ny * 3 + nx;
+            int t0[3], t1[3];  // the lane's tiles
             bool in = on;
             int own = 1;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                image_tiles(r[a], r[a].k_lo + dk[a], nc, P.shift[a], t0[a], t1[a]);
-                in = in && dk[a] < r[a].nk && t0[a] <= t1[a];
+                image_tiles(r[a], PERIODIC ? r[a].k_lo + dk[a] : 0, nc, P.shift[a], t0[a], t1[a]);
+                in = in && (!PERIODIC || (dk[a] < r[a].nk && t0[a] <= t1[a]));
                 own *= t1[a] - t0[a] + 1;
             }
-            unsigned lanes = __ballot_sync(FULLM, in);
-            if (!lanes) continue;
+            unsigned lanes = PERIODIC ? __ballot_sync(FULLM, in) : ~0u;
+            if (PERIODIC && !lanes) return;
             int u0[3], u1[3];
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                if (!in) { t0[a] = INT_MAX; t1[a] = -1; }
+                if (!in) { t0[a] = INT_MAX; t1[a] = -1; }  // no tiles
                 u0[a] = (int)__reduce_min_sync(FULLM, (unsigned)t0[a]);
                 u1[a] = __reduce_max_sync(FULLM, t1[a]);
             }
-            const long long box = (long long)(u1[0] - u0[0] + 1) * (u1[1] - u0[1] + 1) * (u1[2] - u0[2] + 1);
             const unsigned touched = __reduce_add_sync(FULLM, in ? (unsigned)min(own, 1 << 24) : 0u);
-            if (box <= 2LL * touched + 64) {
+            const unsigned wx = u1[0] - u0[0] + 1, wy = u1[1] - u0[1] + 1, wz = u1[2] - u0[2] + 1;
+            if ((unsigned long long)(wx * wy) * wz <= 2ull * touched + 64) {
                 for (int tz = u0[2]; tz <= u1[2]; ++tz) {
                     const bool inz = t0[2] <= tz && tz <= t1[2];
                     for (int ty = u0[1]; ty <= u1[1]; ++ty) {
@@ -217,6 +211,7 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
                     }
                 }
             } else {
+                lanes = __ballot_sync(FULLM, in);
                 while (lanes) {
                     const int l = __ffs(lanes) - 1;
                     lanes &= lanes - 1;
@@ -229,6 +224,17 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
                                 f(J.tile_begin + (tz * J.tiles[1] + ty) * J.tiles[0] + tx, image, 1u << l);
                 }
             }
+        };
+        if constexpr (PERIODIC) {
+            int most[3];  // images per axis
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                most[a] = (int)__reduce_max_sync(FULLM, (unsigned)(on ? r[a].nk : 0));
+            for (int nz = 0; nz < most[2]; ++nz)
+                for (int ny = 0; ny < most[1]; ++ny)
+                    for (int nx = 0; nx < most[0]; ++nx) one_image(nx, ny, nz);
+        } else {
+            one_image(0, 0, 0);
         }
     }
 }
@@ -239,16 +245,19 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
 // nothing.  The cell-range edges (x' -+ h)/L and 1/h are recomputed from it
 // where they are needed (load_dep_rec), with the same rounded operations.
 // counts: the entries of each bundle, counts[bundles] = 0; *pairs += the pairs.
+template <bool PERIODIC>
 __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restrict__ vel,
                            const int* __restrict__ igrp, const float* __restrict__ rk, int n,
                            const __grid_constant__ DepositParams P, float4* __restrict__ rec,
                            uint32_t* __restrict__ counts, unsigned long long* __restrict__ pairs,
                            int* err)
 {
+    __shared__ unsigned long long block_pairs;  // one atomic per block: 0.57 M on one word took 0.3 ms
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int bundles = (n + 31) / 32;
+    if (threadIdx.x == 0) block_pairs = 0ull;
     if (i == 0) counts[bundles] = 0u;
-    if ((i & ~31) >= n) return;
+    __syncthreads();
     bool live = i < n;
     const int ii = live ? i : n - 1;
     const float4 p = pos[ii];
@@ -260,7 +269,7 @@ __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restr
     const bool halo = (P.sign * igrp[ii]) > 0;
     bool skip = !good || (P.density_only && halo);
     float x[3] = {p.x, p.y, p.z};
-    if (P.periodic) {  // global_mesh.cpp:52-61: skip outside the cube, then add the offset
+    if constexpr (PERIODIC) {  // global_mesh.cpp:52-61: skip outside the cube, then add the offset
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             if (x[a] < 0.0f || x[a] >= L) skip = true;
@@ -279,14 +288,16 @@ __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restr
         hi[a] = div_rn_by(__fadd_rn(x[a], h), L, P.rbox);
     }
     uint32_t cnt = 0, np = 0;
-    for_entries(P, lo, hi, live, err, [&](int, int, unsigned m) {
+    for_entries<PERIODIC>(P, lo, hi, live, err, [&](int, int, unsigned m) {
         ++cnt;
         np += (uint32_t)__popc(m);
     });
-    if ((i & 31) == 0) {
+    if ((i & 31) == 0 && i < n) {
         counts[i >> 5] = cnt;
-        if (np) atomicAdd(pairs, (unsigned long long)np);
+        if (np) atomicAdd(&block_pairs, (unsigned long long)np);
     }
+    __syncthreads();
+    if (threadIdx.x == 0 && block_pairs) atomicAdd(pairs, block_pairs);
 }
 
 // ---------------------------------------------------------------------------
@@ -298,6 +309,7 @@ __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restr
 // the same 2.0 ms.
 // entry o is written only when o < cap (the entry arrays' capacity); one beyond
 // it sets ERR_CAP instead
+template <bool PERIODIC>
 __global__ void k_entries(const float4* __restrict__ rec, int n, const __grid_constant__ DepositParams P,
                           const uint32_t* __restrict__ offs, uint32_t* __restrict__ keys,
                           uint2* __restrict__ entry, uint32_t cap, int* err)
@@ -324,9 +336,9 @@ __global__ void k_entries(const float4* __restrict__ rec, int n, const __grid_co
         o += held;
         held = 0;
     };
-    for_entries(P, lo, hi, live, err, [&](int tile, int image, unsigned m) {
+    for_entries<PERIODIC>(P, lo, hi, live, err, [&](int tile, int image, unsigned m) {
         if (lane == held) {
-            key = ((uint32_t)tile << img_bits(P)) | (uint32_t)image;
+            key = PERIODIC ? ((uint32_t)tile << IMG_BITS) | (uint32_t)image : (uint32_t)tile;
             mask = m;
         }
         if (++held == 32) store();
@@ -359,6 +371,21 @@ __global__ void k_sorted_entries(const int* __restrict__ order, const uint2* __r
     first[j] = (uint32_t)__popc(e.y);
 }
 
+constexpr int MERGE_FEW = 8;  // items of a tile that one warp merges by itself
+
+// Pairs per work item, at most `most`.  An item is a serial chain for its warp, so
+// a small set takes short items and all warps: a quarter of the pairs a warp
+// would get if the items were dealt out evenly over 24 warps on 152 SMs, in steps
+// of the 64 pairs between two flushes.  One item length of 4096 pairs left a set of
+// 13,840 particles to 20 warps: 354 us against 18.
+constexpr int ITEM_SHARE = 4 * 24 * 152;
+__device__ __forceinline__ int deposit_seg(const int* __restrict__ counters, int most)
+{
+    const unsigned long long pairs = *reinterpret_cast<const unsigned long long*>(counters + 2);
+    const unsigned long long seg = (pairs / ITEM_SHARE + 64) & ~63ull;
+    return (int)min(seg, (unsigned long long)most);
+}
+
 // tentry[t]: the first entry of tile t (tentry[T]: past the last real tile), by
 // binary search over the sorted keys, in parallel over the tiles.  nitems:
 // seg-pair work items per tile (at least one), nitems[T] = 0.
@@ -373,10 +400,12 @@ __device__ __forceinline__ uint32_t lower_bound(const uint32_t* __restrict__ key
     return lo;
 }
 __global__ void k_tile_items(const uint32_t* __restrict__ keys, uint32_t count,
-                             const uint32_t* __restrict__ first, int total_tiles, int ib, int seg,
-                             uint32_t* __restrict__ tentry, uint32_t* __restrict__ nitems)
+                             const uint32_t* __restrict__ first, int total_tiles, int ib, int most,
+                             uint32_t* __restrict__ tentry, uint32_t* __restrict__ nitems,
+                             const int* __restrict__ counters)
 {
     __shared__ uint32_t e[257];
+    const int seg = deposit_seg(counters, most);
     const int t = blockIdx.x * 256 + threadIdx.x;
     const uint32_t b = lower_bound(keys, count, (uint64_t)min(t, total_tiles) << ib);
     e[threadIdx.x] = b;
@@ -394,7 +423,9 @@ __global__ void k_tile_items(const uint32_t* __restrict__ keys, uint32_t count,
     nitems[t] = max(1u, (c + (uint32_t)seg - 1) / (uint32_t)seg);
 }
 
-// item_tile[i]: the tile of item i; merge: the tiles with several items.  More
+// item_tile[i]: the tile of item i; merge: the tiles with several items, those of
+// up to MERGE_FEW from the front (counters[1] of them), those of more from the
+// back (counters[4]).  More
 // items than the arrays hold (a captured call whose pairs outgrew its capacity)
 // set ERR_CAP.
 __global__ void k_item_list(const uint32_t* __restrict__ item_off, int total_tiles,
@@ -409,7 +440,8 @@ __global__ void k_item_list(const uint32_t* __restrict__ item_off, int total_til
         return;
     }
     for (uint32_t i = i0; i < i1; ++i) item_tile[i] = (uint32_t)t;
-    if (i1 - i0 > 1) merge[atomicAdd(counters + 1, 1)] = (uint32_t)t;
+    if (i1 - i0 > MERGE_FEW) merge[total_tiles - 1 - atomicAdd(counters + 4, 1)] = (uint32_t)t;
+    else if (i1 - i0 > 1) merge[atomicAdd(counters + 1, 1)] = (uint32_t)t;
 }
 
 // The pairs of one work item, 32 at a time: lane l of chunk c has pair 32 c + l.
@@ -557,48 +589,24 @@ __device__ __forceinline__ void write_tile(const WarpTile& S, const DepositParam
     }
 }
 
-__device__ __forceinline__ void block_totals(double sn, double sh, double (*red)[DEP_THREADS / 32],
-                                             const MeshJob& J, int local, int tid)
-{
-    const int lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sn += __shfl_down_sync(FULLM, sn, o);
-        sh += __shfl_down_sync(FULLM, sh, o);
-    }
-    if (lane == 0) {
-        red[0][warp] = sn;
-        red[1][warp] = sh;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double a = 0.0, b = 0.0;
-        for (int w = 0; w < DEP_THREADS / 32; ++w) {
-            a += red[0][w];
-            b += red[1][w];
-        }
-        J.partial[2 * local] = a;
-        J.partial[2 * local + 1] = b;
-    }
-}
-
 __global__ void __launch_bounds__(32 * DEP_WARPS)
 k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositParams P,
                 int total_tiles, const uint32_t* __restrict__ item_off,
                 uint32_t max_items, const uint32_t* __restrict__ item_tile,
                 const uint32_t* __restrict__ tentry, const uint32_t* __restrict__ ekeys,
                 const uint2* __restrict__ list, const uint32_t* __restrict__ first,
-                float* __restrict__ partial, int* __restrict__ next_item)
+                float* __restrict__ partial, int* __restrict__ counters)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     WarpTile& S = reinterpret_cast<WarpTile*>(smem_raw)[threadIdx.x >> 5];
     const bool periodic = P.periodic != 0;
     const uint32_t total_items = min(item_off[total_tiles], max_items);
+    const int most = deposit_seg(counters, P.seg);  // pairs per item
 
     for (;;) {
         int item = 0;
-        if (lane == 0) item = atomicAdd(next_item, 1);
+        if (lane == 0) item = atomicAdd(counters, 1);
         item = __shfl_sync(FULLM, item, 0);
         if ((uint32_t)item >= total_items) break;
         const int tile = (int)item_tile[item];
@@ -608,8 +616,8 @@ k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositP
         const int seg = item - (int)item_off[tile];
         const int nseg = (int)(item_off[tile + 1] - item_off[tile]);
         const uint32_t e0 = tentry[tile], e1 = max(tentry[tile + 1], e0);
-        const uint32_t j0 = first[e0] + (uint32_t)(seg * P.seg);
-        const uint32_t j1 = min(first[e1], j0 + (uint32_t)P.seg);
+        const uint32_t j0 = first[e0] + (uint32_t)(seg * most);
+        const uint32_t j1 = min(first[e1], j0 + (uint32_t)most);
         PairCursor pairs = open_pairs(list, first, e0, e1, j0);
 
         for (int e = lane; e < TC; e += 32) {
@@ -844,7 +852,7 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
               const uint32_t* __restrict__ item_tile, const uint32_t* __restrict__ tentry,
               const uint32_t* __restrict__ ekeys, const uint2* __restrict__ list,
               const uint32_t* __restrict__ first, float* __restrict__ partial,
-              double* __restrict__ item_tot, int* __restrict__ next_item)
+              double* __restrict__ item_tot, int* __restrict__ counters)
 {
     constexpr int MX = TileShape<NCH>::X, MY = TileShape<NCH>::Y, MZ = TileShape<NCH>::Z;
     constexpr int MC = TileShape<NCH>::CELLS;
@@ -857,21 +865,22 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
     const int g = lane >> 2, t = lane & 3;
     const bool periodic = P.periodic != 0;
     const uint32_t total_items = min(item_off[total_tiles], max_items);
+    const int most = deposit_seg(counters, P.seg);  // pairs per item
 
     int item = 0;
-    if (lane == 0) item = atomicAdd(next_item, 1);
+    if (lane == 0) item = atomicAdd(counters, 1);
     item = __shfl_sync(FULLM, item, 0);
     while ((uint32_t)item < total_items) {
         int next = 0;  // the next item's number arrives while this one runs
-        if (lane == 0) next = atomicAdd(next_item, 1);
+        if (lane == 0) next = atomicAdd(counters, 1);
         const int tile = (int)item_tile[item];
         const TileGeo geo = tile_geo(P, tile);
         const MeshJob& J = P.job[geo.job];
         const int nc = geo.nc;
         const int i0 = (int)item_off[tile], nseg = (int)item_off[tile + 1] - i0;
         const uint32_t e0 = tentry[tile], e1 = max(tentry[tile + 1], e0);
-        const uint32_t j0 = first[e0] + (uint32_t)((item - i0) * P.seg);
-        const uint32_t j1 = min(first[e1], j0 + (uint32_t)P.seg);
+        const uint32_t j0 = first[e0] + (uint32_t)((item - i0) * most);
+        const uint32_t j1 = min(first[e1], j0 + (uint32_t)most);
         PairCursor pairs = open_pairs(list, first, e0, e1, j0);
 
 #pragma unroll
@@ -1108,69 +1117,155 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
 // ---------------------------------------------------------------------------
 // (5) merge the partial tiles of multi-segment tiles, in segment order
 // ---------------------------------------------------------------------------
-// item_tot (the tensor-core deposit): the FP64 mass of every item, summed in
-// item order; null: the mass is summed from the merged cells.  A CTA takes every
-// gridDim.x-th tile of the list `merge` (counters[1] tiles with several items).
-__global__ void __launch_bounds__(DEP_THREADS)
-k_merge_tiles(const __grid_constant__ DepositParams P, const uint32_t* __restrict__ item_off,
-              const uint32_t* __restrict__ merge, const int* __restrict__ counters,
-              const float* __restrict__ partial, const double* __restrict__ item_tot)
+// A warp takes 128 cells, four neighbours per lane.  It merges a tile of up to
+// MERGE_FEW items by itself, in item order; for a tile of more, a CTA's 8 warps add
+// an eighth of the items each and the eight sums are added in order (n, c and halo
+// as double-floats throughout).  One thread per cell over all items was a chain of
+// loads: 73 us for the 36 tiles of about 36 items of a 13,840-particle set, so 14.
+// item_tot (the tensor-core deposit): the FP64 mass of every item; null: the
+// mass is summed from the merged cells.
+constexpr int MERGE_WARPS = 8;
+static_assert(MERGE_WARPS <= 32, "one lane per warp's mass");
+
+struct MergeSums {
+    float s[PW][4];  // n hi, lo; c hi, lo; v; halo hi, lo of four cells
+    __device__ __forceinline__ MergeSums()
+    {
+#pragma unroll
+        for (int q = 0; q < PW; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[q][i] = 0.f;
+    }
+    // adds the words at x, word q at x[q * stride]
+    __device__ __forceinline__ void add(const float* __restrict__ x, size_t stride, bool all)
+    {
+        float4 v[PW];
+#pragma unroll
+        for (int q = 0; q < PW; ++q)
+            v[q] = q < 2 || all ? *reinterpret_cast<const float4*>(x + q * stride)
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            auto at = [&](int q) { return i == 0 ? v[q].x : i == 1 ? v[q].y : i == 2 ? v[q].z : v[q].w; };
+            two_sum_acc(s[0][i], s[1][i], at(0));
+            s[1][i] = __fadd_rn(s[1][i], at(1));
+            if (all) {
+                two_sum_acc(s[2][i], s[3][i], at(2));
+                s[3][i] = __fadd_rn(s[3][i], at(3));
+#pragma unroll
+                for (int q = 4; q < 7; ++q) s[q][i] = __fadd_rn(s[q][i], at(q));
+                two_sum_acc(s[7][i], s[8][i], at(7));
+                s[8][i] = __fadd_rn(s[8][i], at(8));
+            }
+        }
+    }
+};
+
+__global__ void __launch_bounds__(32 * MERGE_WARPS)
+k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
+              const uint32_t* __restrict__ item_off, const uint32_t* __restrict__ merge,
+              const int* __restrict__ counters, const float* __restrict__ partial,
+              const double* __restrict__ item_tot)
 {
-    __shared__ double red[2][DEP_THREADS / 32];
+    __shared__ __align__(16) float sums[MERGE_WARPS][PW][128];
+    __shared__ double mass[2][MERGE_WARPS];
     const int cells = 1 << (P.shift[0] + P.shift[1] + P.shift[2]);
-    const int tid = threadIdx.x;
-    const int listed = counters[1];
-    for (int k = blockIdx.x; k < listed; k += gridDim.x) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool all = !P.density_only;
+    const int few = counters[1], many = counters[4];
+
+    // items [a0, a1) of cells [e, e + 3]
+    auto sum_items = [&](int a0, int a1, int e, MergeSums& m) {
+        for (int it = a0; it < a1; ++it)
+            m.add(partial + (size_t)it * cells * PW + e, (size_t)cells, all);
+    };
+    auto store = [&](const TileGeo& g, int e, const MergeSums& m, double& sn, double& sh) {
+        const MeshJob& J = P.job[g.job];
+        const size_t nc = (size_t)g.nc, nmesh = nc * nc * nc;
+        const int ly = (e >> P.shift[0]) & ((1 << P.shift[1]) - 1), lz = e >> (P.shift[0] + P.shift[1]);
+        if (ly >= g.E[1] || lz >= g.E[2]) return;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int lx = (e & ((1 << P.shift[0]) - 1)) + i;
+            if (lx >= g.E[0]) return;
+            const size_t idx = ((size_t)(g.O[2] + lz) * nc + (g.O[1] + ly)) * nc + (g.O[0] + lx);
+            if (!item_tot) {
+                sn += (double)m.s[0][i] + (double)m.s[1][i];
+                sh += (double)m.s[7][i] + (double)m.s[8][i];
+            }
+            J.mesh[idx] = __fadd_rn(m.s[0][i], m.s[1][i]);
+            if (all) {
+                J.mesh[nmesh + idx] = __fadd_rn(m.s[7][i], m.s[8][i]);
+                J.mesh[2 * nmesh + idx] = __fadd_rn(m.s[2][i], m.s[3][i]);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) J.mesh[3 * nmesh + 3 * idx + q] = m.s[4 + q][i];
+            }
+        }
+    };
+    // items [a0, a1)'s masses and the warp's cells', to lane 0
+    auto sum_mass = [&](int a0, int a1, double& sn, double& sh) {
+        if (item_tot)
+            for (int it = a0 + lane; it < a1; it += 32) {
+                sn += item_tot[2 * (size_t)it];
+                sh += item_tot[2 * (size_t)it + 1];
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            sn += __shfl_down_sync(FULLM, sn, o);
+            sh += __shfl_down_sync(FULLM, sh, o);
+        }
+    };
+
+    // ---- tiles of many items first, a CTA each ----
+    for (int k = blockIdx.x; k < many; k += gridDim.x) {
+        const int tile = (int)merge[total_tiles - 1 - k];
+        const int i0 = (int)item_off[tile], i1 = (int)item_off[tile + 1];
+        const int a0 = i0 + (int)((long long)(i1 - i0) * w / MERGE_WARPS);
+        const int a1 = i0 + (int)((long long)(i1 - i0) * (w + 1) / MERGE_WARPS);
+        const TileGeo g = tile_geo(P, tile);
+        double sn = 0.0, sh = 0.0;
+        for (int c = 4 * lane; c < cells; c += 128) {
+            MergeSums m;
+            sum_items(a0, a1, c, m);
+#pragma unroll
+            for (int q = 0; q < PW; ++q)
+                *reinterpret_cast<float4*>(&sums[w][q][4 * lane]) =
+                    make_float4(m.s[q][0], m.s[q][1], m.s[q][2], m.s[q][3]);
+            __syncthreads();
+            if (w == 0) {
+                for (int o = 1; o < MERGE_WARPS; ++o) m.add(&sums[o][0][4 * lane], 128, all);
+                store(g, c, m, sn, sh);
+            }
+            __syncthreads();  // sums is written again
+        }
+        sum_mass(a0, a1, sn, sh);
+        if (lane == 0) {
+            mass[0][w] = sn;
+            mass[1][w] = sh;
+        }
+        __syncthreads();
+        if (threadIdx.x < 2) {
+            double m = 0.0;
+            for (int o = 0; o < MERGE_WARPS; ++o) m += mass[threadIdx.x][o];
+            P.job[g.job].partial[2 * (size_t)g.local + threadIdx.x] = m;
+        }
+        __syncthreads();  // mass is written again
+    }
+    // ---- the others, a warp each ----
+    for (int k = (int)blockIdx.x + (int)gridDim.x * w; k < few; k += (int)gridDim.x * MERGE_WARPS) {
         const int tile = (int)merge[k];
         const int i0 = (int)item_off[tile], i1 = (int)item_off[tile + 1];
         const TileGeo g = tile_geo(P, tile);
-        const MeshJob& J = P.job[g.job];
-        const int nc = g.nc;
-        const size_t nmesh = (size_t)nc * nc * nc;
         double sn = 0.0, sh = 0.0;
-        for (int e = tid; e < cells; e += DEP_THREADS) {
-            float nh = 0.f, nl = 0.f, ch = 0.f, cl = 0.f, vx = 0.f, vy = 0.f, vz = 0.f, hh = 0.f, hl = 0.f;
-#pragma unroll 4
-            for (int it = i0; it < i1; ++it) {
-                const float* pt = partial + (size_t)it * cells * PW;
-                two_sum_acc(nh, nl, pt[e]);
-                nl = __fadd_rn(nl, pt[cells + e]);
-                if (!P.density_only) {
-                    two_sum_acc(ch, cl, pt[2 * cells + e]);
-                    cl = __fadd_rn(cl, pt[3 * cells + e]);
-                    vx = __fadd_rn(vx, pt[4 * cells + e]);
-                    vy = __fadd_rn(vy, pt[5 * cells + e]);
-                    vz = __fadd_rn(vz, pt[6 * cells + e]);
-                    two_sum_acc(hh, hl, pt[7 * cells + e]);
-                    hl = __fadd_rn(hl, pt[8 * cells + e]);
-                }
-            }
-            const int lx = e & ((1 << P.shift[0]) - 1), ly = (e >> P.shift[0]) & ((1 << P.shift[1]) - 1);
-            const int lz = e >> (P.shift[0] + P.shift[1]);
-            if (lx >= g.E[0] || ly >= g.E[1] || lz >= g.E[2]) continue;
-            const size_t idx = ((size_t)(g.O[2] + lz) * nc + (g.O[1] + ly)) * nc + (g.O[0] + lx);
-            sn += (double)nh + (double)nl;
-            sh += (double)hh + (double)hl;
-            J.mesh[idx] = __fadd_rn(nh, nl);
-            if (!P.density_only) {
-                J.mesh[nmesh + idx] = __fadd_rn(hh, hl);
-                J.mesh[2 * nmesh + idx] = __fadd_rn(ch, cl);
-                J.mesh[3 * nmesh + 3 * idx] = vx;
-                J.mesh[3 * nmesh + 3 * idx + 1] = vy;
-                J.mesh[3 * nmesh + 3 * idx + 2] = vz;
-            }
+        for (int c = 4 * lane; c < cells; c += 128) {
+            MergeSums m;
+            sum_items(i0, i1, c, m);
+            store(g, c, m, sn, sh);
         }
-        if (!item_tot) {
-            block_totals(sn, sh, red, J, g.local, tid);
-            __syncthreads();  // red is written again
-        } else if (tid == 0) {
-            double a = 0.0, b = 0.0;
-            for (int it = i0; it < i1; ++it) {
-                a += item_tot[2 * (size_t)it];
-                b += item_tot[2 * (size_t)it + 1];
-            }
-            J.partial[2 * (size_t)g.local] = a;
-            J.partial[2 * (size_t)g.local + 1] = b;
+        sum_mass(i0, i1, sn, sh);
+        if (lane == 0) {
+            P.job[g.job].partial[2 * (size_t)g.local] = sn;
+            P.job[g.job].partial[2 * (size_t)g.local + 1] = sh;
         }
     }
 }
@@ -1263,10 +1358,10 @@ void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, 
                          cudaStream_t s)
 {
     const int bundles = (n + 31) / 32;
-    cudaMemsetAsync(w.counters, 0, 16, s);
-    k_dep_prep<<<(bundles + 7) / 8, 256, 0, s>>>(pos, vel, igrp, rk, n, p, w.rec, w.count,
-                                                 reinterpret_cast<unsigned long long*>(w.counters + 2),
-                                                 err);
+    cudaMemsetAsync(w.counters, 0, 32, s);
+    auto kern = p.periodic ? k_dep_prep<true> : k_dep_prep<false>;
+    kern<<<(bundles + 7) / 8, 256, 0, s>>>(pos, vel, igrp, rk, n, p, w.rec, w.count,
+                                           reinterpret_cast<unsigned long long*>(w.counters + 2), err);
     exclusive_scan_u32(w.count, (size_t)bundles + 1, w.scan_tmp_n, s);
     count_launches(1);
 }
@@ -1275,7 +1370,8 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
                         uint32_t max_items, bool padded, DepositScratch& w, int* err, cudaStream_t s)
 {
     const int T = total_tiles, bundles = (n + 31) / 32;
-    k_entries<<<(bundles + 7) / 8, 256, 0, s>>>(w.rec, n, p, w.count, w.keys0, w.entry, entries, err);
+    auto kern = p.periodic ? k_entries<true> : k_entries<false>;
+    kern<<<(bundles + 7) / 8, 256, 0, s>>>(w.rec, n, p, w.count, w.keys0, w.entry, entries, err);
     count_launches(1);
     if (padded && entries > 0) {  // `entries` is the capacity; the count itself is count[bundles]
         k_pad_entries<<<(entries + 255) / 256, 256, 0, s>>>(w.keys0, w.entry, w.count + bundles, entries,
@@ -1289,7 +1385,7 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
                                                        w.first, err);
     exclusive_scan_u32(w.first, (size_t)entries + 1, w.scan_tmp_e, s);
     k_tile_items<<<T / 256 + 1, 256, 0, s>>>(keys, entries, w.first, T, img_bits(p), p.seg, w.tentry,
-                                             w.item_off);
+                                             w.item_off, w.counters);
     exclusive_scan_u32(w.item_off, (size_t)T + 1, w.scan_tmp_t, s);
     k_item_list<<<(T + 255) / 256, 256, 0, s>>>(w.item_off, T, max_items, w.item_tile, w.merge,
                                                 w.counters, err);
@@ -1312,26 +1408,15 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
                           w.rec, p, T, w.item_off, max_items, w.item_tile, w.tentry, keys, w.list,
                           w.first, w.partial, w.counters);
     }
-    k_merge_tiles<<<std::min(T, 8 * sms), DEP_THREADS, 0, s>>>(p, w.item_off, w.merge, w.counters,
-                                                               w.partial, item_tot);
+    k_merge_tiles<<<4 * sms, 32 * MERGE_WARPS, 0, s>>>(p, T, w.item_off, w.merge, w.counters,
+                                                       w.partial, item_tot);
     count_launches(5);
 }
 
-uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int seg)
+// a partial item per tile, and as many full ones as deposit_seg leaves
+uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int most)
 {
-    return (uint32_t)total_tiles + npairs / (uint32_t)seg + 1;
-}
-
-// An item is a serial chain for its warp, so a small set takes short items and
-// all warps: a quarter of the pairs a warp would get if the items were dealt out
-// evenly (about 2 n per mesh over 24 warps on 152 SMs), in steps of the 64 pairs
-// between two flushes.  One item length of 4096 pairs left a set of 13,840
-// particles to 20 warps: 354 us against 18.
-int deposit_seg(int n, int n_nc, int most)
-{
-    const long long fair = 2LL * n * n_nc / (4 * 24 * 152);
-    const long long seg = (fair + 63) / 64 * 64;
-    return (int)std::max(64LL, std::min(seg, (long long)most));
+    return (uint32_t)total_tiles + std::max((uint32_t)ITEM_SHARE, npairs / (uint32_t)most) + 2;
 }
 
 // partial tiles of multi-item tiles, then each item's FP64 mass (2 doubles)

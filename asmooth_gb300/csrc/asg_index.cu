@@ -13,6 +13,7 @@
 
 #include "asg_common.cuh"
 #include "asg_internal.h"
+#include "asg_keys.cuh"
 
 namespace asg {
 
@@ -26,36 +27,46 @@ struct ParticleRec {  // struct Particle (basic_types.h:10-15), 36 bytes
 };
 static_assert(sizeof(ParticleRec) == 36, "Particle record must be 36 bytes");
 
-__global__ void k_unpack_aos(const ParticleRec* __restrict__ aos, int n, float4* __restrict__ pos,
-                             float4* __restrict__ vel, int* __restrict__ igrp,
-                             float* __restrict__ rkin, int* err)
+// A staged particle is 32 bytes, one memory sector: x, y, z, igrp (int bits) and vx,
+// vy, vz, dens, so that putting the particles in curve order reads one random
+// sector each (four when the fields were staged apart: 1.32 against 0.42 ms for
+// 18.3 M particles).  The unpack kernels also form each particle's key.
+__device__ __forceinline__ void store_staged(float4* __restrict__ rec, int i, float x, float y, float z,
+                                             int igrp, float vx, float vy, float vz, float dens)
+{
+    rec[2 * (size_t)i] = make_float4(x, y, z, __int_as_float(igrp));
+    rec[2 * (size_t)i + 1] = make_float4(vx, vy, vz, dens);
+}
+
+__global__ void k_unpack_aos(const ParticleRec* __restrict__ aos, int n, float4* __restrict__ rec,
+                             float* __restrict__ rkin, KeyGrid grid, uint64_t* __restrict__ keys,
+                             int* err)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float* r = reinterpret_cast<const float*>(aos + i);
     const float x = r[0], y = r[1], z = r[2];
     if (!(isfinite(x) && isfinite(y) && isfinite(z))) atomicOr(err, ERR_NONFINITE);
-    pos[i] = make_float4(x, y, z, __int_as_float(i));
-    vel[i] = make_float4(r[3], r[4], r[5], r[6]);
-    igrp[i] = reinterpret_cast<const int*>(r)[8];
+    store_staged(rec, i, x, y, z, reinterpret_cast<const int*>(r)[8], r[3], r[4], r[5], r[6]);
     rkin[i] = r[7];
+    if (keys) keys[i] = space_key(grid, x, y, z);
 }
 
 __global__ void k_unpack_soa(const float* __restrict__ x3, const float* __restrict__ v3,
                              const float* __restrict__ dens, const int* __restrict__ ig, int n,
-                             float4* __restrict__ pos, float4* __restrict__ vel,
-                             int* __restrict__ igrp, float* __restrict__ rkin, int* err)
+                             float4* __restrict__ rec, KeyGrid grid, uint64_t* __restrict__ keys,
+                             int* err)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float x = x3[3 * (size_t)i], y = x3[3 * (size_t)i + 1], z = x3[3 * (size_t)i + 2];
     if (!(isfinite(x) && isfinite(y) && isfinite(z))) atomicOr(err, ERR_NONFINITE);
-    pos[i] = make_float4(x, y, z, __int_as_float(i));
-    const float d = dens ? dens[i] : 0.0f;
-    vel[i] = v3 ? make_float4(v3[3 * (size_t)i], v3[3 * (size_t)i + 1], v3[3 * (size_t)i + 2], d)
-                : make_float4(0.f, 0.f, 0.f, d);
-    igrp[i] = ig ? ig[i] : 0;
-    rkin[i] = 0.0f;
+    float v[3] = {0.f, 0.f, 0.f};
+    if (v3)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v[a] = v3[3 * (size_t)i + a];
+    store_staged(rec, i, x, y, z, ig ? ig[i] : 0, v[0], v[1], v[2], dens ? dens[i] : 0.0f);
+    if (keys) keys[i] = space_key(grid, x, y, z);
 }
 
 // Mixed-precision input: one int32 cell index c = (cz * grid + cy) * grid + cx
@@ -65,8 +76,8 @@ __global__ void k_unpack_soa(const float* __restrict__ x3, const float* __restri
 // the Python package does the same float32 operations).
 __global__ void k_unpack_quant(const int* __restrict__ cell, const uint16_t* __restrict__ off,
                                const float* __restrict__ v3, int n, int grid, float left, float cs,
-                               float unit, float4* __restrict__ pos, float4* __restrict__ vel,
-                               int* __restrict__ igrp, float* __restrict__ rkin, int* err)
+                               float unit, float4* __restrict__ rec, KeyGrid kgrid,
+                               uint64_t* __restrict__ keys, int* err)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -76,47 +87,43 @@ __global__ void k_unpack_quant(const int* __restrict__ cell, const uint16_t* __r
         atomicOr(err, ERR_BADCELL);
         c = 0;
     }
-    const int cx = c % grid, cy = (c / grid) % grid, cz = c / g2;
-    const float x = __fadd_rn(__fadd_rn(left, __fmul_rn(cs, (float)cx)),
-                              __fmul_rn((float)off[3 * (size_t)i], unit));
-    const float y = __fadd_rn(__fadd_rn(left, __fmul_rn(cs, (float)cy)),
-                              __fmul_rn((float)off[3 * (size_t)i + 1], unit));
-    const float z = __fadd_rn(__fadd_rn(left, __fmul_rn(cs, (float)cz)),
-                              __fmul_rn((float)off[3 * (size_t)i + 2], unit));
-    pos[i] = make_float4(x, y, z, __int_as_float(i));
-    vel[i] = v3 ? make_float4(v3[3 * (size_t)i], v3[3 * (size_t)i + 1], v3[3 * (size_t)i + 2], 0.0f)
-                : make_float4(0.f, 0.f, 0.f, 0.f);
-    igrp[i] = 0;
-    rkin[i] = 0.0f;
+    const int cc[3] = {c % grid, (c / grid) % grid, c / g2};
+    float x[3], v[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        x[a] = __fadd_rn(__fadd_rn(left, __fmul_rn(cs, (float)cc[a])),
+                         __fmul_rn((float)off[3 * (size_t)i + a], unit));
+    if (v3)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v[a] = v3[3 * (size_t)i + a];
+    store_staged(rec, i, x[0], x[1], x[2], 0, v[0], v[1], v[2], 0.0f);
+    keys[i] = space_key(kgrid, x[0], x[1], x[2]);
 }
 
 void launch_unpack_quant(const int* cell, const uint16_t* off, const float* v, int n, int grid,
-                         float left, float cs, float4* pos_in, float4* vel_in, int* igrp_in,
-                         float* rk_in, int* err, cudaStream_t s)
+                         float left, float cs, float4* rec, const KeyGrid& kgrid, uint64_t* keys,
+                         int* err, cudaStream_t s)
 {
     if (n <= 0) return;
     const float unit = cs / 65536.0f;
-    k_unpack_quant<<<(n + 255) / 256, 256, 0, s>>>(cell, off, v, n, grid, left, cs, unit, pos_in,
-                                                    vel_in, igrp_in, rk_in, err);
+    k_unpack_quant<<<(n + 255) / 256, 256, 0, s>>>(cell, off, v, n, grid, left, cs, unit, rec, kgrid,
+                                                    keys, err);
     count_launches(1);
 }
 
-void launch_unpack_aos(const void* aos, int n, float4* pos_in, float4* vel_in, int* igrp_in,
-                       float* rk_in, int* err, cudaStream_t s)
+void launch_unpack_aos(const void* aos, int n, float4* rec, float* rk_in, const KeyGrid& grid,
+                       uint64_t* keys, int* err, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_unpack_aos<<<(n + 255) / 256, 256, 0, s>>>((const ParticleRec*)aos, n, pos_in, vel_in,
-                                                  igrp_in, rk_in, err);
+    k_unpack_aos<<<(n + 255) / 256, 256, 0, s>>>((const ParticleRec*)aos, n, rec, rk_in, grid, keys, err);
     count_launches(1);
 }
 
 void launch_unpack_soa(const float* x, const float* v, const float* dens, const int* igrp, int n,
-                       float4* pos_in, float4* vel_in, int* igrp_in, float* rk_in, int* err,
-                       cudaStream_t s)
+                       float4* rec, const KeyGrid& grid, uint64_t* keys, int* err, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_unpack_soa<<<(n + 255) / 256, 256, 0, s>>>(x, v, dens, igrp, n, pos_in, vel_in, igrp_in,
-                                                  rk_in, err);
+    k_unpack_soa<<<(n + 255) / 256, 256, 0, s>>>(x, v, dens, igrp, n, rec, grid, keys, err);
     count_launches(1);
 }
 
@@ -134,11 +141,11 @@ __global__ void k_bounds_init(int* lohi)
     lohi[1] = (int)0x80000000;
 }
 
-__global__ void k_bounds(const float4* __restrict__ pos, int n, int* lohi)
+__global__ void k_bounds(const float4* __restrict__ rec, int n, int* lohi)
 {
     float lo = INFINITY, hi = -INFINITY;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 p = pos[i];
+        const float4 p = rec[2 * (size_t)i];
         lo = fminf(lo, fminf(p.x, fminf(p.y, p.z)));
         hi = fmaxf(hi, fmaxf(p.x, fmaxf(p.y, p.z)));
     }
@@ -152,31 +159,19 @@ __global__ void k_bounds(const float4* __restrict__ pos, int n, int* lohi)
     }
 }
 
-// space-filling-curve key of each particle: 16 bits per axis over [left,
-// right), with the bounds either given (lohi == nullptr) or read from
-// k_bounds' output; Hilbert order, or Morton order with hilbert == 0
-__global__ void k_space_keys(const float4* __restrict__ pos, int n, float left, float right,
-                             const int* __restrict__ lohi, uint64_t prefix, int hilbert,
-                             uint64_t* __restrict__ keys)
+// keys over the particles' own bounding cube, from k_bounds' output
+__global__ void k_space_keys(const float4* __restrict__ rec, int n, const int* __restrict__ lohi,
+                             int hilbert, uint64_t* __restrict__ keys)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (lohi) {
-        left = fkey_inv(lohi[0]);
-        right = fkey_inv(lohi[1]);
-    }
-    const float w = right - left;
-    const float scale = w > 0.0f ? 65536.0f / w : 1.0f;
-    const float4 p = pos[i];
-    auto cell = [&](float c) -> uint32_t {
-        float t = (c - left) * scale;
-        t = fminf(fmaxf(t, 0.0f), 65535.0f);
-        return (uint32_t)t;
-    };
-    const uint32_t cx = cell(p.x), cy = cell(p.y), cz = cell(p.z);
-    const uint64_t k = hilbert ? hilbert_key48(cx, cy, cz)
-                               : spread3(cx) | (spread3(cy) << 1) | (spread3(cz) << 2);
-    keys[i] = (prefix << 48) | k;
+    KeyGrid g;
+    g.left = fkey_inv(lohi[0]);
+    const float w = fkey_inv(lohi[1]) - g.left;
+    g.scale = w > 0.0f ? 65536.0f / w : 1.0f;
+    g.hilbert = hilbert;
+    const float4 p = rec[2 * (size_t)i];
+    keys[i] = space_key(g, p.x, p.y, p.z);
 }
 
 // ASG_SPACE_CURVE=morton selects Morton order (a tuning and comparison knob)
@@ -189,18 +184,23 @@ static int use_hilbert()
     return h;
 }
 
-void launch_space_keys(const float4* pos_in, int n, float left, float right, int* d_lohi,
-                       uint64_t key_prefix, uint64_t* keys, cudaStream_t s)
+KeyGrid key_grid(float left, float right)
+{
+    KeyGrid g;
+    g.left = left;
+    const float w = right - left;
+    g.scale = w > 0.0f ? 65536.0f / w : 1.0f;
+    g.hilbert = use_hilbert();
+    return g;
+}
+
+void launch_own_keys(const float4* rec, int n, int* d_lohi, uint64_t* keys, cudaStream_t s)
 {
     if (n <= 0) return;
-    if (d_lohi) {
-        k_bounds_init<<<1, 1, 0, s>>>(d_lohi);
-        k_bounds<<<min((n + 255) / 256, 1216), 256, 0, s>>>(pos_in, n, d_lohi);
-        count_launches(2);
-    }
-    k_space_keys<<<(n + 255) / 256, 256, 0, s>>>(pos_in, n, left, right, d_lohi, key_prefix,
-                                                  use_hilbert(), keys);
-    count_launches(1);
+    k_bounds_init<<<1, 1, 0, s>>>(d_lohi);
+    k_bounds<<<min((n + 255) / 256, 1216), 256, 0, s>>>(rec, n, d_lohi);
+    k_space_keys<<<(n + 255) / 256, 256, 0, s>>>(rec, n, d_lohi, use_hilbert(), keys);
+    count_launches(3);
 }
 
 // ---------------------------------------------------------------------------
@@ -376,21 +376,28 @@ k_rs_hist(const K* __restrict__ keys, int n, int passes, int bits, uint32_t* __r
     if (tid == 0) last = atomicAdd(head + RS_PASSES, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
-    // the last block: exclusive scan of each pass's counts, a warp per pass
+    // the last block: exclusive scan of each pass's counts, a warp per pass, a lane
+    // over bins / 32 neighbours
     __threadfence();
     for (int p = tid >> 5; p < passes; p += RS_WARPS) {
-        uint32_t run = 0;
-        for (int d0 = 0; d0 < bins; d0 += 32) {
-            uint32_t* c = hist + (p << bits) + d0 + lane;
-            const uint32_t v = __ldcg(c);
-            uint32_t inc = v;
+        uint32_t* c = hist + (p << bits) + lane * (bins >> 5);
+        uint32_t v[16], sum = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                if ((int)lane >= o) inc += y;
-            }
-            *c = run + inc - v;
-            run += __shfl_sync(0xffffffffu, inc, 31);
+        for (int u = 0; u < 16; ++u) {
+            v[u] = u < bins >> 5 ? __ldcg(c + u) : 0u;
+            sum += v[u];
+        }
+        uint32_t run = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, run, o);
+            if ((int)lane >= o) run += y;
+        }
+        run -= sum;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            if (u < bins >> 5) c[u] = run;
+            run += v[u];
         }
     }
 }
@@ -655,33 +662,6 @@ int radix_sort32(uint32_t* keys0, int* vals0, uint32_t* keys1, int* vals1, int n
                       : radix_sort_t<uint32_t, 8, uint32_t>(keys0, vals0, keys1, vals1, n, p8, iota, temp, err, s);
 }
 
-// perm is a permutation unless the sort gave up (ERR_SORT): then its stray entries
-// are replaced, so that nothing after reads or writes out of range
-__global__ void k_gather(int* __restrict__ perm, const float4* __restrict__ pos_in,
-                         const float4* __restrict__ vel_in, const int* __restrict__ igrp_in,
-                         const float* __restrict__ rk_in, int n, float4* __restrict__ pos,
-                         float4* __restrict__ vel, int* __restrict__ igrp, float* __restrict__ rk)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int o = perm[i];
-    if ((unsigned)o >= (unsigned)n) perm[i] = o = i;
-    pos[i] = pos_in[o];
-    vel[i] = vel_in[o];
-    igrp[i] = igrp_in[o];
-    rk[i] = rk_in[o];
-}
-
-void launch_gather_sorted(int* perm, const float4* pos_in, const float4* vel_in,
-                          const int* igrp_in, const float* rk_in, int n, float4* pos, float4* vel,
-                          int* igrp, float* rk, cudaStream_t s)
-{
-    if (n <= 0) return;
-    k_gather<<<(n + 255) / 256, 256, 0, s>>>(perm, pos_in, vel_in, igrp_in, rk_in, n, pos, vel,
-                                              igrp, rk);
-    count_launches(1);
-}
-
 __global__ void k_iota(int* a, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -691,20 +671,6 @@ void launch_iota(int* a, int n, cudaStream_t s)
 {
     if (n <= 0) return;
     k_iota<<<(n + 255) / 256, 256, 0, s>>>(a, n);
-    count_launches(1);
-}
-
-__global__ void k_check_rk(const float* __restrict__ rk, int n, int* err)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float h = rk[i];
-    if (!(h > 0.0f && h < INFINITY)) atomicOr(err, ERR_ZERO_RK);
-}
-void launch_check_rk(const float* rk, int n, int* err, cudaStream_t s)
-{
-    if (n <= 0) return;
-    k_check_rk<<<(n + 255) / 256, 256, 0, s>>>(rk, n, err);
     count_launches(1);
 }
 
@@ -752,6 +718,54 @@ __device__ __forceinline__ void store_box(float4* box, size_t id, const float (&
     box[2 * id + 1] = make_float4(r[4], r[5], 0.0f, 0.0f);
 }
 
+// The particles in curve order, the boxes of their leaves and, LEAF16 (leaves of
+// 16 particles), of the level above: a block holds 512 particles, the children of
+// one box of level 1.  perm is a permutation unless the sort gave up (ERR_SORT):
+// then its stray entries are replaced, so that nothing after reads or writes out
+// of range.  rk_in == nullptr: no smoothing lengths yet, 0.
+constexpr int GATHER_THREADS = 512;
+template <bool LEAF16>
+__global__ void __launch_bounds__(GATHER_THREADS)
+k_gather(int* __restrict__ perm, const float4* __restrict__ rec, const float* __restrict__ rk_in, int n,
+         float4* __restrict__ pos, float4* __restrict__ vel, int* __restrict__ igrp,
+         float* __restrict__ rk, const __grid_constant__ TreeView t)
+{
+    const int i = blockIdx.x * GATHER_THREADS + threadIdx.x;
+    const bool live = i < n;
+    int o = live ? perm[i] : 0;
+    if ((unsigned)o >= (unsigned)n) {
+        o = i;
+        perm[i] = i;
+    }
+    const float4 p = rec[2 * (size_t)o], v = rec[2 * (size_t)o + 1];
+    if (live) {
+        pos[i] = make_float4(p.x, p.y, p.z, __int_as_float(o));
+        vel[i] = v;
+        igrp[i] = __float_as_int(p.w);
+        rk[i] = rk_in ? rk_in[o] : 0.0f;
+    }
+    if constexpr (LEAF16) {
+        __shared__ float leaf[6][GATHER_THREADS / 16];
+        float4* box = const_cast<float4*>(t.box);
+        const float inf = INFINITY;
+        float b[6] = {live ? p.x : inf, live ? p.y : inf, live ? p.z : inf,
+                      live ? p.x : -inf, live ? p.y : -inf, live ? p.z : -inf};
+        group_box<16>(b);
+        if ((threadIdx.x & 15) == 0) {
+            if (live) store_box(box, (size_t)(i >> 4), b);
+#pragma unroll
+            for (int a = 0; a < 6; ++a) leaf[a][threadIdx.x >> 4] = b[a];
+        }
+        if (t.nlev == 1) return;
+        __syncthreads();
+        if (threadIdx.x >= 32) return;
+#pragma unroll
+        for (int a = 0; a < 6; ++a) b[a] = leaf[a][threadIdx.x];
+        group_box<32>(b);
+        if (threadIdx.x == 0) store_box(box, (size_t)t.off[1] + blockIdx.x, b);
+    }
+}
+
 // level 0: G lanes (16, or 32 for leaves of more particles) per leaf, one
 // coalesced load per lane
 template <int G>
@@ -782,18 +796,30 @@ __global__ void k_up_boxes(const float4* __restrict__ below, int nbelow, float4*
     if ((threadIdx.x & 31) == 0) store_box(box, (size_t)id, b);
 }
 
-void launch_tree_boxes(const float4* pos, const TreeView& t, cudaStream_t s)
+void launch_gather(int* perm, const float4* rec, const float* rk_in, const TreeView& t, float4* pos,
+                   float4* vel, int* igrp, float* rk, cudaStream_t s)
 {
     if (t.n <= 0) return;
     float4* box = const_cast<float4*>(t.box);
-    const int g = t.leaf <= 16 ? 16 : 32;
-    const unsigned nb = (unsigned)(((long long)t.cnt[0] * g + 255) / 256);
-    if (g == 16) k_leaf_boxes<16><<<nb, 256, 0, s>>>(pos, t.n, t.leaf, t.cnt[0], box);
-    else k_leaf_boxes<32><<<nb, 256, 0, s>>>(pos, t.n, t.leaf, t.cnt[0], box);
-    for (int l = 1; l < t.nlev; ++l)
+    const unsigned nb = (unsigned)(((long long)t.n + GATHER_THREADS - 1) / GATHER_THREADS);
+    int l = 2;
+    if (t.leaf == 16) {
+        k_gather<true><<<nb, GATHER_THREADS, 0, s>>>(perm, rec, rk_in, t.n, pos, vel, igrp, rk, t);
+        count_launches(1);
+    } else {
+        k_gather<false><<<nb, GATHER_THREADS, 0, s>>>(perm, rec, rk_in, t.n, pos, vel, igrp, rk, t);
+        const int g = t.leaf <= 16 ? 16 : 32;
+        const unsigned lb = (unsigned)(((long long)t.cnt[0] * g + 255) / 256);
+        if (g == 16) k_leaf_boxes<16><<<lb, 256, 0, s>>>(pos, t.n, t.leaf, t.cnt[0], box);
+        else k_leaf_boxes<32><<<lb, 256, 0, s>>>(pos, t.n, t.leaf, t.cnt[0], box);
+        count_launches(2);
+        l = 1;
+    }
+    for (; l < t.nlev; ++l) {
         k_up_boxes<<<(unsigned)(((long long)t.cnt[l] * 32 + 255) / 256), 256, 0, s>>>(
             box + 2 * t.off[l - 1], t.cnt[l - 1], box + 2 * t.off[l], t.cnt[l]);
-    count_launches(t.nlev);
+        count_launches(1);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -801,47 +827,69 @@ void launch_tree_boxes(const float4* pos, const TreeView& t, cudaStream_t s)
 // ---------------------------------------------------------------------------
 __global__ void k_pack_aos(const int* __restrict__ perm, const float4* __restrict__ pos,
                            const float4* __restrict__ vel, const float* __restrict__ rk,
-                           const float* __restrict__ dens, const int* __restrict__ igrp, int n,
-                           ParticleRec* __restrict__ aos)
+                           const int* __restrict__ igrp, int n, ParticleRec* __restrict__ aos)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int o = perm ? perm[i] : i;  // no perm: the arrays are in output order
+    const int o = perm[i];
     const float4 p = pos[i], v = vel[i];
     float* r = reinterpret_cast<float*>(aos + o);
     r[0] = p.x; r[1] = p.y; r[2] = p.z;
     r[3] = v.x; r[4] = v.y; r[5] = v.z;
-    r[6] = dens ? dens[i] : v.w;
-    r[7] = rk ? rk[i] : 0.0f;
+    r[6] = v.w;
+    r[7] = rk[i];
     reinterpret_cast<int*>(r)[8] = igrp[i];
 }
 
 void launch_pack_aos(const int* perm, const float4* pos, const float4* vel, const float* rk,
-                     const float* dens, const int* igrp, int n, void* aos, cudaStream_t s)
+                     const int* igrp, int n, void* aos, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_pack_aos<<<(n + 255) / 256, 256, 0, s>>>(perm, pos, vel, rk, dens, igrp, n,
+    k_pack_aos<<<(n + 255) / 256, 256, 0, s>>>(perm, pos, vel, rk, igrp, n,
                                                 (ParticleRec*)aos);
     count_launches(1);
 }
 
+// staged records as Particle records, in their order
+__global__ void k_pack_staged(const float4* __restrict__ rec, const float* __restrict__ rk, int n,
+                              ParticleRec* __restrict__ aos)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 p = rec[2 * (size_t)i], v = rec[2 * (size_t)i + 1];
+    float* r = reinterpret_cast<float*>(aos + i);
+    r[0] = p.x; r[1] = p.y; r[2] = p.z;
+    r[3] = v.x; r[4] = v.y; r[5] = v.z;
+    r[6] = v.w;
+    r[7] = rk ? rk[i] : 0.0f;
+    reinterpret_cast<int*>(r)[8] = __float_as_int(p.w);
+}
+
+void launch_pack_staged(const float4* rec, const float* rk, int n, void* aos, cudaStream_t s)
+{
+    if (n <= 0) return;
+    k_pack_staged<<<(n + 255) / 256, 256, 0, s>>>(rec, rk, n, (ParticleRec*)aos);
+    count_launches(1);
+}
+
+// sorted fields to input order; dens is vel.w
 __global__ void k_scatter_fields(const int* __restrict__ perm, const float* __restrict__ rk,
-                                 const float* __restrict__ dens, const int* __restrict__ igrp,
+                                 const float4* __restrict__ vel, const int* __restrict__ igrp,
                                  int n, float* rk_out, float* dens_out, int* igrp_out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int o = perm[i];
     if (rk_out) rk_out[o] = rk[i];
-    if (dens_out) dens_out[o] = dens[i];
+    if (dens_out) dens_out[o] = vel[i].w;
     if (igrp_out) igrp_out[o] = igrp[i];
 }
 
-void launch_scatter_fields(const int* perm, const float* rk, const float* dens, const int* igrp,
+void launch_scatter_fields(const int* perm, const float* rk, const float4* vel, const int* igrp,
                            int n, float* rk_out, float* dens_out, int* igrp_out, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_scatter_fields<<<(n + 255) / 256, 256, 0, s>>>(perm, rk, dens, igrp, n, rk_out, dens_out,
+    k_scatter_fields<<<(n + 255) / 256, 256, 0, s>>>(perm, rk, vel, igrp, n, rk_out, dens_out,
                                                       igrp_out);
     count_launches(1);
 }

@@ -34,22 +34,24 @@ TreeView tree_shape(int n, int leaf);
 size_t tree_box_bytes(int n, int leaf);
 
 // ---- index build (asg_index.cu) -------------------------------------------------
-// unpack reference Particle records (36 B), or SoA device arrays, into the
-// staging arrays (input order; pos.w carries the input index)
-void launch_unpack_aos(const void* aos, int n, float4* pos_in, float4* vel_in, int* igrp_in,
-                       float* rk_in, int* err, cudaStream_t s);
+// Staged particles in input order, rec[2i] = x, y, z, igrp (int bits) and rec[2i + 1]
+// = vx, vy, vz, dens, from reference Particle records (36 B), device arrays or
+// mixed-precision positions (int32 cell index + 3 x uint16 offsets in cells of
+// side cs), with the keys of the particles on a grid (keys may be null)
+struct KeyGrid {
+    float left, scale;  // cell = (x - left) * scale, clamped to 16 bits
+    int hilbert;        // Hilbert order; Morton with ASG_SPACE_CURVE=morton
+};
+KeyGrid key_grid(float left, float right);
+void launch_unpack_aos(const void* aos, int n, float4* rec, float* rk_in, const KeyGrid& grid,
+                       uint64_t* keys, int* err, cudaStream_t s);
 void launch_unpack_soa(const float* x, const float* v, const float* dens, const int* igrp, int n,
-                       float4* pos_in, float4* vel_in, int* igrp_in, float* rk_in, int* err,
-                       cudaStream_t s);
-// mixed-precision positions: int32 cell index + 3 x uint16 offsets in cells of side cs
+                       float4* rec, const KeyGrid& grid, uint64_t* keys, int* err, cudaStream_t s);
 void launch_unpack_quant(const int* cell, const uint16_t* off, const float* v, int n, int grid,
-                         float left, float cs, float4* pos_in, float4* vel_in, int* igrp_in,
-                         float* rk_in, int* err, cudaStream_t s);
-// 48-bit Hilbert keys (16 bits per axis; Morton with ASG_SPACE_CURVE=morton)
-// over [left, right)^3, or over the particles' own bounding cube when d_lohi
-// (2 ints of scratch) is given; key_prefix lands in bits 48+ (batched cubes)
-void launch_space_keys(const float4* pos_in, int n, float left, float right, int* d_lohi,
-                       uint64_t key_prefix, uint64_t* keys, cudaStream_t s);
+                         float left, float cs, float4* rec, const KeyGrid& kgrid, uint64_t* keys,
+                         int* err, cudaStream_t s);
+// keys over the particles' own bounding cube (d_lohi: 2 ints of scratch)
+void launch_own_keys(const float4* rec, int n, int* d_lohi, uint64_t* keys, cudaStream_t s);
 // stable LSD radix sort of (keys, vals) on the low `bits` bits; iota: vals0 is not
 // read, the values are the input positions; ping-pong buffers; returns which
 // buffer (0/1) holds the result.  err |= ERR_SORT if a tile's look-back gives up.
@@ -58,14 +60,11 @@ int radix_sort32(uint32_t* keys0, int* vals0, uint32_t* keys1, int* vals1, int n
                  void* temp, int* err, cudaStream_t s);
 int radix_sort(uint64_t* keys0, int* vals0, uint64_t* keys1, int* vals1, int n, int bits, bool iota,
                void* temp, int* err, cudaStream_t s);
-void launch_gather_sorted(int* perm, const float4* pos_in, const float4* vel_in,
-                          const int* igrp_in, const float* rk_in, int n, float4* pos, float4* vel,
-                          int* igrp, float* rk, cudaStream_t s);
+// the staged particles in the order perm (pos.w: input index), and the boxes of t
+// over them; rk_in may be null (0)
+void launch_gather(int* perm, const float4* rec, const float* rk_in, const TreeView& t, float4* pos,
+                   float4* vel, int* igrp, float* rk, cudaStream_t s);
 void launch_iota(int* a, int n, cudaStream_t s);
-// err |= ERR_ZERO_RK when some rk is not a positive finite number
-void launch_check_rk(const float* rk, int n, int* err, cudaStream_t s);
-// the boxes of every level of t from the sorted positions
-void launch_tree_boxes(const float4* pos, const TreeView& t, cudaStream_t s);
 // exclusive scan of uint32 counts (in place); temp from scan_temp_bytes
 size_t scan_temp_bytes(size_t n);
 void exclusive_scan_u32(uint32_t* data, size_t n, void* temp, cudaStream_t s);
@@ -81,13 +80,15 @@ inline size_t knn_list_words(int n) { return (size_t)((n + 31) / 32) * (KNN_LIST
 // 4 warps per block (tuning; leaves of 16 particles always run 1)
 void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk, int* idx33,
                     int* blist, int* err, cudaStream_t s, int warps = 2);
-// idx33 = input index of the 33rd key, for flagged queries (all = 0) or every query
+// idx33 = input index of the 33rd key, for flagged queries (all = 0) or every query;
+// dexp (n ints, or null) and acc (n uint64) are prepared for launch_dens
 void launch_knn_ties(const float4* pos, const TreeView& t, const float* t33, int* idx33,
-                     int all, int* err, cudaStream_t s);
+                     int all, const float* rk, int* dexp, unsigned long long* acc, int* err,
+                     cudaStream_t s);
 // vel[j].w (dens) += the tent weights j receives as one of the 32 nearest;
-// dexp (n ints) and acc (n uint64) are scratch; blist from launch_knn_t33 or null
+// dexp and acc as launch_knn_ties prepared them; blist from launch_knn_t33 or null
 void launch_dens(const float4* pos, const TreeView& t, const float* t33, const int* idx33,
-                 const int* blist, const float* rk, int* dexp, unsigned long long* acc,
+                 const int* blist, const float* rk, const int* dexp, unsigned long long* acc,
                  float4* vel, cudaStream_t s);
 
 // ---- mesh deposit (asg_deposit.cu) ---------------------------------------------
@@ -110,7 +111,7 @@ struct DepositParams {
     int periodic;
     float offset[3];  // periodic: rank cube offset
     int density_only;
-    int seg;          // pairs per work item of the persistent deposit (tuning, > 0)
+    int seg;          // most pairs per work item of the persistent deposit (tuning, > 0)
     int mma;          // the deposit engine: 1 the tensor cores, 0 the CUDA cores
     int shift[3];     // log2 of the tile edges in cells (deposit_tile_shape)
 };
@@ -137,17 +138,16 @@ struct DepositScratch {
     uint32_t* item_tile;  // [items] tile of each work item
     void* scan_tmp_t;     // scan scratch for T+1 entries
     float* partial;       // [items] partial tiles of multi-segment tiles
-    int* counters;        // work counter of the persistent kernel, length of merge, then
-                          // the number of pairs (64 bits)
+    int* counters;        // 32 bytes: work counter of the persistent kernel, length of merge's
+                          // front, number of pairs (64 bits), length of merge's back
 };
 size_t deposit_prep_bytes(int n);
 size_t deposit_tile_bytes(int total_tiles);
 size_t deposit_entry_bytes(uint32_t entries);
 // the per-entry arrays of w inside one block of deposit_entry_bytes
 void deposit_entry_layout(void* base, uint32_t entries, DepositScratch& w);
-uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int seg);
-// pairs per work item for n particles on n_nc meshes, at most `most`
-int deposit_seg(int n, int n_nc, int most);
+// work items that `npairs` pairs make at most, with at most `most` pairs each
+uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int most);
 int deposit_default_mma();
 size_t deposit_partial_bytes(uint32_t items, int cells);  // of tiles of that many cells
 // pass 1: particle records and entry counts; count[bundles] then holds the number
@@ -186,35 +186,35 @@ void launch_relabel(int* igrp, int n, const uint32_t* scan, const uint32_t* keep
 struct ShellPlan {
     int base[27][27];
 };
-void launch_shell_bins(const float4* pos, int n, float lt, float rt, uint32_t* keys0, int* vals0,
+void launch_shell_bins(const float4* rec, int n, float lt, float rt, uint32_t* keys0, int* vals0,
                        uint32_t* keys1, int* vals1, void* sort_tmp, uint32_t* start, uint32_t* end,
                        const uint32_t** keys, const int** order, int* err, cudaStream_t s);
-void launch_shell_emit(const float4* pos, const float4* vel, const int* igrp, const float* rk,
-                       const uint32_t* keys, const int* order, const uint32_t* start, int n,
-                       const ShellPlan& plan, float L, float4* apos, float4* avel, int* aigrp,
+// staged particles with all copies; rk and ark may both be null
+void launch_shell_emit(const float4* rec, const float* rk, const uint32_t* keys, const int* order,
+                       const uint32_t* start, int n, const ShellPlan& plan, float L, float4* arec,
                        float* ark, cudaStream_t s);
-// keep -bf*L < x < L + bf*L; flags has n_all + 1 words and ends as the exclusive scan
-void launch_shell_filter(const float4* apos, const float4* avel, const int* aigrp, const float* ark,
-                         int n_all, float lo, float hi, uint32_t* flags, void* scan_tmp,
-                         float4* pos, float4* vel, int* igrp, float* rk, cudaStream_t s);
+// keep -bf*L < x < L + bf*L, with keys; flags has n_all + 1 words and ends as the exclusive scan
+void launch_shell_filter(const float4* arec, const float* ark, int n_all, float lo, float hi,
+                         uint32_t* flags, void* scan_tmp, float4* rec, float* rk, const KeyGrid& grid,
+                         uint64_t* out_keys, cudaStream_t s);
 
 // ---- particle file payloads (asg_decode.cu) ----------------------------------------------
-void launch_decode_xv(const float* xv, int n, const float* shift, float4* pos, float4* vel,
-                      int* igrp, float* rk, int* err, cudaStream_t s);
+void launch_decode_xv(const float* xv, int n, const float* shift, float4* rec, int* err, cudaStream_t s);
 size_t zip_scratch_bytes(int ncell);
 // *start: first particle of every cell, ncell + 1 entries (the last = total)
 void launch_zip_counts(const uint8_t* c8, const int* c32, int n32, int ncell, void* scratch,
                        uint32_t** start, int* err, cudaStream_t s);
 void launch_zip_particles(const uint8_t* off, const int16_t* vq, const uint32_t* start, int ncell,
                           int nc, int n, int mesh_scale, float v_r2i, const float* shift,
-                          float4* pos, float4* vel, int* igrp, float* rk, cudaStream_t s);
+                          float4* rec, cudaStream_t s);
 
 // ---- FOF halo catalogue and file formats (asg_output.cu) ----------------------------------
 // records {x[3], v[3], int nfof} of labels 1..nhalo with centre inside (0, boxsize)^3, label
-// order, into out (device, 7*nhalo words) and *nlocal (device); pos/vel/igrp indexed by j,
-// the caller's array index is pos[j].w when w_index else j
+// order, into out (device, 7*nhalo words) and *nlocal (device).  The particles are either
+// sorted arrays (pos.w the caller's array index) or, with igrp null, staged records in the
+// caller's order (pos = rec, vel = rec + 1).
 size_t fof_catalogue_bytes(int n, int nhalo);
-void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp, int n, int w_index,
+void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp, int n,
                           int nhalo, float boxsize, void* scratch, float* out, uint32_t* nlocal,
                           int* err, cudaStream_t s);
 int write_mesh_files(const char* base, int inode, const float* mesh, int nc);
@@ -223,8 +223,11 @@ int write_fof_file(const char* filename, const float* rec, int nlocal);
 // ---- output (asg_index.cu) ------------------------------------------------------------
 // write reference Particle records in input order from the sorted fields
 void launch_pack_aos(const int* perm, const float4* pos, const float4* vel, const float* rk,
-                     const float* dens, const int* igrp, int n, void* aos, cudaStream_t s);
-void launch_scatter_fields(const int* perm, const float* rk, const float* dens, const int* igrp,
+                     const int* igrp, int n, void* aos, cudaStream_t s);
+// the same from staged records (rk may be null: 0)
+void launch_pack_staged(const float4* rec, const float* rk, int n, void* aos, cudaStream_t s);
+// sorted fields to input order (dens is vel.w); outputs may be null
+void launch_scatter_fields(const int* perm, const float* rk, const float4* vel, const int* igrp,
                            int n, float* rk_out, float* dens_out, int* igrp_out, cudaStream_t s);
 
 }  // namespace asg

@@ -316,6 +316,24 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
     }
 }
 
+// dens is summed as 64-bit fixed point per receiver j: a weight w counts as
+// w * 2^(FIX_BITS - e_j), where 2^e_j bounds hinv_j^3.  A query q that has j in
+// its 32-set has rk_j <= 2 rk_q (its 33 nearest lie within 2 rk_q of j), so
+// w <= hinv_q^3 <= 8 hinv_j^3 and every term stays below 2^(FIX_BITS + 3 + a
+// rounding margin).  A lane adds the terms it takes in one leaf (at most 32, in
+// query order) as a double-float and converts the sum to an integer once; the
+// integer atomics make the total independent of the order of the leaves.
+constexpr int FIX_BITS = 40;
+
+
+// e_j with hinv_j^3 <= 2^e_j up to rounding: minus the exponent of rk^3
+__device__ __forceinline__ int dens_exponent(float rk)
+{
+    const float h3 = __fmul_rn(__fmul_rn(rk, rk), rk);
+    const int e = 127 - ((__float_as_int(h3) >> 23) & 0xff);
+    return max(-86, min(86, e));
+}
+
 // The 33rd key of flagged queries: with the exact radius T = t33 each lane
 // counts L = #(d2 < T) and collects the tied indices (d2 == T); the 33rd key is
 // the (33 - L)-th smallest tied index.  A pass keeps the TIE_MAX smallest tied
@@ -326,7 +344,8 @@ constexpr int TIE_PASSES = (K_NN + TIE_MAX - 1) / TIE_MAX;
 
 __global__ void __launch_bounds__(KNN_WARPS * 32)
 k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, const float* __restrict__ t33,
-           int* __restrict__ idx33, int all, int* err)
+           int* __restrict__ idx33, int all, const float* __restrict__ rk, int* __restrict__ dexp,
+           unsigned long long* __restrict__ acc, int* err)
 {
     __shared__ float4 cand[KNN_WARPS][LEAF_MAX];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -334,6 +353,10 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
     const int base = (blockIdx.x * KNN_WARPS + warp) * 32;
     if (base >= n) return;
     const int q = min(base + lane, n - 1);
+    if (dexp && base + lane < n) {  // ready for k_dens_scatter
+        dexp[q] = dens_exponent(rk[q]);
+        acc[q] = 0ull;
+    }
     // unless every index is wanted, only queries flagged by k_knn_t33 (-2) need it
     const bool want = (base + lane < n) && (all || idx33[q] == -2);
     if (!__any_sync(FULL, want)) return;
@@ -416,28 +439,6 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
     }
     if (open) atomicOr(err, ERR_TIES);  // unreachable: need <= 33 <= TIE_PASSES * TIE_MAX
     if (want) idx33[base + lane] = result;
-}
-
-// dens is summed as 64-bit fixed point per receiver j: a weight w counts as
-// w * 2^(FIX_BITS - e_j), where 2^e_j bounds hinv_j^3.  A query q that has j in
-// its 32-set has rk_j <= 2 rk_q (its 33 nearest lie within 2 rk_q of j), so
-// w <= hinv_q^3 <= 8 hinv_j^3 and every term stays below 2^(FIX_BITS + 3 + a
-// rounding margin).  A lane adds the terms it takes in one leaf (at most 32, in
-// query order) as a double-float and converts the sum to an integer once; the
-// integer atomics make the total independent of the order of the leaves.
-constexpr int FIX_BITS = 40;
-
-// e_j with hinv_j^3 < 2^e_j (hinv^3 as the first factor of ker_rn); acc zeroed
-__global__ void k_dens_prep(const float* __restrict__ rk, int n, int* __restrict__ dexp,
-                            unsigned long long* __restrict__ acc)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const float hinv = __fdiv_rn(1.0f, rk[j]);
-    const float h3 = __fmul_rn(__fmul_rn(hinv, hinv), hinv);
-    const int e = ((__float_as_int(h3) >> 23) & 0xff) - 127 + 1;
-    dexp[j] = max(-86, min(86, e));
-    acc[j] = 0ull;
 }
 
 // The warp serves the 32 queries (sources) q of a bundle with their exact radii
@@ -592,26 +593,26 @@ void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk,
 }
 
 void launch_knn_ties(const float4* pos, const TreeView& t, const float* t33, int* idx33,
-                     int all, int* err, cudaStream_t s)
+                     int all, const float* rk, int* dexp, unsigned long long* acc, int* err,
+                     cudaStream_t s)
 {
     if (t.n <= 0) return;
-    k_knn_ties<<<knn_blocks(t.n), KNN_WARPS * 32, 0, s>>>(pos, t, t33, idx33, all, err);
+    k_knn_ties<<<knn_blocks(t.n), KNN_WARPS * 32, 0, s>>>(pos, t, t33, idx33, all, rk, dexp, acc, err);
     count_launches(1);
 }
 
 void launch_dens(const float4* pos, const TreeView& t, const float* t33, const int* idx33,
-                 const int* blist, const float* rk, int* dexp, unsigned long long* acc,
+                 const int* blist, const float* rk, const int* dexp, unsigned long long* acc,
                  float4* vel, cudaStream_t s)
 {
     if (t.n <= 0) return;
     const int nb = (t.n + 255) / 256, nw = (t.n + DENS_WARPS * 32 - 1) / (DENS_WARPS * 32);
-    k_dens_prep<<<nb, 256, 0, s>>>(rk, t.n, dexp, acc);
     if (t.leaf <= 16)
         k_dens_scatter<true><<<nw, DENS_WARPS * 32, 0, s>>>(pos, t, t33, idx33, blist, rk, dexp, acc);
     else
         k_dens_scatter<false><<<nw, DENS_WARPS * 32, 0, s>>>(pos, t, t33, idx33, blist, rk, dexp, acc);
     k_dens_finish<<<nb, 256, 0, s>>>(acc, dexp, t.n, vel);
-    count_launches(3);
+    count_launches(2);
 }
 
 }  // namespace asg

@@ -41,7 +41,7 @@ constexpr int NOALLOC_MAX_DEVICES = 64;
 
 // byte offsets of the arrays carved out of the scratch for n particles
 struct NoallocLayout {
-    size_t pos_in, vel_in, igrp_in, rk_in, keys0, keys1, vals0, vals1, sort_tmp;
+    size_t rec_in, keys0, keys1, vals0, vals1, sort_tmp;
     size_t pos, vel, igrp, rk, t33, idx33, boxes, blist, dacc, dexp, err, total;
 };
 
@@ -56,10 +56,7 @@ static NoallocLayout noalloc_layout(size_t n)
         o = align256(o + bytes);
         return at;
     };
-    L.pos_in = take(16 * n);
-    L.vel_in = take(16 * n);
-    L.igrp_in = take(4 * n);
-    L.rk_in = take(4 * n);
+    L.rec_in = take(32 * n);
     L.keys0 = take(8 * n);
     L.keys1 = take(8 * n);
     L.vals0 = take(4 * n);
@@ -107,18 +104,6 @@ static int scratch_address(int dev, void** out, bool refresh)
     }
     *out = g_scratch_ptr[dev];
     return ASG_OK;
-}
-
-// sorted rk and dens (vel.w) back to input order, in the caller's buffers
-__global__ static void k_noalloc_store(const int* __restrict__ perm, const float* __restrict__ rk,
-                                       const float4* __restrict__ vel, int n,
-                                       float* __restrict__ rk_out, float* __restrict__ dens_out)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int o = perm[i];
-    rk_out[o] = rk[i];
-    dens_out[o] = vel[i].w;
 }
 
 static int noalloc_status(int bits)
@@ -178,26 +163,21 @@ extern "C" int asg_neighbor_search_noalloc(const float* d_x, int np, float left,
         cudaGetLastError();
         return ASG_ERR_CUDA;
     }
-    launch_unpack_soa(d_x, nullptr, d_dens, nullptr, np, F4(L.pos_in), F4(L.vel_in), I(L.igrp_in),
-                      F(L.rk_in), err, s);
-    launch_space_keys(F4(L.pos_in), np, left, right, nullptr, 0,
-                  reinterpret_cast<uint64_t*>(b + L.keys0), s);
+    launch_unpack_soa(d_x, nullptr, d_dens, nullptr, np, F4(L.rec_in), key_grid(left, right),
+                      reinterpret_cast<uint64_t*>(b + L.keys0), err, s);
     const int cur = radix_sort(reinterpret_cast<uint64_t*>(b + L.keys0), I(L.vals0),
                                reinterpret_cast<uint64_t*>(b + L.keys1), I(L.vals1), np, 48,
                                true, b + L.sort_tmp, err, s);
     int* perm = I(cur ? L.vals1 : L.vals0);
-    launch_gather_sorted(perm, F4(L.pos_in), F4(L.vel_in), I(L.igrp_in), F(L.rk_in), np, F4(L.pos),
-                         F4(L.vel), I(L.igrp), F(L.rk), s);
     TreeView t = tree_shape(np, LEAF_DEFAULT);
     t.box = F4(L.boxes);
-    launch_tree_boxes(F4(L.pos), t, s);
+    launch_gather(perm, F4(L.rec_in), nullptr, t, F4(L.pos), F4(L.vel), I(L.igrp), F(L.rk), s);
     launch_knn_t33(F4(L.pos), t, F(L.t33), F(L.rk), I(L.idx33), I(L.blist), err, s);
-    launch_knn_ties(F4(L.pos), t, F(L.t33), I(L.idx33), 0, err, s);
-    launch_check_rk(F(L.rk), np, err, s);
+    launch_knn_ties(F4(L.pos), t, F(L.t33), I(L.idx33), 0, F(L.rk), I(L.dexp),
+                    reinterpret_cast<unsigned long long*>(b + L.dacc), err, s);
     launch_dens(F4(L.pos), t, F(L.t33), I(L.idx33), I(L.blist), F(L.rk), I(L.dexp),
                 reinterpret_cast<unsigned long long*>(b + L.dacc), F4(L.vel), s);
-    k_noalloc_store<<<(np + 255) / 256, 256, 0, s>>>(perm, F(L.rk), F4(L.vel), np, d_rk, d_dens);
-    count_launches(1);
+    launch_scatter_fields(perm, F(L.rk), F4(L.vel), nullptr, np, d_rk, d_dens, nullptr, s);
 
     int bits = 0;
     cudaError_t e = cudaMemcpyAsync(&bits, err, sizeof(int), cudaMemcpyDeviceToHost, s);

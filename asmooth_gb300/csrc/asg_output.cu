@@ -52,15 +52,16 @@ static CatLayout cat_layout(int n, int nhalo)
 
 size_t fof_catalogue_bytes(int n, int nhalo) { return cat_layout(n, nhalo).total; }
 
-// the label of the particle at position i of the caller's array, and its
-// position j in pos/vel (label 0: in no halo)
+// the label of the particle at position i of the caller's array, and its place j
+// in pos/vel (label 0: in no halo).  igrp: sorted arrays, pos.w the position;
+// null: staged records, the label in pos.w
 __global__ void k_cat_keys(const float4* __restrict__ pos, const int* __restrict__ igrp, int n,
-                           int w_index, int nhalo, uint32_t* __restrict__ keys, int* __restrict__ vals)
+                           int nhalo, uint32_t* __restrict__ keys, int* __restrict__ vals)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const int lab = igrp[j];
-    const int i = w_index ? __float_as_int(pos[j].w) : j;
+    const int w = __float_as_int(pos[igrp ? (size_t)j : 2 * (size_t)j].w);
+    const int lab = igrp ? igrp[j] : w, i = igrp ? w : j;
     keys[i] = (lab >= 1 && lab <= nhalo) ? (uint32_t)lab : 0u;
     vals[i] = j;
 }
@@ -94,7 +95,7 @@ struct CatRows {
 template <int T, class Sync>
 __device__ __forceinline__ float cat_sum(CatRows<T>& R, int tid, uint32_t s, uint32_t e,
                                          const float4* __restrict__ pos,
-                                         const float4* __restrict__ vel,
+                                         const float4* __restrict__ vel, int stride,
                                          const int* __restrict__ order, Sync sync)
 {
     float sum = 0.f;
@@ -103,8 +104,8 @@ __device__ __forceinline__ float cat_sum(CatRows<T>& R, int tid, uint32_t s, uin
     int j = s + tid < e ? order[s + tid] : 0;
     auto fetch = [&](uint32_t m) {
         if (m + tid < e) {
-            p = pos[j];
-            v = vel[j];
+            p = pos[(size_t)j * stride];
+            v = vel[(size_t)j * stride];
         }
         if (m + T + tid < e) j = order[m + T + tid];
     };
@@ -148,7 +149,7 @@ __device__ __forceinline__ void cat_record(int lane, float sum, uint32_t members
 }
 
 __global__ void __launch_bounds__(CAT_THREADS)
-k_cat_sums(const float4* __restrict__ pos, const float4* __restrict__ vel,
+k_cat_sums(const float4* __restrict__ pos, const float4* __restrict__ vel, int stride,
            const int* __restrict__ order, const uint32_t* __restrict__ start,
            const uint32_t* __restrict__ end, int nhalo, int nbig, float boxsize,
            float* __restrict__ rec, uint32_t* __restrict__ flags)
@@ -163,7 +164,7 @@ k_cat_sums(const float4* __restrict__ pos, const float4* __restrict__ vel,
         for (int h = blockIdx.x; h < nhalo; h += nbig) {
             const uint32_t s = start[h + 1], e = end[h + 1];
             if (e - s <= CAT_BIG) continue;
-            const float sum = cat_sum<CAT_THREADS>(R.block, tid, s, e, pos, vel, order,
+            const float sum = cat_sum<CAT_THREADS>(R.block, tid, s, e, pos, vel, stride, order,
                                                    [] { __syncthreads(); });
             if (w == 0) cat_record(lane, sum, e - s, boxsize, rec + (size_t)REC_WORDS * h, flags + h);
         }
@@ -172,7 +173,7 @@ k_cat_sums(const float4* __restrict__ pos, const float4* __restrict__ vel,
     const int h = ((int)blockIdx.x - nbig) * W + w;  // a warp per halo
     const uint32_t s = h < nhalo ? start[h + 1] : 0u, e = h < nhalo ? end[h + 1] : 0u;
     if (h >= nhalo || e - s > CAT_BIG) return;
-    const float sum = cat_sum<32>(R.warp[w], lane, s, e, pos, vel, order, [] { __syncwarp(); });
+    const float sum = cat_sum<32>(R.warp[w], lane, s, e, pos, vel, stride, order, [] { __syncwarp(); });
     cat_record(lane, sum, e - s, boxsize, rec + (size_t)REC_WORDS * h, flags + h);
 }
 
@@ -190,7 +191,7 @@ __global__ void k_cat_compact(const float* __restrict__ rec, const uint32_t* __r
     for (int k = 0; k < REC_WORDS; ++k) b[k] = a[k];
 }
 
-void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp, int n, int w_index,
+void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp, int n,
                           int nhalo, float boxsize, void* scratch, float* out, uint32_t* nlocal,
                           int* err, cudaStream_t s)
 {
@@ -203,7 +204,7 @@ void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp,
     cudaMemsetAsync(b + L.end, 0, 4 * H, s);
     cudaMemsetAsync(b + L.flags, 0, 4 * H, s);
     if (n > 0) {
-        k_cat_keys<<<(n + 255) / 256, 256, 0, s>>>(pos, igrp, n, w_index, nhalo, U(L.keys0),
+        k_cat_keys<<<(n + 255) / 256, 256, 0, s>>>(pos, igrp, n, nhalo, U(L.keys0),
                                                     I(L.vals0));
         int bits = 0;
         while (bits < 31 && (nhalo >> bits) != 0) ++bits;
@@ -216,7 +217,7 @@ void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp,
         if (nhalo > 0) {
             const int nbig = nhalo < 8192 ? nhalo : 8192, per = CAT_THREADS / 32;
             k_cat_sums<<<nbig + (nhalo + per - 1) / per, CAT_THREADS, 0, s>>>(
-                pos, vel, order, U(L.start), U(L.end), nhalo, nbig, boxsize,
+                pos, vel, igrp ? 1 : 2, order, U(L.start), U(L.end), nhalo, nbig, boxsize,
                 reinterpret_cast<float*>(b + L.rec), U(L.flags));
             count_launches(1);
         }

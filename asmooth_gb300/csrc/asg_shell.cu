@@ -15,15 +15,16 @@
 // tie-breaks.)
 #include "asg_common.cuh"
 #include "asg_internal.h"
+#include "asg_keys.cuh"
 
 namespace asg {
 
-__global__ void k_shell_bins(const float4* __restrict__ pos, int n, float lt, float rt,
+__global__ void k_shell_bins(const float4* __restrict__ rec, int n, float lt, float rt,
                              uint32_t* __restrict__ keys)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 p = pos[i];
+    const float4 p = rec[2 * (size_t)i];
     const int bx = (p.x >= lt) + (p.x > rt);
     const int by = (p.y >= lt) + (p.y > rt);
     const int bz = (p.z >= lt) + (p.z > rt);
@@ -41,26 +42,20 @@ __global__ void k_shell_bounds(const uint32_t* __restrict__ keys, int n, uint32_
 }
 
 // interior particles first, unchanged
-__global__ void k_shell_interior(const float4* __restrict__ pos, const float4* __restrict__ vel,
-                                 const int* __restrict__ igrp, const float* __restrict__ rk, int n,
-                                 float4* __restrict__ apos, float4* __restrict__ avel,
-                                 int* __restrict__ aigrp, float* __restrict__ ark)
+__global__ void k_shell_interior(const float4* __restrict__ rec, const float* __restrict__ rk, int n,
+                                 float4* __restrict__ arec, float* __restrict__ ark)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    apos[i] = pos[i];
-    avel[i] = vel[i];
-    aigrp[i] = igrp[i];
-    ark[i] = rk[i];
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 2LL * n) return;
+    arec[i] = rec[i];
+    if (rk && i < n) ark[i] = rk[i];
 }
 
 // every copy of the bin-sorted particle m, at its group's offset + rank in the bin
-__global__ void k_shell_emit(const float4* __restrict__ pos, const float4* __restrict__ vel,
-                             const int* __restrict__ igrp, const float* __restrict__ rk,
+__global__ void k_shell_emit(const float4* __restrict__ rec, const float* __restrict__ rk,
                              const uint32_t* __restrict__ keys, const int* __restrict__ order,
                              const uint32_t* __restrict__ start, int n, ShellPlan plan, float L,
-                             float4* __restrict__ apos, float4* __restrict__ avel,
-                             int* __restrict__ aigrp, float* __restrict__ ark)
+                             float4* __restrict__ arec, float* __restrict__ ark)
 {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n) return;
@@ -68,10 +63,9 @@ __global__ void k_shell_emit(const float4* __restrict__ pos, const float4* __res
     if (b == 13) return;
     const int i = order[m];
     const uint32_t r = (uint32_t)m - start[b];
-    const float4 p = pos[i];
-    const float4 v = vel[i];
-    const int g = igrp[i];
-    const float h = rk[i];
+    const float4 p = rec[2 * (size_t)i];
+    const float4 v = rec[2 * (size_t)i + 1];
+    const float h = rk ? rk[i] : 0.0f;
     for (int d = 0; d < 27; ++d) {
         const int base = plan.base[b][d];
         if (base < 0) continue;
@@ -79,46 +73,43 @@ __global__ void k_shell_emit(const float4* __restrict__ pos, const float4* __res
         const float sx = __fmul_rn((float)(d % 3 - 1), L);
         const float sy = __fmul_rn((float)((d / 3) % 3 - 1), L);
         const float sz = __fmul_rn((float)(d / 9 - 1), L);
-        apos[dst] = make_float4(__fsub_rn(p.x, sx), __fsub_rn(p.y, sy), __fsub_rn(p.z, sz), p.w);
-        avel[dst] = v;
-        aigrp[dst] = g;
-        ark[dst] = h;
+        arec[2 * dst] = make_float4(__fsub_rn(p.x, sx), __fsub_rn(p.y, sy), __fsub_rn(p.z, sz), p.w);
+        arec[2 * dst + 1] = v;
+        if (rk) ark[dst] = h;
     }
 }
 
-__global__ void k_shell_keep(const float4* __restrict__ apos, int n, float lo, float hi,
+__global__ void k_shell_keep(const float4* __restrict__ arec, int n, float lo, float hi,
                              uint32_t* __restrict__ flags)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const float4 p = apos[k];
+    const float4 p = arec[2 * (size_t)k];
     flags[k] = (lo < p.x && p.x < hi && lo < p.y && p.y < hi && lo < p.z && p.z < hi) ? 1u : 0u;
 }
 
-// stable compaction; pos.w becomes the index in the shelled set
-__global__ void k_shell_compact(const float4* __restrict__ apos, const float4* __restrict__ avel,
-                                const int* __restrict__ aigrp, const float* __restrict__ ark, int n,
-                                const uint32_t* __restrict__ scan, float4* __restrict__ pos,
-                                float4* __restrict__ vel, int* __restrict__ igrp,
-                                float* __restrict__ rk)
+// stable compaction, with the keys of the kept particles
+__global__ void k_shell_compact(const float4* __restrict__ arec, const float* __restrict__ ark, int n,
+                                const uint32_t* __restrict__ scan, float4* __restrict__ rec,
+                                float* __restrict__ rk, KeyGrid grid, uint64_t* __restrict__ keys)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n || scan[k + 1] == scan[k]) return;
     const uint32_t o = scan[k];
-    const float4 p = apos[k];
-    pos[o] = make_float4(p.x, p.y, p.z, __int_as_float((int)o));
-    vel[o] = avel[k];
-    igrp[o] = aigrp[k];
-    rk[o] = ark[k];
+    const float4 p = arec[2 * (size_t)k];
+    rec[2 * (size_t)o] = p;
+    rec[2 * (size_t)o + 1] = arec[2 * (size_t)k + 1];
+    if (rk) rk[o] = ark[k];
+    keys[o] = space_key(grid, p.x, p.y, p.z);
 }
 
-void launch_shell_bins(const float4* pos, int n, float lt, float rt, uint32_t* keys0, int* vals0,
+void launch_shell_bins(const float4* rec, int n, float lt, float rt, uint32_t* keys0, int* vals0,
                        uint32_t* keys1, int* vals1, void* sort_tmp, uint32_t* start, uint32_t* end,
                        const uint32_t** keys, const int** order, int* err, cudaStream_t s)
 {
     cudaMemsetAsync(start, 0, 27 * sizeof(uint32_t), s);
     cudaMemsetAsync(end, 0, 27 * sizeof(uint32_t), s);
-    k_shell_bins<<<(n + 255) / 256, 256, 0, s>>>(pos, n, lt, rt, keys0);
+    k_shell_bins<<<(n + 255) / 256, 256, 0, s>>>(rec, n, lt, rt, keys0);
     const int cur = radix_sort32(keys0, vals0, keys1, vals1, n, 5, true, sort_tmp, err, s);
     *keys = cur ? keys1 : keys0;
     *order = cur ? vals1 : vals0;
@@ -126,26 +117,23 @@ void launch_shell_bins(const float4* pos, int n, float lt, float rt, uint32_t* k
     count_launches(2);
 }
 
-void launch_shell_emit(const float4* pos, const float4* vel, const int* igrp, const float* rk,
-                       const uint32_t* keys, const int* order, const uint32_t* start, int n,
-                       const ShellPlan& plan, float L, float4* apos, float4* avel, int* aigrp,
+void launch_shell_emit(const float4* rec, const float* rk, const uint32_t* keys, const int* order,
+                       const uint32_t* start, int n, const ShellPlan& plan, float L, float4* arec,
                        float* ark, cudaStream_t s)
 {
-    k_shell_interior<<<(n + 255) / 256, 256, 0, s>>>(pos, vel, igrp, rk, n, apos, avel, aigrp, ark);
-    k_shell_emit<<<(n + 255) / 256, 256, 0, s>>>(pos, vel, igrp, rk, keys, order, start, n, plan, L,
-                                                  apos, avel, aigrp, ark);
+    k_shell_interior<<<(unsigned)((2LL * n + 255) / 256), 256, 0, s>>>(rec, rk, n, arec, ark);
+    k_shell_emit<<<(n + 255) / 256, 256, 0, s>>>(rec, rk, keys, order, start, n, plan, L, arec, ark);
     count_launches(2);
 }
 
-void launch_shell_filter(const float4* apos, const float4* avel, const int* aigrp, const float* ark,
-                         int n_all, float lo, float hi, uint32_t* flags, void* scan_tmp,
-                         float4* pos, float4* vel, int* igrp, float* rk, cudaStream_t s)
+void launch_shell_filter(const float4* arec, const float* ark, int n_all, float lo, float hi,
+                         uint32_t* flags, void* scan_tmp, float4* rec, float* rk, const KeyGrid& grid,
+                         uint64_t* out_keys, cudaStream_t s)
 {
     cudaMemsetAsync(flags + n_all, 0, sizeof(uint32_t), s);
-    k_shell_keep<<<(n_all + 255) / 256, 256, 0, s>>>(apos, n_all, lo, hi, flags);
+    k_shell_keep<<<(n_all + 255) / 256, 256, 0, s>>>(arec, n_all, lo, hi, flags);
     exclusive_scan_u32(flags, (size_t)n_all + 1, scan_tmp, s);
-    k_shell_compact<<<(n_all + 255) / 256, 256, 0, s>>>(apos, avel, aigrp, ark, n_all, flags, pos,
-                                                         vel, igrp, rk);
+    k_shell_compact<<<(n_all + 255) / 256, 256, 0, s>>>(arec, ark, n_all, flags, rec, rk, grid, out_keys);
     count_launches(2);
 }
 
