@@ -11,8 +11,8 @@
 // (membership is bit-exact; the reference numbers groups in kd-tree order).
 //
 // SO halos (mark_halo_particles, nbr_search.cpp:140-165, driven by the loop at
-// clumping_tree_main.cpp:474-485): one warp per halo walks the tree with the
-// halo's sphere; lanes test bucket particles with d2 < r*r and set igrp = -1.
+// clumping_tree_main.cpp:474-485): a halo's warps walk the tree with its sphere;
+// lanes test bucket particles with d2 < r*r and set igrp = -1.
 #include <climits>
 
 #include "asg_common.cuh"
@@ -217,44 +217,73 @@ void launch_relabel(int* igrp, int n, const uint32_t* scan, const uint32_t* keep
 // ---------------------------------------------------------------------------
 // SO halos
 // ---------------------------------------------------------------------------
-constexpr int MH_WARPS = 4;
+// A halo's warps walk the upper levels together and take the groups of 32 leaves in
+// turn; within a group they load 32 particles at a time, all loads independent. A
+// leaf at a time on one warp was a chain of dependent loads, as long as the largest
+// halo: 299 us for 102 halos of a 377,000-particle set, so 20.
+constexpr int MH_WARPS = 8;
+// warps per halo: 8 while few halos leave the chip idle (64 halos 18 us, 53 with one
+// warp each), else 1, a walk of the upper levels costing more than most halos' leaves:
+// 4864 halos 54 against 62 us, 20,000 halos 173 against 131.
+constexpr int MH_MANY = 32 * 152;
+static int mark_split(int nh) { return nh <= MH_MANY ? MH_WARPS : 1; }
 
 __global__ void __launch_bounds__(MH_WARPS * 32)
 k_mark_halos(const float4* __restrict__ pos, const __grid_constant__ TreeView t, const float* __restrict__ halos, int nh,
-             float left, float right, int* __restrict__ igrp, long long* __restrict__ counts,
+             int split, float left, float right, int* __restrict__ igrp, long long* __restrict__ counts,
              double* __restrict__ mass8)
 {
+    __shared__ int found[MH_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.x * MH_WARPS + warp;
-    if (h >= nh) return;
-    const float cx = halos[5 * (size_t)h], cy = halos[5 * (size_t)h + 1],
-                cz = halos[5 * (size_t)h + 2], r = halos[5 * (size_t)h + 3],
-                mass = halos[5 * (size_t)h + 4];
-    const bool inside = left < cx && cx < right && left < cy && cy < right && left < cz && cz < right;
-    if (!inside) {
-        if (lane == 0) { counts[h] = 0; mass8[h] = 0.0; }
-        return;
+    const int h = (blockIdx.x * MH_WARPS + warp) / split, share = warp % split;
+    int cnt = 0;
+    bool inside = false;
+    if (h < nh) {
+        const float cx = halos[5 * (size_t)h], cy = halos[5 * (size_t)h + 1],
+                    cz = halos[5 * (size_t)h + 2], r = halos[5 * (size_t)h + 3];
+        inside = left < cx && cx < right && left < cy && cy < right && left < cz && cz < right;
+        const float r2 = __fmul_rn(r, r);
+        const float bound = prune_bound(r2);
+        const float4 c4 = make_float4(cx, cy, cz, 0.f);
+        auto pass = [&](const TreeBox& c, int, int) { return point_box_fast(c4, c) <= bound; };
+        const int per = t.leaf <= 16 ? 2 : 1, width = 32 / per;
+        int turn = 0;
+        if (inside)
+            tree_walk_groups(t, pass, [&](int g) {
+                if (turn++ % split != share) return true;
+                const unsigned m = group_leaves(t, g, pass);
+                // a warp's load covers `per` leaves; four loads in flight
+                for (int l0 = 0; l0 < 32; l0 += 4 * per) {
+                    if (!(m >> l0 & (unsigned)((1ull << 4 * per) - 1))) continue;
+                    float4 p[4];
+                    int at[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int l = l0 + per * u + lane / width;
+                        const int i = (g * 32 + l) * t.leaf + lane % width;
+                        const bool on = l < 32 && (m >> l & 1u) && lane % width < t.leaf && i < t.n;
+                        at[u] = on ? i : -1;
+                        p[u] = on ? pos[i] : make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        // norm2(x, particle[i].x) with x the halo centre (nbr_search.cpp:149)
+                        const bool hit = at[u] >= 0 && norm2_rn(cx, cy, cz, p[u].x, p[u].y, p[u].z) < r2;
+                        if (hit) igrp[at[u]] = -1;
+                        cnt += hit ? 1 : 0;
+                    }
+                }
+                return true;
+            });
     }
-    const float r2 = __fmul_rn(r, r);
-    const float bound = prune_bound(r2);
-    const float4 c4 = make_float4(cx, cy, cz, 0.f);
-    long long cnt = 0;
-    tree_walk(t, [&](const TreeBox& c, int, int) { return point_box_fast(c4, c) <= bound; },
-              [&](int id) {
-                  const int first = id * t.leaf, nb = leaf_count(t, id);
-                  bool hit = false;
-                  if (lane < nb) {
-                      const float4 p = pos[first + lane];
-                      // norm2(x, particle[i].x) with x the halo centre (nbr_search.cpp:149)
-                      hit = norm2_rn(cx, cy, cz, p.x, p.y, p.z) < r2;
-                      if (hit) igrp[first + lane] = -1;
-                  }
-                  cnt += __popc(__ballot_sync(FM, hit));
-                  return true;
-              });
-    if (lane == 0) {
-        counts[h] = cnt;
-        mass8[h] = (double)__fdiv_rn(mass, 8.0f);  // h[i].mass/8.0f (:483)
+    cnt = (int)__reduce_add_sync(FM, (unsigned)cnt);
+    if (lane == 0) found[warp] = cnt;
+    __syncthreads();
+    if (h < nh && share == 0 && lane == 0) {
+        long long sum = 0;
+        for (int w = 0; w < split; ++w) sum += found[warp + w];
+        counts[h] = sum;
+        mass8[h] = inside ? (double)__fdiv_rn(halos[5 * (size_t)h + 4], 8.0f) : 0.0;  // h[i].mass/8.0f (:483)
     }
 }
 
@@ -263,8 +292,9 @@ void launch_mark_halos(const float4* pos, const TreeView& t, const float* halos,
                        cudaStream_t s)
 {
     if (nh <= 0 || t.n <= 0) return;
-    k_mark_halos<<<(nh + MH_WARPS - 1) / MH_WARPS, MH_WARPS * 32, 0, s>>>(
-        pos, t, halos, nh, left, right, igrp, counts, mass8);
+    const int split = mark_split(nh);
+    k_mark_halos<<<(unsigned)(((long long)nh * split + MH_WARPS - 1) / MH_WARPS), MH_WARPS * 32, 0, s>>>(
+        pos, t, halos, nh, split, left, right, igrp, counts, mass8);
     count_launches(1);
 }
 

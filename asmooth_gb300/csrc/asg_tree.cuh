@@ -63,16 +63,20 @@ __device__ __forceinline__ int leaf_count(const TreeView& t, int id)
     return min(t.leaf, t.n - id * t.leaf);
 }
 
-// Visits, in a fixed order, every leaf all of whose ancestors pass: pass(box,
-// level, id) is asked by each lane for its own child, leaf(id) is called by the
-// whole warp (and may end the walk by returning false).  Lane l keeps the
-// pending children of the node open at level l.
-template <class Pass, class Leaf>
-__device__ __forceinline__ void tree_walk(const TreeView& t, Pass pass, Leaf leaf)
+// Visits, in a fixed order, every group of 32 leaves (32 g ... 32 g + 31) all of whose
+// ancestors pass: pass(box, level, id) is asked by each lane for its own child,
+// group(g) is called by the whole warp (and may end the walk by returning false).
+// Lane l keeps the pending children of the node open at level l.
+template <class Pass, class Group>
+__device__ __forceinline__ void tree_walk_groups(const TreeView& t, Pass pass, Group group)
 {
     constexpr unsigned ALL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    int L = t.nlev - 1, g = 0;
+    const int lane = threadIdx.x & 31, top = t.nlev - 1;
+    if (top == 0) {
+        group(0);
+        return;
+    }
+    int L = top, g = 0;
     unsigned pending = 0;
     auto open = [&]() {
         const unsigned id = (unsigned)g * 32u + (unsigned)lane;
@@ -85,21 +89,43 @@ __device__ __forceinline__ void tree_walk(const TreeView& t, Pass pass, Leaf lea
     for (;;) {
         const unsigned m = __shfl_sync(ALL, pending, L);
         if (!m) {
-            if (L == t.nlev - 1) return;
+            if (L == top) return;
             ++L;
             g >>= 5;
             continue;
         }
         if (lane == L) pending = m & (m - 1);
         const int id = g * 32 + __ffs(m) - 1;
-        if (L == 0) {
-            if (!leaf(id)) return;
+        if (L == 1) {
+            if (!group(id)) return;
         } else {
             --L;
             g = id;
             open();
         }
     }
+}
+
+// the leaves of group g that pass, as a mask
+template <class Pass>
+__device__ __forceinline__ unsigned group_leaves(const TreeView& t, int g, Pass pass)
+{
+    const unsigned id = (unsigned)g * 32u + (threadIdx.x & 31);
+    bool ok = id < (unsigned)t.cnt[0];
+    if (ok) ok = pass(tree_box(t, 0, (int)id), 0, (int)id);
+    return __ballot_sync(0xffffffffu, ok);
+}
+
+// Visits, in a fixed order, every leaf all of whose ancestors pass; leaf(id) is
+// called by the whole warp and may end the walk by returning false.
+template <class Pass, class Leaf>
+__device__ __forceinline__ void tree_walk(const TreeView& t, Pass pass, Leaf leaf)
+{
+    tree_walk_groups(t, pass, [&](int g) {
+        for (unsigned m = group_leaves(t, g, pass); m; m &= m - 1)
+            if (!leaf(g * 32 + __ffs(m) - 1)) return false;
+        return true;
+    });
 }
 
 }  // namespace asg
