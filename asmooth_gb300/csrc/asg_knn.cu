@@ -51,6 +51,7 @@ constexpr unsigned FULL = 0xffffffffu;
 constexpr int KNN_SLOTS = 32;
 constexpr int KNN_CHUNK = 16;  // candidates between two checks
 static_assert(KNN_SLOTS >= KNN_QUEUE + KNN_CHUNK, "a chunk must fit behind a full flush");
+static_assert(KNN_SLOTS == K_NN - 1 && KNN_SLOTS % KNN_QUEUE == 0 && 3 * KNN_CHUNK >= 32, "a list handed over");
 
 // A warp's shared memory in k_knn_t33, addressed with 32-bit shared addresses: a
 // lane's words lie at `column` (4 x lane into the struct) plus a constant.
@@ -100,12 +101,21 @@ __device__ __forceinline__ void knn_take(float (&v)[KNN_QUEUE], unsigned q0)
     }
 }
 
+// Merges KNN_QUEUE ascending values into the ascending top-33 a[].  tie_out ("a
+// particle outside a[] has d2 == a[32]") stays exact: the values dropped by the
+// merge are all >= the 34th smallest t34, so one of them ties the new a[32] exactly
+// when t34 == a[32]; an earlier tie survives only while a[32] is unchanged.
+__device__ __forceinline__ void knn_take_sorted(float (&a)[K_NN], float (&v)[KNN_QUEUE], bool& tie_out)
+{
+    const float old = a[K_NN - 1];
+    const float t34 = knn_merge33(a, v);
+    const float top = a[K_NN - 1];
+    tie_out = (top == old && tie_out) || t34 == top;
+}
+
 // Merges the up to KNN_QUEUE newest candidates of a lane's queue (at `column`;
 // `slot`: its next free slot) into its ascending top-33 a[] and refills their
-// slots with +inf.  tie_out ("a particle outside a[] has d2 == a[32]") stays
-// exact: the values dropped by the merge are all >= the 34th smallest t34, so
-// one of them ties the new a[32] exactly when t34 == a[32]; an earlier tie
-// survives only while a[32] is unchanged.
+// slots with +inf.
 __device__ __forceinline__ void knn_flush(float (&a)[K_NN], unsigned column, unsigned& slot,
                                           bool& tie_out)
 {
@@ -113,10 +123,17 @@ __device__ __forceinline__ void knn_flush(float (&a)[K_NN], unsigned column, uns
     float v[KNN_QUEUE];
     knn_take<0>(v, slot);
     knn_sort16(v);
-    const float old = a[K_NN - 1];
-    const float t34 = knn_merge33(a, v);
-    const float top = a[K_NN - 1];
-    tie_out = (top == old && tie_out) || t34 == top;
+    knn_take_sorted(a, v, tie_out);
+}
+
+// the largest of SPLIT warps' shared values of a lane, 128 bytes apart
+template <int SPLIT>
+__device__ __forceinline__ float knn_shared_bound(unsigned at)
+{
+    float r = lds_f32<0>(at);
+    if constexpr (SPLIT >= 2) r = fmaxf(r, lds_f32<128>(at));
+    if constexpr (SPLIT >= 4) r = fmaxf(r, fmaxf(lds_f32<256>(at), lds_f32<384>(at)));
+    return r;
 }
 
 // four candidates against the lane's query: the distances two at a time in
@@ -166,17 +183,36 @@ __device__ __forceinline__ void knn_scan(unsigned warp_base, f32x2 qx, f32x2 qy,
 // beyond the largest radius of the bundle.  Keys of the levels above wait in
 // shared memory.  A leaf is scanned if some lane's own radius reaches its box.
 // LEAF16: leaves of 16 particles (the default), one chunk each.
-template <int T33_WARPS, bool LEAF16>
-__global__ void __launch_bounds__(T33_WARPS * 32, 32 / T33_WARPS)
+//
+// SPLIT > 1 (few bundles): the block's SPLIT warps search for the same bundle, each
+// in the leaves of its own (leaf number mod SPLIT), and merge their lists at the
+// end, since one warp's search is a serial chain of some 50 us.  Any SPLIT lists
+// whose SHARE-th values lie within r hold 33 particles within r, so the largest of
+// these values bounds t33 from above: it goes with a[32] into the pruning radius
+// (read without synchronisation: values only shrink, an old one is a looser bound).
+// Particles that it shuts out lie beyond t33, so ties stay exact.  4099 particles
+// 56 -> 28 us, 13,840 in Plummer spheres 75 -> 42.
+template <int T33_WARPS, bool LEAF16, int SPLIT>
+__global__ void __launch_bounds__(T33_WARPS * 32, (SPLIT > 1 ? 16 : 32) / T33_WARPS)
 k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
           float* __restrict__ t33, float* __restrict__ rk, int* __restrict__ idx33,
           int* __restrict__ blist, int* err)
 {
+    static_assert(SPLIT == 1 || (SPLIT == T33_WARPS && LEAF16), "one bundle per block");
+    constexpr int SHARE = (K_NN + SPLIT - 1) / SPLIT;
     __shared__ __align__(16) KnnWarp smem[T33_WARPS];
-    const int lane = threadIdx.x & 31;
+    __shared__ float shares[SPLIT > 1 ? SPLIT : 1][32];  // each warp's a[SHARE - 1]
+    __shared__ int listed;                               // leaves in the bundle's list
+    const int lane = threadIdx.x & 31, part = SPLIT > 1 ? threadIdx.x >> 5 : 0;
     const int n = t.n;
-    const int base = (blockIdx.x * T33_WARPS + (threadIdx.x >> 5)) * 32;
+    const int base = SPLIT > 1 ? blockIdx.x * 32 : (blockIdx.x * T33_WARPS + (threadIdx.x >> 5)) * 32;
     if (base >= n) return;
+    if constexpr (SPLIT > 1) {
+        shares[part][lane] = INFINITY;
+        if (threadIdx.x == 0) listed = 0;
+        __syncthreads();
+    }
+    const unsigned share_at = (unsigned)__cvta_generic_to_shared(&shares[0][lane]);
     KnnWarp& S = smem[threadIdx.x >> 5];
     const unsigned warp_base = (unsigned)__cvta_generic_to_shared(&S);
     const unsigned column = warp_base + 4u * (unsigned)lane;
@@ -215,7 +251,25 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
         g = own0 >> 5;
         const int id = g * 32 + lane;
         if (id < t.cnt[0]) key = id >= own0 && id <= own1 ? (unsigned)lane : child_key(0, id);
+        if (id % SPLIT != part) key = ~0u;
     }
+    // the newest `cnt` entries into the bundle's list
+    auto write_list = [&](int cnt) {
+        int at = nlist - cnt;
+        if constexpr (SPLIT > 1) {
+            if (lane == 0) at = atomicAdd(&listed, cnt);
+            at = __shfl_sync(FULL, at, 0);
+        }
+        if (lane < cnt && at + cnt <= KNN_LIST)
+            blist[(size_t)(base >> 5) * (KNN_LIST + 1) + 1 + at + lane] = entry;
+    };
+    // a lane's t33 is at most this
+    float limit = INFINITY;
+    auto shrink = [&]() {
+        limit = a[K_NN - 1];
+        if constexpr (SPLIT > 1) limit = fminf(limit, knn_shared_bound<SPLIT>(share_at));
+        bound = max(__reduce_max_sync(FULL, __float_as_uint(prune_bound(limit))) | 31u, 63u);
+    };
     int top = 0;  // the highest level opened so far
     for (;;) {
         // ---- the leaves of group g, nearest first ----
@@ -227,12 +281,11 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
             const float4* bp = t.box + 2 * (size_t)id;
             const TreeBox c = {bp[0], bp[1]};
             if (!__any_sync(FULL, point_box_fast(make_float4(lo2(qx), lo2(qy), lo2(qz), 0.f), c) <=
-                                      prune_bound(a[K_NN - 1])))
+                                      prune_bound(SPLIT > 1 ? limit : a[K_NN - 1])))
                 continue;
             if (lane == (nlist & 31)) entry = id;
             ++nlist;
-            if (blist && (nlist & 31) == 0 && nlist <= KNN_LIST)
-                blist[(size_t)(base >> 5) * (KNN_LIST + 1) + 1 + nlist - 32 + lane] = entry;
+            if (blist && (nlist & 31) == 0) write_list(32);
             const int cnt = LEAF16 ? 16 : leaf_count(t, id);
             for (int c0 = 0; c0 < cnt; c0 += KNN_CHUNK) {
                 __syncwarp();  // every lane is done with the chunk before it
@@ -247,12 +300,13 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
                     sts_f32<C + 2 * ROW>(column, p.z);
                 }
                 __syncwarp();
-                knn_scan<0>(warp_base, qx, qy, qz, a[K_NN - 1], slot);
+                knn_scan<0>(warp_base, qx, qy, qz, SPLIT > 1 ? limit : a[K_NN - 1], slot);
                 if (__any_sync(FULL, slot > column + QUEUE_ROW * KNN_QUEUE)) {
                     knn_flush(a, column, slot, tie_out);
-                    bound = max(__reduce_max_sync(FULL, __float_as_uint(prune_bound(a[K_NN - 1]))) | 31u,
-                                63u);
+                    if constexpr (SPLIT > 1) sts_f32<0>(share_at + 128u * part, a[SHARE - 1]);
+                    else shrink();
                 }
+                if constexpr (SPLIT > 1) shrink();
                 if (LEAF16) break;
             }
         }
@@ -288,7 +342,7 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
                 k = c < t.cnt[L] ? child_key(L, c) : ~0u;
                 if (L == 0) {
                     g = id;
-                    key = k;
+                    key = c % SPLIT == part ? k : ~0u;
                     found = true;
                     break;
                 }
@@ -301,11 +355,40 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
     if (__any_sync(FULL, slot > column)) knn_flush(a, column, slot, tie_out);
     // every leaf any lane's final radius reaches was scanned, so the list is
     // complete for k_dens_scatter unless it overflowed
-    if (blist) {
-        int* bl = blist + (size_t)(base >> 5) * (KNN_LIST + 1);
-        if (nlist <= KNN_LIST && lane < (nlist & 31)) bl[1 + (nlist & ~31) + lane] = entry;
-        if (lane == 0) bl[0] = nlist > KNN_LIST ? -1 : nlist;
+    if (blist && (nlist & 31)) write_list(nlist & 31);
+    if constexpr (SPLIT > 1) {
+        __syncthreads();  // nobody prunes by the shared values any more
+        // pairs of warps, pairs of pairs ...: the upper one hands its list over in its
+        // queue's memory, and in `shares` the value of a particle that it left out
+#pragma unroll
+        for (int step = 1; step < SPLIT; step *= 2) {
+            if (part % (2 * step) == step) {
+#pragma unroll
+                for (int k = 0; k < K_NN - 1; ++k) S.queue[k][lane] = a[k];
+                (&S.cand[0][0])[lane] = a[K_NN - 1];
+                shares[part][lane] = tie_out ? a[K_NN - 1] : -1.0f;
+            }
+            __syncthreads();
+            if (part % (2 * step) == 0) {
+                KnnWarp& G = smem[part + step];
+                for (int k0 = 0; k0 < K_NN; k0 += KNN_QUEUE) {
+                    const float first = k0 < KNN_SLOTS ? G.queue[k0][lane] : (&G.cand[0][0])[lane];
+                    if (!__any_sync(FULL, first <= a[K_NN - 1])) break;
+                    float v[KNN_QUEUE];
+                    v[0] = first;
+#pragma unroll
+                    for (int k = 1; k < KNN_QUEUE; ++k)
+                        v[k] = k0 < KNN_SLOTS ? G.queue[k0 + k][lane] : INFINITY;
+                    knn_take_sorted(a, v, tie_out);
+                }
+                tie_out |= shares[part + step][lane] == a[K_NN - 1];
+            }
+            __syncthreads();
+        }
+        nlist = listed;
+        if (part) return;
     }
+    if (blist && lane == 0) blist[(size_t)(base >> 5) * (KNN_LIST + 1)] = nlist > KNN_LIST ? -1 : nlist;
     if (base + lane < n) {
         const float v = a[K_NN - 1];
         t33[base + lane] = v;
@@ -453,22 +536,25 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
 // HALVES (leaves of at most 16 particles): both half-warps hold the leaf's
 // receivers and take every second query, so no lane idles; their integer sums
 // are added by a shuffle before the atomic.
+// PARTS: nparts warps share a bundle's leaves where bundles are few.
 // Bound by instruction issue (82% of slots busy, 11.3 K warp instructions per
-// bundle, of which the distances and weights are half): 7.10 -> 6.47 ms on the
+// bundle, of which the distances and weights are half): 7.10 -> 6.09 ms on the
 // 256^3 step against radix-tree buckets of 22 particles on average.
-template <bool HALVES>
+template <bool HALVES, bool PARTS>
 __global__ void __launch_bounds__(DENS_WARPS * 32)
 k_dens_scatter(const float4* __restrict__ pos, const __grid_constant__ TreeView t, const float* __restrict__ t33,
                const int* __restrict__ idx33, const int* __restrict__ blist,
                const float* __restrict__ rk, const int* __restrict__ dexp,
-               unsigned long long* __restrict__ acc)
+               unsigned long long* __restrict__ acc, int nparts)
 {
     // the queries that reach the leaf at hand: x, y, z, t33 and hinv, hinv^3,
     // idx33 (int bits), then entries that take nothing
     __shared__ float4 qlist[DENS_WARPS][2][32 + 3];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = t.n;
-    const int base = (blockIdx.x * DENS_WARPS + warp) * 32;
+    const int parts = PARTS ? nparts : 1;
+    const int unit = blockIdx.x * DENS_WARPS + warp, part = unit % parts;
+    const int base = unit / parts * 32;
     if (base >= n) return;
     const bool valid = base + lane < n;
     const int q = min(base + lane, n - 1);
@@ -545,7 +631,7 @@ k_dens_scatter(const float4* __restrict__ pos, const __grid_constant__ TreeView 
         for (int i0 = 0; i0 < nlist; i0 += 32) {
             const int cnt = min(32, nlist - i0);
             const int e = lane < cnt ? bl[1 + i0 + lane] : 0;
-            for (int i = 0; i < cnt; ++i) visit(__shfl_sync(FULL, e, i));
+            for (int i = part; i < cnt; i += parts) visit(__shfl_sync(FULL, e, i));
         }
         return;
     }
@@ -555,7 +641,7 @@ k_dens_scatter(const float4* __restrict__ pos, const __grid_constant__ TreeView 
     for (int o = 16; o > 0; o >>= 1) reach = fmaxf(reach, __shfl_xor_sync(FULL, reach, o));
     tree_walk(t, [&](const TreeBox& c, int, int) { return boxes_dist2_fast(box, c) <= reach; },
               [&](int id) {
-                  visit(id);
+                  if (id % parts == part) visit(id);
                   return true;
               });
 }
@@ -573,6 +659,15 @@ __global__ void k_dens_finish(const unsigned long long* __restrict__ acc,
     vel[j] = v;
 }
 
+// Bundles up to which k_knn_t33 puts 4 and 2 warps on each: a search of 20,000 uniform
+// particles takes 60 us with 1, 41 with 2, 40 with 4; 65,000 80, 72, 96; 90,000 87, 89,
+// 120; in Plummer spheres 20,000 87, 61, 52; 65,000 99, 79, 98; 130,000 139, 125, 169.
+// (8 warps: never better than 4.)
+constexpr int KNN_SPLIT4 = 5 * 152, KNN_SPLIT2 = 18 * 152;
+// and k_dens_scatter 8, 4 and 2 (4099 uniform particles 45, 29, 23 and 17 us with 1, 2,
+// 4 and 8; 30,000 49, 35, 27 with 1, 2, 4; 130,000 71, 66 with 1, 2, 200,000 100, 101)
+constexpr int DENS_SPLIT8 = 152, DENS_SPLIT4 = 18 * 152, DENS_SPLIT2 = 32 * 152;
+
 static int knn_blocks(int n) { return (n + KNN_WARPS * 32 - 1) / (KNN_WARPS * 32); }
 
 void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk, int* idx33,
@@ -586,9 +681,16 @@ void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk,
     // Leaves of 16 run one warp per block, so that every warp that ends makes
     // room at once: 11.02 against 11.44 ms in blocks of 2 on the 256^3 step
     // (persistent warps that take bundles by ticket: 11.53).
-    if (t.leaf == 16) run(k_knn_t33<1, true>, 1);
-    else if (warps == 4) run(k_knn_t33<4, false>, 4);
-    else run(k_knn_t33<2, false>, 2);
+    if (t.leaf == 16) {
+        const int bundles = (t.n + 31) / 32;
+        auto split = [&](auto kern, int w) {
+            kern<<<bundles, 32 * w, 0, s>>>(pos, t, t33, rk, idx33, blist, err);
+        };
+        if (bundles <= KNN_SPLIT4) split(k_knn_t33<4, true, 4>, 4);
+        else if (bundles <= KNN_SPLIT2) split(k_knn_t33<2, true, 2>, 2);
+        else run(k_knn_t33<1, true, 1>, 1);
+    } else if (warps == 4) run(k_knn_t33<4, false, 1>, 4);
+    else run(k_knn_t33<2, false, 1>, 2);
     count_launches(1);
 }
 
@@ -606,11 +708,12 @@ void launch_dens(const float4* pos, const TreeView& t, const float* t33, const i
                  float4* vel, cudaStream_t s)
 {
     if (t.n <= 0) return;
-    const int nb = (t.n + 255) / 256, nw = (t.n + DENS_WARPS * 32 - 1) / (DENS_WARPS * 32);
-    if (t.leaf <= 16)
-        k_dens_scatter<true><<<nw, DENS_WARPS * 32, 0, s>>>(pos, t, t33, idx33, blist, rk, dexp, acc);
-    else
-        k_dens_scatter<false><<<nw, DENS_WARPS * 32, 0, s>>>(pos, t, t33, idx33, blist, rk, dexp, acc);
+    const int nb = (t.n + 255) / 256, bundles = (t.n + 31) / 32;
+    const int parts = bundles <= DENS_SPLIT8 ? 8 : bundles <= DENS_SPLIT4 ? 4 : bundles <= DENS_SPLIT2 ? 2 : 1;
+    const unsigned nw = (unsigned)(((long long)bundles * parts + DENS_WARPS - 1) / DENS_WARPS);
+    auto kern = parts > 1 ? (t.leaf <= 16 ? k_dens_scatter<true, true> : k_dens_scatter<false, true>)
+                          : (t.leaf <= 16 ? k_dens_scatter<true, false> : k_dens_scatter<false, false>);
+    kern<<<nw, DENS_WARPS * 32, 0, s>>>(pos, t, t33, idx33, blist, rk, dexp, acc, parts);
     k_dens_finish<<<nb, 256, 0, s>>>(acc, dexp, t.n, vel);
     count_launches(2);
 }
