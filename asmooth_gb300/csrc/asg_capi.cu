@@ -182,6 +182,7 @@ void phase_end(asg_ctx* ctx)
 // engine behind any large device-to-host copy in flight on another stream.
 __global__ void k_read_words(const uint32_t* a, const uint32_t* b, const uint32_t* c, uint32_t* out)
 {
+    grid_begin();
     out[0] = *a;
     if (b) out[1] = *b;
     if (c) out[2] = *c;
@@ -190,7 +191,7 @@ __global__ void k_read_words(const uint32_t* a, const uint32_t* b, const uint32_
 static int read_words(asg_ctx* ctx, const uint32_t* a, const uint32_t* b = nullptr,
                       const uint32_t* c = nullptr)
 {
-    k_read_words<<<1, 1, 0, ctx->s>>>(a, b, c, ctx->h_u32_dev);
+    launch(k_read_words, 1, 1, 0, ctx->s, a, b, c, ctx->h_u32_dev);
     count_launches(1);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(ctx->s));
@@ -969,6 +970,7 @@ int asg_run_fof(asg_ctx* ctx, float ll, int* ngroup)
 
 __global__ static void k_label_range(const int* igrp, int n, int ngrp, int* err)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n && (igrp[i] < 0 || igrp[i] > ngrp)) atomicOr(err, ERR_RANGE);
 }
@@ -984,7 +986,7 @@ int asg_run_remove_small_groups(asg_ctx* ctx, int ngrp, int* nhalo)
     if (int r = grow(ctx, ctx->lab_cnt, 4 * nl)) return r;
     if (int r = grow(ctx, ctx->lab_scan, 4 * nl)) return r;
     if (int r = grow(ctx, ctx->scan_tmp, scan_temp_bytes(nl))) return r;
-    k_label_range<<<(n + 255) / 256, 256, 0, ctx->s>>>(P<int>(ctx->igrp), n, ngrp, ctx->d_err);
+    launch(k_label_range, (n + 255) / 256, 256, 0, ctx->s, P<int>(ctx->igrp), n, ngrp, ctx->d_err);
     count_launches(1);
     if (int r = finish(ctx, "remove_small_groups")) {
         return fail(ctx, r == ASG_ERR_RANGE ? ASG_ERR_ARG : r, "group labels outside [0, ngrp]");

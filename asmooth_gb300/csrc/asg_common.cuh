@@ -29,6 +29,34 @@ constexpr int ERR_BADCELL = 128;   // mixed-precision cell index outside the gri
 constexpr int ERR_SORT = 512;      // a radix sort's look-back gave up
 constexpr int ERR_CAP = 256;       // more deposit pairs than a pre-sized pair array holds
 
+// ---- launches that overlap ---------------------------------------------------
+// Every kernel is launched with `launch`, which lets the device set its grid up
+// while the kernel before it in the stream still runs, and begins with
+// grid_begin(), which waits until that kernel is complete and its writes are
+// visible, then lets the next one be set up in turn.  Between short kernels the setup
+// was 1.5 to 2 us each: 8 launches of a 4099-particle search 109 -> 95 us, 34 of a step
+// of 377 k particles 999 -> 926.
+__device__ __forceinline__ void grid_begin()
+{
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" : : : "memory");
+}
+
+template <class... Params, class... Args>
+inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchAttribute overlap;
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &overlap;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // ---- exact float helpers (reference expression order) ----------------------
 
 // norm2 (nbr_search.cpp:20-25): ((dx*dx + dy*dy) + dz*dz), no contraction

@@ -17,6 +17,7 @@ namespace asg {
 __global__ void k_decode_xv(const float* __restrict__ xv, int n, float s0, float s1, float s2,
                             float4* __restrict__ rec, int* err)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float* r = xv + 6 * (size_t)i;
@@ -28,6 +29,7 @@ __global__ void k_decode_xv(const float* __restrict__ xv, int n, float s0, float
 
 __global__ void k_zip_big(const uint8_t* __restrict__ c8, int ncell, uint32_t* __restrict__ flag)
 {
+    grid_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < ncell) flag[c] = c8[c] == 255 ? 1u : 0u;
     if (c == ncell) flag[c] = 0u;
@@ -38,6 +40,7 @@ __global__ void k_zip_counts(const uint8_t* __restrict__ c8, const uint32_t* __r
                              const int* __restrict__ c32, int n32, int ncell,
                              uint32_t* __restrict__ counts, int* err)
 {
+    grid_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c > ncell) return;
     if (c == ncell) {
@@ -62,6 +65,7 @@ __global__ void k_zip_particles(const uint8_t* __restrict__ off, const int16_t* 
                                 float scale, float v_r2i, float s0, float s1, float s2,
                                 float4* __restrict__ rec)
 {
+    grid_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     // the cell c with start[c] <= p < start[c + 1] (empty cells have equal starts)
@@ -88,7 +92,7 @@ __global__ void k_zip_particles(const uint8_t* __restrict__ off, const int16_t* 
 void launch_decode_xv(const float* xv, int n, const float* shift, float4* rec, int* err, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_decode_xv<<<(n + 255) / 256, 256, 0, s>>>(xv, n, shift[0], shift[1], shift[2], rec, err);
+    launch(k_decode_xv, (n + 255) / 256, 256, 0, s, xv, n, shift[0], shift[1], shift[2], rec, err);
     count_launches(1);
 }
 
@@ -107,9 +111,9 @@ void launch_zip_counts(const uint8_t* c8, const int* c32, int n32, int ncell, vo
     uint32_t* counts = reinterpret_cast<uint32_t*>(b + a);
     void* tmp = b + 2 * a;
     const unsigned grid = (unsigned)((C1 + 255) / 256);
-    k_zip_big<<<grid, 256, 0, s>>>(c8, ncell, rank);
+    launch(k_zip_big, grid, 256, 0, s, c8, ncell, rank);
     exclusive_scan_u32(rank, C1, tmp, s);
-    k_zip_counts<<<grid, 256, 0, s>>>(c8, rank, c32, n32, ncell, counts, err);
+    launch(k_zip_counts, grid, 256, 0, s, c8, rank, c32, n32, ncell, counts, err);
     exclusive_scan_u32(counts, C1, tmp, s);  // counts -> first particle of each cell
     count_launches(2);
     *start = counts;
@@ -120,7 +124,7 @@ void launch_zip_particles(const uint8_t* off, const int16_t* vq, const uint32_t*
                           float4* rec, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_zip_particles<<<(n + 255) / 256, 256, 0, s>>>(off, vq, start, ncell, nc, n, (float)mesh_scale,
+    launch(k_zip_particles, (n + 255) / 256, 256, 0, s, off, vq, start, ncell, nc, n, (float)mesh_scale,
                                                      v_r2i, shift[0], shift[1], shift[2], rec);
     count_launches(1);
 }

@@ -252,6 +252,7 @@ __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restr
                            uint32_t* __restrict__ counts, unsigned long long* __restrict__ pairs,
                            int* err)
 {
+    grid_begin();
     __shared__ unsigned long long block_pairs;  // one atomic per block: 0.57 M on one word took 0.3 ms
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int bundles = (n + 31) / 32;
@@ -314,6 +315,7 @@ __global__ void k_entries(const float4* __restrict__ rec, int n, const __grid_co
                           const uint32_t* __restrict__ offs, uint32_t* __restrict__ keys,
                           uint2* __restrict__ entry, uint32_t cap, int* err)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if ((i & ~31) >= n) return;
     const int lane = threadIdx.x & 31;
@@ -351,6 +353,7 @@ __global__ void k_entries(const float4* __restrict__ rec, int n, const __grid_co
 __global__ void k_pad_entries(uint32_t* __restrict__ keys, uint2* __restrict__ entry,
                               const uint32_t* __restrict__ count, uint32_t cap, uint32_t pad_key)
 {
+    grid_begin();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= cap || j < *count) return;
     keys[j] = pad_key;
@@ -362,6 +365,7 @@ __global__ void k_sorted_entries(const int* __restrict__ order, const uint2* __r
                                  uint32_t count, uint2* __restrict__ list, uint32_t* __restrict__ first,
                                  const int* __restrict__ err)
 {
+    grid_begin();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j == count) first[j] = 0u;
     if (j >= count) return;
@@ -404,6 +408,7 @@ __global__ void k_tile_items(const uint32_t* __restrict__ keys, uint32_t count,
                              uint32_t* __restrict__ tentry, uint32_t* __restrict__ nitems,
                              const int* __restrict__ counters)
 {
+    grid_begin();
     __shared__ uint32_t e[257];
     const int seg = deposit_seg(counters, most);
     const int t = blockIdx.x * 256 + threadIdx.x;
@@ -432,6 +437,7 @@ __global__ void k_item_list(const uint32_t* __restrict__ item_off, int total_til
                             uint32_t max_items, uint32_t* __restrict__ item_tile,
                             uint32_t* __restrict__ merge, int* __restrict__ counters, int* err)
 {
+    grid_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total_tiles) return;
     const uint32_t i0 = item_off[t], i1 = item_off[t + 1];
@@ -597,6 +603,7 @@ k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositP
                 const uint2* __restrict__ list, const uint32_t* __restrict__ first,
                 float* __restrict__ partial, int* __restrict__ counters)
 {
+    grid_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     WarpTile& S = reinterpret_cast<WarpTile*>(smem_raw)[threadIdx.x >> 5];
@@ -854,6 +861,7 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
               const uint32_t* __restrict__ first, float* __restrict__ partial,
               double* __restrict__ item_tot, int* __restrict__ counters)
 {
+    grid_begin();
     constexpr int MX = TileShape<NCH>::X, MY = TileShape<NCH>::Y, MZ = TileShape<NCH>::Z;
     constexpr int MC = TileShape<NCH>::CELLS;
     constexpr int NB = NCH == 1 ? 1 : 3;  // column blocks: n (8 z) or n halo | c vx | vy vz (4 z each)
@@ -1167,6 +1175,7 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
               const int* __restrict__ counters, const float* __restrict__ partial,
               const double* __restrict__ item_tot)
 {
+    grid_begin();
     __shared__ __align__(16) float sums[MERGE_WARPS][PW][128];
     __shared__ double mass[2][MERGE_WARPS];
     const int cells = 1 << (P.shift[0] + P.shift[1] + P.shift[2]);
@@ -1350,7 +1359,7 @@ static void launch_persistent(void (*kern)(KArgs...), int dev, int sms, int thre
     }
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-    kern<<<sms * (per_sm > 0 ? per_sm : 1), threads, smem, s>>>(args...);
+    launch(kern, sms * (per_sm > 0 ? per_sm : 1), threads, smem, s, args...);
 }
 
 void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, const float* rk,
@@ -1360,7 +1369,7 @@ void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, 
     const int bundles = (n + 31) / 32;
     cudaMemsetAsync(w.counters, 0, 32, s);
     auto kern = p.periodic ? k_dep_prep<true> : k_dep_prep<false>;
-    kern<<<(bundles + 7) / 8, 256, 0, s>>>(pos, vel, igrp, rk, n, p, w.rec, w.count,
+    launch(kern, (bundles + 7) / 8, 256, 0, s, pos, vel, igrp, rk, n, p, w.rec, w.count,
                                            reinterpret_cast<unsigned long long*>(w.counters + 2), err);
     exclusive_scan_u32(w.count, (size_t)bundles + 1, w.scan_tmp_n, s);
     count_launches(1);
@@ -1371,23 +1380,23 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
 {
     const int T = total_tiles, bundles = (n + 31) / 32;
     auto kern = p.periodic ? k_entries<true> : k_entries<false>;
-    kern<<<(bundles + 7) / 8, 256, 0, s>>>(w.rec, n, p, w.count, w.keys0, w.entry, entries, err);
+    launch(kern, (bundles + 7) / 8, 256, 0, s, w.rec, n, p, w.count, w.keys0, w.entry, entries, err);
     count_launches(1);
     if (padded && entries > 0) {  // `entries` is the capacity; the count itself is count[bundles]
-        k_pad_entries<<<(entries + 255) / 256, 256, 0, s>>>(w.keys0, w.entry, w.count + bundles, entries,
+        launch(k_pad_entries, (entries + 255) / 256, 256, 0, s, w.keys0, w.entry, w.count + bundles, entries,
                                                             (uint32_t)T << img_bits(p));
         count_launches(1);
     }
     const int cur = radix_sort32(w.keys0, w.vals0, w.keys1, w.vals1, (int)entries,
                                  key_bits(padded ? T + 1 : T, img_bits(p)), true, w.sort_tmp, err, s);
     const uint32_t* keys = cur ? w.keys1 : w.keys0;
-    k_sorted_entries<<<entries / 256 + 1, 256, 0, s>>>(cur ? w.vals1 : w.vals0, w.entry, entries, w.list,
+    launch(k_sorted_entries, entries / 256 + 1, 256, 0, s, cur ? w.vals1 : w.vals0, w.entry, entries, w.list,
                                                        w.first, err);
     exclusive_scan_u32(w.first, (size_t)entries + 1, w.scan_tmp_e, s);
-    k_tile_items<<<T / 256 + 1, 256, 0, s>>>(keys, entries, w.first, T, img_bits(p), p.seg, w.tentry,
+    launch(k_tile_items, T / 256 + 1, 256, 0, s, keys, entries, w.first, T, img_bits(p), p.seg, w.tentry,
                                              w.item_off, w.counters);
     exclusive_scan_u32(w.item_off, (size_t)T + 1, w.scan_tmp_t, s);
-    k_item_list<<<(T + 255) / 256, 256, 0, s>>>(w.item_off, T, max_items, w.item_tile, w.merge,
+    launch(k_item_list, (T + 255) / 256, 256, 0, s, w.item_off, T, max_items, w.item_tile, w.merge,
                                                 w.counters, err);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -1408,7 +1417,7 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
                           w.rec, p, T, w.item_off, max_items, w.item_tile, w.tentry, keys, w.list,
                           w.first, w.partial, w.counters);
     }
-    k_merge_tiles<<<4 * sms, 32 * MERGE_WARPS, 0, s>>>(p, T, w.item_off, w.merge, w.counters,
+    launch(k_merge_tiles, 4 * sms, 32 * MERGE_WARPS, 0, s, p, T, w.item_off, w.merge, w.counters,
                                                        w.partial, item_tot);
     count_launches(5);
 }
@@ -1436,6 +1445,7 @@ __global__ void __launch_bounds__(256)
 k_reduce_partials(const __grid_constant__ DepositParams P, const double* __restrict__ in,
                   double* __restrict__ out)
 {
+    grid_begin();
     __shared__ double r[2][256];
     const int k = blockIdx.y, B = gridDim.x;
     const MeshJob& J = P.job[k];
@@ -1465,19 +1475,20 @@ void launch_deposit_totals(const DepositParams& p, int total_tiles, double* tota
 {
     const unsigned k = (unsigned)p.n_jobs;
     if (total_tiles <= REDUCE_MIN) {
-        k_reduce_partials<<<dim3(1, k), 256, 0, s>>>(p, nullptr, totals);
+        launch(k_reduce_partials, dim3(1, k), 256, 0, s, p, nullptr, totals);
         count_launches(1);
         return;
     }
     double* part = totals + 2 * p.n_jobs;
-    k_reduce_partials<<<dim3(REDUCE_BLOCKS, k), 256, 0, s>>>(p, nullptr, part);
-    k_reduce_partials<<<dim3(1, k), 256, 0, s>>>(p, part, totals);
+    launch(k_reduce_partials, dim3(REDUCE_BLOCKS, k), 256, 0, s, p, nullptr, part);
+    launch(k_reduce_partials, dim3(1, k), 256, 0, s, p, part, totals);
     count_launches(2);
 }
 
 // write_mesh_separate normalisation (coarse_mesh.cpp:158-171), in place
 __global__ void k_normalise(float* __restrict__ mesh, size_t nmesh, float vol)
 {
+    grid_begin();
     const size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nmesh) return;
     float* n = mesh;
@@ -1501,7 +1512,7 @@ __global__ void k_normalise(float* __restrict__ mesh, size_t nmesh, float vol)
 void launch_normalise(float* mesh, int nc, float vol, cudaStream_t s)
 {
     const size_t nmesh = (size_t)nc * nc * nc;
-    k_normalise<<<(unsigned)((nmesh + 255) / 256), 256, 0, s>>>(mesh, nmesh, vol);
+    launch(k_normalise, (unsigned)((nmesh + 255) / 256), 256, 0, s, mesh, nmesh, vol);
     count_launches(1);
 }
 

@@ -63,6 +63,7 @@ __device__ __forceinline__ int uf_union(int* P, int a, int b)
 __global__ void __launch_bounds__(FOF_WARPS * 32)
 k_fof_link(const float4* __restrict__ pos, const __grid_constant__ TreeView t, float ll2, int* P, int* err)
 {
+    grid_begin();
     __shared__ float4 cand[FOF_WARPS][LEAF_MAX];  // x, y, z, root
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = t.n;
@@ -118,7 +119,7 @@ void launch_fof_link(const float4* pos, const TreeView& t, float ll, int* parent
 {
     if (t.n <= 0) return;
     const float ll2 = ll * ll;  // host float multiply: fl(ll*ll) as in fof.cpp:86
-    k_fof_link<<<(t.n + FOF_WARPS * 32 - 1) / (FOF_WARPS * 32), FOF_WARPS * 32, 0, s>>>(
+    launch(k_fof_link, (t.n + FOF_WARPS * 32 - 1) / (FOF_WARPS * 32), FOF_WARPS * 32, 0, s, 
         pos, t, ll2, parent, err);
     count_launches(1);
 }
@@ -128,6 +129,7 @@ void launch_fof_link(const float4* pos, const TreeView& t, float ll, int* parent
 // a group lie close together; then mark[minin[root]] = 1
 __global__ void k_fof_root(const float4* __restrict__ pos, int n, int* P, int* minin)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = i < n ? uf_find(P, i) : -1;
     const int w = i < n ? __float_as_int(pos[i].w) : 0;
@@ -138,6 +140,7 @@ __global__ void k_fof_root(const float4* __restrict__ pos, int n, int* P, int* m
 }
 __global__ void k_fof_mark(int n, const int* P, const int* minin, int* mark)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (P[i] == i) mark[minin[i]] = 1;
@@ -148,14 +151,15 @@ void launch_fof_finish(const float4* pos, int n, int* parent, int* minin, int* m
 {
     if (n <= 0) return;
     const int nb = (n + 255) / 256;
-    k_fof_root<<<nb, 256, 0, s>>>(pos, n, parent, minin);
-    k_fof_mark<<<nb, 256, 0, s>>>(n, parent, minin, mark);
+    launch(k_fof_root, nb, 256, 0, s, pos, n, parent, minin);
+    launch(k_fof_mark, nb, 256, 0, s, n, parent, minin, mark);
     count_launches(2);
 }
 
 __global__ void k_fof_label(int n, const int* __restrict__ P, const int* __restrict__ minin,
                             const uint32_t* __restrict__ scan, int* __restrict__ igrp)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     igrp[i] = (int)scan[minin[P[i]]] + 1;
@@ -166,7 +170,7 @@ void launch_fof_label(const float4* pos, int n, const int* parent, const int* mi
 {
     (void)pos;
     if (n <= 0) return;
-    k_fof_label<<<(n + 255) / 256, 256, 0, s>>>(n, parent, minin, scan, igrp_sorted);
+    launch(k_fof_label, (n + 255) / 256, 256, 0, s, n, parent, minin, scan, igrp_sorted);
     count_launches(1);
 }
 
@@ -177,6 +181,7 @@ void launch_fof_label(const float4* pos, int n, const int* parent, const int* mi
 // counters a queue (345 us on a 128^3 cube).
 __global__ void k_count_labels(const int* __restrict__ igrp, int n, uint32_t* counts)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int g = i < n ? igrp[i] : -1;
     const unsigned peers = __match_any_sync(FM, g);
@@ -185,23 +190,25 @@ __global__ void k_count_labels(const int* __restrict__ igrp, int n, uint32_t* co
 void launch_count_labels(const int* igrp, int n, uint32_t* counts, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_count_labels<<<(n + 255) / 256, 256, 0, s>>>(igrp, n, counts);
+    launch(k_count_labels, (n + 255) / 256, 256, 0, s, igrp, n, counts);
     count_launches(1);
 }
 __global__ void k_keep_mask(uint32_t* counts, int ngrp, int threshold)
 {
+    grid_begin();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g > ngrp) return;
     counts[g] = (g > 0 && counts[g] >= (uint32_t)threshold) ? 1u : 0u;
 }
 void launch_keep_mask(uint32_t* counts, int ngrp, int threshold, cudaStream_t s)
 {
-    k_keep_mask<<<(ngrp + 1 + 255) / 256, 256, 0, s>>>(counts, ngrp, threshold);
+    launch(k_keep_mask, (ngrp + 1 + 255) / 256, 256, 0, s, counts, ngrp, threshold);
     count_launches(1);
 }
 __global__ void k_relabel(int* igrp, int n, const uint32_t* __restrict__ scan,
                           const uint32_t* __restrict__ keep)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int g = igrp[i];
@@ -210,7 +217,7 @@ __global__ void k_relabel(int* igrp, int n, const uint32_t* __restrict__ scan,
 void launch_relabel(int* igrp, int n, const uint32_t* scan, const uint32_t* keep, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_relabel<<<(n + 255) / 256, 256, 0, s>>>(igrp, n, scan, keep);
+    launch(k_relabel, (n + 255) / 256, 256, 0, s, igrp, n, scan, keep);
     count_launches(1);
 }
 
@@ -233,6 +240,7 @@ k_mark_halos(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
              int split, float left, float right, int* __restrict__ igrp, long long* __restrict__ counts,
              double* __restrict__ mass8)
 {
+    grid_begin();
     __shared__ int found[MH_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = (blockIdx.x * MH_WARPS + warp) / split, share = warp % split;
@@ -293,7 +301,7 @@ void launch_mark_halos(const float4* pos, const TreeView& t, const float* halos,
 {
     if (nh <= 0 || t.n <= 0) return;
     const int split = mark_split(nh);
-    k_mark_halos<<<(unsigned)(((long long)nh * split + MH_WARPS - 1) / MH_WARPS), MH_WARPS * 32, 0, s>>>(
+    launch(k_mark_halos, (unsigned)(((long long)nh * split + MH_WARPS - 1) / MH_WARPS), MH_WARPS * 32, 0, s, 
         pos, t, halos, nh, split, left, right, igrp, counts, mass8);
     count_launches(1);
 }

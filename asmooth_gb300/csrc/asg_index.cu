@@ -44,6 +44,7 @@ __global__ void k_unpack_aos(const ParticleRec* __restrict__ aos, int n, float4*
                              float* __restrict__ rkin, KeyGrid grid, uint64_t* __restrict__ keys,
                              int* err)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float* r = reinterpret_cast<const float*>(aos + i);
@@ -59,6 +60,7 @@ __global__ void k_unpack_soa(const float* __restrict__ x3, const float* __restri
                              float4* __restrict__ rec, KeyGrid grid, uint64_t* __restrict__ keys,
                              int* err)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float x = x3[3 * (size_t)i], y = x3[3 * (size_t)i + 1], z = x3[3 * (size_t)i + 2];
@@ -81,6 +83,7 @@ __global__ void k_unpack_quant(const int* __restrict__ cell, const uint16_t* __r
                                float unit, float4* __restrict__ rec, KeyGrid kgrid,
                                uint64_t* __restrict__ keys, int* err)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int c = cell[i];
@@ -108,7 +111,7 @@ void launch_unpack_quant(const int* cell, const uint16_t* off, const float* v, i
 {
     if (n <= 0) return;
     const float unit = cs / 65536.0f;
-    k_unpack_quant<<<(n + 255) / 256, 256, 0, s>>>(cell, off, v, n, grid, left, cs, unit, rec, kgrid,
+    launch(k_unpack_quant, (n + 255) / 256, 256, 0, s, cell, off, v, n, grid, left, cs, unit, rec, kgrid,
                                                     keys, err);
     count_launches(1);
 }
@@ -117,7 +120,7 @@ void launch_unpack_aos(const void* aos, int n, float4* rec, float* rk_in, const 
                        uint64_t* keys, int* err, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_unpack_aos<<<(n + 255) / 256, 256, 0, s>>>((const ParticleRec*)aos, n, rec, rk_in, grid, keys, err);
+    launch(k_unpack_aos, (n + 255) / 256, 256, 0, s, (const ParticleRec*)aos, n, rec, rk_in, grid, keys, err);
     count_launches(1);
 }
 
@@ -125,7 +128,7 @@ void launch_unpack_soa(const float* x, const float* v, const float* dens, const 
                        float4* rec, const KeyGrid& grid, uint64_t* keys, int* err, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_unpack_soa<<<(n + 255) / 256, 256, 0, s>>>(x, v, dens, igrp, n, rec, grid, keys, err);
+    launch(k_unpack_soa, (n + 255) / 256, 256, 0, s, x, v, dens, igrp, n, rec, grid, keys, err);
     count_launches(1);
 }
 
@@ -139,12 +142,14 @@ __device__ __forceinline__ float fkey_inv(int i) { return __int_as_float(i >= 0 
 
 __global__ void k_bounds_init(int* lohi)
 {
+    grid_begin();
     lohi[0] = 0x7fffffff;
     lohi[1] = (int)0x80000000;
 }
 
 __global__ void k_bounds(const float4* __restrict__ rec, int n, int* lohi)
 {
+    grid_begin();
     float lo = INFINITY, hi = -INFINITY;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 p = rec[2 * (size_t)i];
@@ -165,6 +170,7 @@ __global__ void k_bounds(const float4* __restrict__ rec, int n, int* lohi)
 __global__ void k_space_keys(const float4* __restrict__ rec, int n, const int* __restrict__ lohi,
                              int hilbert, uint64_t* __restrict__ keys)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     KeyGrid g;
@@ -199,9 +205,9 @@ KeyGrid key_grid(float left, float right)
 void launch_own_keys(const float4* rec, int n, int* d_lohi, uint64_t* keys, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_bounds_init<<<1, 1, 0, s>>>(d_lohi);
-    k_bounds<<<min((n + 255) / 256, 1216), 256, 0, s>>>(rec, n, d_lohi);
-    k_space_keys<<<(n + 255) / 256, 256, 0, s>>>(rec, n, d_lohi, use_hilbert(), keys);
+    launch(k_bounds_init, 1, 1, 0, s, d_lohi);
+    launch(k_bounds, min((n + 255) / 256, 1216), 256, 0, s, rec, n, d_lohi);
+    launch(k_space_keys, (n + 255) / 256, 256, 0, s, rec, n, d_lohi, use_hilbert(), keys);
     count_launches(3);
 }
 
@@ -214,6 +220,7 @@ constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(uint32_t* data, size_t n, uint32_t* sums)
 {
+    grid_begin();
     __shared__ uint32_t warp_tot[32];
     const size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
     uint32_t v[SCAN_ITEMS];
@@ -254,6 +261,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(uint32_t* data, siz
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_add(uint32_t* data, size_t n, const uint32_t* offs)
 {
+    grid_begin();
     const uint32_t o = offs[blockIdx.x];
     const size_t base = (size_t)blockIdx.x * SCAN_TILE;
     for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS)
@@ -275,11 +283,11 @@ void exclusive_scan_u32(uint32_t* data, size_t n, void* temp, cudaStream_t s)
     if (n == 0) return;
     const size_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     uint32_t* sums = (uint32_t*)temp;
-    k_scan_tiles<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(data, n, nb > 1 ? sums : nullptr);
+    launch(k_scan_tiles, (unsigned)nb, SCAN_THREADS, 0, s, data, n, nb > 1 ? sums : nullptr);
     count_launches(1);
     if (nb > 1) {
         exclusive_scan_u32(sums, nb, sums + nb, s);
-        k_scan_add<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(data, n, sums);
+        launch(k_scan_add, (unsigned)nb, SCAN_THREADS, 0, s, data, n, sums);
         count_launches(1);
     }
 }
@@ -346,6 +354,7 @@ template <class K>
 __global__ void __launch_bounds__(RS_THREADS)
 k_rs_hist(const K* __restrict__ keys, int n, int passes, int bits, uint32_t* __restrict__ head)
 {
+    grid_begin();
     __shared__ uint32_t h[RS_HIST];
     __shared__ bool last;
     const int bins = 1 << bits, tid = threadIdx.x;
@@ -430,6 +439,7 @@ k_rs_pass(const K* __restrict__ kin, const int* __restrict__ vin, K* __restrict_
           int* __restrict__ vout, int n, int shift, uint32_t* __restrict__ ticket,
           const uint32_t* __restrict__ start, S* state, int* err)
 {
+    grid_begin();
     constexpr int BINS = 1 << BITS, PER = BINS / RS_THREADS;  // digits per thread, neighbours
     constexpr int ROUNDS = RS_ROUNDS<K>;
     extern __shared__ __align__(16) unsigned char rs_smem[];
@@ -619,6 +629,7 @@ __global__ void __cluster_dims__(RSC_CTAS, 1, 1) __launch_bounds__(RSC_THREADS)
 k_rs_cluster(const K* __restrict__ kin, const int* __restrict__ vin, K* __restrict__ kout,
              int* __restrict__ vout, int n, int passes)
 {
+    grid_begin();
     extern __shared__ __align__(16) unsigned char rs_smem[];
     using Mem = RsCluster<K, R>;
     Mem& M = *reinterpret_cast<Mem*>(rs_smem);
@@ -768,7 +779,7 @@ static bool rs_cluster_t(const K* kin, const int* vin, K* kout, int* vout, int n
         checked.fetch_or(bit);
     }
     if (!(possible.load() & bit)) return false;
-    k_rs_cluster<K, R, CTAS><<<CTAS, RSC_THREADS, cfg.dynamicSmemBytes, s>>>(kin, vin, kout, vout, n, passes);
+    launch(k_rs_cluster<K, R, CTAS>, CTAS, RSC_THREADS, cfg.dynamicSmemBytes, s, kin, vin, kout, vout, n, passes);
     count_launches(1);
     return true;
 }
@@ -817,12 +828,12 @@ static int radix_sort_t(K* keys0, int* vals0, K* keys1, int* vals1, int n, int p
     const size_t per_pass = (size_t)ntiles * BINS;
     cudaMemsetAsync(temp, 0, 4 * (RS_HEAD + RS_HIST) + sizeof(S) * per_pass * passes, s);
     const int blocks = std::min(4 * sms, (int)(((long long)n + 8 * RS_THREADS - 1) / (8 * RS_THREADS)));
-    k_rs_hist<K><<<blocks, RS_THREADS, 0, s>>>(keys0, n, passes, BITS, head);
+    launch(k_rs_hist<K>, blocks, RS_THREADS, 0, s, keys0, n, passes, BITS, head);
     K* kb[2] = {keys0, keys1};
     int* vb[2] = {vals0, vals1};
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
-        k_rs_pass<K, BITS, S><<<ntiles, RS_THREADS, sizeof(RsSmem<K, BITS>), s>>>(
+        launch(k_rs_pass<K, BITS, S>, ntiles, RS_THREADS, sizeof(RsSmem<K, BITS>), s, 
             kb[cur], p == 0 && iota ? nullptr : vb[cur], kb[cur ^ 1], vb[cur ^ 1], n, p * BITS,
             head + p, head + RS_HEAD + p * BINS, state + per_pass * p, err);
         cur ^= 1;
@@ -862,13 +873,14 @@ int radix_sort32(uint32_t* keys0, int* vals0, uint32_t* keys1, int* vals1, int n
 
 __global__ void k_iota(int* a, int n)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[i] = i;
 }
 void launch_iota(int* a, int n, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_iota<<<(n + 255) / 256, 256, 0, s>>>(a, n);
+    launch(k_iota, (n + 255) / 256, 256, 0, s, a, n);
     count_launches(1);
 }
 
@@ -928,6 +940,7 @@ k_gather(int* __restrict__ perm, const float4* __restrict__ rec, const float* __
          float4* __restrict__ pos, float4* __restrict__ vel, int* __restrict__ igrp,
          float* __restrict__ rk, const __grid_constant__ TreeView t)
 {
+    grid_begin();
     const int i = blockIdx.x * GATHER_THREADS + threadIdx.x;
     const bool live = i < n;
     int o = live ? perm[i] : 0;
@@ -970,6 +983,7 @@ template <int G>
 __global__ void k_leaf_boxes(const float4* __restrict__ pos, int n, int leaf, int nleaf,
                              float4* __restrict__ box)
 {
+    grid_begin();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long id = t / G;
     const int r = (int)(t % G);
@@ -985,6 +999,7 @@ __global__ void k_leaf_boxes(const float4* __restrict__ pos, int n, int leaf, in
 __global__ void k_up_boxes(const float4* __restrict__ below, int nbelow, float4* __restrict__ box,
                            int nbox)
 {
+    grid_begin();
     const long long id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     if (id >= nbox) return;
     const long long c = min(id * 32 + (threadIdx.x & 31), (long long)nbelow - 1);
@@ -1002,19 +1017,19 @@ void launch_gather(int* perm, const float4* rec, const float* rk_in, const TreeV
     const unsigned nb = (unsigned)(((long long)t.n + GATHER_THREADS - 1) / GATHER_THREADS);
     int l = 2;
     if (t.leaf == 16) {
-        k_gather<true><<<nb, GATHER_THREADS, 0, s>>>(perm, rec, rk_in, t.n, pos, vel, igrp, rk, t);
+        launch(k_gather<true>, nb, GATHER_THREADS, 0, s, perm, rec, rk_in, t.n, pos, vel, igrp, rk, t);
         count_launches(1);
     } else {
-        k_gather<false><<<nb, GATHER_THREADS, 0, s>>>(perm, rec, rk_in, t.n, pos, vel, igrp, rk, t);
+        launch(k_gather<false>, nb, GATHER_THREADS, 0, s, perm, rec, rk_in, t.n, pos, vel, igrp, rk, t);
         const int g = t.leaf <= 16 ? 16 : 32;
         const unsigned lb = (unsigned)(((long long)t.cnt[0] * g + 255) / 256);
-        if (g == 16) k_leaf_boxes<16><<<lb, 256, 0, s>>>(pos, t.n, t.leaf, t.cnt[0], box);
-        else k_leaf_boxes<32><<<lb, 256, 0, s>>>(pos, t.n, t.leaf, t.cnt[0], box);
+        if (g == 16) launch(k_leaf_boxes<16>, lb, 256, 0, s, pos, t.n, t.leaf, t.cnt[0], box);
+        else launch(k_leaf_boxes<32>, lb, 256, 0, s, pos, t.n, t.leaf, t.cnt[0], box);
         count_launches(2);
         l = 1;
     }
     for (; l < t.nlev; ++l) {
-        k_up_boxes<<<(unsigned)(((long long)t.cnt[l] * 32 + 255) / 256), 256, 0, s>>>(
+        launch(k_up_boxes, (unsigned)(((long long)t.cnt[l] * 32 + 255) / 256), 256, 0, s, 
             box + 2 * t.off[l - 1], t.cnt[l - 1], box + 2 * t.off[l], t.cnt[l]);
         count_launches(1);
     }
@@ -1027,6 +1042,7 @@ __global__ void k_pack_aos(const int* __restrict__ perm, const float4* __restric
                            const float4* __restrict__ vel, const float* __restrict__ rk,
                            const int* __restrict__ igrp, int n, ParticleRec* __restrict__ aos)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int o = perm[i];
@@ -1043,7 +1059,7 @@ void launch_pack_aos(const int* perm, const float4* pos, const float4* vel, cons
                      const int* igrp, int n, void* aos, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_pack_aos<<<(n + 255) / 256, 256, 0, s>>>(perm, pos, vel, rk, igrp, n,
+    launch(k_pack_aos, (n + 255) / 256, 256, 0, s, perm, pos, vel, rk, igrp, n,
                                                 (ParticleRec*)aos);
     count_launches(1);
 }
@@ -1052,6 +1068,7 @@ void launch_pack_aos(const int* perm, const float4* pos, const float4* vel, cons
 __global__ void k_pack_staged(const float4* __restrict__ rec, const float* __restrict__ rk, int n,
                               ParticleRec* __restrict__ aos)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = rec[2 * (size_t)i], v = rec[2 * (size_t)i + 1];
@@ -1066,7 +1083,7 @@ __global__ void k_pack_staged(const float4* __restrict__ rec, const float* __res
 void launch_pack_staged(const float4* rec, const float* rk, int n, void* aos, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_pack_staged<<<(n + 255) / 256, 256, 0, s>>>(rec, rk, n, (ParticleRec*)aos);
+    launch(k_pack_staged, (n + 255) / 256, 256, 0, s, rec, rk, n, (ParticleRec*)aos);
     count_launches(1);
 }
 
@@ -1075,6 +1092,7 @@ __global__ void k_scatter_fields(const int* __restrict__ perm, const float* __re
                                  const float4* __restrict__ vel, const int* __restrict__ igrp,
                                  int n, float* rk_out, float* dens_out, int* igrp_out)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int o = perm[i];
@@ -1087,7 +1105,7 @@ void launch_scatter_fields(const int* perm, const float* rk, const float4* vel, 
                            int n, float* rk_out, float* dens_out, int* igrp_out, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_scatter_fields<<<(n + 255) / 256, 256, 0, s>>>(perm, rk, vel, igrp, n, rk_out, dens_out,
+    launch(k_scatter_fields, (n + 255) / 256, 256, 0, s, perm, rk, vel, igrp, n, rk_out, dens_out,
                                                       igrp_out);
     count_launches(1);
 }

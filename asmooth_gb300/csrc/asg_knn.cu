@@ -198,6 +198,7 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
           float* __restrict__ t33, float* __restrict__ rk, int* __restrict__ idx33,
           int* __restrict__ blist, int* err)
 {
+    grid_begin();
     static_assert(SPLIT == 1 || (SPLIT == T33_WARPS && LEAF16), "one bundle per block");
     constexpr int SHARE = (K_NN + SPLIT - 1) / SPLIT;
     __shared__ __align__(16) KnnWarp smem[T33_WARPS];
@@ -430,6 +431,7 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
            int* __restrict__ idx33, int all, const float* __restrict__ rk, int* __restrict__ dexp,
            unsigned long long* __restrict__ acc, int* err)
 {
+    grid_begin();
     __shared__ float4 cand[KNN_WARPS][LEAF_MAX];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = t.n;
@@ -547,6 +549,7 @@ k_dens_scatter(const float4* __restrict__ pos, const __grid_constant__ TreeView 
                const float* __restrict__ rk, const int* __restrict__ dexp,
                unsigned long long* __restrict__ acc, int nparts)
 {
+    grid_begin();
     // the queries that reach the leaf at hand: x, y, z, t33 and hinv, hinv^3,
     // idx33 (int bits), then entries that take nothing
     __shared__ float4 qlist[DENS_WARPS][2][32 + 3];
@@ -650,6 +653,7 @@ k_dens_scatter(const float4* __restrict__ pos, const __grid_constant__ TreeView 
 __global__ void k_dens_finish(const unsigned long long* __restrict__ acc,
                               const int* __restrict__ dexp, int n, float4* __restrict__ vel)
 {
+    grid_begin();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const double scale = __longlong_as_double((long long)(1023 + dexp[j] - FIX_BITS) << 52);
@@ -675,7 +679,7 @@ void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk,
 {
     if (t.n <= 0) return;
     auto run = [&](auto kern, int w) {
-        kern<<<(unsigned)(((long long)t.n + 32 * w - 1) / (32 * w)), 32 * w, 0, s>>>(
+        launch(kern, (unsigned)(((long long)t.n + 32 * w - 1) / (32 * w)), 32 * w, 0, s, 
             pos, t, t33, rk, idx33, blist, err);
     };
     // Leaves of 16 run one warp per block, so that every warp that ends makes
@@ -684,7 +688,7 @@ void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk,
     if (t.leaf == 16) {
         const int bundles = (t.n + 31) / 32;
         auto split = [&](auto kern, int w) {
-            kern<<<bundles, 32 * w, 0, s>>>(pos, t, t33, rk, idx33, blist, err);
+            launch(kern, bundles, 32 * w, 0, s, pos, t, t33, rk, idx33, blist, err);
         };
         if (bundles <= KNN_SPLIT4) split(k_knn_t33<4, true, 4>, 4);
         else if (bundles <= KNN_SPLIT2) split(k_knn_t33<2, true, 2>, 2);
@@ -699,7 +703,7 @@ void launch_knn_ties(const float4* pos, const TreeView& t, const float* t33, int
                      cudaStream_t s)
 {
     if (t.n <= 0) return;
-    k_knn_ties<<<knn_blocks(t.n), KNN_WARPS * 32, 0, s>>>(pos, t, t33, idx33, all, rk, dexp, acc, err);
+    launch(k_knn_ties, knn_blocks(t.n), KNN_WARPS * 32, 0, s, pos, t, t33, idx33, all, rk, dexp, acc, err);
     count_launches(1);
 }
 
@@ -713,8 +717,8 @@ void launch_dens(const float4* pos, const TreeView& t, const float* t33, const i
     const unsigned nw = (unsigned)(((long long)bundles * parts + DENS_WARPS - 1) / DENS_WARPS);
     auto kern = parts > 1 ? (t.leaf <= 16 ? k_dens_scatter<true, true> : k_dens_scatter<false, true>)
                           : (t.leaf <= 16 ? k_dens_scatter<true, false> : k_dens_scatter<false, false>);
-    kern<<<nw, DENS_WARPS * 32, 0, s>>>(pos, t, t33, idx33, blist, rk, dexp, acc, parts);
-    k_dens_finish<<<nb, 256, 0, s>>>(acc, dexp, t.n, vel);
+    launch(kern, nw, DENS_WARPS * 32, 0, s, pos, t, t33, idx33, blist, rk, dexp, acc, parts);
+    launch(k_dens_finish, nb, 256, 0, s, acc, dexp, t.n, vel);
     count_launches(2);
 }
 

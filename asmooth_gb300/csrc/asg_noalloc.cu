@@ -77,9 +77,9 @@ static NoallocLayout noalloc_layout(size_t n)
     return L;
 }
 
-// 248 bytes per particle in the arrays above plus the radix sort's scratch
-// (radix_sort_temp_bytes) and 256-byte alignment of every array: 304 bytes
-// per particle and 64 KB cover them (noalloc_layout checks the total)
+// About 142 bytes per particle in the arrays above plus the radix sort's scratch
+// (radix_sort_temp_bytes) and 256-byte alignment of every array: 304 bytes per
+// particle and 64 KB cover them (the call checks the total)
 constexpr size_t NOALLOC_BYTES = 304u * (size_t)NOALLOC_MAX_N + 64u * 1024u;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];

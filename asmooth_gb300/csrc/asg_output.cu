@@ -58,6 +58,7 @@ size_t fof_catalogue_bytes(int n, int nhalo) { return cat_layout(n, nhalo).total
 __global__ void k_cat_keys(const float4* __restrict__ pos, const int* __restrict__ igrp, int n,
                            int nhalo, uint32_t* __restrict__ keys, int* __restrict__ vals)
 {
+    grid_begin();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int w = __float_as_int(pos[igrp ? (size_t)j : 2 * (size_t)j].w);
@@ -70,6 +71,7 @@ __global__ void k_cat_keys(const float4* __restrict__ pos, const int* __restrict
 __global__ void k_cat_bounds(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ start,
                              uint32_t* __restrict__ end, const int* __restrict__ err)
 {
+    grid_begin();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n || (*err & ERR_SORT)) return;
     const uint32_t lab = keys[m];
@@ -154,6 +156,7 @@ k_cat_sums(const float4* __restrict__ pos, const float4* __restrict__ vel, int s
            const uint32_t* __restrict__ end, int nhalo, int nbig, float boxsize,
            float* __restrict__ rec, uint32_t* __restrict__ flags)
 {
+    grid_begin();
     constexpr int W = CAT_THREADS / 32;
     __shared__ __align__(16) union Rows {
         CatRows<CAT_THREADS> block;
@@ -182,6 +185,7 @@ k_cat_sums(const float4* __restrict__ pos, const float4* __restrict__ vel, int s
 __global__ void k_cat_compact(const float* __restrict__ rec, const uint32_t* __restrict__ scan,
                               int nhalo, float* __restrict__ out, uint32_t* __restrict__ nlocal)
 {
+    grid_begin();
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h == 0) *nlocal = scan[nhalo];
     if (h >= nhalo || scan[h + 1] == scan[h]) return;
@@ -204,7 +208,7 @@ void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp,
     cudaMemsetAsync(b + L.end, 0, 4 * H, s);
     cudaMemsetAsync(b + L.flags, 0, 4 * H, s);
     if (n > 0) {
-        k_cat_keys<<<(n + 255) / 256, 256, 0, s>>>(pos, igrp, n, nhalo, U(L.keys0),
+        launch(k_cat_keys, (n + 255) / 256, 256, 0, s, pos, igrp, n, nhalo, U(L.keys0),
                                                     I(L.vals0));
         int bits = 0;
         while (bits < 31 && (nhalo >> bits) != 0) ++bits;
@@ -212,18 +216,18 @@ void launch_fof_catalogue(const float4* pos, const float4* vel, const int* igrp,
                                      false, b + L.sort_tmp, err, s);
         const uint32_t* keys = U(cur ? L.keys1 : L.keys0);
         const int* order = I(cur ? L.vals1 : L.vals0);
-        k_cat_bounds<<<(n + 255) / 256, 256, 0, s>>>(keys, n, U(L.start), U(L.end), err);
+        launch(k_cat_bounds, (n + 255) / 256, 256, 0, s, keys, n, U(L.start), U(L.end), err);
         count_launches(2);
         if (nhalo > 0) {
             const int nbig = nhalo < 8192 ? nhalo : 8192, per = CAT_THREADS / 32;
-            k_cat_sums<<<nbig + (nhalo + per - 1) / per, CAT_THREADS, 0, s>>>(
+            launch(k_cat_sums, nbig + (nhalo + per - 1) / per, CAT_THREADS, 0, s, 
                 pos, vel, igrp ? 1 : 2, order, U(L.start), U(L.end), nhalo, nbig, boxsize,
                 reinterpret_cast<float*>(b + L.rec), U(L.flags));
             count_launches(1);
         }
     }
     exclusive_scan_u32(U(L.flags), H, b + L.scan_tmp, s);  // in place: flags -> offsets
-    k_cat_compact<<<(unsigned)((H + 255) / 256), 256, 0, s>>>(
+    launch(k_cat_compact, (unsigned)((H + 255) / 256), 256, 0, s, 
         reinterpret_cast<const float*>(b + L.rec), U(L.flags), nhalo, out, nlocal);
     count_launches(1);
 }

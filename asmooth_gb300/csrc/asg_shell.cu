@@ -22,6 +22,7 @@ namespace asg {
 __global__ void k_shell_bins(const float4* __restrict__ rec, int n, float lt, float rt,
                              uint32_t* __restrict__ keys)
 {
+    grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = rec[2 * (size_t)i];
@@ -34,6 +35,7 @@ __global__ void k_shell_bins(const float4* __restrict__ rec, int n, float lt, fl
 __global__ void k_shell_bounds(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ start,
                                uint32_t* __restrict__ end)
 {
+    grid_begin();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n) return;
     const uint32_t b = keys[m];
@@ -45,6 +47,7 @@ __global__ void k_shell_bounds(const uint32_t* __restrict__ keys, int n, uint32_
 __global__ void k_shell_interior(const float4* __restrict__ rec, const float* __restrict__ rk, int n,
                                  float4* __restrict__ arec, float* __restrict__ ark)
 {
+    grid_begin();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2LL * n) return;
     arec[i] = rec[i];
@@ -57,6 +60,7 @@ __global__ void k_shell_emit(const float4* __restrict__ rec, const float* __rest
                              const uint32_t* __restrict__ start, int n, ShellPlan plan, float L,
                              float4* __restrict__ arec, float* __restrict__ ark)
 {
+    grid_begin();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n) return;
     const int b = (int)keys[m];
@@ -82,6 +86,7 @@ __global__ void k_shell_emit(const float4* __restrict__ rec, const float* __rest
 __global__ void k_shell_keep(const float4* __restrict__ arec, int n, float lo, float hi,
                              uint32_t* __restrict__ flags)
 {
+    grid_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const float4 p = arec[2 * (size_t)k];
@@ -93,6 +98,7 @@ __global__ void k_shell_compact(const float4* __restrict__ arec, const float* __
                                 const uint32_t* __restrict__ scan, float4* __restrict__ rec,
                                 float* __restrict__ rk, KeyGrid grid, uint64_t* __restrict__ keys)
 {
+    grid_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n || scan[k + 1] == scan[k]) return;
     const uint32_t o = scan[k];
@@ -109,11 +115,11 @@ void launch_shell_bins(const float4* rec, int n, float lt, float rt, uint32_t* k
 {
     cudaMemsetAsync(start, 0, 27 * sizeof(uint32_t), s);
     cudaMemsetAsync(end, 0, 27 * sizeof(uint32_t), s);
-    k_shell_bins<<<(n + 255) / 256, 256, 0, s>>>(rec, n, lt, rt, keys0);
+    launch(k_shell_bins, (n + 255) / 256, 256, 0, s, rec, n, lt, rt, keys0);
     const int cur = radix_sort32(keys0, vals0, keys1, vals1, n, 5, true, sort_tmp, err, s);
     *keys = cur ? keys1 : keys0;
     *order = cur ? vals1 : vals0;
-    k_shell_bounds<<<(n + 255) / 256, 256, 0, s>>>(*keys, n, start, end);
+    launch(k_shell_bounds, (n + 255) / 256, 256, 0, s, *keys, n, start, end);
     count_launches(2);
 }
 
@@ -121,8 +127,8 @@ void launch_shell_emit(const float4* rec, const float* rk, const uint32_t* keys,
                        const uint32_t* start, int n, const ShellPlan& plan, float L, float4* arec,
                        float* ark, cudaStream_t s)
 {
-    k_shell_interior<<<(unsigned)((2LL * n + 255) / 256), 256, 0, s>>>(rec, rk, n, arec, ark);
-    k_shell_emit<<<(n + 255) / 256, 256, 0, s>>>(rec, rk, keys, order, start, n, plan, L, arec, ark);
+    launch(k_shell_interior, (unsigned)((2LL * n + 255) / 256), 256, 0, s, rec, rk, n, arec, ark);
+    launch(k_shell_emit, (n + 255) / 256, 256, 0, s, rec, rk, keys, order, start, n, plan, L, arec, ark);
     count_launches(2);
 }
 
@@ -131,9 +137,9 @@ void launch_shell_filter(const float4* arec, const float* ark, int n_all, float 
                          uint64_t* out_keys, cudaStream_t s)
 {
     cudaMemsetAsync(flags + n_all, 0, sizeof(uint32_t), s);
-    k_shell_keep<<<(n_all + 255) / 256, 256, 0, s>>>(arec, n_all, lo, hi, flags);
+    launch(k_shell_keep, (n_all + 255) / 256, 256, 0, s, arec, n_all, lo, hi, flags);
     exclusive_scan_u32(flags, (size_t)n_all + 1, scan_tmp, s);
-    k_shell_compact<<<(n_all + 255) / 256, 256, 0, s>>>(arec, ark, n_all, flags, rec, rk, grid, out_keys);
+    launch(k_shell_compact, (n_all + 255) / 256, 256, 0, s, arec, ark, n_all, flags, rec, rk, grid, out_keys);
     count_launches(2);
 }
 
