@@ -43,6 +43,13 @@ struct MeshBuf {
     size_t words = 0;
 };
 
+// words that the device stores for the host; `number` comes last, in a line of its own
+struct HostWords {
+    uint32_t number, pad[31];
+    int err;
+    uint32_t word[64];
+};
+
 }  // namespace
 
 struct asg_ctx {
@@ -51,7 +58,12 @@ struct asg_ctx {
     cudaStream_t s_out = nullptr;      // per-particle outputs copied out while the deposit runs
     cudaEvent_t fields_ready = nullptr;
     int* d_err = nullptr;
-    int* h_err = nullptr;  // pinned
+    HostWords* host = nullptr;      // pinned, mapped: what fetch() brings
+    HostWords* host_dev = nullptr;  // its device address
+    uint32_t fetches = 0;
+    int polls = 0;  // looks at host->number before a synchronisation
+    unsigned char* h_mark = nullptr;  // pinned: the halos' counts and masses
+    size_t h_mark_bytes = 0;
     std::string last;
 
     // loaded particle set
@@ -80,8 +92,6 @@ struct asg_ctx {
     bool dec_rk = false;    // they have smoothing lengths
     uint32_t dep_npairs = 0, dep_nentries = 0;
     int dep_tiles_n = 0, dep_cells = 0;  // tiles of the last deposit, cells of one
-    uint32_t* h_u32 = nullptr;      // pinned, mapped
-    uint32_t* h_u32_dev = nullptr;  // its device address
     float mesh_boxsize = 0.0f;
     std::vector<MeshBuf> meshes;
 
@@ -177,34 +187,53 @@ void phase_end(asg_ctx* ctx)
     ctx->open_phase = -1;
 }
 
-// Reads up to three device words into ctx->h_u32 and waits for them.  A kernel
-// stores them through the mapped host words: a copy would queue on the copy
-// engine behind any large device-to-host copy in flight on another stream.
-__global__ void k_read_words(const uint32_t* a, const uint32_t* b, const uint32_t* c, uint32_t* out)
+// `n` words at p
+struct Words {
+    const void* p = nullptr;
+    int n = 0;
+};
+
+__global__ void k_report(Words a, Words b, Words c, const int* err, HostWords* out, uint32_t number)
 {
     grid_begin();
-    out[0] = *a;
-    if (b) out[1] = *b;
-    if (c) out[2] = *c;
+    const int i = threadIdx.x;
+    const Words w = i < a.n ? a : i < a.n + b.n ? b : c;
+    const int at = i < a.n ? i : i < a.n + b.n ? i - a.n : i - a.n - b.n;
+    if (i < a.n + b.n + c.n) out->word[i] = static_cast<const uint32_t*>(w.p)[at];
+    if (i == 0) out->err = *err;
+    __threadfence_system();
+    __syncthreads();
+    if (i == 0) asm volatile("st.release.sys.global.u32 [%0], %1;" : : "l"(&out->number), "r"(number) : "memory");
 }
 
-static int read_words(asg_ctx* ctx, const uint32_t* a, const uint32_t* b = nullptr,
-                      const uint32_t* c = nullptr)
+// Waits for the work queued on ctx->s and brings the error word and up to 64 other
+// words to ctx->host.  A kernel stores them through the mapped host memory and the
+// host watches for its number: a copy of a few bytes and the end of a
+// synchronisation took 8 us more, and the copy would queue on the copy engine behind
+// any large device-to-host copy on another stream.  After HOST_POLLS looks (a few
+// milliseconds; a synchronisation spins as long as it takes) the host waits for the
+// stream instead, which also reports what made the kernels fail.  No looks where the
+// device is set to block or yield in a synchronisation.
+constexpr int HOST_POLLS = 1000000;
+static int fetch(asg_ctx* ctx, Words a = {}, Words b = {}, Words c = {})
 {
-    launch(k_read_words, 1, 1, 0, ctx->s, a, b, c, ctx->h_u32_dev);
+    const uint32_t number = ++ctx->fetches;
+    launch(k_report, 1, 64, 0, ctx->s, a, b, c, ctx->d_err, ctx->host_dev, number);
     count_launches(1);
     CK(cudaGetLastError());
+    for (int i = 0; i < ctx->polls; ++i)
+        if (__atomic_load_n(&ctx->host->number, __ATOMIC_ACQUIRE) == number) return 0;
     CK(cudaStreamSynchronize(ctx->s));
     return 0;
 }
 
-// wait for the queued work and report device-side and launch errors
-int finish(asg_ctx* ctx, const char* what)
+// wait for the queued work and report device-side and launch errors; `a` as fetch()
+int finish(asg_ctx* ctx, const char* what, Words a = {})
 {
-    CK(cudaMemcpyAsync(ctx->h_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->s));
-    CK(cudaStreamSynchronize(ctx->s));
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(ctx, e, what);
+    if (int r = fetch(ctx, a)) {
+        cudaGetLastError();
+        return fail(ctx, r, std::string(what) + ": " + ctx->last);
+    }
     for (auto& pe : ctx->pending) {
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, pe.second.first, pe.second.second) == cudaSuccess)
@@ -213,7 +242,7 @@ int finish(asg_ctx* ctx, const char* what)
     ctx->pending.clear();
     ctx->ev_used = 0;
     ctx->open_phase = -1;
-    const int bits = *ctx->h_err;
+    const int bits = ctx->host->err;
     if (bits) {
         CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->s));
         CK(cudaStreamSynchronize(ctx->s));
@@ -221,6 +250,15 @@ int finish(asg_ctx* ctx, const char* what)
                     std::string(what) + ": device error bits " + std::to_string(bits));
     }
     return ASG_OK;
+}
+
+// finish() with the FP64 totals of n_nc meshes into totals (null: none)
+int finish_totals(asg_ctx* ctx, const char* what, int n_nc, double* totals)
+{
+    if (!totals) return finish(ctx, what);
+    const int r = finish(ctx, what, Words{ctx->totals.p, 4 * n_nc});
+    if (r != ASG_ERR_CUDA) std::memcpy(totals, ctx->host->word, 16 * (size_t)n_nc);
+    return r;
 }
 
 TreeView tree_view(asg_ctx* ctx)
@@ -434,9 +472,12 @@ int asg_create(asg_ctx** out, int device)
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->s_out, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->fields_ready, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_err, sizeof(int));
-    if (e == cudaSuccess) e = cudaHostAlloc(&ctx->h_u32, 4 * sizeof(uint32_t), cudaHostAllocMapped);
-    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&ctx->h_u32_dev, ctx->h_u32, 0);
+    if (e == cudaSuccess) e = cudaHostAlloc(&ctx->host, sizeof(HostWords), cudaHostAllocMapped);
+    if (e == cudaSuccess) std::memset(ctx->host, 0, sizeof(HostWords));
+    unsigned flags = 0;
+    if (e == cudaSuccess) e = cudaGetDeviceFlags(&flags);
+    if (!(flags & (cudaDeviceScheduleBlockingSync | cudaDeviceScheduleYield))) ctx->polls = HOST_POLLS;
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&ctx->host_dev, ctx->host, 0);
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->s);
     if (e != cudaSuccess) {
@@ -471,8 +512,8 @@ void asg_destroy(asg_ctx* ctx)
     }
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     if (ctx->d_err) cudaFree(ctx->d_err);
-    if (ctx->h_err) cudaFreeHost(ctx->h_err);
-    if (ctx->h_u32) cudaFreeHost(ctx->h_u32);
+    if (ctx->host) cudaFreeHost(ctx->host);
+    if (ctx->h_mark) cudaFreeHost(ctx->h_mark);
     if (ctx->s) cudaStreamDestroy(ctx->s);
     if (ctx->s_out) {
         cudaStreamSynchronize(ctx->s_out);
@@ -536,12 +577,10 @@ static int load_shell(asg_ctx* ctx, int np, float boxsize, float bf, int* np_wit
     const int* order = nullptr;
     launch_shell_bins(F4(L.rec), np, lt, rt, U(L.k0), I(L.v0), U(L.k1), I(L.v1), b + L.tmp,
                       U(L.start), U(L.end), &keys, &order, ctx->d_err, ctx->s);
+    if (int r = fetch(ctx, {b + L.start, 27}, {b + L.end, 27})) return r;
     uint32_t se[54];
-    CK(cudaMemcpyAsync(se, b + L.start, 27 * 4, cudaMemcpyDeviceToHost, ctx->s));
-    CK(cudaMemcpyAsync(se + 27, b + L.end, 27 * 4, cudaMemcpyDeviceToHost, ctx->s));
-    CK(cudaMemcpyAsync(ctx->h_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->s));
-    CK(cudaStreamSynchronize(ctx->s));
-    if (*ctx->h_err & ERR_SORT) return finish(ctx, "shell sort");
+    std::memcpy(se, ctx->host->word, sizeof(se));
+    if (ctx->host->err & ERR_SORT) return finish(ctx, "shell sort");
     // the reference's send loop order (exchange_buffer.cpp:120-150): source bin, then direction
     ShellPlan plan;
     size_t off = (size_t)np;
@@ -575,10 +614,10 @@ static int load_shell(asg_ctx* ctx, int np, float boxsize, float bf, int* np_wit
                         P<float4>(ctx->rec_in), rk ? P<float>(ctx->rk_in) : nullptr,
                         key_grid(-dx, boxsize + dx), P<uint64_t>(ctx->keys0), ctx->s);
     phase_end(ctx);
-    if (int r = read_words(ctx, flags + n_all, flags + np)) return r;
-    const int n = (int)ctx->h_u32[0];
+    if (int r = fetch(ctx, {flags + n_all, 1}, {flags + np, 1})) return r;
+    const int n = (int)ctx->host->word[0];
     if (np_with) *np_with = n;
-    if (np_local) *np_local = (int)ctx->h_u32[1];
+    if (np_local) *np_local = (int)ctx->host->word[1];
     if (n < K_NN) return fail(ctx, ASG_ERR_FEW, "fewer than 33 particles with the shell");
     ctx->n = n;
     ctx->left = -dx;
@@ -756,10 +795,9 @@ int asg_decode_zip(asg_ctx* ctx, const uint8_t* zip0, const int16_t* zip1, const
     uint32_t* start = nullptr;
     launch_zip_counts(raw, reinterpret_cast<const int*>(raw + o3), n_zip3, ncell, ctx->dec_scan.p,
                       &start, ctx->d_err, ctx->s);
-    CK(cudaMemcpyAsync(ctx->h_u32, start + ncell, 4, cudaMemcpyDeviceToHost, ctx->s));
-    if (int r = finish(ctx, "decode_zip counts")) return r;
-    if (ctx->h_u32[0] != (uint32_t)np_local)  // file_reader2.cpp:261-264
-        return fail(ctx, ASG_ERR_ARG, "zip cell counts sum to " + std::to_string(ctx->h_u32[0]) +
+    if (int r = finish(ctx, "decode_zip counts", {start + ncell, 1})) return r;
+    if (ctx->host->word[0] != (uint32_t)np_local)  // file_reader2.cpp:261-264
+        return fail(ctx, ASG_ERR_ARG, "zip cell counts sum to " + std::to_string(ctx->host->word[0]) +
                                           ", the header says " + std::to_string(np_local));
     unsigned char* b = P<unsigned char>(ctx->sh_in);
     launch_zip_particles(raw + o0, reinterpret_cast<const int16_t*>(raw + o1), start, ncell, nc,
@@ -905,23 +943,30 @@ static int queue_mark(asg_ctx* ctx, const asg_halo* halos, int nh)
                       ctx->right, P<int>(ctx->igrp), P<long long>(ctx->hcount),
                       P<double>(ctx->hmass), ctx->s);
     phase_end(ctx);
+    const size_t bytes = 8 * (size_t)nh;
+    if (ctx->h_mark_bytes < 2 * bytes) {
+        if (ctx->h_mark) cudaFreeHost(ctx->h_mark);
+        ctx->h_mark = nullptr;
+        ctx->h_mark_bytes = 0;
+        CK(cudaMallocHost(&ctx->h_mark, 2 * bytes));
+        ctx->h_mark_bytes = 2 * bytes;
+    }
+    CK(cudaMemcpyAsync(ctx->h_mark, ctx->hcount.p, bytes, cudaMemcpyDeviceToHost, ctx->s));
+    CK(cudaMemcpyAsync(ctx->h_mark + bytes, ctx->hmass.p, bytes, cudaMemcpyDeviceToHost, ctx->s));
     return 0;
 }
 
+// after finish()
 static int collect_mark(asg_ctx* ctx, int nh, long* np_halo, double* m_halo)
 {
     long tot = 0;
     double mh = 0.0;
     if (nh > 0) {
-        std::vector<long long> cnt((size_t)nh);
-        std::vector<double> m8((size_t)nh);
-        CK(cudaMemcpy(cnt.data(), ctx->hcount.p, sizeof(long long) * (size_t)nh,
-                      cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(m8.data(), ctx->hmass.p, sizeof(double) * (size_t)nh,
-                      cudaMemcpyDeviceToHost));
+        const long long* cnt = reinterpret_cast<const long long*>(ctx->h_mark);
+        const double* m8 = reinterpret_cast<const double*>(ctx->h_mark) + nh;
         for (int i = 0; i < nh; ++i) {  // halo order, as the reference's serial loop
-            tot += (long)cnt[(size_t)i];
-            mh += m8[(size_t)i];
+            tot += (long)cnt[i];
+            mh += m8[i];
         }
     }
     if (np_halo) *np_halo = tot;
@@ -961,10 +1006,8 @@ int asg_run_fof(asg_ctx* ctx, float ll, int* ngroup)
     launch_fof_label(P<float4>(ctx->pos), n, P<int>(ctx->uf), P<int>(ctx->minin),
                      P<uint32_t>(ctx->mark), P<int>(ctx->igrp), ctx->s);
     phase_end(ctx);
-    uint32_t ng = 0;
-    CK(cudaMemcpyAsync(&ng, P<uint32_t>(ctx->mark) + n, 4, cudaMemcpyDeviceToHost, ctx->s));
-    if (int r = finish(ctx, "fof")) return r;
-    *ngroup = (int)ng;
+    if (int r = finish(ctx, "fof", {P<uint32_t>(ctx->mark) + n, 1})) return r;
+    *ngroup = (int)ctx->host->word[0];
     return 0;
 }
 
@@ -999,11 +1042,8 @@ int asg_run_remove_small_groups(asg_ctx* ctx, int ngrp, int* nhalo)
     exclusive_scan_u32(P<uint32_t>(ctx->lab_scan), nl, ctx->scan_tmp.p, ctx->s);
     launch_relabel(P<int>(ctx->igrp), n, P<uint32_t>(ctx->lab_scan), P<uint32_t>(ctx->lab_cnt),
                    ctx->s);
-    uint32_t nh = 0;
-    CK(cudaMemcpyAsync(&nh, P<uint32_t>(ctx->lab_scan) + ngrp + 1, 4, cudaMemcpyDeviceToHost,
-                       ctx->s));
-    if (int r = finish(ctx, "remove_small_groups")) return r;
-    *nhalo = (int)nh;
+    if (int r = finish(ctx, "remove_small_groups", {P<uint32_t>(ctx->lab_scan) + ngrp + 1, 1})) return r;
+    *nhalo = (int)ctx->host->word[0];
     return 0;
 }
 
@@ -1095,10 +1135,10 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
         have = *cap;
     } else {
         const uint32_t* pairs = reinterpret_cast<uint32_t*>(w.counters + 2);
-        if (int r = read_words(ctx, w.count + (B1 - 1), pairs, pairs + 1)) return r;
-        have.entries = ctx->h_u32[0];
-        have.pairs = ctx->h_u32[1];
-        if (ctx->h_u32[2] || have.pairs > (uint32_t)INT_MAX) {  // past the 32-bit pair numbers
+        if (int r = fetch(ctx, {w.count + (B1 - 1), 1}, {pairs, 2})) return r;
+        have.entries = ctx->host->word[0];
+        have.pairs = ctx->host->word[1];
+        if (ctx->host->word[2] || have.pairs > (uint32_t)INT_MAX) {  // past the 32-bit pair numbers
             phase_end(ctx);
             if (!p.mma) return fail(ctx, ASG_ERR_ARG, "more than 2^31 - 1 (particle, tile) pairs");
             return queue_deposit(ctx, boxsize, ncs, n_nc, sign, periodic, coords, density_only, cap,
@@ -1159,9 +1199,7 @@ int asg_run_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, int s
     CK(cudaSetDevice(ctx->device));
     if (int r = queue_deposit(ctx, boxsize, ncs, n_nc, sign, periodic, coords, density_only))
         return r;
-    if (totals)
-        CK(cudaMemcpyAsync(totals, ctx->totals.p, 16 * (size_t)n_nc, cudaMemcpyDeviceToHost, ctx->s));
-    return finish(ctx, "deposit");
+    return finish_totals(ctx, "deposit", n_nc, totals);
 }
 
 float* asg_mesh_device(asg_ctx* ctx, int k)
@@ -1357,9 +1395,8 @@ static int run_catalogue(asg_ctx* ctx, const float4* pos, const float4* vel, con
                          ctx->s);
     if (nhalo > 0) CK(cudaMemcpyAsync(out, ob, sizeof(asg_fof_halo) * (size_t)nhalo,
                                       cudaMemcpyDeviceToHost, ctx->s));
-    CK(cudaMemcpyAsync(ctx->h_u32, ob + o_cnt, 4, cudaMemcpyDeviceToHost, ctx->s));
-    if (int r = finish(ctx, "fof_halos")) return r;
-    *nlocal = (int)ctx->h_u32[0];
+    if (int r = finish(ctx, "fof_halos", {ob + o_cnt, 1})) return r;
+    *nlocal = (int)ctx->host->word[0];
     return ASG_OK;
 }
 
@@ -1537,9 +1574,7 @@ int asg_smooth(asg_ctx* ctx, asg_particle* p, int np, float left, float right, f
     if (!rd) queue_mesh_out(ctx, n_nc, meshes);
     CK(cudaStreamSynchronize(ctx->s_out));  // the records and meshes are out before any return
     if (rd) return rd;
-    if (totals)
-        CK(cudaMemcpyAsync(totals, ctx->totals.p, 16 * (size_t)n_nc, cudaMemcpyDeviceToHost, ctx->s));
-    if (int r = finish(ctx, "smooth")) return r;
+    if (int r = finish_totals(ctx, "smooth", n_nc, totals)) return r;
     return collect_mark(ctx, nh, np_halo, m_halo);
 }
 
@@ -1576,9 +1611,7 @@ int asg_smooth_quantised(asg_ctx* ctx, const int* cell, const uint16_t* off, con
     if (!rd) queue_mesh_out(ctx, n_nc, meshes);
     CK(cudaStreamSynchronize(ctx->s_out));  // rk, dens and the meshes are out before any return
     if (rd) return rd;
-    if (totals)
-        CK(cudaMemcpyAsync(totals, ctx->totals.p, 16 * (size_t)n_nc, cudaMemcpyDeviceToHost, ctx->s));
-    return finish(ctx, "smooth_quantised");
+    return finish_totals(ctx, "smooth_quantised", n_nc, totals);
 }
 
 }  // extern "C"
