@@ -105,6 +105,20 @@ __device__ __forceinline__ f32x2 sq2_rn(f32x2 d)
     return r;
 }
 
+// fl(a * b) likewise, a product of -0 becoming +0
+__device__ __forceinline__ f32x2 mul2_rn(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(0ull));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2_rn(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 // norm2_rn from the point (ax, ay, az), each coordinate given twice, to two
 // points (their x, y and z pairs): the same roundings in the same order
 __device__ __forceinline__ f32x2 norm2_rn_x2(f32x2 ax, f32x2 ay, f32x2 az, f32x2 bx, f32x2 by,
@@ -221,6 +235,15 @@ __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x)
     const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bp)), __fsub_rn(x, bp));
     hi = s;
     lo = __fadd_rn(lo, e);
+}
+// two_sum_acc of two elements: the same operations, packed
+__device__ __forceinline__ void two_sum_acc_x2(f32x2& hi, f32x2& lo, f32x2 x)
+{
+    const f32x2 s = add2_rn(hi, x);
+    const f32x2 bp = sub2_rn(s, hi);
+    const f32x2 e = add2_rn(sub2_rn(hi, sub2_rn(s, bp)), sub2_rn(x, bp));
+    hi = s;
+    lo = add2_rn(lo, e);
 }
 
 // ---- Morton keys ------------------------------------------------------------

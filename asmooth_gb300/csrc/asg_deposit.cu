@@ -451,44 +451,48 @@ __global__ void k_item_list(const uint32_t* __restrict__ item_off, int total_til
 }
 
 // The pairs of one work item, 32 at a time: lane l of chunk c has pair 32 c + l.
-// A chunk spans at most 32 entries, which the lanes load together.
+// A chunk spans at most 32 entries, which the lanes load together; the entries then
+// place their particles one after another, a lane of the bundle each (about four
+// entries a chunk; searching each pair's entry and bit took twice the instructions).
 struct PairCursor {
     const uint2* list;
     const uint32_t* first;
     uint32_t at, end;  // the entry of the next chunk's first pair, the tile's last + 1
+    uint32_t f;        // of entry at + lane, loaded a chunk ahead: its first pair
+    uint2 e;           // and itself
 
-    // particle and entry number of pair j (consecutive over the lanes, from the
-    // chunk's first pair on, all but the first chunk following the one before);
-    // lanes with j >= j1 get -1
-    __device__ __forceinline__ int take(uint32_t j, uint32_t j1, uint32_t& which)
+    __device__ __forceinline__ void load()
+    {
+        const uint32_t mine = at + (threadIdx.x & 31);
+        f = mine < end ? first[mine] : 0xffffffffu;
+        e = mine < end ? list[mine] : make_uint2(0u, 0u);
+    }
+
+    // particle and entry number of pair j0 + lane (j0 from chunk to chunk 32 on);
+    // lanes past j1 get -1.  box: 32 words of the warp's shared memory
+    __device__ __forceinline__ int take(uint32_t j0, uint32_t j1, int2* box, uint32_t& which)
     {
         const int lane = threadIdx.x & 31;
-        const uint32_t mine = at + lane;
-        const uint32_t f = mine < end ? first[mine] : 0xffffffffu;
-        const uint2 e = mine < end ? list[mine] : make_uint2(0u, 0u);
-        int l = 0;  // the last of the 32 entries that starts at or before pair j
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1)
-            if (__shfl_sync(FULLM, f, l + s) <= j) l += s;
-        const uint32_t start = __shfl_sync(FULLM, f, l);
-        unsigned m = __shfl_sync(FULLM, e.y, l);
-        const uint32_t w = __shfl_sync(FULLM, e.x, l);
-        which = at + l;
-        // on to the entry of the pair after lane 31's
-        at += __shfl_sync(FULLM, l + (j - start + 1u == (uint32_t)__popc(m) ? 1 : 0), 31);
-        if (j >= j1) return -1;
-        // the (j - start)-th set bit of the mask
-        int k = (int)(j - start), bit = 0;
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1) {
-            const int c = __popc(m & ((1u << s) - 1u));
-            if (k >= c) {
-                k -= c;
-                m >>= s;
-                bit += s;
-            }
+        const uint32_t stop = min(j0 + 32u, j1);
+        const int n = __popc(__ballot_sync(FULLM, f < stop));  // first[] rises: the lanes below n
+        for (int k = 0; k < n; ++k) {
+            const uint32_t start = __shfl_sync(FULLM, f, k), m = __shfl_sync(FULLM, e.y, k);
+            const uint32_t w = __shfl_sync(FULLM, e.x, k);
+            const uint32_t to = start + (uint32_t)__popc(m & lanemask_lt()) - j0;  // wraps before j0
+            if ((m >> lane & 1u) && to < 32u) box[to] = make_int2((int)(w * 32u) + lane, k);
         }
-        return (int)(w * 32u) + bit;
+        __syncwarp();
+        const int2 got = box[lane];
+        const uint32_t j = j0 + (uint32_t)lane;
+        which = at + (uint32_t)got.y;
+        // on to the last of these entries, or past it when its pairs end here
+        if (n > 0) {
+            const uint32_t last = __shfl_sync(FULLM, f + (uint32_t)__popc(e.y), n - 1);
+            at += (uint32_t)(n - 1) + (last <= stop ? 1u : 0u);
+        }
+        load();
+        __syncwarp();  // `box` may be written again
+        return j < j1 ? got.x : -1;
     }
 };
 __device__ __forceinline__ PairCursor open_pairs(const uint2* __restrict__ list,
@@ -500,7 +504,9 @@ __device__ __forceinline__ PairCursor open_pairs(const uint2* __restrict__ list,
         const uint32_t mid = lo + ((hi - lo) >> 1);
         if (first[mid] <= j0) lo = mid; else hi = mid;
     }
-    return {list, first, lo, e1};
+    PairCursor c{list, first, lo, e1, 0u, make_uint2(0u, 0u)};
+    c.load();
+    return c;
 }
 
 // ---------------------------------------------------------------------------
@@ -642,7 +648,7 @@ k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositP
             float4 val = make_float4(0.f, 0.f, 0.f, 0.f);
             {
                 uint32_t which;
-                const int i = pairs.take(c0 + lane, j1, which);
+                const int i = pairs.take(c0, j1, reinterpret_cast<int2*>(S.w), which);
                 if (i >= 0) {
                     const int combo = periodic ? (int)(ekeys[which] & ((1u << IMG_BITS) - 1u)) : 0;
                     const int dk[3] = {combo % 3, (combo / 3) % 3, combo / 9};
@@ -775,17 +781,27 @@ k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositP
 // One warp per item and CTA: no barriers, and a warp that waits for its own
 // loads or its mma.sync chains leaves the SM to 23 others (8 KB of shared memory
 // each): 70% of issue slots busy against 48% with two warps per 8 x 8 x 8 item and
-// 16 warps per SM.  Bound by instruction issue, 44 warp instructions per pair, of
-// which the 1-D weights take two thirds.  9.22 -> 7.02 ms on the 256^3 step's
-// 120 M pairs; on 160^3 cells, n alone, 0.27 ms for 512 k particles.
+// 16 warps per SM.  Bound by instruction issue and, more than by the tensor cores, by
+// the ALU pipe (half rate: selects, comparisons, min/max, integer), so roundings to
+// TF32 and two-sums run on the FMA pipe, two values per instruction where they can:
+// 9.22 -> 7.02 -> 6.29 ms on the 256^3 step's 120 M pairs (of the last part, packed
+// two-sums in the flush and the placed entries took 0.20 ms, the splitting by FMAs
+// 0.38, the centre cell outside the loop 0.07, entries loaded a chunk ahead 0.05); on
+// 160^3 cells, n alone, 0.27 -> 0.23 ms for 512 k particles.  Two cells of an axis at
+// a time in packed arithmetic gained nothing: the ALU part stays.
 constexpr int MMA_FLUSH = 64;  // pairs between flushes of the fragments
 
 template <int NCH>
 struct MmaWarp {
-    // [word][lane]: 8 hi, 8 lo of n/halo; of c/vx; 8 of vy/vz (n alone: 16 hi, 16 lo)
-    float acc[NCH == 1 ? 32 : 40][32];
-    // per pair of the chunk: wx | wy | wz | dens, vx, vy, vz (n alone: padding)
-    float w[32][NCH == 1 ? 28 : 20];
+    // [words r, r + 1][lane]: 8 hi, 8 lo of n/halo; of c/vx; 8 of vy/vz (n alone: 16 hi, 16 lo)
+    float2 acc[NCH == 1 ? 16 : 20][32];
+    __device__ __forceinline__ float sum(int r, int lane) const  // word r
+    {
+        return r & 1 ? acc[r >> 1][lane].y : acc[r >> 1][lane].x;
+    }
+    // per pair of the chunk: wx | wy | wz | n, halo (1 or 0), dens, vx, vy, vz (n alone:
+    // padding); the row lengths spread a K step's four rows over all banks
+    float w[32][NCH == 1 ? 28 : 24];
 };
 
 __device__ __forceinline__ uint32_t tf32_rna(float x)
@@ -802,6 +818,20 @@ __device__ __forceinline__ void tf32_split(float x, uint32_t& hi, uint32_t& lo)
 {
     hi = tf32_rna(x);
     lo = __float_as_uint(__fsub_rn(x, __uint_as_float(hi)));
+}
+// tf32_split of two weights (|x| <= 1: no overflow) on the FMA pipe, which has room
+// where the ALU pipe of the integer rounding has none: hi by the splitting with the
+// constant 2^13 + 1 (T. J. Dekker, "A floating-point technique for extending the
+// available precision", Numer. Math. 18, 1971), also x rounded to 11 bits
+__device__ __forceinline__ void tf32_split_x2(f32x2 x, uint32_t& h0, uint32_t& h1, uint32_t& l0, uint32_t& l1)
+{
+    const f32x2 c = mul2_rn(x, pack2(8193.0f, 8193.0f));
+    const f32x2 hi = add2_rn(c, sub2_rn(x, c));
+    const f32x2 lo = sub2_rn(x, hi);
+    h0 = __float_as_uint(lo2(hi));
+    h1 = __float_as_uint(hi2(hi));
+    l0 = __float_as_uint(lo2(lo));
+    l1 = __float_as_uint(hi2(lo));
 }
 __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
                                          uint32_t b1)
@@ -841,7 +871,7 @@ __device__ __forceinline__ void df_mul_df(float& hi, float& lo, float bh, float 
 __device__ __forceinline__ float tent_side_rn(float a, float b)
 {
     const float p = fminf(fabsf(a), fabsf(b)), q = fmaxf(fabsf(a), fabsf(b));
-    const float u = fmaxf(__fsub_rn(1.0f, p), 0.0f);
+    const float u = __saturatef(__fsub_rn(1.0f, p));  // p >= 0
     const float tail = __fmul_rn(__fmul_rn(0.5f, u), u);
     const float mid = __fmul_rn(__fsub_rn(b, a), __fmaf_rn(-0.5f, fabsf(__fadd_rn(a, b)), 1.0f));
     return q >= 1.0f ? tail : mid;
@@ -885,6 +915,7 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
         const TileGeo geo = tile_geo(P, tile);
         const MeshJob& J = P.job[geo.job];
         const int nc = geo.nc;
+        const float rdx = __fmul_rn(J.ncf, P.rbox);  // about 1 / dx
         const int i0 = (int)item_off[tile], nseg = (int)item_off[tile + 1] - i0;
         const uint32_t e0 = tentry[tile], e1 = max(tentry[tile + 1], e0);
         const uint32_t j0 = first[e0] + (uint32_t)((item - i0) * most);
@@ -892,7 +923,7 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
         PairCursor pairs = open_pairs(list, first, e0, e1, j0);
 
 #pragma unroll
-        for (int k = 0; k < (int)(sizeof(S.acc) / sizeof(S.acc[0])); ++k) S.acc[k][lane] = 0.f;
+        for (int k = 0; k < (int)(sizeof(S.acc) / sizeof(S.acc[0])); ++k) S.acc[k][lane] = make_float2(0.f, 0.f);
         float C[RB][NB][4];
 #pragma unroll
         for (int m = 0; m < RB; ++m)
@@ -902,24 +933,28 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
                 for (int i = 0; i < 4; ++i) C[m][b][i] = 0.f;
         float tn_hi = 0.f, tn_lo = 0.f, th_hi = 0.f, th_lo = 0.f;  // this lane's pairs' totals
 
-        // adds the fragments into the lane's sums and clears them
+        // adds the fragments into the lane's sums and clears them, two words at a time
         auto flush = [&]() {
 #pragma unroll
             for (int m = 0; m < RB; ++m)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = 4 * m + i;
+                for (int i = 0; i < 4; i += 2) {
+                    const int r = (4 * m + i) / 2;
 #pragma unroll
                     for (int b = 0; b < (NB < 2 ? NB : 2); ++b) {
-                        float hi = S.acc[2 * R * b + r][lane], lo = S.acc[2 * R * b + R + r][lane];
-                        two_sum_acc(hi, lo, C[m][b][i]);
-                        S.acc[2 * R * b + r][lane] = hi;
-                        S.acc[2 * R * b + R + r][lane] = lo;
+                        f32x2* hi = reinterpret_cast<f32x2*>(&S.acc[R * b + r][lane]);
+                        f32x2* lo = reinterpret_cast<f32x2*>(&S.acc[R * b + R / 2 + r][lane]);
+                        f32x2 h = *hi, l = *lo;
+                        two_sum_acc_x2(h, l, pack2(C[m][b][i], C[m][b][i + 1]));
+                        *hi = h;
+                        *lo = l;
                     }
-                    if constexpr (NB > 2)
-                        S.acc[4 * R + r][lane] = __fadd_rn(S.acc[4 * R + r][lane], C[m][2][i]);
+                    if constexpr (NB > 2) {
+                        f32x2* v = reinterpret_cast<f32x2*>(&S.acc[2 * R + r][lane]);
+                        *v = add2_rn(*v, pack2(C[m][2][i], C[m][2][i + 1]));
+                    }
 #pragma unroll
-                    for (int b = 0; b < NB; ++b) C[m][b][i] = 0.f;
+                    for (int b = 0; b < NB; ++b) C[m][b][i] = C[m][b][i + 1] = 0.f;
                 }
         };
 
@@ -932,7 +967,7 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
             bool halo = false;
             {
                 uint32_t which;
-                const int i = pairs.take(c0 + lane, j1, which);
+                const int i = pairs.take(c0, j1, reinterpret_cast<int2*>(S.w), which);
                 float* wl = S.w[lane];
                 float4* wz4 = reinterpret_cast<float4*>(wl);
 #pragma unroll
@@ -959,32 +994,45 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
                     if (i < 0 || r1 <= r0) r0 = r1 = 0;
                     const int any0 = (int)__reduce_min_sync(FULLM, (unsigned)(r1 > r0 ? r0 : MX));
                     const int any1 = (int)__reduce_max_sync(FULLM, (unsigned)r1);
+                    // the cell around the particle, by the signs of its edges (an FMA's
+                    // sign is exact; the guess is off by one at most)
+                    int fc = __float2int_rd(__fmul_rn(xs[a], rdx));
+                    {
+                        const float f = (float)fc;
+                        fc += (__fmaf_rn(__fadd_rn(f, 1.0f), J.dx, -xs[a]) < 0.0f ? 1 : 0) -
+                              (__fmaf_rn(f, J.dx, -xs[a]) >= 0.0f ? 1 : 0);
+                    }
+                    const float ff = (float)fc;
+                    const float ca = __fmul_rn(__fmaf_rn(ff, J.dx, -xs[a]), hinv);
+                    const float cb = __fmul_rn(__fmaf_rn(__fadd_rn(ff, 1.0f), J.dx, -xs[a]), hinv);
+                    const float wc = tent_centre_rn(ca, cb);
+                    const int centre = ca < 0.0f && cb > 0.0f ? (int)((unsigned)fc - (unsigned)sh) : -1;
                     // cell c covers [fi*dx, (fi+1)*dx] with fi = c + sh (see k_deposit_items)
                     float fi = (float)(any0 + sh);
                     float e0 = __fmul_rn(__fmaf_rn(fi, J.dx, -xs[a]), hinv);
                     float sh_ = 0.f, sl_ = 0.f;
-                    const unsigned mine = ((1u << r1) - 1u) & ~((1u << r0) - 1u);  // cells [r0, r1)
+                    const unsigned len = (unsigned)(r1 - r0);
                     for (int c = any0; c < any1; ++c) {
                         fi = __fadd_rn(fi, 1.0f);
                         const float e1 = __fmul_rn(__fmaf_rn(fi, J.dx, -xs[a]), hinv);
                         float wv = tent_side_rn(e0, e1);
-                        const bool centre = e0 < 0.0f && e1 > 0.0f;
-                        if (__any_sync(FULLM, centre)) {
-                            const float wc = tent_centre_rn(e0, e1);
-                            wv = centre ? wc : wv;
-                        }
-                        wv = (mine >> c) & 1u ? wv : 0.0f;
+                        wv = c == centre ? wc : wv;
+                        wv = (unsigned)(c - r0) < len ? wv : 0.0f;
                         wl[at[a] + c] = wv;
-                        two_sum_acc_nonneg(sh_, sl_, wv);
+                        two_sum_acc(sh_, sl_, wv);
                         e0 = e1;
                     }
                     if (a == 0) { mh = sh_; ml = sl_; }
                     else df_mul_df(mh, ml, sh_, sl_);
-                    if (a == 1) rows = mine;
+                    if (a == 1) rows = ((1u << r1) - 1u) & ~((1u << r0) - 1u);
                 }
                 // a halo particle counts in the halo channel only
                 if constexpr (NCH > 1)
-                    wz4[4] = halo ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(B.w, Cc.w, D.x, D.y);
+                {
+                    wz4[4] = halo ? make_float4(0.f, 1.f, 0.f, 0.f) : make_float4(1.f, 0.f, B.w, Cc.w);
+                    *reinterpret_cast<float2*>(wl + MX + MY + MZ + 4) =
+                        halo ? make_float2(0.f, 0.f) : make_float2(D.x, D.y);
+                }
                 if (!halo) {
                     two_sum_acc(tn_hi, tn_lo, mh);
                     tn_lo = __fadd_rn(tn_lo, ml);
@@ -993,7 +1041,6 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
                     th_lo = __fadd_rn(th_lo, ml);
                 }
             }
-            const unsigned halos = __ballot_sync(FULLM, halo);
             __syncwarp();
             // ---- K steps of 8 pairs: pairs 8s + t and 8s + t + 4 for this lane ----
             const int cnt = (int)min(32u, j1 - c0);
@@ -1007,17 +1054,16 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
                 const float zb = wb[MX + MY + (NCH == 1 ? g : g & 3)];
                 uint32_t bh[NB][2], bl[NB][2];
                 if constexpr (NCH == 1) {
-                    tf32_split(za, bh[0][0], bl[0][0]);
-                    tf32_split(zb, bh[0][1], bl[0][1]);
+                    tf32_split_x2(pack2(za, zb), bh[0][0], bh[0][1], bl[0][0], bl[0][1]);
                 } else {
-                    const unsigned hs = halos >> (s8 + t);
-                    tf32_split((hs & 1u) == (unsigned)(g >> 2) ? za : 0.0f, bh[0][0], bl[0][0]);
-                    tf32_split(((hs >> 4) & 1u) == (unsigned)(g >> 2) ? zb : 0.0f, bh[0][1], bl[0][1]);
+                    // n, halo: a weight times 1 or 0
+                    const int at = MX + MY + MZ + (g >> 2);
+                    tf32_split_x2(pack2(__fmul_rn(za, wa[at]), __fmul_rn(zb, wb[at])), bh[0][0], bh[0][1],
+                                  bl[0][0], bl[0][1]);
 #pragma unroll
                     for (int b = 1; b < NB; ++b) {
-                        const int at = MX + MY + MZ + 2 * (b - 1) + (g >> 2);
-                        tf32_split(__fmul_rn(za, wa[at]), bh[b][0], bl[b][0]);
-                        tf32_split(__fmul_rn(zb, wb[at]), bh[b][1], bl[b][1]);
+                        tf32_split(__fmul_rn(za, wa[at + 2 * b]), bh[b][0], bl[b][0]);
+                        tf32_split(__fmul_rn(zb, wb[at + 2 * b]), bh[b][1], bl[b][1]);
                     }
                 }
                 // two row blocks at a time, those this K step touches, both in one
@@ -1033,10 +1079,10 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
 #pragma unroll
                         for (int m = 0; m < 2; ++m) {
                             if (!U[m]) continue;
-                            tf32_split(__fmul_rn(xa, m ? ya.z : ya.x), ah[m][0], al[m][0]);
-                            tf32_split(__fmul_rn(xa, m ? ya.w : ya.y), ah[m][1], al[m][1]);
-                            tf32_split(__fmul_rn(xb, m ? yb.z : yb.x), ah[m][2], al[m][2]);
-                            tf32_split(__fmul_rn(xb, m ? yb.w : yb.y), ah[m][3], al[m][3]);
+                            tf32_split_x2(mul2_rn(pack2(xa, xa), m ? pack2(ya.z, ya.w) : pack2(ya.x, ya.y)),
+                                          ah[m][0], ah[m][1], al[m][0], al[m][1]);
+                            tf32_split_x2(mul2_rn(pack2(xb, xb), m ? pack2(yb.z, yb.w) : pack2(yb.x, yb.y)),
+                                          ah[m][2], ah[m][3], al[m][2], al[m][3]);
                         }
 #pragma unroll
                         for (int m = 0; m < 2; ++m)
@@ -1083,16 +1129,16 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
             for (int r = 0; r < R; ++r) {
                 const int y = r >> 1, z = 2 * (NCH == 1 ? t : t & 1) + (r & 1);
                 const int e = (z * MY + y) * MX + g;
-                pt[(low ? 0 : 7) * MC + e] = S.acc[r][lane];
-                pt[(low ? 1 : 8) * MC + e] = S.acc[R + r][lane];
+                pt[(low ? 0 : 7) * MC + e] = S.sum(r, lane);
+                pt[(low ? 1 : 8) * MC + e] = S.sum(R + r, lane);
                 if constexpr (NCH > 1) {
                     if (low) {
-                        pt[2 * MC + e] = S.acc[2 * R + r][lane];
-                        pt[3 * MC + e] = S.acc[3 * R + r][lane];
+                        pt[2 * MC + e] = S.sum(2 * R + r, lane);
+                        pt[3 * MC + e] = S.sum(3 * R + r, lane);
                     } else {
-                        pt[4 * MC + e] = __fadd_rn(S.acc[2 * R + r][lane], S.acc[3 * R + r][lane]);
+                        pt[4 * MC + e] = __fadd_rn(S.sum(2 * R + r, lane), S.sum(3 * R + r, lane));
                     }
-                    pt[(low ? 5 : 6) * MC + e] = S.acc[4 * R + r][lane];
+                    pt[(low ? 5 : 6) * MC + e] = S.sum(4 * R + r, lane);
                 }
             }
             if (lane == 0) {
@@ -1106,11 +1152,11 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
                 const int y = r >> 1, z = 2 * (NCH == 1 ? t : t & 1) + (r & 1);
                 if (g >= geo.E[0] || y >= geo.E[1] || z >= geo.E[2]) continue;
                 const size_t idx = ((size_t)(geo.O[2] + z) * nc + (geo.O[1] + y)) * nc + (geo.O[0] + g);
-                J.mesh[(low ? 0 : nmesh) + idx] = __fadd_rn(S.acc[r][lane], S.acc[R + r][lane]);
+                J.mesh[(low ? 0 : nmesh) + idx] = __fadd_rn(S.sum(r, lane), S.sum(R + r, lane));
                 if constexpr (NCH > 1) {
                     J.mesh[low ? 2 * nmesh + idx : 3 * nmesh + 3 * idx] =
-                        __fadd_rn(S.acc[2 * R + r][lane], S.acc[3 * R + r][lane]);
-                    J.mesh[3 * nmesh + 3 * idx + (low ? 1 : 2)] = S.acc[4 * R + r][lane];
+                        __fadd_rn(S.sum(2 * R + r, lane), S.sum(3 * R + r, lane));
+                    J.mesh[3 * nmesh + 3 * idx + (low ? 1 : 2)] = S.sum(4 * R + r, lane);
                 }
             }
             if (lane == 0) {
