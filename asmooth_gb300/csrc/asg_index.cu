@@ -259,10 +259,23 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(uint32_t* data, siz
     }
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_add(uint32_t* data, size_t n, const uint32_t* offs)
+// adds each tile's offset: the sum of the tiles before it, which the block forms
+// itself when they are few (scanned == 0: offs holds the tiles' sums), one launch less
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_add(uint32_t* data, size_t n, const uint32_t* offs,
+                                                           int scanned)
 {
     grid_begin();
-    const uint32_t o = offs[blockIdx.x];
+    __shared__ uint32_t warp_tot[32];
+    uint32_t o;
+    if (scanned) {
+        o = offs[blockIdx.x];
+    } else {
+        const uint32_t v = threadIdx.x < blockIdx.x ? offs[threadIdx.x] : 0u;
+        const uint32_t w = __reduce_add_sync(0xffffffffu, v);
+        if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = w;
+        __syncthreads();
+        o = __reduce_add_sync(0xffffffffu, warp_tot[threadIdx.x & 31]);
+    }
     const size_t base = (size_t)blockIdx.x * SCAN_TILE;
     for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS)
         if (base + k < n) data[base + k] += o;
@@ -286,8 +299,9 @@ void exclusive_scan_u32(uint32_t* data, size_t n, void* temp, cudaStream_t s)
     launch(k_scan_tiles, (unsigned)nb, SCAN_THREADS, 0, s, data, n, nb > 1 ? sums : nullptr);
     count_launches(1);
     if (nb > 1) {
-        exclusive_scan_u32(sums, nb, sums + nb, s);
-        launch(k_scan_add, (unsigned)nb, SCAN_THREADS, 0, s, data, n, sums);
+        const bool few = nb <= SCAN_THREADS;
+        if (!few) exclusive_scan_u32(sums, nb, sums + nb, s);
+        launch(k_scan_add, (unsigned)nb, SCAN_THREADS, 0, s, data, n, sums, few ? 0 : 1);
         count_launches(1);
     }
 }
@@ -602,16 +616,17 @@ k_rs_pass(const K* __restrict__ kin, const int* __restrict__ vin, K* __restrict_
 }
 
 // ---- up to RSC_MAX elements: one launch on a cluster of 8 or 16 blocks ----
-// Small sorts are bound by the latency of a pass (8 us, of 7 launches and a memset).
-// Here the elements stay in the cluster: block b holds positions [b T, (b + 1) T) in
-// registers, ranks them as k_rs_pass does, the blocks read one another's digit
-// counts, and every element goes straight to its new place in the shared memory of
-// the block it belongs to.  Missing elements have all bits set and stay last.
-// Unpack, 48-bit sort and gather together: 4099 particles 73 -> 35 us, 13,840 76 ->
-// 39, 32,768 82 -> 56, 65,536 92 -> 84, where the line is drawn.  8 blocks up to
-// 8192 elements (35 us; 16 blocks 37), 16 above (13,840: 39; 8 blocks 47).
+// Small sorts are bound by the latency of a pass (5 to 8 us each, and a histogram and
+// a memset before them).  Here the elements stay in the cluster: block b holds
+// positions [b T, (b + 1) T) in registers, ranks them as k_rs_pass does, the blocks read
+// one another's digit counts, and every element goes straight to its new place in the
+// shared memory of the block it belongs to.  Missing elements have all bits set and
+// stay last.  Unpack, 48-bit sort and gather together: 4099 particles 54 -> 32 us,
+// 13,840 61 -> 38, 32,768 64 -> 54; above that the cluster is slower (50,000: 67 and
+// 79).  8 blocks up to 8192 elements (2 us less than 16), 16 above (13,840: 9 us less
+// than 8).
 constexpr int RSC_THREADS = 1024, RSC_WARPS = RSC_THREADS / 32, RSC_BINS = 256;
-constexpr int RSC_MAX = 16 * RSC_THREADS * 4;
+constexpr int RSC_MAX = 16 * RSC_THREADS * 2;
 
 template <class K, int R>
 struct RsCluster {
@@ -792,8 +807,7 @@ static bool rs_cluster(const K* keys0, const int* vals0, K* keys1, int* vals1, i
     const int* vin = iota ? nullptr : vals0;
     if (n <= 8 * RSC_THREADS) return rs_cluster_t<K, 1, 8>(keys0, vin, keys1, vals1, n, passes, s);
     if (n <= 16 * RSC_THREADS) return rs_cluster_t<K, 1, 16>(keys0, vin, keys1, vals1, n, passes, s);
-    if (n <= 32 * RSC_THREADS) return rs_cluster_t<K, 2, 16>(keys0, vin, keys1, vals1, n, passes, s);
-    return rs_cluster_t<K, 4, 16>(keys0, vin, keys1, vals1, n, passes, s);
+    return rs_cluster_t<K, 2, 16>(keys0, vin, keys1, vals1, n, passes, s);
 }
 
 // 32-bit tile states hold counts below 2^30
@@ -1087,27 +1101,50 @@ void launch_pack_staged(const float4* rec, const float* rk, int n, void* aos, cu
     count_launches(1);
 }
 
-// sorted fields to input order; dens is vel.w
+// Sorted fields to input order; dens is vel.w.  The stores go to random places.  Where
+// the fields together are larger than SCATTER_L2, they are written one at a time, each
+// in slices of that size (the particles of input positions [first, first + count)), so
+// that the L2 takes all stores to a sector before it goes to memory: rk and dens of
+// 18.3 M particles 728 -> 314 us (80 and 96 MB; 60 MB, two slices each, 425; both
+// fields in two slices 392).  A slice reads all its input again, so from more than
+// SCATTER_SLICES on there is one.
+constexpr long long SCATTER_L2 = 80LL << 20;
+constexpr int SCATTER_SLICES = 5;
 __global__ void k_scatter_fields(const int* __restrict__ perm, const float* __restrict__ rk,
                                  const float4* __restrict__ vel, const int* __restrict__ igrp,
-                                 int n, float* rk_out, float* dens_out, int* igrp_out)
+                                 int n, int first, int count, float* rk_out, float* dens_out, int* igrp_out)
 {
     grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int o = perm[i];
-    if (rk_out) rk_out[o] = rk[i];
-    if (dens_out) dens_out[o] = vel[i].w;
-    if (igrp_out) igrp_out[o] = igrp[i];
+    const int o = __ldcs(perm + i);
+    if ((unsigned)(o - first) >= (unsigned)count) return;
+    if (rk_out) rk_out[o] = __ldcs(rk + i);
+    if (dens_out) dens_out[o] = __ldcs(&vel[i].w);
+    if (igrp_out) igrp_out[o] = __ldcs(igrp + i);
 }
 
 void launch_scatter_fields(const int* perm, const float* rk, const float4* vel, const int* igrp,
                            int n, float* rk_out, float* dens_out, int* igrp_out, cudaStream_t s)
 {
     if (n <= 0) return;
-    launch(k_scatter_fields, (n + 255) / 256, 256, 0, s, perm, rk, vel, igrp, n, rk_out, dens_out,
-                                                      igrp_out);
-    count_launches(1);
+    auto run = [&](float* r, float* d, int* g) {
+        const int fields = (r != nullptr) + (d != nullptr) + (g != nullptr);
+        int slices = (int)((4LL * n * fields - 1) / SCATTER_L2) + 1;
+        if (slices > SCATTER_SLICES) slices = 1;
+        const int count = (n + slices - 1) / slices;
+        for (int k = 0; k < slices; ++k)
+            launch(k_scatter_fields, (n + 255) / 256, 256, 0, s, perm, rk, vel, igrp, n, k * count, count, r, d, g);
+        count_launches(slices);
+    };
+    const int fields = (rk_out != nullptr) + (dens_out != nullptr) + (igrp_out != nullptr);
+    if (4LL * n * fields <= SCATTER_L2) {
+        run(rk_out, dens_out, igrp_out);
+        return;
+    }
+    if (rk_out) run(rk_out, nullptr, nullptr);
+    if (dens_out) run(nullptr, dens_out, nullptr);
+    if (igrp_out) run(nullptr, nullptr, igrp_out);
 }
 
 }  // namespace asg

@@ -1,5 +1,5 @@
 """GPU tests of the index at the sizes where its sort changes (one cluster of 8
-blocks, of 16 with 1, 2 and 4 elements per thread, many blocks): with the
+blocks, of 16 with 1 and 2 elements per thread, many blocks): with the
 particles in an order that the sort has to undo and half of them in ties, the
 33rd keys equal the oracle's exactly, and the input order does not show in the
 result: rk of a shuffled set is the shuffled rk."""
