@@ -904,7 +904,7 @@ static int run_knn(asg_ctx* ctx)
                    P<int>(ctx->idx33), P<int>(ctx->blist), ctx->d_err, ctx->s, ctx->knn_warps);
     phase_end(ctx);
     phase_begin(ctx, ASG_PH_TIES);  // only bundles with an exact tie at the 33rd distance
-    launch_knn_ties(P<float4>(ctx->pos), t, P<float>(ctx->t33), P<int>(ctx->idx33), 0,
+    launch_knn_ties(P<float4>(ctx->pos), t, P<float>(ctx->t33), P<int>(ctx->idx33), 0, P<int>(ctx->blist),
                     P<float>(ctx->rk), P<int>(ctx->dexp), P<unsigned long long>(ctx->dacc),
                     ctx->d_err, ctx->s);
     phase_end(ctx);
@@ -1264,7 +1264,7 @@ int asg_get_knn(asg_ctx* ctx, float* t33, int* idx33)
     if (int r = grow(ctx, ctx->minin, 4 * n)) return r;
     if (!ctx->idx33_all) {  // the hot path resolves idx33 only where the 33rd value is tied
         launch_knn_ties(P<float4>(ctx->pos), tree_view(ctx), P<float>(ctx->t33),
-                        P<int>(ctx->idx33), 1, nullptr, nullptr, nullptr, ctx->d_err, ctx->s);
+                        P<int>(ctx->idx33), 1, nullptr, nullptr, nullptr, nullptr, ctx->d_err, ctx->s);
         ctx->idx33_all = true;
     }
     launch_scatter_fields(ctx->perm, P<float>(ctx->t33), nullptr, P<int>(ctx->idx33), ctx->n,

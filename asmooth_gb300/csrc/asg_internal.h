@@ -85,8 +85,8 @@ void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk,
 // idx33 = input index of the 33rd key, for flagged queries (all = 0) or every query;
 // dexp (n ints, or null) and acc (n uint64) are prepared for launch_dens
 void launch_knn_ties(const float4* pos, const TreeView& t, const float* t33, int* idx33,
-                     int all, const float* rk, int* dexp, unsigned long long* acc, int* err,
-                     cudaStream_t s);
+                     int all, const int* blist, const float* rk, int* dexp, unsigned long long* acc,
+                     int* err, cudaStream_t s);
 // vel[j].w (dens) += the tent weights j receives as one of the 32 nearest;
 // dexp and acc as launch_knn_ties prepared them; blist from launch_knn_t33 or null
 void launch_dens(const float4* pos, const TreeView& t, const float* t33, const int* idx33,

@@ -425,11 +425,15 @@ __device__ __forceinline__ int dens_exponent(float rk)
 // deeper one runs another pass with the floor at its last kept index, so any
 // number of ties resolves in at most TIE_PASSES = ceil(33 / TIE_MAX) passes.
 constexpr int TIE_PASSES = (K_NN + TIE_MAX - 1) / TIE_MAX;
+// Mostly a bundle has one such query, if any, and the kernel lasts as long as one
+// bundle: 24 -> 10 us at 377 k particles, 40 -> 18 with a zip decode's rounded
+// positions.
+constexpr int TIE_FEW = 8;  // queries of a bundle up to which each is resolved by itself
 
 __global__ void __launch_bounds__(KNN_WARPS * 32)
 k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, const float* __restrict__ t33,
-           int* __restrict__ idx33, int all, const float* __restrict__ rk, int* __restrict__ dexp,
-           unsigned long long* __restrict__ acc, int* err)
+           int* __restrict__ idx33, int all, const int* __restrict__ blist, const float* __restrict__ rk,
+           int* __restrict__ dexp, unsigned long long* __restrict__ acc, int* err)
 {
     grid_begin();
     __shared__ float4 cand[KNN_WARPS][LEAF_MAX];
@@ -447,6 +451,58 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
     if (!__any_sync(FULL, want)) return;
     const float4 xq = pos[q];
     const float T = t33[q], bound = prune_bound(T);
+    // few queries, and the leaves that k_knn_t33 scanned: one query at a time, a leaf's
+    // box or a particle per lane; the k-th smallest tied index in lane k
+    unsigned few = __ballot_sync(FULL, want);
+    const int* bl = blist ? blist + (size_t)(base >> 5) * (KNN_LIST + 1) : nullptr;
+    const int nlist = bl && t.leaf <= 16 ? bl[0] : -1;
+    if (nlist >= 0 && __popc(few) <= TIE_FEW) {
+        bool left = false;  // a query that this form cannot resolve
+        for (; few; few &= few - 1) {
+            const int l = __ffs(few) - 1;
+            const float x = __shfl_sync(FULL, xq.x, l), y = __shfl_sync(FULL, xq.y, l), z = __shfl_sync(FULL, xq.z, l);
+            const float Tl = __shfl_sync(FULL, T, l), bl_ = prune_bound(Tl);
+            int less = 0, eq = 0, tie = INT_MAX;
+            for (int i0 = 0; i0 < nlist; i0 += 32) {
+                const int e = i0 + lane < nlist ? bl[1 + i0 + lane] : 0;
+                unsigned m = __ballot_sync(FULL, i0 + lane < nlist &&
+                                                     point_box_fast(make_float4(x, y, z, 0.f), tree_box(t, 0, e)) <= bl_);
+                while (m) {  // two leaves, a half-warp each
+                    const int l0 = __ffs(m) - 1;
+                    m &= m - 1;
+                    const int l1 = m ? __ffs(m) - 1 : -1;
+                    m &= m - 1;
+                    const int mine = lane < 16 ? l0 : l1;
+                    const int id = __shfl_sync(FULL, e, mine < 0 ? 0 : mine);
+                    const bool have = mine >= 0 && (lane & 15) < leaf_count(t, id);
+                    const float4 c = pos[have ? id * t.leaf + (lane & 15) : 0];
+                    const float d2 = norm2_rn(x, y, z, c.x, c.y, c.z);
+                    less += __popc(__ballot_sync(FULL, have && d2 < Tl));
+                    unsigned ties = __ballot_sync(FULL, have && d2 == Tl);
+                    eq += __popc(ties);
+                    for (; ties; ties &= ties - 1) {
+                        const int v = __shfl_sync(FULL, __float_as_int(c.w), __ffs(ties) - 1);
+                        const int up = __shfl_up_sync(FULL, tie, 1);
+                        const int at = __popc(__ballot_sync(FULL, tie < v));
+                        tie = lane < at ? tie : lane == at ? v : up;
+                    }
+                }
+            }
+            const int rank = K_NN - less;  // position of the 33rd key among all the ties
+            const int found = __shfl_sync(FULL, tie, (rank - 1) & 31);
+            if (rank < 1 || rank > eq) {
+                if (lane == l) {
+                    atomicOr(err, ERR_FEW);
+                    idx33[q] = -1;
+                }
+            } else if (rank <= 32) {
+                if (lane == l) idx33[q] = found;
+            } else {
+                left = true;
+            }
+        }
+        if (!left) return;
+    }
     int nless = 0, neq = 0;
     int need = 0;          // rank of the wanted index among the ties above floor
     int floor_idx = -1;    // this pass keeps tied indices > floor_idx
@@ -699,11 +755,11 @@ void launch_knn_t33(const float4* pos, const TreeView& t, float* t33, float* rk,
 }
 
 void launch_knn_ties(const float4* pos, const TreeView& t, const float* t33, int* idx33,
-                     int all, const float* rk, int* dexp, unsigned long long* acc, int* err,
-                     cudaStream_t s)
+                     int all, const int* blist, const float* rk, int* dexp, unsigned long long* acc,
+                     int* err, cudaStream_t s)
 {
     if (t.n <= 0) return;
-    launch(k_knn_ties, knn_blocks(t.n), KNN_WARPS * 32, 0, s, pos, t, t33, idx33, all, rk, dexp, acc, err);
+    launch(k_knn_ties, knn_blocks(t.n), KNN_WARPS * 32, 0, s, pos, t, t33, idx33, all, blist, rk, dexp, acc, err);
     count_launches(1);
 }
 

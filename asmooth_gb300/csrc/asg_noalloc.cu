@@ -173,7 +173,7 @@ extern "C" int asg_neighbor_search_noalloc(const float* d_x, int np, float left,
     t.box = F4(L.boxes);
     launch_gather(perm, F4(L.rec_in), nullptr, t, F4(L.pos), F4(L.vel), I(L.igrp), F(L.rk), s);
     launch_knn_t33(F4(L.pos), t, F(L.t33), F(L.rk), I(L.idx33), I(L.blist), err, s);
-    launch_knn_ties(F4(L.pos), t, F(L.t33), I(L.idx33), 0, F(L.rk), I(L.dexp),
+    launch_knn_ties(F4(L.pos), t, F(L.t33), I(L.idx33), 0, I(L.blist), F(L.rk), I(L.dexp),
                     reinterpret_cast<unsigned long long*>(b + L.dacc), err, s);
     launch_dens(F4(L.pos), t, F(L.t33), I(L.idx33), I(L.blist), F(L.rk), I(L.dexp),
                 reinterpret_cast<unsigned long long*>(b + L.dacc), F4(L.vel), s);
