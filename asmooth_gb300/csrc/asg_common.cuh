@@ -264,7 +264,7 @@ __host__ __device__ __forceinline__ uint64_t spread3(uint32_t v)
 // turned into the transposed index by undoing the curve's inversions and
 // exchanges level by level, Gray-decoded, then interleaved x-major.  Every
 // 3k-bit prefix of the key is one octree cell of level k, as with a Morton
-// key, so the radix tree over sorted keys is built the same way; consecutive
+// key; consecutive
 // keys are always face-adjacent cells, so 32 consecutive particles are more
 // compact than in Morton order.
 __host__ __device__ __forceinline__ uint64_t hilbert_key48(uint32_t x, uint32_t y, uint32_t z)

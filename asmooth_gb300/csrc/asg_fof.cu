@@ -32,7 +32,9 @@ __device__ __forceinline__ int uf_find(int* P, int x)
         if (p == x) return x;
         const int g = __ldcg(P + p);
         if (g == p) return p;
-        atomicCAS(P + x, p, g);  // path halving: g is an ancestor of x
+        // path halving: g is an ancestor of x.  A plain store could put it over the root
+        // that k_fof_root wrote meanwhile
+        atomicCAS(P + x, p, g);
         x = g;
     }
 }

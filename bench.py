@@ -4,7 +4,7 @@ smoothing length, particle density, adaptive deposit at nc = 64, 128, 256) on
 the 256^3-particle NFW-clustered cube of side 512 with its 8-unit periodic
 shell, seeded synthetic data.
 
-One step = index build (Morton sort + radix tree) + neighbour search + dens +
+One step = index build (Hilbert sort + box tree) + neighbour search + dens +
 deposit of all three meshes for one cube.  `value` times steps with inputs
 resident in HBM (CUDA events on the library's stream; L2 is flushed before
 every step and the inputs are larger than L2).  `e2e` times the public C-ABI

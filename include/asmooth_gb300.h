@@ -312,12 +312,12 @@ int asg_batch_set_item_quantised(asg_batch* batch, int item, const int* cell, co
  * stream i % streams, each stream with its own scratch (about 300 bytes per
  * particle of the largest item), forked and joined inside the one graph. */
 int asg_batch_set_streams(asg_batch* batch, int streams);
-/* Optional autotuner: times the largest item with tree bucket sizes 16, 24, 32,
+/* Optional autotuner: times the largest item with tree leaf sizes 16, 24, 32,
  * deposit work items of 2048, 4096, 8192 pairs, 2 or 4 warps per block of the
  * neighbour search and each deposit engine, and keeps the fastest; *leaf and
  * *seg receive the first two choices. */
 int asg_batch_tune(asg_batch* batch, int* leaf, int* seg);
-/* The batch's configuration (tuned or default): tree bucket size, deposit
+/* The batch's configuration (tuned or default): tree leaf size, deposit
  * work-item length, neighbour-search warps per block and the deposit engine
  * (1: tensor cores, one warp per work item; 0: CUDA cores).
  * Any pointer may be NULL. */
