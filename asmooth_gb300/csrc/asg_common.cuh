@@ -194,23 +194,7 @@ __device__ __forceinline__ float max3f(float a, float b, float c)
     return r;
 }
 
-// Squared distance from a point to an AABB in the cheaper FMA form, for
-// pruning only: compare it against prune_bound(t), never against t itself.
-// Per axis d = fl(lo - q) (or fl(q - hi)) is at most |fl(p - q)| for every
-// point p of the box (rounding is monotone); the FMA sum is at most
-// (dx^2 + dy^2 + dz^2)(1 + u)^3 and norm2_rn(q, p) is at least
-// (px^2 + py^2 + pz^2)(1 - u)^3 (u = 2^-24), so the result is at most
-// norm2_rn(q, p)(1 + 6.1u) for every p in the box.
-__device__ __forceinline__ float box_dist2_fast(float qx, float qy, float qz, float lx, float ly,
-                                                float lz, float hx, float hy, float hz)
-{
-    const float dx = max3f(lx - qx, qx - hx, 0.0f);
-    const float dy = max3f(ly - qy, qy - hy, 0.0f);
-    const float dz = max3f(lz - qz, qz - hz, 0.0f);
-    return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-}
-
-// the bound that box_dist2_fast is compared against for a threshold t on
+// the bound that a pruning distance (asg_tree.cuh) is compared against for a threshold t on
 // norm2_rn: fl(t (1 + 2^-21)) >= t (1 + 6.9u) > t (1 + 6.1u), so a box holding
 // a point with norm2_rn <= t is never pruned (t = +inf stays +inf)
 __device__ __forceinline__ float prune_bound(float t) { return __fmul_rn(t, 1.0f + 0x1p-21f); }

@@ -938,8 +938,8 @@ __device__ __forceinline__ void group_box(float (&r)[6])
 }
 __device__ __forceinline__ void store_box(float4* box, size_t id, const float (&r)[6])
 {
-    box[2 * id] = make_float4(r[0], r[1], r[2], r[3]);
-    box[2 * id + 1] = make_float4(r[4], r[5], 0.0f, 0.0f);
+    box[2 * id] = make_float4(r[0], r[3], r[1], r[4]);
+    box[2 * id + 1] = make_float4(r[2], r[5], 0.0f, 0.0f);
 }
 
 // The particles in curve order, the boxes of their leaves and, LEAF16 (leaves of
@@ -1018,7 +1018,7 @@ __global__ void k_up_boxes(const float4* __restrict__ below, int nbelow, float4*
     if (id >= nbox) return;
     const long long c = min(id * 32 + (threadIdx.x & 31), (long long)nbelow - 1);
     const float4 u = below[2 * c], v = below[2 * c + 1];
-    float b[6] = {u.x, u.y, u.z, u.w, v.x, v.y};
+    float b[6] = {u.x, u.z, v.x, u.y, u.w, v.y};
     group_box<32>(b);
     if ((threadIdx.x & 31) == 0) store_box(box, (size_t)id, b);
 }

@@ -281,7 +281,7 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
             const int id = g * 32 + (int)(m & 31u);
             const float4* bp = t.box + 2 * (size_t)id;
             const TreeBox c = {bp[0], bp[1]};
-            if (!__any_sync(FULL, point_box_fast(make_float4(lo2(qx), lo2(qy), lo2(qz), 0.f), c) <=
+            if (!__any_sync(FULL, point_box_fast(qx, qy, qz, c) <=
                                       prune_bound(SPLIT > 1 ? limit : a[K_NN - 1])))
                 continue;
             if (lane == (nlist & 31)) entry = id;
@@ -516,9 +516,9 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
         for (int k = 0; k < TIE_MAX; ++k) tie[k] = INT_MAX;
         // the box of the queries still open and their largest radius
         TreeBox box;
-        box.a = open ? make_float4(xq.x, xq.y, xq.z, xq.x)
-                     : make_float4(INFINITY, INFINITY, INFINITY, -INFINITY);
-        box.b = open ? make_float4(xq.y, xq.z, 0.f, 0.f) : make_float4(-INFINITY, -INFINITY, 0.f, 0.f);
+        box.a = open ? make_float4(xq.x, xq.x, xq.y, xq.y)
+                     : make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+        box.b = open ? make_float4(xq.z, xq.z, 0.f, 0.f) : make_float4(INFINITY, -INFINITY, 0.f, 0.f);
         float reach = open ? bound : 0.0f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
