@@ -380,13 +380,16 @@ constexpr int MERGE_FEW = 8;  // items of a tile that one warp merges by itself
 // Pairs per work item, at most `most`.  An item is a serial chain for its warp, so
 // a small set takes short items and all warps: a quarter of the pairs a warp
 // would get if the items were dealt out evenly over 24 warps on 152 SMs, in steps
-// of the 64 pairs between two flushes.  One item length of 4096 pairs left a set of
-// 13,840 particles to 20 warps: 354 us against 18.
+// of the 64 pairs between two flushes; half of them for n alone, whose larger
+// partial tiles cost more to merge (the deposit of 512 k particles on 160^3 cells 381
+// -> 363 us; with all channels a half costs 5% more on 1.2 to 2.5 M particles).  One
+// item length of 4096 pairs left a set of 13,840 particles to 20 warps: 354 us
+// against 18.
 constexpr int ITEM_SHARE = 4 * 24 * 152;
-__device__ __forceinline__ int deposit_seg(const int* __restrict__ counters, int most)
+__device__ __forceinline__ int deposit_seg(const int* __restrict__ counters, int most, bool n_alone)
 {
     const unsigned long long pairs = *reinterpret_cast<const unsigned long long*>(counters + 2);
-    const unsigned long long seg = (pairs / ITEM_SHARE + 64) & ~63ull;
+    const unsigned long long seg = (pairs / (n_alone ? ITEM_SHARE / 2 : ITEM_SHARE) + 64) & ~63ull;
     return (int)min(seg, (unsigned long long)most);
 }
 
@@ -416,13 +419,13 @@ __device__ __forceinline__ uint32_t lower_bound(const uint32_t* __restrict__ key
 }
 constexpr int TI_THREADS = 256, TI_TILES = TI_THREADS - 1;  // the last thread finds the next block's first
 __global__ void k_tile_items(const uint32_t* __restrict__ keys, uint32_t count,
-                             const uint32_t* __restrict__ first, int total_tiles, int ib, int most,
+                             const uint32_t* __restrict__ first, int total_tiles, int ib, int most, bool n_alone,
                              uint32_t* __restrict__ tentry, uint32_t* __restrict__ nitems,
                              const int* __restrict__ counters)
 {
     grid_begin();
     __shared__ uint32_t e[TI_THREADS];
-    const int seg = deposit_seg(counters, most);
+    const int seg = deposit_seg(counters, most, n_alone);
     const long long tt = (long long)blockIdx.x * TI_TILES + threadIdx.x;
     const int t = (int)min(tt, (long long)total_tiles + 1);
     const uint32_t b = lower_bound(keys, count, (uint64_t)min(t, total_tiles) << ib);
@@ -627,7 +630,7 @@ k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositP
     WarpTile& S = reinterpret_cast<WarpTile*>(smem_raw)[threadIdx.x >> 5];
     const bool periodic = P.periodic != 0;
     const uint32_t total_items = min(item_off[total_tiles], max_items);
-    const int most = deposit_seg(counters, P.seg);  // pairs per item
+    const int most = deposit_seg(counters, P.seg, P.density_only != 0);  // pairs per item
 
     for (;;) {
         int item = 0;
@@ -915,7 +918,7 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
     const int g = lane >> 2, t = lane & 3;
     const bool periodic = P.periodic != 0;
     const uint32_t total_items = min(item_off[total_tiles], max_items);
-    const int most = deposit_seg(counters, P.seg);  // pairs per item
+    const int most = deposit_seg(counters, P.seg, P.density_only != 0);  // pairs per item
 
     int item = 0;
     if (lane == 0) item = atomicAdd(counters, 1);
@@ -1451,7 +1454,8 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
     launch(k_sorted_entries, entries / 256 + 1, 256, 0, s, cur ? w.vals1 : w.vals0, w.entry, entries, w.list,
                                                        w.first, err);
     exclusive_scan_u32(w.first, (size_t)entries + 1, w.scan_tmp_e, s);
-    launch(k_tile_items, T / TI_TILES + 1, TI_THREADS, 0, s, keys, entries, w.first, T, img_bits(p), p.seg, w.tentry,
+    launch(k_tile_items, T / TI_TILES + 1, TI_THREADS, 0, s, keys, entries, w.first, T, img_bits(p), p.seg,
+           p.density_only != 0, w.tentry,
                                              w.item_off, w.counters);
     exclusive_scan_u32(w.item_off, (size_t)T + 1, w.scan_tmp_t, s);
     launch(k_item_list, (T + 255) / 256, 256, 0, s, w.item_off, T, max_items, w.item_tile, w.merge,
