@@ -112,12 +112,6 @@ __device__ __forceinline__ f32x2 mul2_rn(f32x2 a, f32x2 b)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(0ull));
     return r;
 }
-__device__ __forceinline__ f32x2 fma2_rn(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 
 // norm2_rn from the point (ax, ay, az), each coordinate given twice, to two
 // points (their x, y and z pairs): the same roundings in the same order

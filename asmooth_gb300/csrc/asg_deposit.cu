@@ -858,15 +858,7 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// double-float (hi, lo) helpers in FP32 arithmetic: exact product of a
-// double-float and a float (two_prod by FMA), and accumulation
-__device__ __forceinline__ void df_mul(float& hi, float& lo, float b)
-{
-    const float p = __fmul_rn(hi, b);
-    const float e = fmaf(hi, b, -p);
-    hi = p;
-    lo = fmaf(lo, b, e);
-}
+// product of two double-floats (hi, lo) in FP32 arithmetic (two_prod by FMA)
 __device__ __forceinline__ void df_mul_df(float& hi, float& lo, float bh, float bl)
 {
     const float p = __fmul_rn(hi, bh);
