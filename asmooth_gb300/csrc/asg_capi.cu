@@ -1928,7 +1928,6 @@ int asg_batch_tune(asg_batch* b, int* leaf, int* seg)
     if (!b) return ASG_ERR_ARG;
     asg_ctx* ctx = b->ctx;
     CK(cudaSetDevice(ctx->device));
-    if (int r = alloc_set(ctx, b->max_n)) return r;
     int item = 0;  // the largest item
     for (int i = 1; i < b->n_items; ++i)
         if (b->np[(size_t)i] > b->np[(size_t)item]) item = i;
@@ -1937,11 +1936,12 @@ int asg_batch_tune(asg_batch* b, int* leaf, int* seg)
     const int leaves[] = {16, 24, 32}, segs[] = {2048, 4096, 8192}, warps[] = {2, 4}, mmas[] = {1, 0};
     float best = INFINITY;
     int bl = ctx->leaf, bs = ctx->dep_seg, bw = ctx->knn_warps, bm = ctx->dep_mma;
-    for (int l : leaves)
+    for (int l : leaves) {
+        ctx->leaf = l;
+        if (int r = alloc_set(ctx, b->max_n)) return r;  // smaller leaves have more boxes
         for (int sg : segs)
             for (int w : warps)
                 for (int m : mmas) {
-                    ctx->leaf = l;
                     ctx->dep_seg = sg;
                     ctx->knn_warps = w;
                     ctx->dep_mma = m;
@@ -1961,6 +1961,7 @@ int asg_batch_tune(asg_batch* b, int* leaf, int* seg)
                         bm = m;
                     }
                 }
+    }
     ctx->leaf = bl;
     ctx->dep_seg = bs;
     ctx->knn_warps = bw;

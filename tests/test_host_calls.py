@@ -1,0 +1,80 @@
+"""CPU tests of what the host code asks of the device: the library's object files
+linked against a CUDA runtime that only keeps a log (host_checks/fake_cudart.cpp).
+No kernel runs, so these cover sizes, launches and call order alone."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    from asmooth_gb300 import _lib
+    from asmooth_gb300 import build as B
+
+    objs = [os.path.join(B.CSRC, "_build", u + ".o") for u in B.UNITS]
+    B.build(force=not all(os.path.exists(o) and os.path.getmtime(o) >= B._sources_mtime() for o in objs))
+    so = str(tmp_path_factory.mktemp("fake") / "libasg_fake.so")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(B.nvcc())))
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", B.CSRC, "-I",
+                    os.path.join(cuda, "include"), os.path.join(HERE, "host_checks", "fake_cudart.cpp"),
+                    *objs, "-o", so, "-lpthread"], check=True, capture_output=True)
+    lib = C.CDLL(so)
+    for name, (res, args) in _lib.SIGNATURES.items():
+        getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
+    lib.fake_log.restype = C.c_char_p
+    lib.fake_counts.argtypes = [C.c_uint32, C.c_ulonglong, C.c_ulonglong]
+    lib.fake_counts(0, 0, 0)
+    return lib
+
+
+def log(fake):
+    lines = [ln.split() for ln in fake.fake_log().decode().splitlines()]
+    fake.fake_clear()
+    return lines
+
+
+def context(fake):
+    h = C.c_void_p()
+    assert fake.asg_create(C.byref(h), 0) == 0
+    return h
+
+
+def batch(fake, ctx, sizes, ncs=(8,)):
+    """a batch of cubes of these particle counts, positions all zero"""
+    k = len(sizes)
+    n = np.asarray(sizes, np.int32)
+    lo, hi = np.zeros(k, np.float32), np.full(k, 10, np.float32)
+    nc = np.asarray(ncs, np.int32)
+    b = C.c_void_p()
+    p = lambda a: C.c_void_p(a.ctypes.data)  # noqa: E731
+    assert fake.asg_batch_create(ctx, k, p(n), None, p(lo), p(hi), p(hi), p(nc), len(nc), -1, C.byref(b)) == 0
+    return b
+
+
+def boxes_short(lines):
+    return [ln for ln in lines if ln[0] == "boxes" and int(ln[1]) > int(ln[2])]
+
+
+@pytest.mark.parametrize("leaf", ["", "1", "17", "24", "32"])
+def test_tuned_leaf_sizes_fit_the_box_array(fake, monkeypatch, leaf):
+    """The tuner's index builds keep to the tree's box array whatever leaf size the
+    context starts from, and so does a later, larger batch of the same context, which
+    starts from the leaf size that the first one chose (the largest here)."""
+    if leaf:
+        monkeypatch.setenv("ASG_LEAF_SIZE", leaf)
+    ctx = context(fake)
+    for sizes in ([3000, 2000], [90000, 4000], [200000]):
+        b = batch(fake, ctx, sizes)
+        chosen = C.c_int(0)
+        assert fake.asg_batch_tune(b, C.byref(chosen), None) == 0 and chosen.value == 32
+        assert fake.asg_batch_run(b) == 0
+        fake.asg_batch_destroy(b)
+    lines = log(fake)
+    assert sum(ln[0] == "boxes" for ln in lines) > 100
+    assert not boxes_short(lines)
+    fake.asg_destroy(ctx)
