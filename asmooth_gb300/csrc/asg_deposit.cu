@@ -447,7 +447,7 @@ __global__ void k_tile_items(const uint32_t* __restrict__ keys, uint32_t count,
 // up to MERGE_FEW from the front (counters[1] of them), those of more from the
 // back (counters[4]).  More
 // items than the arrays hold (a captured call whose pairs outgrew its capacity)
-// set ERR_CAP.
+// set ERR_CAP; those that they hold run all the same, so each has its tile.
 __global__ void k_item_list(const uint32_t* __restrict__ item_off, int total_tiles,
                             uint32_t max_items, uint32_t* __restrict__ item_tile,
                             uint32_t* __restrict__ merge, int* __restrict__ counters, int* err)
@@ -456,11 +456,11 @@ __global__ void k_item_list(const uint32_t* __restrict__ item_off, int total_til
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total_tiles) return;
     const uint32_t i0 = item_off[t], i1 = item_off[t + 1];
+    for (uint32_t i = i0; i < min(i1, max_items); ++i) item_tile[i] = (uint32_t)t;
     if (i1 > max_items) {
         atomicOr(err, ERR_CAP);
         return;
     }
-    for (uint32_t i = i0; i < i1; ++i) item_tile[i] = (uint32_t)t;
     if (i1 - i0 > MERGE_FEW) merge[total_tiles - 1 - atomicAdd(counters + 4, 1)] = (uint32_t)t;
     else if (i1 - i0 > 1) merge[atomicAdd(counters + 1, 1)] = (uint32_t)t;
 }
