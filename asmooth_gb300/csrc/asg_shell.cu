@@ -32,12 +32,13 @@ __global__ void k_shell_bins(const float4* __restrict__ rec, int n, float lt, fl
     keys[i] = (uint32_t)(bx + 3 * by + 9 * bz);
 }
 
+// (none when the sort gave up: its output is not all written then)
 __global__ void k_shell_bounds(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ start,
-                               uint32_t* __restrict__ end)
+                               uint32_t* __restrict__ end, const int* __restrict__ err)
 {
     grid_begin();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= n) return;
+    if (m >= n || (*err & ERR_SORT)) return;
     const uint32_t b = keys[m];
     if (m == 0 || keys[m - 1] != b) start[b] = (uint32_t)m;
     if (m == n - 1 || keys[m + 1] != b) end[b] = (uint32_t)m + 1;
@@ -119,7 +120,7 @@ void launch_shell_bins(const float4* rec, int n, float lt, float rt, uint32_t* k
     const int cur = radix_sort32(keys0, vals0, keys1, vals1, n, 5, true, sort_tmp, err, s);
     *keys = cur ? keys1 : keys0;
     *order = cur ? vals1 : vals0;
-    launch(k_shell_bounds, (n + 255) / 256, 256, 0, s, *keys, n, start, end);
+    launch(k_shell_bounds, (n + 255) / 256, 256, 0, s, *keys, n, start, end, err);
     count_launches(2);
 }
 

@@ -29,3 +29,19 @@ int main()
     assert (int(out[0]) != 0) == (room < len(want))
     if room >= len(want):
         assert out[2] == "2 1"
+
+
+@pytest.mark.parametrize("gave_up", [False, True])
+def test_shell_bounds_after_a_sort_that_gave_up(tmp_path, gave_up):
+    """k_shell_bounds reads bin numbers from the sort's output.  When the sort gave up
+    (ERR_SORT) some of that output was never written: no bounds then, and no store."""
+    out = K.run(tmp_path, K.constants("ERR_SORT") + K.kernel_text("asg_shell", "k_shell_bounds") + f"""
+int main()
+{{
+    std::vector<uint32_t> keys = {{0, 0, 3, 3, 3, 13, 26}}, start(27, 0u), end(27, 0u);
+    int err = {int(gave_up)} ? ERR_SORT : 0;
+    if (err) keys = {{0, 0, 0xcdcdcdcd, 3, 28, 0x7fffffff, 26}};
+    run(1, 32, [&] {{ k_shell_bounds(keys.data(), (int)keys.size(), start.data(), end.data(), &err); }});
+    for (int b : {{0, 3, 13, 26}}) std::printf("%u %u ", start[b], end[b]);
+}}""")
+    assert out.split() == (["0"] * 8 if gave_up else "0 2 2 5 5 6 6 7".split())
