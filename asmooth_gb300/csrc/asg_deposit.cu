@@ -360,17 +360,22 @@ __global__ void k_pad_entries(uint32_t* __restrict__ keys, uint2* __restrict__ e
     entry[j] = make_uint2(0u, 0u);
 }
 
-// the entries in key order, and their pair counts (then scanned in place)
+// the entries in key order, and their pair counts (then scanned in place, in 32 bits:
+// a captured call whose pairs outgrew them sets ERR_CAP and has none)
 __global__ void k_sorted_entries(const int* __restrict__ order, const uint2* __restrict__ entry,
-                                 uint32_t count, uint2* __restrict__ list, uint32_t* __restrict__ first,
-                                 const int* __restrict__ err)
+                                 uint32_t count, const unsigned long long* __restrict__ pairs,
+                                 uint2* __restrict__ list, uint32_t* __restrict__ first, int* err)
 {
     grid_begin();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j == count) first[j] = 0u;
+    const bool many = *pairs > (unsigned long long)INT_MAX;
+    if (j == count) {
+        first[j] = 0u;
+        if (many) atomicOr(err, ERR_CAP);
+    }
     if (j >= count) return;
     // not in order when the sort gave up: no pairs at all
-    const uint2 e = (*err & ERR_SORT) ? make_uint2(0u, 0u) : entry[order[j]];
+    const uint2 e = many || (*err & ERR_SORT) ? make_uint2(0u, 0u) : entry[order[j]];
     list[j] = e;
     first[j] = (uint32_t)__popc(e.y);
 }
@@ -1443,8 +1448,8 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
     const int cur = radix_sort32(w.keys0, w.vals0, w.keys1, w.vals1, (int)entries,
                                  key_bits(padded ? T + 1 : T, img_bits(p)), true, w.sort_tmp, err, s);
     const uint32_t* keys = cur ? w.keys1 : w.keys0;
-    launch(k_sorted_entries, entries / 256 + 1, 256, 0, s, cur ? w.vals1 : w.vals0, w.entry, entries, w.list,
-                                                       w.first, err);
+    launch(k_sorted_entries, entries / 256 + 1, 256, 0, s, cur ? w.vals1 : w.vals0, w.entry, entries,
+           reinterpret_cast<const unsigned long long*>(w.counters + 2), w.list, w.first, err);
     exclusive_scan_u32(w.first, (size_t)entries + 1, w.scan_tmp_e, s);
     launch(k_tile_items, T / TI_TILES + 1, TI_THREADS, 0, s, keys, entries, w.first, T, img_bits(p), p.seg,
            p.density_only != 0, w.tentry,

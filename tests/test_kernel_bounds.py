@@ -45,3 +45,23 @@ int main()
     for (int b : {{0, 3, 13, 26}}) std::printf("%u %u ", start[b], end[b]);
 }}""")
     assert out.split() == (["0"] * 8 if gave_up else "0 2 2 5 5 6 6 7".split())
+
+
+@pytest.mark.parametrize("pairs", [7, 2 ** 31 - 1, 2 ** 31, 2 ** 33])
+def test_entries_of_more_pairs_than_numbers(tmp_path, pairs):
+    """k_sorted_entries numbers the pairs in 32 bits.  A captured call whose pairs
+    outgrew these has no pairs and reports ERR_CAP."""
+    out = K.run(tmp_path, K.constants("ERR_SORT", "ERR_CAP") + K.kernel_text("asg_deposit", "k_sorted_entries") + f"""
+int main()
+{{
+    const int order[] = {{2, 0, 1}};
+    const uint2 entry[] = {{{{5, 0x7}}, {{6, 0xffffffff}}, {{9, 0x80000001}}}};
+    const unsigned long long pairs = {pairs}ull;
+    std::vector<uint2> list(3);
+    std::vector<uint32_t> first(4, 77u);
+    int err = 0;
+    run(1, 32, [&] {{ k_sorted_entries(order, entry, 3u, &pairs, list.data(), first.data(), &err); }});
+    for (uint32_t f : first) std::printf("%u ", f);
+    std::printf("%d %d", list[0].x, err == ERR_CAP);
+}}""")
+    assert out.split() == ("2 3 32 0 9 0" if pairs < 2 ** 31 else "0 0 0 0 0 1").split()
