@@ -92,6 +92,7 @@ struct asg_ctx {
     bool dec_rk = false;    // they have smoothing lengths
     uint32_t dep_npairs = 0, dep_nentries = 0;
     int dep_tiles_n = 0, dep_cells = 0;  // tiles of the last deposit, cells of one
+    bool dep_large = false;  // its pairs needed the larger tiles
     float mesh_boxsize = 0.0f;
     std::vector<MeshBuf> meshes;
 
@@ -1047,9 +1048,11 @@ int asg_run_remove_small_groups(asg_ctx* ctx, int ngrp, int* nhalo)
     return 0;
 }
 
-// entries and pairs that a deposit's arrays hold
+// entries and pairs that a deposit's arrays hold, and whether its pairs need the
+// larger tiles
 struct DepositCap {
     uint32_t entries = 0, pairs = 0;
+    bool large_tiles = false;
 };
 
 // no cap: the arrays are sized from the counts (one host synchronisation); with a
@@ -1073,6 +1076,7 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     p.periodic = periodic ? 1 : 0;
     p.density_only = density_only ? 1 : 0;
     p.seg = ctx->dep_seg;
+    if (cap) large_tiles = cap->large_tiles;
     p.mma = large_tiles ? 0 : ctx->dep_mma;
     for (int d = 0; d < 3; ++d) p.offset[d] = periodic && coords ? boxsize * (float)coords[d] : 0.0f;
     // the pair keys hold tile << 5 | image in 32 bits: meshes of more tiles than
@@ -1159,6 +1163,7 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     if (!cap) {
         ctx->dep_npairs = have.pairs;
         ctx->dep_nentries = have.entries;
+        ctx->dep_large = large_tiles;
     }
     ctx->dep_tiles_n = tiles;
     ctx->dep_cells = 1 << (p.shift[0] + p.shift[1] + p.shift[2]);
@@ -1706,14 +1711,18 @@ int batch_plan(asg_batch* b)
     }
     b->cap.assign((size_t)b->n_items, DepositCap{});
     uint32_t max_entries = 0, max_items = 0;
+    size_t max_partial = 0;
     for (int i = 0; i < b->n_items; ++i) {
         asg_ctx* c = b->sub[(size_t)i % S];
         if (int r = batch_queue_item(b, c, i, nullptr)) return fail(ctx, r, c->last);
         DepositCap& cap = b->cap[(size_t)i];  // headroom for inputs that change between runs
         cap.entries = c->dep_nentries + c->dep_nentries / 16 + 4096;
         cap.pairs = c->dep_npairs + c->dep_npairs / 16 + 4096;
+        cap.large_tiles = c->dep_large;
         max_entries = std::max(max_entries, cap.entries);
-        max_items = std::max(max_items, deposit_max_items(c->dep_tiles_n, cap.pairs, c->dep_seg));
+        const uint32_t items = deposit_max_items(c->dep_tiles_n, cap.pairs, c->dep_seg);
+        max_items = std::max(max_items, items);
+        max_partial = std::max(max_partial, deposit_partial_bytes(items, c->dep_cells));
     }
     for (asg_ctx* c : b->sub)
         if (int r = finish(c, "batch plan")) return fail(ctx, r, c->last);
@@ -1721,7 +1730,7 @@ int batch_plan(asg_batch* b)
     for (asg_ctx* c : b->sub) {
         int r = grow(c, c->dep_pairs, deposit_entry_bytes(max_entries));
         if (!r) r = grow(c, c->dep_sort, radix_sort_temp_bytes((int)max_entries));
-        if (!r) r = grow(c, c->dep_partial, deposit_partial_bytes(max_items, c->dep_cells) + 16);
+        if (!r) r = grow(c, c->dep_partial, max_partial + 16);
         if (!r) r = grow(c, c->dep_items, 4 * (size_t)max_items);
         if (r) return fail(ctx, r, "batch: deposit reserve");
     }

@@ -78,3 +78,30 @@ def test_tuned_leaf_sizes_fit_the_box_array(fake, monkeypatch, leaf):
     assert sum(ln[0] == "boxes" for ln in lines) > 100
     assert not boxes_short(lines)
     fake.asg_destroy(ctx)
+
+
+def kernels(lines, *names):
+    """(kernel, grid, block) of the launches of these kernels, in order"""
+    return [(n, int(ln[2]), int(ln[3])) for ln in lines if ln[0] == "launch"
+            for n in names if f"{len(n)}{n}" in ln[1]]
+
+
+@pytest.mark.parametrize("small,large", [(10 ** 6, 10 ** 6), (2 ** 31 - 1, 2 ** 29), (2 ** 31, 2 ** 29),
+                                         (2 ** 33, 2 ** 31 - 1)])
+def test_captured_deposit_takes_the_planned_tiles(fake, small, large):
+    """A batch item with more pairs than 32 bits number takes the larger tiles in the
+    planning pass, and so it does in the graph, whose capture allocates nothing."""
+    ctx = context(fake)
+    b = batch(fake, ctx, [5000, 4000], ncs=(16, 32))
+    fake.fake_counts(1000, small, large)
+    log(fake)
+    assert fake.asg_batch_run(b) == 0
+    lines = log(fake)
+    fake.fake_counts(0, 0, 0)
+    at = [ln[0] for ln in lines].index("capture")
+    plan = [k[0] for k in kernels(lines[:at], "k_deposit_mma", "k_deposit_items")]
+    graph = [k[0] for k in kernels(lines[at:], "k_deposit_mma", "k_deposit_items")]
+    assert not any(ln[0] == "malloc" for ln in lines[at:])
+    assert plan == graph == 2 * ["k_deposit_mma" if small < 2 ** 31 else "k_deposit_items"]
+    fake.asg_batch_destroy(b)
+    fake.asg_destroy(ctx)
