@@ -70,7 +70,8 @@ struct asg_ctx {
     int n = 0;
     float left = 0.f, right = 0.f;
     bool loaded = false, knn_done = false, idx33_all = false;
-    int leaf = LEAF_DEFAULT;  // particles per tree leaf
+    int leaf = LEAF_DEFAULT;  // particles per tree leaf, of the next index build
+    int tree_leaf = LEAF_DEFAULT;  // and of the loaded set's tree
     int dep_seg = 4096;  // pairs per deposit work item, at most
     int knn_warps = 2;   // warps per block of the neighbour search (2 or 4)
     int dep_mma = deposit_default_mma();  // deposit engine: tensor cores (1) or CUDA cores (0)
@@ -264,7 +265,7 @@ int finish_totals(asg_ctx* ctx, const char* what, int n_nc, double* totals)
 
 TreeView tree_view(asg_ctx* ctx)
 {
-    TreeView t = tree_shape(ctx->n, ctx->leaf);
+    TreeView t = tree_shape(ctx->n, ctx->tree_leaf);
     t.box = P<float4>(ctx->boxes);
     return t;
 }
@@ -298,6 +299,7 @@ int alloc_set(asg_ctx* ctx, int n)
 int build_index(asg_ctx* ctx, bool with_rk)
 {
     const int n = ctx->n;
+    ctx->tree_leaf = ctx->leaf;
     const int cur = radix_sort(P<uint64_t>(ctx->keys0), P<int>(ctx->vals0), P<uint64_t>(ctx->keys1),
                                P<int>(ctx->vals1), n, 48, true, ctx->sort_tmp.p, ctx->d_err, ctx->s);
     ctx->perm = cur ? P<int>(ctx->vals1) : P<int>(ctx->vals0);

@@ -7,10 +7,12 @@
 //   load <kernel>                              (cudaFuncGetAttributes)
 //   malloc <bytes>
 //   boxes <bytes the tree takes> <bytes from its start to the end of its block>
+//   tree <kernel> <particles per leaf>         (the tree that a kernel builds or walks)
 // k_report (the words that a call brings to the host) is carried out, and so are
 // the two counts of k_dep_prep, with the numbers that fake_counts() was given.
 #include <sys/mman.h>
 
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -31,6 +33,7 @@ std::map<const void*, void*> g_var_at;
 std::map<char*, size_t> g_blocks;
 uint32_t g_entries = 0;
 unsigned long long g_pairs_small = 0, g_pairs_large = 0;
+int g_timed = 0, g_fastest = INT_MAX;
 
 void line(const std::string& s) { g_log += s + "\n"; }
 std::string num(unsigned long long v) { return std::to_string(v); }
@@ -55,6 +58,8 @@ void launched(const std::string& k, dim3 grid, dim3 block, size_t smem, void** a
 {
     line("launch " + k + " " + num((unsigned long long)grid.x * grid.y * grid.z) + " " + num(block.x) + " " +
          num(smem));
+    const int tree = is(k, "k_gather") ? 8 : is(k, "k_fof_link") || is(k, "k_mark_halos") || is(k, "k_knn_ties") ? 1 : -1;
+    if (tree >= 0) line("tree " + k + " " + num(static_cast<TreeView*>(a[tree])->leaf));
     if (is(k, "k_report")) {
         HostWords* out = *static_cast<HostWords**>(a[4]);
         int at = 0;
@@ -107,6 +112,13 @@ void fake_counts(uint32_t entries, unsigned long long pairs_small_tiles, unsigne
     g_entries = entries;
     g_pairs_small = pairs_small_tiles;
     g_pairs_large = pairs_large_tiles;
+}
+
+// of the times that are asked for, the n-th from now on is the shortest
+void fake_fastest(int n)
+{
+    g_timed = 0;
+    g_fastest = n;
 }
 
 void** __cudaRegisterFatBinary(void*)
@@ -257,8 +269,7 @@ cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t)
 {
-    static float next = 1000.0f;  // every setting that is timed beats the one before it
-    *ms = next *= 0.999f;
+    *ms = (float)std::abs((long long)++g_timed - g_fastest);
     return cudaSuccess;
 }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) { return handle(x); }

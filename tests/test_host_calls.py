@@ -28,8 +28,14 @@ def fake(tmp_path_factory):
         getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
     lib.fake_log.restype = C.c_char_p
     lib.fake_counts.argtypes = [C.c_uint32, C.c_ulonglong, C.c_ulonglong]
-    lib.fake_counts(0, 0, 0)
     return lib
+
+
+@pytest.fixture(autouse=True)
+def fresh(fake):
+    fake.fake_counts(0, 0, 0)
+    fake.fake_fastest(10 ** 6)
+    fake.fake_clear()
 
 
 def log(fake):
@@ -94,14 +100,32 @@ def test_captured_deposit_takes_the_planned_tiles(fake, small, large):
     ctx = context(fake)
     b = batch(fake, ctx, [5000, 4000], ncs=(16, 32))
     fake.fake_counts(1000, small, large)
-    log(fake)
     assert fake.asg_batch_run(b) == 0
     lines = log(fake)
-    fake.fake_counts(0, 0, 0)
     at = [ln[0] for ln in lines].index("capture")
     plan = [k[0] for k in kernels(lines[:at], "k_deposit_mma", "k_deposit_items")]
     graph = [k[0] for k in kernels(lines[at:], "k_deposit_mma", "k_deposit_items")]
     assert not any(ln[0] == "malloc" for ln in lines[at:])
     assert plan == graph == 2 * ["k_deposit_mma" if small < 2 ** 31 else "k_deposit_items"]
+    fake.asg_batch_destroy(b)
+    fake.asg_destroy(ctx)
+
+
+def test_tuned_context_walks_the_tree_it_built(fake):
+    """The tuner leaves the largest item loaded, with a tree of the last leaf size it
+    timed; calls on that set walk that tree, whatever leaf size was chosen."""
+    ctx = context(fake)
+    b = batch(fake, ctx, [3000, 2000])
+    fake.fake_fastest(2)
+    chosen, groups = C.c_int(0), C.c_int(0)
+    assert fake.asg_batch_tune(b, C.byref(chosen), None) == 0 and chosen.value == 16
+    assert fake.asg_run_fof(ctx, 0.5, C.byref(groups)) == 0
+    halo = np.zeros(5, np.float32)
+    assert fake.asg_run_mark_halos(ctx, halo.ctypes.data, 1, None, None) == 0
+    assert fake.asg_get_knn(ctx, None, None) == 0
+    trees = [ln for ln in log(fake) if ln[0] == "tree"]
+    assert ["k_mark_halos" in trees[-2][1], "k_knn_ties" in trees[-1][1]] == [True, True]
+    built = [int(t[2]) for t in trees if "k_gather" in t[1]][-1]
+    assert [int(t[2]) for t in trees[-3:]] == 3 * [built]
     fake.asg_batch_destroy(b)
     fake.asg_destroy(ctx)
