@@ -1934,28 +1934,38 @@ int asg_batch_set_item_quantised(asg_batch* b, int item, const int* cell, const 
     return ASG_OK;
 }
 
-int asg_batch_tune(asg_batch* b, int* leaf, int* seg)
+// the four settings that the tuner chooses
+struct Tuning {
+    int leaf, seg, warps, mma;
+};
+static Tuning tuning_of(const asg_ctx* ctx) { return {ctx->leaf, ctx->dep_seg, ctx->knn_warps, ctx->dep_mma}; }
+static void set_tuning(asg_ctx* ctx, const Tuning& t)
 {
-    if (!b) return ASG_ERR_ARG;
+    ctx->leaf = t.leaf;
+    ctx->dep_seg = t.seg;
+    ctx->knn_warps = t.warps;
+    ctx->dep_mma = t.mma;
+}
+
+// times the largest item with every setting; the context is left at the last one
+static int tune_settings(asg_batch* b, Tuning& fastest)
+{
     asg_ctx* ctx = b->ctx;
-    CK(cudaSetDevice(ctx->device));
     int item = 0;  // the largest item
     for (int i = 1; i < b->n_items; ++i)
         if (b->np[(size_t)i] > b->np[(size_t)item]) item = i;
-    // tree bucket size x deposit work-item length x neighbour-search warps per
+    // tree leaf size x deposit work-item length x neighbour-search warps per
     // block x deposit engine (tensor cores or CUDA cores)
     const int leaves[] = {16, 24, 32}, segs[] = {2048, 4096, 8192}, warps[] = {2, 4}, mmas[] = {1, 0};
     float best = INFINITY;
-    int bl = ctx->leaf, bs = ctx->dep_seg, bw = ctx->knn_warps, bm = ctx->dep_mma;
     for (int l : leaves) {
         ctx->leaf = l;
         if (int r = alloc_set(ctx, b->max_n)) return r;  // smaller leaves have more boxes
         for (int sg : segs)
             for (int w : warps)
                 for (int m : mmas) {
-                    ctx->dep_seg = sg;
-                    ctx->knn_warps = w;
-                    ctx->dep_mma = m;
+                    const Tuning t{l, sg, w, m};
+                    set_tuning(ctx, t);
                     float ms = 0.0f;
                     for (int rep = 0; rep < 2; ++rep) {  // the first repetition warms up
                         CK(cudaEventRecord(b->e0, ctx->s));
@@ -1966,21 +1976,27 @@ int asg_batch_tune(asg_batch* b, int* leaf, int* seg)
                     }
                     if (ms < best) {
                         best = ms;
-                        bl = l;
-                        bs = sg;
-                        bw = w;
-                        bm = m;
+                        fastest = t;
                     }
                 }
     }
-    ctx->leaf = bl;
-    ctx->dep_seg = bs;
-    ctx->knn_warps = bw;
-    ctx->dep_mma = bm;
-    batch_drop_graph(b);  // a new configuration needs a new plan and capture
-    if (leaf) *leaf = bl;
-    if (seg) *seg = bs;
     return finish(ctx, "batch tune");
+}
+
+int asg_batch_tune(asg_batch* b, int* leaf, int* seg)
+{
+    if (!b) return ASG_ERR_ARG;
+    asg_ctx* ctx = b->ctx;
+    CK(cudaSetDevice(ctx->device));
+    batch_drop_graph(b);  // its buffers may move, and a new configuration needs a new plan and capture
+    const Tuning before = tuning_of(ctx);
+    Tuning t = before;
+    const int r = tune_settings(b, t);
+    if (r) t = before;
+    set_tuning(ctx, t);
+    if (leaf) *leaf = t.leaf;
+    if (seg) *seg = t.seg;
+    return r;
 }
 
 int asg_batch_config(asg_batch* b, int* leaf, int* seg, int* knn_warps, int* deposit_engine)

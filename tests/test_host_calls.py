@@ -129,3 +129,23 @@ def test_tuned_context_walks_the_tree_it_built(fake):
     assert [int(t[2]) for t in trees[-3:]] == 3 * [built]
     fake.asg_batch_destroy(b)
     fake.asg_destroy(ctx)
+
+
+def test_tuner_that_fails_leaves_the_configuration(fake, monkeypatch):
+    """... and no graph that holds buffers which it may have moved."""
+    monkeypatch.setenv("ASG_LEAF_SIZE", "24")
+    ctx = context(fake)
+    b = batch(fake, ctx, [3000])
+    v = [C.c_int(0) for _ in range(8)]
+    assert fake.asg_batch_config(b, *[C.byref(t) for t in v[:4]]) == 0 and v[0].value == 24
+    assert fake.asg_batch_run(b) == 0
+    fake.fake_counts(10, 2 ** 33, 2 ** 33)  # more pairs than either tile shape can number
+    assert fake.asg_batch_tune(b, None, None) != 0
+    assert fake.asg_batch_config(b, *[C.byref(t) for t in v[4:]]) == 0
+    assert [t.value for t in v[4:]] == [t.value for t in v[:4]]
+    fake.fake_counts(10, 100, 100)
+    log(fake)
+    assert fake.asg_batch_run(b) == 0
+    assert ["capture"] in log(fake)
+    fake.asg_batch_destroy(b)
+    fake.asg_destroy(ctx)
