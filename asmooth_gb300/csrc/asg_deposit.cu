@@ -154,11 +154,17 @@ __device__ __forceinline__ void image_tiles(const AxisRange& r, int k, int nc, i
 // mesh and image the warp goes through the tiles of the union of its lanes' tile
 // boxes; where that holds many more tiles than the lanes touch (particles far
 // apart), through each lane's own tiles, one lane after another.  Either way the
-// particles of a tile come in lane order.
-template <bool PERIODIC, class F>
+// particles of a tile come in lane order.  Of `parts` warps with the same bundle (a
+// power of two), each takes the rows of tiles whose y + z falls to it.
+// count(entries, pairs) instead of f with COUNT: the lanes' own boxes give the pairs,
+// and a row of tiles is one union of bit masks.
+template <bool PERIODIC, bool COUNT, class F>
 __device__ __forceinline__ void for_entries(const DepositParams& P, const float (&lo)[3],
-                                            const float (&hi)[3], bool live, int* err, F f)
+                                            const float (&hi)[3], bool live, int part, int parts, int* err,
+                                            F f)
 {
+    // the first row of tiles from y on, at z, that falls to this warp
+    auto first_row = [&](int y, int z) { return y + ((part - y - z) & (parts - 1)); };
     for (int jb = 0; jb < P.n_jobs; ++jb) {
         const MeshJob& J = P.job[jb];
         const int nc = J.nc;
@@ -180,12 +186,12 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
             const int image = nz * 9 + ny * 3 + nx;
             int t0[3], t1[3];  // the lane's tiles
             bool in = on;
-            int own = 1;
+            unsigned own = 1;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 image_tiles(r[a], PERIODIC ? r[a].k_lo + dk[a] : 0, nc, P.shift[a], t0[a], t1[a]);
                 in = in && (!PERIODIC || (dk[a] < r[a].nk && t0[a] <= t1[a]));
-                own *= t1[a] - t0[a] + 1;
+                own *= (unsigned)(t1[a] - t0[a] + 1);
             }
             unsigned lanes = PERIODIC ? __ballot_sync(FULLM, in) : ~0u;
             if (PERIODIC && !lanes) return;
@@ -196,17 +202,27 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
                 u0[a] = (int)__reduce_min_sync(FULLM, (unsigned)t0[a]);
                 u1[a] = __reduce_max_sync(FULLM, t1[a]);
             }
-            const unsigned touched = __reduce_add_sync(FULLM, in ? (unsigned)min(own, 1 << 24) : 0u);
+            if (!in) own = 0;
+            const unsigned touched = __reduce_add_sync(FULLM, min(own, 1u << 24));
             const unsigned wx = u1[0] - u0[0] + 1, wy = u1[1] - u0[1] + 1, wz = u1[2] - u0[2] + 1;
+            if constexpr (COUNT) f(0u, part == 0 ? own : 0u);
             if ((unsigned long long)(wx * wy) * wz <= 2ull * touched + 64) {
                 for (int tz = u0[2]; tz <= u1[2]; ++tz) {
                     const bool inz = t0[2] <= tz && tz <= t1[2];
-                    for (int ty = u0[1]; ty <= u1[1]; ++ty) {
+                    for (int ty = first_row(u0[1], tz); ty <= u1[1]; ty += parts) {
                         const bool iny = inz && t0[1] <= ty && ty <= t1[1];
-                        int tile = J.tile_begin + (tz * J.tiles[1] + ty) * J.tiles[0] + u0[0];
-                        for (int tx = u0[0]; tx <= u1[0]; ++tx, ++tile) {
-                            const unsigned m = __ballot_sync(FULLM, iny && t0[0] <= tx && tx <= t1[0]);
-                            if (m) f(tile, image, m);
+                        if constexpr (COUNT) {
+                            for (int tx = u0[0]; tx <= u1[0]; tx += 32) {
+                                const int a = max(t0[0] - tx, 0), b = min(t1[0] - tx, 31);
+                                const unsigned bits = (2u << (b & 31)) - (1u << (a & 31));
+                                f((unsigned)__popc(__reduce_or_sync(FULLM, iny && a <= b ? bits : 0u)), 0u);
+                            }
+                        } else {
+                            int tile = J.tile_begin + (tz * J.tiles[1] + ty) * J.tiles[0] + u0[0];
+                            for (int tx = u0[0]; tx <= u1[0]; ++tx, ++tile) {
+                                const unsigned m = __ballot_sync(FULLM, iny && t0[0] <= tx && tx <= t1[0]);
+                                if (m) f(tile, image, m);
+                            }
                         }
                     }
                 }
@@ -219,9 +235,12 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
                     const int y0 = __shfl_sync(FULLM, t0[1], l), y1 = __shfl_sync(FULLM, t1[1], l);
                     const int z0 = __shfl_sync(FULLM, t0[2], l), z1 = __shfl_sync(FULLM, t1[2], l);
                     for (int tz = z0; tz <= z1; ++tz)
-                        for (int ty = y0; ty <= y1; ++ty)
-                            for (int tx = x0; tx <= x1; ++tx)
-                                f(J.tile_begin + (tz * J.tiles[1] + ty) * J.tiles[0] + tx, image, 1u << l);
+                        for (int ty = first_row(y0, tz); ty <= y1; ty += parts)
+                            if constexpr (COUNT)
+                                f((unsigned)(x1 - x0 + 1), 0u);
+                            else
+                                for (int tx = x0; tx <= x1; ++tx)
+                                    f(J.tile_begin + (tz * J.tiles[1] + ty) * J.tiles[0] + tx, image, 1u << l);
                 }
             }
         };
@@ -244,20 +263,21 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
 // -h when the particle deposits into the halo channel, 0 when it deposits
 // nothing.  The cell-range edges (x' -+ h)/L and 1/h are recomputed from it
 // where they are needed (load_dep_rec), with the same rounded operations.
-// counts: the entries of each bundle, counts[bundles] = 0; *pairs += the pairs.
+// counts: the entries of each part of each bundle, then 0; *pairs += the pairs.
 template <bool PERIODIC>
 __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restrict__ vel,
-                           const int* __restrict__ igrp, const float* __restrict__ rk, int n,
+                           const int* __restrict__ igrp, const float* __restrict__ rk, int n, int parts,
                            const __grid_constant__ DepositParams P, float4* __restrict__ rec,
                            uint32_t* __restrict__ counts, unsigned long long* __restrict__ pairs,
                            int* err)
 {
     grid_begin();
     __shared__ unsigned long long block_pairs;  // one atomic per block: 0.57 M on one word took 0.3 ms
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int unit = (blockIdx.x * blockDim.x + threadIdx.x) / 32, part = unit & (parts - 1);
+    const int i = unit / parts * 32 + (threadIdx.x & 31);
     const int bundles = (n + 31) / 32;
     if (threadIdx.x == 0) block_pairs = 0ull;
-    if (i == 0) counts[bundles] = 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) counts[bundles * parts] = 0u;
     __syncthreads();
     bool live = i < n;
     const int ii = live ? i : n - 1;
@@ -277,7 +297,7 @@ __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restr
             x[a] = __fadd_rn(x[a], P.offset[a]);
         }
     }
-    if (live) {
+    if (live && part == 0) {
         rec[2 * (size_t)i] = make_float4(x[0], x[1], x[2], skip ? 0.0f : (halo ? -h : h));
         rec[2 * (size_t)i + 1] = make_float4(v.w, v.x, v.y, v.z);
     }
@@ -288,15 +308,16 @@ __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restr
         lo[a] = div_rn_by(__fsub_rn(x[a], h), L, P.rbox);
         hi[a] = div_rn_by(__fadd_rn(x[a], h), L, P.rbox);
     }
-    uint32_t cnt = 0, np = 0;
-    for_entries<PERIODIC>(P, lo, hi, live, err, [&](int, int, unsigned m) {
-        ++cnt;
-        np += (uint32_t)__popc(m);
+    uint32_t cnt = 0;
+    unsigned long long np = 0;  // this lane's
+    for_entries<PERIODIC, true>(P, lo, hi, live, part, parts, err, [&](unsigned entries, unsigned pairs) {
+        cnt += entries;
+        np += pairs;
     });
-    if ((i & 31) == 0 && i < n) {
-        counts[i >> 5] = cnt;
-        if (np) atomicAdd(&block_pairs, (unsigned long long)np);
-    }
+    if ((i & 31) == 0 && i < n) counts[unit] = cnt;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(FULLM, np, o);
+    if ((i & 31) == 0 && np) atomicAdd(&block_pairs, np);
     __syncthreads();
     if (threadIdx.x == 0 && block_pairs) atomicAdd(pairs, block_pairs);
 }
@@ -311,19 +332,20 @@ __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restr
 // entry o is written only when o < cap (the entry arrays' capacity); one beyond
 // it sets ERR_CAP instead
 template <bool PERIODIC>
-__global__ void k_entries(const float4* __restrict__ rec, int n, const __grid_constant__ DepositParams P,
+__global__ void k_entries(const float4* __restrict__ rec, int n, int parts, const __grid_constant__ DepositParams P,
                           const uint32_t* __restrict__ offs, uint32_t* __restrict__ keys,
                           uint2* __restrict__ entry, uint32_t cap, int* err)
 {
     grid_begin();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((i & ~31) >= n) return;
     const int lane = threadIdx.x & 31;
+    const int unit = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int i = unit / parts * 32 + lane;
+    if ((i & ~31) >= n) return;
     float4 a, b, c, d;
     load_dep_rec(rec, min(i, n - 1), P.boxsize, P.rbox, a, b, c, d);
     const bool live = i < n && !(__float_as_int(d.z) & FLAG_SKIP);
     const float lo[3] = {b.x, b.y, b.z}, hi[3] = {c.x, c.y, c.z};
-    uint32_t o = offs[i >> 5];  // the next group of up to 32 entries goes here
+    uint32_t o = offs[unit];    // the next group of up to 32 entries goes here
     int held = 0;               // entries held by the lanes below it
     uint32_t key = 0, mask = 0;
     auto store = [&]() {
@@ -338,7 +360,7 @@ __global__ void k_entries(const float4* __restrict__ rec, int n, const __grid_co
         o += held;
         held = 0;
     };
-    for_entries<PERIODIC>(P, lo, hi, live, err, [&](int tile, int image, unsigned m) {
+    for_entries<PERIODIC, false>(P, lo, hi, live, unit & (parts - 1), parts, err, [&](int tile, int image, unsigned m) {
         if (lane == held) {
             key = PERIODIC ? ((uint32_t)tile << IMG_BITS) | (uint32_t)image : (uint32_t)tile;
             mask = m;
@@ -1342,6 +1364,20 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
 // ---------------------------------------------------------------------------
 size_t deposit_prep_bytes(int n) { return 32 * (size_t)n; }
 
+// A warp goes through a bundle's tiles one after another: with few bundles and wide
+// supports on a fine mesh, few warps had a long way (64 particles with supports of 120
+// cells of a 256^3 mesh 8.8 ms, a thread per particle 0.8, 16 warps per bundle 0.8).
+// As many as make 4096 warps: 13,840 particles on a mesh of 6 cells per mean
+// separation 391 us with 1, 281 with 8, of 1 cell 73 and 71; 32,768 647, 560 with 4
+// and 87, 84; above that a bundle's fixed cost (ranges, unions) is most of it.
+int deposit_parts(int n)
+{
+    const long long bundles = ((long long)n + 31) / 32;
+    int parts = 1;
+    while (parts < 16 && 2 * parts * bundles <= 4096) parts *= 2;
+    return parts;
+}
+
 void deposit_tile_shape(DepositParams& p)
 {
     p.shift[0] = 3;
@@ -1424,24 +1460,24 @@ void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, 
                          int n, const DepositParams& p, DepositScratch& w, int* err,
                          cudaStream_t s)
 {
-    const int bundles = (n + 31) / 32;
+    const int parts = deposit_parts(n), units = (n + 31) / 32 * parts;
     cudaMemsetAsync(w.counters, 0, 32, s);
     auto kern = p.periodic ? k_dep_prep<true> : k_dep_prep<false>;
-    launch(kern, (bundles + 7) / 8, 256, 0, s, pos, vel, igrp, rk, n, p, w.rec, w.count,
-                                           reinterpret_cast<unsigned long long*>(w.counters + 2), err);
-    exclusive_scan_u32(w.count, (size_t)bundles + 1, w.scan_tmp_n, s);
+    launch(kern, (units + 7) / 8, 256, 0, s, pos, vel, igrp, rk, n, parts, p, w.rec, w.count,
+           reinterpret_cast<unsigned long long*>(w.counters + 2), err);
+    exclusive_scan_u32(w.count, (size_t)units + 1, w.scan_tmp_n, s);
     count_launches(1);
 }
 
 void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t entries,
                         uint32_t max_items, bool padded, DepositScratch& w, int* err, cudaStream_t s)
 {
-    const int T = total_tiles, bundles = (n + 31) / 32;
+    const int T = total_tiles, parts = deposit_parts(n), units = (n + 31) / 32 * parts;
     auto kern = p.periodic ? k_entries<true> : k_entries<false>;
-    launch(kern, (bundles + 7) / 8, 256, 0, s, w.rec, n, p, w.count, w.keys0, w.entry, entries, err);
+    launch(kern, (units + 7) / 8, 256, 0, s, w.rec, n, parts, p, w.count, w.keys0, w.entry, entries, err);
     count_launches(1);
-    if (padded && entries > 0) {  // `entries` is the capacity; the count itself is count[bundles]
-        launch(k_pad_entries, (entries + 255) / 256, 256, 0, s, w.keys0, w.entry, w.count + bundles, entries,
+    if (padded && entries > 0) {  // `entries` is the capacity; the count itself is the last of `count`
+        launch(k_pad_entries, (entries + 255) / 256, 256, 0, s, w.keys0, w.entry, w.count + units, entries,
                                                             (uint32_t)T << img_bits(p));
         count_launches(1);
     }

@@ -123,8 +123,8 @@ void deposit_tile_shape(DepositParams& p);
 // those of them that touch a tile), work items
 struct DepositScratch {
     float4* rec;          // [2n] x', y', z', h (-h: halo channel, 0: skipped) | dens, v
-    uint32_t* count;      // [bundles+1] entries per bundle, then their exclusive scan
-    void* scan_tmp_n;     // scan scratch for bundles+1 entries
+    uint32_t* count;      // [units+1] entries per part of a bundle, then their exclusive scan
+    void* scan_tmp_n;     // scan scratch for units+1 entries
     uint2* entry;         // [entries] bundle, lane mask, as emitted
     uint2* list;          // [entries] the same in key order
     uint32_t* keys0;      // [entries] tile << 5 | image (periodic), else tile; ping-pong with keys1
@@ -144,6 +144,8 @@ struct DepositScratch {
                           // front, number of pairs (64 bits), length of merge's back
 };
 size_t deposit_prep_bytes(int n);
+// warps that share the making of a bundle's entries (units = bundles * parts)
+int deposit_parts(int n);
 size_t deposit_tile_bytes(int total_tiles);
 size_t deposit_entry_bytes(uint32_t entries);
 // the per-entry arrays of w inside one block of deposit_entry_bytes
@@ -152,13 +154,13 @@ void deposit_entry_layout(void* base, uint32_t entries, DepositScratch& w);
 uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int most);
 int deposit_default_mma();
 size_t deposit_partial_bytes(uint32_t items, int cells);  // of tiles of that many cells
-// pass 1: particle records and entry counts; count[bundles] then holds the number
+// pass 1: particle records and entry counts; count[units] then holds the number
 // of entries, counters[2..3] the number of pairs
 void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, const float* rk,
                          int n, const DepositParams& p, DepositScratch& w, int* err,
                          cudaStream_t s);
 // pass 2: emit and sort the entries, deposit every (tile, segment), merge multi-segment tiles.
-// padded = false: `entries` is the exact number (read back from count[bundles]);
+// padded = false: `entries` is the exact number (read back from count[units]);
 // padded = true: it is the arrays' capacity, the number stays on the device
 // (no host synchronisation, e.g. under stream capture) and a larger one sets ERR_CAP,
 // as do more than max_items work items
