@@ -180,12 +180,13 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
             on = false;
         }
         if (!__any_sync(FULLM, on)) continue;
-        // one image of the mesh per axis (nx, ny, nz: the lane's 0th, 1st or 2nd)
-        auto one_image = [&](int nx, int ny, int nz) {
+        // one image of the mesh per axis (nx, ny, nz: the lane's 0th, 1st or 2nd), of
+        // the lanes of `group`
+        auto one_image = [&](bool group, int nx, int ny, int nz) {
             const int dk[3] = {nx, ny, nz};
             const int image = nz * 9 + ny * 3 + nx;
             int t0[3], t1[3];  // the lane's tiles
-            bool in = on;
+            bool in = group;
             unsigned own = 1;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
@@ -245,15 +246,31 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
             }
         };
         if constexpr (PERIODIC) {
-            int most[3];  // images per axis
+            // The lanes of the same first image go together: their n-th images lie together,
+            // while those of a lane that reaches over the mesh's edge and of its neighbour
+            // that does not lie at opposite ends of the mesh, and a union of both is all of
+            // it (262,144 particles on 383^3 cells 6.1 -> 5.0 ms, 13,840 on 95^3 485 -> 422
+            // us).  All lanes together where the mesh has few tiles, as each group costs what
+            // 64 tiles do (4096 particles on 31^3 92, in groups 96), and where the bundle's
+            // particles are far apart (more than 8 groups).
+            const int first = (r[0].k_lo & 1023) | (r[1].k_lo & 1023) << 10 | (r[2].k_lo & 1023) << 20;
+            const unsigned same = __match_any_sync(FULLM, on ? first : -1);
+            unsigned leaders = __ballot_sync(FULLM, on && (same & lanemask_lt()) == 0u);
+            const bool together = __popc(leaders) > 8 || J.tiles[0] * J.tiles[1] * J.tiles[2] < 64 * parts;
+            if (together) leaders &= 0u - leaders;
+            for (; leaders; leaders &= leaders - 1) {
+                const int lead = __shfl_sync(FULLM, first, __ffs(leaders) - 1);
+                const bool group = on && (together || first == lead);
+                int most[3];  // images per axis
 #pragma unroll
-            for (int a = 0; a < 3; ++a)
-                most[a] = (int)__reduce_max_sync(FULLM, (unsigned)(on ? r[a].nk : 0));
-            for (int nz = 0; nz < most[2]; ++nz)
-                for (int ny = 0; ny < most[1]; ++ny)
-                    for (int nx = 0; nx < most[0]; ++nx) one_image(nx, ny, nz);
+                for (int a = 0; a < 3; ++a)
+                    most[a] = (int)__reduce_max_sync(FULLM, (unsigned)(group ? r[a].nk : 0));
+                for (int nz = 0; nz < most[2]; ++nz)
+                    for (int ny = 0; ny < most[1]; ++ny)
+                        for (int nx = 0; nx < most[0]; ++nx) one_image(group, nx, ny, nz);
+            }
         } else {
-            one_image(0, 0, 0);
+            one_image(on, 0, 0, 0);
         }
     }
 }
@@ -1366,15 +1383,17 @@ size_t deposit_prep_bytes(int n) { return 32 * (size_t)n; }
 
 // A warp goes through a bundle's tiles one after another: with few bundles and wide
 // supports on a fine mesh, few warps had a long way (64 particles with supports of 120
-// cells of a 256^3 mesh 8.8 ms, a thread per particle 0.8, 16 warps per bundle 0.8).
+// cells of a 256^3 mesh 8.8 ms, a thread per particle 0.8, 32 warps per bundle 0.6).
 // As many as make 4096 warps: 13,840 particles on a mesh of 6 cells per mean
 // separation 391 us with 1, 281 with 8, of 1 cell 73 and 71; 32,768 647, 560 with 4
-// and 87, 84; above that a bundle's fixed cost (ranges, unions) is most of it.
-int deposit_parts(int n)
+// and 87, 84; above that a bundle's fixed cost (ranges, unions) is most of it.  A
+// periodic mesh has more tiles per bundle: 8192 (131,072 particles 2.71, 2.57 ms with 2
+// and 220, 216 us), and a bundle of particles far apart the most.
+int deposit_parts(int n, bool periodic)
 {
     const long long bundles = ((long long)n + 31) / 32;
-    int parts = 1;
-    while (parts < 16 && 2 * parts * bundles <= 4096) parts *= 2;
+    int parts = bundles <= 32 ? 32 : 1;
+    while (parts < 16 && 2 * parts * bundles <= (periodic ? 8192 : 4096)) parts *= 2;
     return parts;
 }
 
@@ -1460,7 +1479,7 @@ void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, 
                          int n, const DepositParams& p, DepositScratch& w, int* err,
                          cudaStream_t s)
 {
-    const int parts = deposit_parts(n), units = (n + 31) / 32 * parts;
+    const int parts = deposit_parts(n, p.periodic != 0), units = (n + 31) / 32 * parts;
     cudaMemsetAsync(w.counters, 0, 32, s);
     auto kern = p.periodic ? k_dep_prep<true> : k_dep_prep<false>;
     launch(kern, (units + 7) / 8, 256, 0, s, pos, vel, igrp, rk, n, parts, p, w.rec, w.count,
@@ -1472,7 +1491,7 @@ void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, 
 void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t entries,
                         uint32_t max_items, bool padded, DepositScratch& w, int* err, cudaStream_t s)
 {
-    const int T = total_tiles, parts = deposit_parts(n), units = (n + 31) / 32 * parts;
+    const int T = total_tiles, parts = deposit_parts(n, p.periodic != 0), units = (n + 31) / 32 * parts;
     auto kern = p.periodic ? k_entries<true> : k_entries<false>;
     launch(kern, (units + 7) / 8, 256, 0, s, w.rec, n, parts, p, w.count, w.keys0, w.entry, entries, err);
     count_launches(1);

@@ -145,7 +145,7 @@ struct DepositScratch {
 };
 size_t deposit_prep_bytes(int n);
 // warps that share the making of a bundle's entries (units = bundles * parts)
-int deposit_parts(int n);
+int deposit_parts(int n, bool periodic);
 size_t deposit_tile_bytes(int total_tiles);
 size_t deposit_entry_bytes(uint32_t entries);
 // the per-entry arrays of w inside one block of deposit_entry_bytes

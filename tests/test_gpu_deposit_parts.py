@@ -1,6 +1,6 @@
 """GPU test of the making of the deposit's entries: bundle counts on both sides of
-every change in the number of warps that share a bundle (powers of two up to 16,
-1 from 4097 bundles on), with particles spread over the box, in clumps, and at the
+every change in the number of warps that share a bundle (32 up to 1024 particles, then
+powers of two from 16 down to 1), with particles spread over the box, in clumps, and at the
 seams of the periodic mesh, so that a bundle's particles reach tiles in one row of
 more than 32, in few and in many images.  Every cell is within DEP_TOL of the
 oracle's FP64 sums of the library's weights (below float32's normal range, of its
@@ -40,10 +40,11 @@ def particles(kind, n, nc):
 
 
 @pytest.mark.parametrize("mode", ["plain", "periodic", "density"])
-@pytest.mark.parametrize("kind,n,nc", [("spread", 6, 280), ("seams", 64, 61), ("seams", 1000, 33),
+@pytest.mark.parametrize("kind,n,nc", [("spread", 6, 280), ("seams", 64, 61), ("seams", 1000, 33), ("seams", 1024, 80), ("seams", 1025, 64),
                                        ("clumps", 8192, 40), ("seams", 8193, 40), ("spread", 16384, 50),
                                        ("seams", 16385, 50), ("spread", 32768, 40), ("seams", 32769, 41),
-                                       ("clumps", 65536, 33), ("seams", 65537, 33), ("seams", 131073, 40)])
+                                       ("clumps", 65536, 33), ("seams", 65537, 33), ("seams", 131072, 40), ("clumps", 131073, 40),
+                                       ("seams", 262145, 33)])
 def test_deposit_parts(gpu_ctx, oracle, mode, kind, n, nc):
     x, v, dens, rk, igrp = particles(kind, n, nc)
     p = api.make_particles(x, v, dens=dens, rk=rk, igrp=igrp)
