@@ -1120,7 +1120,8 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     const int n = ctx->n;
     const size_t T1 = (size_t)tiles + 1;
     if (int r = grow(ctx, ctx->dep_rec, deposit_prep_bytes(n))) return r;
-    const size_t B1 = ((size_t)n + 31) / 32 * (size_t)deposit_parts(n, periodic != 0) + 1;
+    p.log_parts = deposit_log_parts(n, periodic != 0, tiles);
+    const size_t B1 = (((size_t)n + 31) / 32 << p.log_parts) + 1;
     if (int r = grow(ctx, ctx->dep_pcount, 4 * B1 + scan_temp_bytes(B1))) return r;
     if (int r = grow(ctx, ctx->dep_tiles, deposit_tile_bytes(tiles))) return r;
     if (int r = grow(ctx, ctx->dep_counter, 32)) return r;

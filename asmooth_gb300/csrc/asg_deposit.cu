@@ -154,17 +154,18 @@ __device__ __forceinline__ void image_tiles(const AxisRange& r, int k, int nc, i
 // mesh and image the warp goes through the tiles of the union of its lanes' tile
 // boxes; where that holds many more tiles than the lanes touch (particles far
 // apart), through each lane's own tiles, one lane after another.  Either way the
-// particles of a tile come in lane order.  Of `parts` warps with the same bundle (a
-// power of two), each takes the rows of tiles whose y + z falls to it.
+// particles of a tile come in lane order.  SPLIT: of the warps with the same bundle
+// (a power of two; a template, as reading their number costs 2% of a large deposit)
+// each takes the rows of tiles whose y + z falls to it.
 // count(entries, pairs) instead of f with COUNT: the lanes' own boxes give the pairs,
 // and a row of tiles is one union of bit masks.
-template <bool PERIODIC, bool COUNT, class F>
+template <bool PERIODIC, bool SPLIT, bool COUNT, class F>
 __device__ __forceinline__ void for_entries(const DepositParams& P, const float (&lo)[3],
-                                            const float (&hi)[3], bool live, int part, int parts, int* err,
-                                            F f)
+                                            const float (&hi)[3], bool live, int part, int* err, F f)
 {
+    const int parts = SPLIT ? 1 << P.log_parts : 1;
     // the first row of tiles from y on, at z, that falls to this warp
-    auto first_row = [&](int y, int z) { return y + ((part - y - z) & (parts - 1)); };
+    auto first_row = [&](int y, int z) { return SPLIT ? y + ((part - y - z) & (parts - 1)) : y; };
     for (int jb = 0; jb < P.n_jobs; ++jb) {
         const MeshJob& J = P.job[jb];
         const int nc = J.nc;
@@ -206,18 +207,22 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
             if (!in) own = 0;
             const unsigned touched = __reduce_add_sync(FULLM, min(own, 1u << 24));
             const unsigned wx = u1[0] - u0[0] + 1, wy = u1[1] - u0[1] + 1, wz = u1[2] - u0[2] + 1;
-            if constexpr (COUNT) f(0u, part == 0 ? own : 0u);
+            if constexpr (COUNT) f(0u, !SPLIT || part == 0 ? own : 0u);
             if ((unsigned long long)(wx * wy) * wz <= 2ull * touched + 64) {
+                // of 32 tiles from x on, those that the lane touches
+                auto touches = [&](int x) {
+                    const int a = max(t0[0] - x, 0), b = min(t1[0] - x, 31);
+                    return a <= b ? (2u << (b & 31)) - (1u << (a & 31)) : 0u;
+                };
+                const unsigned first32 = COUNT ? touches(u0[0]) : 0u;
                 for (int tz = u0[2]; tz <= u1[2]; ++tz) {
                     const bool inz = t0[2] <= tz && tz <= t1[2];
                     for (int ty = first_row(u0[1], tz); ty <= u1[1]; ty += parts) {
                         const bool iny = inz && t0[1] <= ty && ty <= t1[1];
                         if constexpr (COUNT) {
-                            for (int tx = u0[0]; tx <= u1[0]; tx += 32) {
-                                const int a = max(t0[0] - tx, 0), b = min(t1[0] - tx, 31);
-                                const unsigned bits = (2u << (b & 31)) - (1u << (a & 31));
-                                f((unsigned)__popc(__reduce_or_sync(FULLM, iny && a <= b ? bits : 0u)), 0u);
-                            }
+                            f((unsigned)__popc(__reduce_or_sync(FULLM, iny ? first32 : 0u)), 0u);
+                            for (int tx = u0[0] + 32; tx <= u1[0]; tx += 32)
+                                f((unsigned)__popc(__reduce_or_sync(FULLM, iny ? touches(tx) : 0u)), 0u);
                         } else {
                             int tile = J.tile_begin + (tz * J.tiles[1] + ty) * J.tiles[0] + u0[0];
                             for (int tx = u0[0]; tx <= u1[0]; ++tx, ++tile) {
@@ -251,12 +256,12 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
             // that does not lie at opposite ends of the mesh, and a union of both is all of
             // it (262,144 particles on 383^3 cells 6.1 -> 5.0 ms, 13,840 on 95^3 485 -> 422
             // us).  All lanes together where the mesh has few tiles, as each group costs what
-            // 64 tiles do (4096 particles on 31^3 92, in groups 96), and where the bundle's
+            // 128 tiles do (4096 particles on 31^3 92, in groups 96), and where the bundle's
             // particles are far apart (more than 8 groups).
             const int first = (r[0].k_lo & 1023) | (r[1].k_lo & 1023) << 10 | (r[2].k_lo & 1023) << 20;
             const unsigned same = __match_any_sync(FULLM, on ? first : -1);
             unsigned leaders = __ballot_sync(FULLM, on && (same & lanemask_lt()) == 0u);
-            const bool together = __popc(leaders) > 8 || J.tiles[0] * J.tiles[1] * J.tiles[2] < 64 * parts;
+            const bool together = __popc(leaders) > 8 || J.tiles[0] * J.tiles[1] * J.tiles[2] < 128 * parts;
             if (together) leaders &= 0u - leaders;
             for (; leaders; leaders &= leaders - 1) {
                 const int lead = __shfl_sync(FULLM, first, __ffs(leaders) - 1);
@@ -281,20 +286,21 @@ __device__ __forceinline__ void for_entries(const DepositParams& P, const float 
 // nothing.  The cell-range edges (x' -+ h)/L and 1/h are recomputed from it
 // where they are needed (load_dep_rec), with the same rounded operations.
 // counts: the entries of each part of each bundle, then 0; *pairs += the pairs.
-template <bool PERIODIC>
+template <bool PERIODIC, bool SPLIT>
 __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restrict__ vel,
-                           const int* __restrict__ igrp, const float* __restrict__ rk, int n, int parts,
+                           const int* __restrict__ igrp, const float* __restrict__ rk, int n,
                            const __grid_constant__ DepositParams P, float4* __restrict__ rec,
                            uint32_t* __restrict__ counts, unsigned long long* __restrict__ pairs,
                            int* err)
 {
     grid_begin();
     __shared__ unsigned long long block_pairs;  // one atomic per block: 0.57 M on one word took 0.3 ms
-    const int unit = (blockIdx.x * blockDim.x + threadIdx.x) / 32, part = unit & (parts - 1);
-    const int i = unit / parts * 32 + (threadIdx.x & 31);
+    const int log_parts = SPLIT ? P.log_parts : 0;
+    const int unit = (blockIdx.x * blockDim.x + threadIdx.x) / 32, part = unit & ((1 << log_parts) - 1);
+    const int i = (unit >> log_parts) * 32 + (threadIdx.x & 31);
     const int bundles = (n + 31) / 32;
     if (threadIdx.x == 0) block_pairs = 0ull;
-    if (blockIdx.x == 0 && threadIdx.x == 0) counts[bundles * parts] = 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) counts[bundles << log_parts] = 0u;
     __syncthreads();
     bool live = i < n;
     const int ii = live ? i : n - 1;
@@ -327,14 +333,16 @@ __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restr
     }
     uint32_t cnt = 0;
     unsigned long long np = 0;  // this lane's
-    for_entries<PERIODIC, true>(P, lo, hi, live, part, parts, err, [&](unsigned entries, unsigned pairs) {
+    for_entries<PERIODIC, SPLIT, true>(P, lo, hi, live, part, err, [&](unsigned entries, unsigned pairs) {
         cnt += entries;
         np += pairs;
     });
-    if ((i & 31) == 0 && i < n) counts[unit] = cnt;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(FULLM, np, o);
-    if ((i & 31) == 0 && np) atomicAdd(&block_pairs, np);
+    const unsigned np_lo = __reduce_add_sync(FULLM, (unsigned)np & 0xffffffu);
+    const unsigned np_hi = __reduce_add_sync(FULLM, (unsigned)(np >> 24));
+    if ((i & 31) == 0 && i < n) {
+        counts[unit] = cnt;
+        if (!SPLIT || part == 0) atomicAdd(&block_pairs, ((unsigned long long)np_hi << 24) + np_lo);
+    }
     __syncthreads();
     if (threadIdx.x == 0 && block_pairs) atomicAdd(pairs, block_pairs);
 }
@@ -348,15 +356,16 @@ __global__ void k_dep_prep(const float4* __restrict__ pos, const float4* __restr
 // the same 2.0 ms.
 // entry o is written only when o < cap (the entry arrays' capacity); one beyond
 // it sets ERR_CAP instead
-template <bool PERIODIC>
-__global__ void k_entries(const float4* __restrict__ rec, int n, int parts, const __grid_constant__ DepositParams P,
+template <bool PERIODIC, bool SPLIT>
+__global__ void k_entries(const float4* __restrict__ rec, int n, const __grid_constant__ DepositParams P,
                           const uint32_t* __restrict__ offs, uint32_t* __restrict__ keys,
                           uint2* __restrict__ entry, uint32_t cap, int* err)
 {
     grid_begin();
     const int lane = threadIdx.x & 31;
     const int unit = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
-    const int i = unit / parts * 32 + lane;
+    const int log_parts = SPLIT ? P.log_parts : 0;
+    const int i = (unit >> log_parts) * 32 + lane;
     if ((i & ~31) >= n) return;
     float4 a, b, c, d;
     load_dep_rec(rec, min(i, n - 1), P.boxsize, P.rbox, a, b, c, d);
@@ -377,7 +386,7 @@ __global__ void k_entries(const float4* __restrict__ rec, int n, int parts, cons
         o += held;
         held = 0;
     };
-    for_entries<PERIODIC, false>(P, lo, hi, live, unit & (parts - 1), parts, err, [&](int tile, int image, unsigned m) {
+    for_entries<PERIODIC, SPLIT, false>(P, lo, hi, live, unit & ((1 << log_parts) - 1), err, [&](int tile, int image, unsigned m) {
         if (lane == held) {
             key = PERIODIC ? ((uint32_t)tile << IMG_BITS) | (uint32_t)image : (uint32_t)tile;
             mask = m;
@@ -1384,17 +1393,22 @@ size_t deposit_prep_bytes(int n) { return 32 * (size_t)n; }
 // A warp goes through a bundle's tiles one after another: with few bundles and wide
 // supports on a fine mesh, few warps had a long way (64 particles with supports of 120
 // cells of a 256^3 mesh 8.8 ms, a thread per particle 0.8, 32 warps per bundle 0.6).
-// As many as make 4096 warps: 13,840 particles on a mesh of 6 cells per mean
-// separation 391 us with 1, 281 with 8, of 1 cell 73 and 71; 32,768 647, 560 with 4
-// and 87, 84; above that a bundle's fixed cost (ranges, unions) is most of it.  A
-// periodic mesh has more tiles per bundle: 8192 (131,072 particles 2.71, 2.57 ms with 2
-// and 220, 216 us), and a bundle of particles far apart the most.
-int deposit_parts(int n, bool periodic)
+// As many as make 4096 warps, whose counts one scan launch takes: 13,840 particles on
+// a mesh of 6 cells per mean separation 391 us with 1, 281 with 8; 32,768 647, 577 with
+// 2.  Above that, and where the meshes hold few tiles (256 per warp), a bundle's
+// fixed cost (ranges, unions) is most of it: 32,768 on 32^3 cells 82 us with 1, 87 with
+// 8.  A periodic mesh has more tiles and images per bundle: 8192 warps (131,072
+// particles at 6 cells 2.71, 2.57 ms with 2) and 128 tiles; a bundle of particles far
+// apart goes through all images (64 on 24^3 cells 294 us with 1, 146 with 4).
+int deposit_log_parts(int n, bool periodic, long long total_tiles)
 {
     const long long bundles = ((long long)n + 31) / 32;
-    int parts = bundles <= 32 ? 32 : 1;
-    while (parts < 16 && 2 * parts * bundles <= (periodic ? 8192 : 4096)) parts *= 2;
-    return parts;
+    const bool far_apart = bundles <= 32;
+    const long long most = std::min(total_tiles / (!periodic ? 256 : far_apart ? 16 : 128),
+                                    far_apart ? 32ll : std::min(16ll, (periodic ? 8192 : 4095) / bundles));
+    int log_parts = 0;
+    while ((2ll << log_parts) <= most) ++log_parts;
+    return log_parts;
 }
 
 void deposit_tile_shape(DepositParams& p)
@@ -1479,10 +1493,11 @@ void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, 
                          int n, const DepositParams& p, DepositScratch& w, int* err,
                          cudaStream_t s)
 {
-    const int parts = deposit_parts(n, p.periodic != 0), units = (n + 31) / 32 * parts;
+    const int units = (n + 31) / 32 << p.log_parts;
     cudaMemsetAsync(w.counters, 0, 32, s);
-    auto kern = p.periodic ? k_dep_prep<true> : k_dep_prep<false>;
-    launch(kern, (units + 7) / 8, 256, 0, s, pos, vel, igrp, rk, n, parts, p, w.rec, w.count,
+    auto kern = p.periodic ? (p.log_parts ? k_dep_prep<true, true> : k_dep_prep<true, false>)
+                           : (p.log_parts ? k_dep_prep<false, true> : k_dep_prep<false, false>);
+    launch(kern, (units + 7) / 8, 256, 0, s, pos, vel, igrp, rk, n, p, w.rec, w.count,
            reinterpret_cast<unsigned long long*>(w.counters + 2), err);
     exclusive_scan_u32(w.count, (size_t)units + 1, w.scan_tmp_n, s);
     count_launches(1);
@@ -1491,9 +1506,10 @@ void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, 
 void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t entries,
                         uint32_t max_items, bool padded, DepositScratch& w, int* err, cudaStream_t s)
 {
-    const int T = total_tiles, parts = deposit_parts(n, p.periodic != 0), units = (n + 31) / 32 * parts;
-    auto kern = p.periodic ? k_entries<true> : k_entries<false>;
-    launch(kern, (units + 7) / 8, 256, 0, s, w.rec, n, parts, p, w.count, w.keys0, w.entry, entries, err);
+    const int T = total_tiles, units = (n + 31) / 32 << p.log_parts;
+    auto kern = p.periodic ? (p.log_parts ? k_entries<true, true> : k_entries<true, false>)
+                           : (p.log_parts ? k_entries<false, true> : k_entries<false, false>);
+    launch(kern, (units + 7) / 8, 256, 0, s, w.rec, n, p, w.count, w.keys0, w.entry, entries, err);
     count_launches(1);
     if (padded && entries > 0) {  // `entries` is the capacity; the count itself is the last of `count`
         launch(k_pad_entries, (entries + 255) / 256, 256, 0, s, w.keys0, w.entry, w.count + units, entries,

@@ -116,6 +116,7 @@ struct DepositParams {
     int seg;          // most pairs per work item of the persistent deposit (tuning, > 0)
     int mma;          // the deposit engine: 1 the tensor cores, 0 the CUDA cores
     int shift[3];     // log2 of the tile edges in cells (deposit_tile_shape)
+    int log_parts;    // log2 of the warps that make a bundle's entries (deposit_log_parts)
 };
 // the tile shape of the engine p.mma
 void deposit_tile_shape(DepositParams& p);
@@ -144,8 +145,8 @@ struct DepositScratch {
                           // front, number of pairs (64 bits), length of merge's back
 };
 size_t deposit_prep_bytes(int n);
-// warps that share the making of a bundle's entries (units = bundles * parts)
-int deposit_parts(int n, bool periodic);
+// log2 of the warps that share the making of a bundle's entries (units = bundles << log_parts)
+int deposit_log_parts(int n, bool periodic, long long total_tiles);
 size_t deposit_tile_bytes(int total_tiles);
 size_t deposit_entry_bytes(uint32_t entries);
 // the per-entry arrays of w inside one block of deposit_entry_bytes

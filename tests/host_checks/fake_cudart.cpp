@@ -71,10 +71,10 @@ void launched(const std::string& k, dim3 grid, dim3 block, size_t smem, void** a
         out->err = **static_cast<const int**>(a[3]);
         out->number = *static_cast<uint32_t*>(a[5]);
     } else if (is(k, "k_dep_prep")) {
-        const int n = *static_cast<int*>(a[4]), parts = *static_cast<int*>(a[5]);
-        const DepositParams& p = *static_cast<DepositParams*>(a[6]);
-        (*static_cast<uint32_t**>(a[8]))[(n + 31) / 32 * parts] = g_entries;
-        **static_cast<unsigned long long**>(a[9]) = p.shift[1] < 3 ? g_pairs_small : g_pairs_large;
+        const int n = *static_cast<int*>(a[4]);
+        const DepositParams& p = *static_cast<DepositParams*>(a[5]);
+        (*static_cast<uint32_t**>(a[7]))[(n + 31) / 32 << p.log_parts] = g_entries;
+        **static_cast<unsigned long long**>(a[8]) = p.shift[1] < 3 ? g_pairs_small : g_pairs_large;
     } else if (is(k, "k_gather")) {
         const TreeView& t = *static_cast<TreeView*>(a[8]);
         char* at = (char*)t.box;
