@@ -93,7 +93,7 @@ struct asg_ctx {
     bool dec_rk = false;    // they have smoothing lengths
     uint32_t dep_npairs = 0, dep_nentries = 0;
     int dep_tiles_n = 0, dep_cells = 0;  // tiles of the last deposit, cells of one
-    bool dep_large = false;  // its pairs needed the larger tiles
+    int dep_shape = 0;  // its tiles (Tiles)
     float mesh_boxsize = 0.0f;
     std::vector<MeshBuf> meshes;
 
@@ -1050,18 +1050,21 @@ int asg_run_remove_small_groups(asg_ctx* ctx, int ngrp, int* nhalo)
     return 0;
 }
 
-// entries and pairs that a deposit's arrays hold, and whether its pairs need the
-// larger tiles
+// Tiles that a deposit of many pairs takes in turn: the engine's own, wider ones on
+// the tensor cores, and the CUDA cores' 8^3.
+enum Tiles { TILES_OWN, TILES_WIDE, TILES_LARGE };
+
+// entries and pairs that a deposit's arrays hold, and its tiles
 struct DepositCap {
     uint32_t entries = 0, pairs = 0;
-    bool large_tiles = false;
+    int tiles = TILES_OWN;
 };
 
 // no cap: the arrays are sized from the counts (one host synchronisation); with a
 // cap: arrays of that capacity, no synchronisation (stream capture)
 static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, int sign,
                          int periodic, const int* coords, int density_only,
-                         const DepositCap* cap = nullptr, bool large_tiles = false)
+                         const DepositCap* cap = nullptr, int shape = TILES_OWN)
 {
     if (!ncs || n_nc <= 0 || n_nc > MAX_MESHES) return fail(ctx, ASG_ERR_ARG, "1..8 meshes");
     if (!(boxsize > 0.0f) || !std::isfinite(boxsize)) return fail(ctx, ASG_ERR_ARG, "boxsize");
@@ -1078,8 +1081,9 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     p.periodic = periodic ? 1 : 0;
     p.density_only = density_only ? 1 : 0;
     p.seg = ctx->dep_seg;
-    if (cap) large_tiles = cap->large_tiles;
-    p.mma = large_tiles ? 0 : ctx->dep_mma;
+    if (cap) shape = cap->tiles;
+    p.mma = shape == TILES_LARGE ? 0 : ctx->dep_mma;
+    p.wide = shape == TILES_WIDE ? 1 : 0;
     for (int d = 0; d < 3; ++d) p.offset[d] = periodic && coords ? boxsize * (float)coords[d] : 0.0f;
     // the pair keys hold tile << 5 | image in 32 bits: meshes of more tiles than
     // that allows take the engine with the larger tiles
@@ -1141,15 +1145,20 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     if (cap) {
         have = *cap;
     } else {
-        const uint32_t* pairs = reinterpret_cast<uint32_t*>(w.counters + 2);
-        if (int r = fetch(ctx, {w.count + (B1 - 1), 1}, {pairs, 2})) return r;
+        if (int r = fetch(ctx, {w.count + (B1 - 1), 1}, {w.counters + 2, 2})) return r;
         have.entries = ctx->host->word[0];
         have.pairs = ctx->host->word[1];
-        if (ctx->host->word[2] || have.pairs > (uint32_t)INT_MAX) {  // past the 32-bit pair numbers
+        const unsigned long long pairs_made = have.pairs | (unsigned long long)ctx->host->word[2] << 32;
+        const bool many = pairs_made > INT_MAX;  // past the 32-bit pair numbers
+        if (many && !p.mma) {
             phase_end(ctx);
-            if (!p.mma) return fail(ctx, ASG_ERR_ARG, "more than 2^31 - 1 (particle, tile) pairs");
-            return queue_deposit(ctx, boxsize, ncs, n_nc, sign, periodic, coords, density_only, cap,
-                                 true);  // larger tiles, fewer pairs
+            return fail(ctx, ASG_ERR_ARG, "more than 2^31 - 1 (particle, tile) pairs");
+        }
+        const bool wide = p.mma && !density_only && !p.wide && pairs_made > deposit_wide_pairs(n);
+        if (many || wide) {  // larger tiles, fewer pairs
+            phase_end(ctx);
+            return queue_deposit(ctx, boxsize, ncs, n_nc, sign, periodic, coords, density_only, nullptr,
+                                 wide ? TILES_WIDE : TILES_LARGE);
         }
     }
     if (int r = grow(ctx, ctx->dep_pairs, deposit_entry_bytes(have.entries))) return r;
@@ -1166,7 +1175,7 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     if (!cap) {
         ctx->dep_npairs = have.pairs;
         ctx->dep_nentries = have.entries;
-        ctx->dep_large = large_tiles;
+        ctx->dep_shape = shape;
     }
     ctx->dep_tiles_n = tiles;
     ctx->dep_cells = 1 << (p.shift[0] + p.shift[1] + p.shift[2]);
@@ -1721,7 +1730,7 @@ int batch_plan(asg_batch* b)
         DepositCap& cap = b->cap[(size_t)i];  // headroom for inputs that change between runs
         cap.entries = c->dep_nentries + c->dep_nentries / 16 + 4096;
         cap.pairs = c->dep_npairs + c->dep_npairs / 16 + 4096;
-        cap.large_tiles = c->dep_large;
+        cap.tiles = c->dep_shape;
         max_entries = std::max(max_entries, cap.entries);
         const uint32_t items = deposit_max_items(c->dep_tiles_n, cap.pairs, c->dep_seg);
         max_items = std::max(max_items, items);

@@ -52,9 +52,10 @@ constexpr int TC = TS * TS * TS;   // cells of such a tile
 // 256^3 step's three meshes; 4.5 with 8 x 8 x 8, 8.2 with 4 x 4 x 4).  n alone: 8
 // x 8 x 8, whose one channel takes no more registers and whose meshes are the
 // finest (on 160^3 cells for 512 k particles 13 pairs per particle, 33 with 8 x 4 x 4).
-template <int NCH>
+// WIDE: 8 x 8 x 4 for the six channels of wide supports (deposit_wide_pairs).
+template <int NCH, bool WIDE>
 struct TileShape {
-    static constexpr int X = 8, Y = NCH == 1 ? 8 : 4, Z = NCH == 1 ? 8 : 4;
+    static constexpr int X = 8, Y = NCH == 1 || WIDE ? 8 : 4, Z = NCH == 1 ? 8 : 4;
     static constexpr int CELLS = X * Y * Z;
 };
 constexpr int PW = 9;              // partial words per cell
@@ -859,17 +860,18 @@ k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositP
 // a time in packed arithmetic gained nothing: the ALU part stays.
 constexpr int MMA_FLUSH = 64;  // pairs between flushes of the fragments
 
-template <int NCH>
+template <int NCH, bool WIDE>
 struct MmaWarp {
-    // [words r, r + 1][lane]: 8 hi, 8 lo of n/halo; of c/vx; 8 of vy/vz (n alone: 16 hi, 16 lo)
-    float2 acc[NCH == 1 ? 16 : 20][32];
+    static constexpr int R = 2 * TileShape<NCH, WIDE>::Y;  // cells per lane and column block
+    // [words r, r + 1][lane]: R hi, R lo of n/halo; of c/vx; R of vy/vz (n alone: R hi, R lo)
+    float2 acc[(NCH == 1 ? 2 : 5) * R / 2][32];
     __device__ __forceinline__ float sum(int r, int lane) const  // word r
     {
         return r & 1 ? acc[r >> 1][lane].y : acc[r >> 1][lane].x;
     }
     // per pair of the chunk: wx | wy | wz | n, halo (1 or 0), dens, vx, vy, vz (n alone:
     // padding); the row lengths spread a K step's four rows over all banks
-    float w[32][NCH == 1 ? 28 : 24];
+    float w[32][NCH == 1 ? 28 : WIDE ? 40 : 24];
 };
 
 __device__ __forceinline__ uint32_t tf32_rna(float x)
@@ -942,8 +944,8 @@ __device__ __forceinline__ float tent_centre_rn(float a, float b)
     return __fadd_rn(__fmul_rn(t, __fmaf_rn(-0.5f, t, 1.0f)), __fmul_rn(s, __fmaf_rn(-0.5f, s, 1.0f)));
 }
 
-template <int NCH>
-__global__ void __launch_bounds__(32, 24)
+template <int NCH, bool WIDE>
+__global__ void __launch_bounds__(32, WIDE ? 14 : 24)
 k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositParams P, int total_tiles,
               const uint32_t* __restrict__ item_off, uint32_t max_items,
               const uint32_t* __restrict__ item_tile, const uint32_t* __restrict__ tentry,
@@ -952,13 +954,13 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
               double* __restrict__ item_tot, int* __restrict__ counters)
 {
     grid_begin();
-    constexpr int MX = TileShape<NCH>::X, MY = TileShape<NCH>::Y, MZ = TileShape<NCH>::Z;
-    constexpr int MC = TileShape<NCH>::CELLS;
+    using Shape = TileShape<NCH, WIDE>;
+    constexpr int MX = Shape::X, MY = Shape::Y, MZ = Shape::Z, MC = Shape::CELLS;
     constexpr int NB = NCH == 1 ? 1 : 3;  // column blocks: n (8 z) or n halo | c vx | vy vz (4 z each)
     constexpr int RB = MY / 2;            // row blocks: 8 x and 2 y
     constexpr int R = 4 * RB;             // cells per lane and column block
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    MmaWarp<NCH>& S = *reinterpret_cast<MmaWarp<NCH>*>(smem_raw);
+    MmaWarp<NCH, WIDE>& S = *reinterpret_cast<MmaWarp<NCH, WIDE>*>(smem_raw);
     const int lane = threadIdx.x;
     const int g = lane >> 2, t = lane & 3;
     const bool periodic = P.periodic != 0;
@@ -1089,7 +1091,7 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
                 // a halo particle counts in the halo channel only
                 if constexpr (NCH > 1)
                 {
-                    wz4[4] = halo ? make_float4(0.f, 1.f, 0.f, 0.f) : make_float4(1.f, 0.f, B.w, Cc.w);
+                    wz4[(MX + MY + MZ) / 4] = halo ? make_float4(0.f, 1.f, 0.f, 0.f) : make_float4(1.f, 0.f, B.w, Cc.w);
                     *reinterpret_cast<float2*>(wl + MX + MY + MZ + 4) =
                         halo ? make_float2(0.f, 0.f) : make_float2(D.x, D.y);
                 }
@@ -1413,8 +1415,10 @@ int deposit_log_parts(int n, bool periodic, long long total_tiles)
 
 void deposit_tile_shape(DepositParams& p)
 {
+    const bool small = p.mma && !p.density_only;
     p.shift[0] = 3;
-    p.shift[1] = p.shift[2] = p.mma && !p.density_only ? 2 : 3;
+    p.shift[1] = small && !p.wide ? 2 : 3;
+    p.shift[2] = small ? 2 : 3;
 }
 
 size_t deposit_tile_bytes(int total_tiles)
@@ -1450,6 +1454,19 @@ static int key_bits(int total_tiles, int ib)
     int b = 0;
     while ((1 << b) < total_tiles) ++b;
     return b + ib;
+}
+
+// Above this many pairs with 8 x 4 x 4 tiles, six channels go through the preparation
+// again with 8 x 8 x 4 ones: wide supports fill the tiles, and a pair's weights are
+// formed for twice the cells.
+// 262,144 particles at 6 cells per mean separation (182 pairs per particle) 3.91 ->
+// 3.79 ms, in halos 3.81 -> 3.55, periodic 5.09 -> 4.66; at 4 cells (75) 1.46 and 1.45, at
+// 2 (28) 0.39 and 0.49.  Below 8 M pairs the second preparation and the longer items of
+// fewer warps are not made up: 13,840 particles at 6 cells 0.28 and 0.36 ms, 32,768
+// 0.56 both, 65,536 1.06 both and periodic 1.50 -> 1.46.
+unsigned long long deposit_wide_pairs(int n)
+{
+    return std::max(64ull * (unsigned long long)n, 8ull << 20);
 }
 
 // the default deposit engine: 1 the tensor cores, 0 the CUDA cores
@@ -1534,14 +1551,13 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
     double* item_tot = nullptr;
     if (p.mma) {
         item_tot = deposit_item_totals(w.partial, max_items, p);
-        if (p.density_only)
-            launch_persistent(k_deposit_mma<1>, dev, sms, 32, sizeof(MmaWarp<1>), s, w.rec, p, T,
-                              w.item_off, max_items, w.item_tile, w.tentry, keys, w.list, w.first,
-                              w.partial, item_tot, w.counters);
-        else
-            launch_persistent(k_deposit_mma<6>, dev, sms, 32, sizeof(MmaWarp<6>), s, w.rec, p, T,
-                              w.item_off, max_items, w.item_tile, w.tentry, keys, w.list, w.first,
-                              w.partial, item_tot, w.counters);
+        auto run = [&](auto kern, size_t smem) {
+            launch_persistent(kern, dev, sms, 32, smem, s, w.rec, p, T, w.item_off, max_items, w.item_tile,
+                              w.tentry, keys, w.list, w.first, w.partial, item_tot, w.counters);
+        };
+        if (p.density_only) run(k_deposit_mma<1, false>, sizeof(MmaWarp<1, false>));
+        else if (p.wide) run(k_deposit_mma<6, true>, sizeof(MmaWarp<6, true>));
+        else run(k_deposit_mma<6, false>, sizeof(MmaWarp<6, false>));
     } else {
         launch_persistent(k_deposit_items, dev, sms, 32 * DEP_WARPS, DEP_WARPS * sizeof(WarpTile), s,
                           w.rec, p, T, w.item_off, max_items, w.item_tile, w.tentry, keys, w.list,

@@ -115,6 +115,7 @@ struct DepositParams {
     int density_only;
     int seg;          // most pairs per work item of the persistent deposit (tuning, > 0)
     int mma;          // the deposit engine: 1 the tensor cores, 0 the CUDA cores
+    int wide;         // tensor cores, six channels: the wider tiles
     int shift[3];     // log2 of the tile edges in cells (deposit_tile_shape)
     int log_parts;    // log2 of the warps that make a bundle's entries (deposit_log_parts)
 };
@@ -147,6 +148,8 @@ struct DepositScratch {
 size_t deposit_prep_bytes(int n);
 // log2 of the warps that share the making of a bundle's entries (units = bundles << log_parts)
 int deposit_log_parts(int n, bool periodic, long long total_tiles);
+// pairs from which on six channels take the wider tiles
+unsigned long long deposit_wide_pairs(int n);
 size_t deposit_tile_bytes(int total_tiles);
 size_t deposit_entry_bytes(uint32_t entries);
 // the per-entry arrays of w inside one block of deposit_entry_bytes

@@ -354,7 +354,8 @@ const char* asg_phase_name(int phase);
  * register-resident FMA-chain kernel over all SMs: the FP32 roofline ceiling. */
 int asg_measure_fp32_peak(asg_ctx* ctx, double* tflops);
 /* Work statistics of the last deposit: (particle, mesh tile) pairs deposited,
- * mesh tiles (8x4x4 cells; 8^3 for density-only meshes and on the CUDA cores),
+ * mesh tiles (8x4x4 cells, 8x8x4 where supports reach many of them; 8^3 for
+ * density-only meshes and on the CUDA cores),
  * work items run. */
 int asg_deposit_stats(asg_ctx* ctx, long long* pairs, long long* tiles, long long* items);
 

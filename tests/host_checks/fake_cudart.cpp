@@ -32,7 +32,7 @@ std::map<const void*, size_t> g_vars;
 std::map<const void*, void*> g_var_at;
 std::map<char*, size_t> g_blocks;
 uint32_t g_entries = 0;
-unsigned long long g_pairs_small = 0, g_pairs_large = 0;
+unsigned long long g_pairs[3] = {};
 int g_timed = 0, g_fastest = INT_MAX;
 
 void line(const std::string& s) { g_log += s + "\n"; }
@@ -74,7 +74,7 @@ void launched(const std::string& k, dim3 grid, dim3 block, size_t smem, void** a
         const int n = *static_cast<int*>(a[4]);
         const DepositParams& p = *static_cast<DepositParams*>(a[5]);
         (*static_cast<uint32_t**>(a[7]))[(n + 31) / 32 << p.log_parts] = g_entries;
-        **static_cast<unsigned long long**>(a[8]) = p.shift[1] < 3 ? g_pairs_small : g_pairs_large;
+        **static_cast<unsigned long long**>(a[8]) = g_pairs[p.shift[1] < 3 ? 0 : p.shift[2] < 3 ? 1 : 2];
     } else if (is(k, "k_gather")) {
         const TreeView& t = *static_cast<TreeView*>(a[8]);
         char* at = (char*)t.box;
@@ -107,11 +107,14 @@ extern "C" {
 
 const char* fake_log() { return g_log.c_str(); }
 void fake_clear() { g_log.clear(); }
-void fake_counts(uint32_t entries, unsigned long long pairs_small_tiles, unsigned long long pairs_large_tiles)
+// entries, and the pairs with tiles of 8 x 4 x 4, 8 x 8 x 4 and 8 x 8 x 8 cells
+void fake_counts(uint32_t entries, unsigned long long pairs844, unsigned long long pairs884,
+                 unsigned long long pairs888)
 {
     g_entries = entries;
-    g_pairs_small = pairs_small_tiles;
-    g_pairs_large = pairs_large_tiles;
+    g_pairs[0] = pairs844;
+    g_pairs[1] = pairs884;
+    g_pairs[2] = pairs888;
 }
 
 // of the times that are asked for, the n-th from now on is the shortest

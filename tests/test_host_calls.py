@@ -27,13 +27,13 @@ def fake(tmp_path_factory):
     for name, (res, args) in _lib.SIGNATURES.items():
         getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
     lib.fake_log.restype = C.c_char_p
-    lib.fake_counts.argtypes = [C.c_uint32, C.c_ulonglong, C.c_ulonglong]
+    lib.fake_counts.argtypes = [C.c_uint32] + 3 * [C.c_ulonglong]
     return lib
 
 
 @pytest.fixture(autouse=True)
 def fresh(fake):
-    fake.fake_counts(0, 0, 0)
+    fake.fake_counts(0, 0, 0, 0)
     fake.fake_fastest(10 ** 6)
     fake.fake_clear()
 
@@ -86,27 +86,28 @@ def test_tuned_leaf_sizes_fit_the_box_array(fake, monkeypatch, leaf):
     fake.asg_destroy(ctx)
 
 
-def kernels(lines, *names):
-    """(kernel, grid, block) of the launches of these kernels, in order"""
-    return [(n, int(ln[2]), int(ln[3])) for ln in lines if ln[0] == "launch"
-            for n in names if f"{len(n)}{n}" in ln[1]]
-
-
-@pytest.mark.parametrize("small,large", [(10 ** 6, 10 ** 6), (2 ** 31 - 1, 2 ** 29), (2 ** 31, 2 ** 29),
-                                         (2 ** 33, 2 ** 31 - 1)])
-def test_captured_deposit_takes_the_planned_tiles(fake, small, large):
-    """A batch item with more pairs than 32 bits number takes the larger tiles in the
-    planning pass, and so it does in the graph, whose capture allocates nothing."""
+@pytest.mark.parametrize("pairs,tiles", [
+    ((10 ** 6, 10 ** 6, 10 ** 6), "own"),
+    ((8 * 2 ** 20, 2 ** 22, 2 ** 21), "own"),  # the line of deposit_wide_pairs for few particles
+    ((8 * 2 ** 20 + 1, 2 ** 22, 2 ** 21), "wide"),
+    ((2 ** 31, 2 ** 30, 2 ** 29), "wide"),
+    ((2 ** 33, 2 ** 31 - 1, 2 ** 30), "wide"),
+    ((2 ** 33, 2 ** 31, 2 ** 31 - 1), "large")])
+def test_captured_deposit_takes_the_planned_tiles(fake, pairs, tiles):
+    """A batch item with many pairs, or with more than 32 bits number, takes larger
+    tiles in the planning pass, and so it does in the graph, whose capture allocates
+    nothing."""
     ctx = context(fake)
     b = batch(fake, ctx, [5000, 4000], ncs=(16, 32))
-    fake.fake_counts(1000, small, large)
+    fake.fake_counts(1000, *pairs)
     assert fake.asg_batch_run(b) == 0
     lines = log(fake)
     at = [ln[0] for ln in lines].index("capture")
-    plan = [k[0] for k in kernels(lines[:at], "k_deposit_mma", "k_deposit_items")]
-    graph = [k[0] for k in kernels(lines[at:], "k_deposit_mma", "k_deposit_items")]
+    want = {"own": "k_deposit_mmaILi6ELb0E", "wide": "k_deposit_mmaILi6ELb1E", "large": "k_deposit_items"}[tiles]
+    for part in (lines[:at], lines[at:]):
+        ran = [ln[1] for ln in part if ln[0] == "launch" and "k_deposit_" in ln[1]]
+        assert len(ran) == 2 and all(want in k for k in ran)
     assert not any(ln[0] == "malloc" for ln in lines[at:])
-    assert plan == graph == 2 * ["k_deposit_mma" if small < 2 ** 31 else "k_deposit_items"]
     fake.asg_batch_destroy(b)
     fake.asg_destroy(ctx)
 
@@ -139,11 +140,11 @@ def test_tuner_that_fails_leaves_the_configuration(fake, monkeypatch):
     v = [C.c_int(0) for _ in range(8)]
     assert fake.asg_batch_config(b, *[C.byref(t) for t in v[:4]]) == 0 and v[0].value == 24
     assert fake.asg_batch_run(b) == 0
-    fake.fake_counts(10, 2 ** 33, 2 ** 33)  # more pairs than either tile shape can number
+    fake.fake_counts(10, 2 ** 33, 2 ** 33, 2 ** 33)  # more pairs than any tile shape can number
     assert fake.asg_batch_tune(b, None, None) != 0
     assert fake.asg_batch_config(b, *[C.byref(t) for t in v[4:]]) == 0
     assert [t.value for t in v[4:]] == [t.value for t in v[:4]]
-    fake.fake_counts(10, 100, 100)
+    fake.fake_counts(10, 100, 100, 100)
     log(fake)
     assert fake.asg_batch_run(b) == 0
     assert ["capture"] in log(fake)
