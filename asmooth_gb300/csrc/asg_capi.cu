@@ -92,7 +92,8 @@ struct asg_ctx {
     int dec_n = 0;          // particles of the last decode (in sh_in), 0 = none
     bool dec_rk = false;    // they have smoothing lengths
     uint32_t dep_npairs = 0, dep_nentries = 0;
-    int dep_tiles_n = 0, dep_cells = 0;  // tiles of the last deposit, cells of one
+    int dep_tiles_n = 0;        // tiles of the last deposit
+    size_t dep_item_words = 0;  // and the words of an item's partial tile
     int dep_shape = 0;  // its tiles (Tiles)
     float mesh_boxsize = 0.0f;
     std::vector<MeshBuf> meshes;
@@ -1163,10 +1164,8 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
     }
     if (int r = grow(ctx, ctx->dep_pairs, deposit_entry_bytes(have.entries))) return r;
     if (int r = grow(ctx, ctx->dep_sort, radix_sort_temp_bytes((int)have.entries))) return r;
-    const uint32_t max_items = deposit_max_items(tiles, have.pairs, p.seg);
-    if (int r = grow(ctx, ctx->dep_partial,
-                     deposit_partial_bytes(max_items, 1 << (p.shift[0] + p.shift[1] + p.shift[2])) + 16))
-        return r;
+    const uint32_t max_items = deposit_max_items(tiles, have.pairs, p.seg, p.density_only != 0);
+    if (int r = grow(ctx, ctx->dep_partial, deposit_partial_bytes(max_items, deposit_item_words(p)) + 16)) return r;
     if (int r = grow(ctx, ctx->dep_items, 4 * (size_t)max_items)) return r;
     deposit_entry_layout(ctx->dep_pairs.p, have.entries, w);
     w.item_tile = P<uint32_t>(ctx->dep_items);
@@ -1178,7 +1177,7 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
         ctx->dep_shape = shape;
     }
     ctx->dep_tiles_n = tiles;
-    ctx->dep_cells = 1 << (p.shift[0] + p.shift[1] + p.shift[2]);
+    ctx->dep_item_words = deposit_item_words(p);
     launch_deposit_run(n, p, tiles, have.entries, max_items, cap != nullptr, w, ctx->d_err, ctx->s);
     launch_deposit_totals(p, tiles, P<double>(ctx->totals), ctx->s);
     phase_end(ctx);
@@ -1732,9 +1731,9 @@ int batch_plan(asg_batch* b)
         cap.pairs = c->dep_npairs + c->dep_npairs / 16 + 4096;
         cap.tiles = c->dep_shape;
         max_entries = std::max(max_entries, cap.entries);
-        const uint32_t items = deposit_max_items(c->dep_tiles_n, cap.pairs, c->dep_seg);
+        const uint32_t items = deposit_max_items(c->dep_tiles_n, cap.pairs, c->dep_seg, false);
         max_items = std::max(max_items, items);
-        max_partial = std::max(max_partial, deposit_partial_bytes(items, c->dep_cells));
+        max_partial = std::max(max_partial, deposit_partial_bytes(items, c->dep_item_words));
     }
     for (asg_ctx* c : b->sub)
         if (int r = finish(c, "batch plan")) return fail(ctx, r, c->last);

@@ -58,7 +58,8 @@ struct TileShape {
     static constexpr int X = 8, Y = NCH == 1 || WIDE ? 8 : 4, Z = NCH == 1 ? 8 : 4;
     static constexpr int CELLS = X * Y * Z;
 };
-constexpr int PW = 9;              // partial words per cell
+constexpr int PW = 9, PW_ALONE = 2;  // partial words per cell: all channels, n alone
+__host__ __device__ inline int partial_words(const DepositParams& P) { return P.density_only ? PW_ALONE : PW; }
 constexpr int IMG_BITS = 5;        // periodic images per pair: up to 3 x 3 x 3
 // key bits of the image index: none without periodic images (every pair is
 // image 0), so the pair sort needs fewer passes
@@ -797,12 +798,14 @@ k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositP
 
         // ---- write: final tile when alone, partial tile otherwise ----
         if (nseg > 1) {
-            float* pt = partial + (size_t)item * TC * PW;
+            float* pt = partial + (size_t)item * TC * partial_words(P);
             for (int e = lane; e < TC; e += 32) {
                 const int slot = tile_slot(e & (TS - 1), (e >> 3) & (TS - 1), e >> 6);
                 const float4 A = S.a[slot];
                 const float4 B = S.b[slot];
-                pt[e] = A.x; pt[TC + e] = A.y; pt[2 * TC + e] = A.z; pt[3 * TC + e] = A.w;
+                pt[e] = A.x; pt[TC + e] = A.y;
+                if (P.density_only) continue;
+                pt[2 * TC + e] = A.z; pt[3 * TC + e] = A.w;
                 pt[4 * TC + e] = B.x; pt[5 * TC + e] = B.y; pt[6 * TC + e] = B.z;
                 pt[7 * TC + e] = B.w; pt[8 * TC + e] = S.hl[slot];
             }
@@ -1186,7 +1189,7 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
         }
         const bool low = NCH == 1 || t < 2;  // the lane's channels: n, c, vy, else halo, vx, vz
         if (nseg > 1) {
-            float* pt = partial + (size_t)item * MC * PW;
+            float* pt = partial + (size_t)item * MC * (NCH == 1 ? PW_ALONE : PW);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const int y = r >> 1, z = 2 * (NCH == 1 ? t : t & 1) + (r & 1);
@@ -1289,12 +1292,13 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
     const int cells = 1 << (P.shift[0] + P.shift[1] + P.shift[2]);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const bool all = !P.density_only;
+    const int words = partial_words(P);
     const int few = counters[1], many = counters[4];
 
     // items [a0, a1) of cells [e, e + 3]
     auto sum_items = [&](int a0, int a1, int e, MergeSums& m) {
         for (int it = a0; it < a1; ++it)
-            m.add(partial + (size_t)it * cells * PW + e, (size_t)cells, all);
+            m.add(partial + (size_t)it * cells * words + e, (size_t)cells, all);
     };
     auto store = [&](const TileGeo& g, int e, const MergeSums& m, double& sn, double& sh) {
         const MeshJob& J = P.job[g.job];
@@ -1483,8 +1487,7 @@ int deposit_default_mma()
 // per-item FP64 masses after the partial tiles of deposit_max_items items
 static double* deposit_item_totals(float* partial, uint32_t items, const DepositParams& p)
 {
-    const size_t cells = (size_t)1 << (p.shift[0] + p.shift[1] + p.shift[2]);
-    const size_t off = ((size_t)items * cells * PW * sizeof(float) + 15) & ~size_t(15);
+    const size_t off = ((size_t)items * deposit_item_words(p) * sizeof(float) + 15) & ~size_t(15);
     return reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(partial) + off);
 }
 
@@ -1568,17 +1571,24 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
     count_launches(5);
 }
 
-// a partial item per tile, and as many full ones as deposit_seg leaves
-uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int most)
+// Work items that `npairs` pairs or fewer make: a partial one per tile, and as many
+// full ones as deposit_seg leaves, of 64 pairs at least.  (Room for ITEM_SHARE whatever
+// the pairs took 76 MB for the smallest deposit of six channels, 303 for n alone.)
+uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int most, bool n_alone)
 {
-    return (uint32_t)total_tiles + std::max((uint32_t)ITEM_SHARE, npairs / (uint32_t)most) + 2;
+    const uint32_t share = n_alone ? ITEM_SHARE / 2 : ITEM_SHARE;
+    return (uint32_t)total_tiles + std::max(std::min(share, npairs / 64), npairs / (uint32_t)most) + 2;
+}
+
+size_t deposit_item_words(const DepositParams& p)
+{
+    return (size_t)partial_words(p) << (p.shift[0] + p.shift[1] + p.shift[2]);
 }
 
 // partial tiles of multi-item tiles, then each item's FP64 mass (2 doubles)
-size_t deposit_partial_bytes(uint32_t items, int cells)
+size_t deposit_partial_bytes(uint32_t items, size_t item_words)
 {
-    return (((size_t)items * cells * PW * sizeof(float) + 15) & ~size_t(15)) +
-           16 * (size_t)items;
+    return (((size_t)items * item_words * sizeof(float) + 15) & ~size_t(15)) + 16 * (size_t)items;
 }
 
 // FP64 totals of every mesh from its tiles' partial sums: block (b, mesh) adds a

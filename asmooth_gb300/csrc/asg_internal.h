@@ -155,9 +155,10 @@ size_t deposit_entry_bytes(uint32_t entries);
 // the per-entry arrays of w inside one block of deposit_entry_bytes
 void deposit_entry_layout(void* base, uint32_t entries, DepositScratch& w);
 // work items that `npairs` pairs make at most, with at most `most` pairs each
-uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int most);
+uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int most, bool n_alone);
 int deposit_default_mma();
-size_t deposit_partial_bytes(uint32_t items, int cells);  // of tiles of that many cells
+size_t deposit_item_words(const DepositParams& p);  // of an item's partial tile
+size_t deposit_partial_bytes(uint32_t items, size_t item_words);
 // pass 1: particle records and entry counts; count[units] then holds the number
 // of entries, counters[2..3] the number of pairs
 void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, const float* rk,

@@ -150,3 +150,43 @@ def test_tuner_that_fails_leaves_the_configuration(fake, monkeypatch):
     assert ["capture"] in log(fake)
     fake.asg_batch_destroy(b)
     fake.asg_destroy(ctx)
+
+
+@pytest.mark.parametrize("density_only", [0, 1])
+def test_small_deposits_take_little_memory(fake, density_only):
+    """A deposit's partial tiles are sized by its pairs: a few MB for a few particles."""
+    ctx = context(fake)
+    x = np.zeros((100, 3), np.float32)
+    assert fake.asg_load_particles_device(ctx, x.ctypes.data, None, None, None, 100, 0.0, 1.0) == 0
+    fake.fake_counts(50, 1000, 500, 300)
+    log(fake)
+    nc = np.asarray([16], np.int32)
+    assert fake.asg_run_deposit(ctx, 1.0, nc.ctypes.data, 1, -1, 0, None, density_only, None) == 0
+    assert sum(int(ln[1]) for ln in log(fake) if ln[0] == "malloc") < 4 << 20
+    fake.asg_destroy(ctx)
+
+
+@pytest.mark.parametrize("n_alone", [False, True])
+def test_items_fit_the_room_for_them(fake, n_alone):
+    """deposit_max_items covers the items that k_tile_items makes of any split of the
+    pairs over the tiles, also when a plan has room for more pairs than there are."""
+    room = getattr(fake, "_ZN3asg17deposit_max_itemsEijib")
+    room.restype, room.argtypes = C.c_uint32, [C.c_int, C.c_uint32, C.c_int, C.c_bool]
+    share = 4 * 24 * 152 // (2 if n_alone else 1)
+    rng = np.random.default_rng(2)
+    for pairs in [0, 1, 63, 64, 65, 10_000, 500_000, 933_888, 933_889, 20_000_000, 2 ** 31 - 1]:
+        for most in (2048, 4096, 8192):
+            seg = min((pairs // share + 64) & ~63, most)
+            for tiles in (1, 7, 3000):
+                even = np.full(tiles, pairs // tiles)
+                even[0] += pairs - even.sum()
+                some = rng.multinomial(pairs, rng.dirichlet(np.full(tiles, 0.1)))
+                # as many tiles as there can be with one pair over a full item
+                full = np.zeros(tiles, np.int64)
+                k = min(tiles, pairs // (seg + 1))
+                full[:k] = seg + 1
+                full[0] += pairs - full.sum()
+                for c in (even, some, full):
+                    items = int(np.maximum(1, -(-c // seg)).sum())
+                    for planned in (pairs, min(pairs + pairs // 16 + 4096, 2 ** 32 - 1)):
+                        assert items <= room(tiles, planned, most, n_alone)
