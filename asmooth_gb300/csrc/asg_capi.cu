@@ -73,7 +73,7 @@ struct asg_ctx {
     int leaf = LEAF_DEFAULT;  // particles per tree leaf, of the next index build
     int tree_leaf = LEAF_DEFAULT;  // and of the loaded set's tree
     int dep_seg = 4096;  // pairs per deposit work item, at most
-    int knn_warps = 2;   // warps per block of the neighbour search (2 or 4)
+    int knn_warps = 2;   // warps per block of the neighbour search (2 or 4), leaves but 16
     int dep_mma = deposit_default_mma();  // deposit engine: tensor cores (1) or CUDA cores (0)
     int* perm = nullptr;       // sorted position -> input index
 
@@ -467,7 +467,7 @@ int asg_create(asg_ctx** out, int device)
         const int v = std::atoi(e);
         if (v >= 1 && v <= LEAF_MAX) ctx->leaf = v;
     }
-    if (const char* e = std::getenv("ASG_KNN_WARPS")) {  // tuning knob: 2 or 4 warps per block
+    if (const char* e = std::getenv("ASG_KNN_WARPS")) {  // tuning knob: 2 or 4 warps per block, leaves but 16
         const int v = std::atoi(e);
         if (v == 2 || v == 4) ctx->knn_warps = v;
     }
@@ -1964,14 +1964,16 @@ static int tune_settings(asg_batch* b, Tuning& fastest)
     for (int i = 1; i < b->n_items; ++i)
         if (b->np[(size_t)i] > b->np[(size_t)item]) item = i;
     // tree leaf size x deposit work-item length x neighbour-search warps per
-    // block x deposit engine (tensor cores or CUDA cores)
+    // block (leaves of 16 have their own) x deposit engine (tensor cores or CUDA cores)
     const int leaves[] = {16, 24, 32}, segs[] = {2048, 4096, 8192}, warps[] = {2, 4}, mmas[] = {1, 0};
+    const int own_warps = ctx->knn_warps;
     float best = INFINITY;
     for (int l : leaves) {
         ctx->leaf = l;
         if (int r = alloc_set(ctx, b->max_n)) return r;  // smaller leaves have more boxes
         for (int sg : segs)
-            for (int w : warps)
+            for (int w : warps) {
+                if (l == 16 && w != own_warps) continue;
                 for (int m : mmas) {
                     const Tuning t{l, sg, w, m};
                     set_tuning(ctx, t);
@@ -1988,6 +1990,7 @@ static int tune_settings(asg_batch* b, Tuning& fastest)
                         fastest = t;
                     }
                 }
+            }
     }
     return finish(ctx, "batch tune");
 }

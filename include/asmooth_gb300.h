@@ -314,12 +314,13 @@ int asg_batch_set_item_quantised(asg_batch* batch, int item, const int* cell, co
 int asg_batch_set_streams(asg_batch* batch, int streams);
 /* Optional autotuner: times the largest item with tree leaf sizes 16, 24, 32,
  * deposit work items of 2048, 4096, 8192 pairs, 2 or 4 warps per block of the
- * neighbour search and each deposit engine, and keeps the fastest; *leaf and
- * *seg receive the first two choices. */
+ * neighbour search (leaves of 16 particles run it in blocks of their own, of one
+ * warp, or of 2 or 4 per bundle of a small set) and each deposit engine, and keeps
+ * the fastest; *leaf and *seg receive the first two choices. */
 int asg_batch_tune(asg_batch* batch, int* leaf, int* seg);
 /* The batch's configuration (tuned or default): tree leaf size, deposit
- * work-item length, neighbour-search warps per block and the deposit engine
- * (1: tensor cores, one warp per work item; 0: CUDA cores).
+ * work-item length, neighbour-search warps per block (without effect for leaves of
+ * 16) and the deposit engine (1: tensor cores, one warp per work item; 0: CUDA cores).
  * Any pointer may be NULL. */
 int asg_batch_config(asg_batch* batch, int* leaf, int* seg, int* knn_warps, int* deposit_engine);
 int asg_batch_run(asg_batch* batch);

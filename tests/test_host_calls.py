@@ -190,3 +190,16 @@ def test_items_fit_the_room_for_them(fake, n_alone):
                     items = int(np.maximum(1, -(-c // seg)).sum())
                     for planned in (pairs, min(pairs + pairs // 16 + 4096, 2 ** 32 - 1)):
                         assert items <= room(tiles, planned, most, n_alone)
+
+
+def test_tuner_times_no_setting_twice(fake):
+    """Leaves of 16 run the search in blocks of their own, so the warps per block are
+    no setting there: 3 x 2 settings with leaves of 16, 3 x 2 x 2 with each other size,
+    two passes each."""
+    ctx = context(fake)
+    b = batch(fake, ctx, [3000])
+    assert fake.asg_batch_tune(b, None, None) == 0
+    searches = [tuple(ln[1:4]) for ln in log(fake) if ln[0] == "launch" and "k_knn_t33" in ln[1]]
+    assert len(searches) == 2 * (6 + 12 + 12)
+    fake.asg_batch_destroy(b)
+    fake.asg_destroy(ctx)
