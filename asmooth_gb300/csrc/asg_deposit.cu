@@ -1492,21 +1492,21 @@ static double* deposit_item_totals(float* partial, uint32_t items, const Deposit
 }
 
 // a persistent kernel: as many CTAs as fit on every SM at once, its dynamic
-// shared memory allowed once per device (function attributes are per device)
-template <class... KArgs, class... Args>
-static void launch_persistent(void (*kern)(KArgs...), int dev, int sms, int threads, size_t smem,
-                              cudaStream_t s, Args... args)
+// shared memory allowed once per device (function attributes are per device).  The
+// kernel is a template argument: kernels of one signature share a function's statics
+template <auto Kern, class... Args>
+static void launch_persistent(int dev, int sms, int threads, size_t smem, cudaStream_t s, Args... args)
 {
     static std::atomic<unsigned long long> attr_set{0};  // one bit per device, per kernel
     const unsigned long long bit = 1ull << (dev & 63);
     if (!(attr_set.load() & bit)) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(Kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         attr_set.fetch_or(bit);
     }
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-    launch(kern, sms * (per_sm > 0 ? per_sm : 1), threads, smem, s, args...);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, Kern, threads, smem);
+    launch(Kern, sms * (per_sm > 0 ? per_sm : 1), threads, smem, s, args...);
 }
 
 void launch_deposit_prep(const float4* pos, const float4* vel, const int* igrp, const float* rk,
@@ -1554,17 +1554,22 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
     double* item_tot = nullptr;
     if (p.mma) {
         item_tot = deposit_item_totals(w.partial, max_items, p);
-        auto run = [&](auto kern, size_t smem) {
-            launch_persistent(kern, dev, sms, 32, smem, s, w.rec, p, T, w.item_off, max_items, w.item_tile,
-                              w.tentry, keys, w.list, w.first, w.partial, item_tot, w.counters);
+        auto run = [&](auto nch, auto wide) {
+            constexpr int N = decltype(nch)::value;
+            constexpr bool W = decltype(wide)::value;
+            launch_persistent<k_deposit_mma<N, W>>(dev, sms, 32, sizeof(MmaWarp<N, W>), s, w.rec, p, T, w.item_off,
+                                                   max_items, w.item_tile, w.tentry, keys, w.list, w.first,
+                                                   w.partial, item_tot, w.counters);
         };
-        if (p.density_only) run(k_deposit_mma<1, false>, sizeof(MmaWarp<1, false>));
-        else if (p.wide) run(k_deposit_mma<6, true>, sizeof(MmaWarp<6, true>));
-        else run(k_deposit_mma<6, false>, sizeof(MmaWarp<6, false>));
+        using One = std::integral_constant<int, 1>;
+        using Six = std::integral_constant<int, 6>;
+        if (p.density_only) run(One{}, std::false_type{});
+        else if (p.wide) run(Six{}, std::true_type{});
+        else run(Six{}, std::false_type{});
     } else {
-        launch_persistent(k_deposit_items, dev, sms, 32 * DEP_WARPS, DEP_WARPS * sizeof(WarpTile), s,
-                          w.rec, p, T, w.item_off, max_items, w.item_tile, w.tentry, keys, w.list,
-                          w.first, w.partial, w.counters);
+        launch_persistent<k_deposit_items>(dev, sms, 32 * DEP_WARPS, DEP_WARPS * sizeof(WarpTile), s, w.rec, p,
+                                           T, w.item_off, max_items, w.item_tile, w.tentry, keys, w.list,
+                                           w.first, w.partial, w.counters);
     }
     launch(k_merge_tiles, 4 * sms, 32 * MERGE_WARPS, 0, s, p, T, w.item_off, w.merge, w.counters,
                                                        w.partial, item_tot);

@@ -3,6 +3,7 @@ linked against a CUDA runtime that only keeps a log (host_checks/fake_cudart.cpp
 No kernel runs, so these cover sizes, launches and call order alone."""
 import ctypes as C
 import os
+import shutil
 import subprocess
 
 import numpy as np
@@ -11,9 +12,20 @@ import pytest
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
+def bind(so):
+    from asmooth_gb300 import _lib
+
+    lib = C.CDLL(so)
+    for name, (res, args) in _lib.SIGNATURES.items():
+        getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
+    lib.fake_log.restype = C.c_char_p
+    lib.fake_counts.argtypes = [C.c_uint32] + 3 * [C.c_ulonglong]
+    lib.path = so
+    return lib
+
+
 @pytest.fixture(scope="module")
 def fake(tmp_path_factory):
-    from asmooth_gb300 import _lib
     from asmooth_gb300 import build as B
 
     objs = [os.path.join(B.CSRC, "_build", u + ".o") for u in B.UNITS]
@@ -23,12 +35,13 @@ def fake(tmp_path_factory):
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", B.CSRC, "-I",
                     os.path.join(cuda, "include"), os.path.join(HERE, "host_checks", "fake_cudart.cpp"),
                     *objs, "-o", so, "-lpthread"], check=True, capture_output=True)
-    lib = C.CDLL(so)
-    for name, (res, args) in _lib.SIGNATURES.items():
-        getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
-    lib.fake_log.restype = C.c_char_p
-    lib.fake_counts.argtypes = [C.c_uint32] + 3 * [C.c_ulonglong]
-    return lib
+    return bind(so)
+
+
+@pytest.fixture
+def fresh_fake(fake, tmp_path):
+    """the library as in a process that has made no call yet"""
+    return bind(shutil.copy(fake.path, str(tmp_path / "libasg_fresh.so")))
 
 
 @pytest.fixture(autouse=True)
@@ -203,3 +216,23 @@ def test_tuner_times_no_setting_twice(fake):
     assert len(searches) == 2 * (6 + 12 + 12)
     fake.asg_batch_destroy(b)
     fake.asg_destroy(ctx)
+
+
+def test_every_persistent_kernel_gets_its_attributes(fresh_fake):
+    """The deposit kernels share a signature; each has its shared memory and carve-out
+    set before its first launch."""
+    ctx = context(fresh_fake)
+    x = np.zeros((100, 3), np.float32)
+    assert fresh_fake.asg_load_particles_device(ctx, x.ctypes.data, None, None, None, 100, 0.0, 1.0) == 0
+    nc = np.asarray([16], np.int32)
+    for density_only, pairs in ((0, 1000), (1, 1000), (0, 2 ** 30), (0, 2 ** 33)):
+        fresh_fake.fake_counts(50, pairs, pairs, pairs // 8)
+        assert fresh_fake.asg_run_deposit(ctx, 1.0, nc.ctypes.data, 1, -1, 0, None, density_only, None) == 0
+    lines = log(fresh_fake)
+    kernels = {ln[1] for ln in lines if ln[0] == "launch" and "k_deposit_" in ln[1]}
+    assert len(kernels) == 4
+    smem, carveout = "8", "9"  # cudaFuncAttribute
+    for k in kernels:
+        first = next(i for i, ln in enumerate(lines) if ln[:2] == ["launch", k])
+        assert {ln[2] for ln in lines[:first] if ln[:2] == ["attr", k]} == {smem, carveout}
+    fresh_fake.asg_destroy(ctx)
