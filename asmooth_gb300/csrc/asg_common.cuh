@@ -57,6 +57,15 @@ inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem
     cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
+// loads a kernel on the current device now: with lazy loading its first launch would,
+// and may take device memory for it
+template <class... Params>
+inline bool kernel_loaded(void (*kernel)(Params...))
+{
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, kernel) == cudaSuccess;
+}
+
 // ---- exact float helpers (reference expression order) ----------------------
 
 // norm2 (nbr_search.cpp:20-25): ((dx*dx + dy*dy) + dz*dz), no contraction

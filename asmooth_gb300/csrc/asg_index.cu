@@ -764,9 +764,9 @@ k_rs_cluster(const K* __restrict__ kin, const int* __restrict__ vin, K* __restri
     }
 }
 
-// false: the device cannot run such a cluster
+// sets the kernel up on the current device, once; false: it cannot run such a cluster
 template <class K, int R, int CTAS>
-static bool rs_cluster_t(const K* kin, const int* vin, K* kout, int* vout, int n, int passes, cudaStream_t s)
+static bool rs_cluster_ready()
 {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -776,7 +776,6 @@ static bool rs_cluster_t(const K* kin, const int* vin, K* kout, int* vout, int n
     cfg.gridDim = dim3(CTAS);
     cfg.blockDim = dim3(RSC_THREADS);
     cfg.dynamicSmemBytes = sizeof(RsCluster<K, R>);
-    cfg.stream = s;
     if (!(checked.load() & bit)) {
         auto* f = k_rs_cluster<K, R, CTAS>;
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
@@ -793,8 +792,14 @@ static bool rs_cluster_t(const K* kin, const int* vin, K* kout, int* vout, int n
         if (ok) possible.fetch_or(bit);
         checked.fetch_or(bit);
     }
-    if (!(possible.load() & bit)) return false;
-    launch(k_rs_cluster<K, R, CTAS>, CTAS, RSC_THREADS, cfg.dynamicSmemBytes, s, kin, vin, kout, vout, n, passes);
+    return (possible.load() & bit) != 0;
+}
+
+template <class K, int R, int CTAS>
+static bool rs_cluster_t(const K* kin, const int* vin, K* kout, int* vout, int n, int passes, cudaStream_t s)
+{
+    if (!rs_cluster_ready<K, R, CTAS>()) return false;
+    launch(k_rs_cluster<K, R, CTAS>, CTAS, RSC_THREADS, sizeof(RsCluster<K, R>), s, kin, vin, kout, vout, n, passes);
     count_launches(1);
     return true;
 }
@@ -822,6 +827,17 @@ size_t radix_sort_temp_bytes(int n)
     return 4 * (RS_HEAD + RS_HIST) + states + 256;
 }
 
+// allows k_rs_pass its shared memory on the current device, once
+template <class K, int BITS, class S>
+static void rs_pass_ready(int dev)
+{
+    static std::atomic<unsigned long long> attr_set{0};  // one bit per device
+    if (attr_set.load() & (1ull << (dev & 63))) return;
+    cudaFuncSetAttribute(k_rs_pass<K, BITS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(RsSmem<K, BITS>));
+    attr_set.fetch_or(1ull << (dev & 63));
+}
+
 template <class K, int BITS, class S>
 static int radix_sort_t(K* keys0, int* vals0, K* keys1, int* vals1, int n, int passes, bool iota,
                         void* temp, int* err, cudaStream_t s)
@@ -831,12 +847,7 @@ static int radix_sort_t(K* keys0, int* vals0, K* keys1, int* vals1, int n, int p
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    static std::atomic<unsigned long long> attr_set{0};  // one bit per device
-    if (!(attr_set.load() & (1ull << (dev & 63)))) {
-        cudaFuncSetAttribute(k_rs_pass<K, BITS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(RsSmem<K, BITS>));
-        attr_set.fetch_or(1ull << (dev & 63));
-    }
+    rs_pass_ready<K, BITS, S>(dev);
     uint32_t* head = static_cast<uint32_t*>(temp);
     S* state = reinterpret_cast<S*>(head + RS_HEAD + RS_HIST);
     const size_t per_pass = (size_t)ntiles * BINS;
@@ -1145,6 +1156,25 @@ void launch_scatter_fields(const int* perm, const float* rk, const float4* vel, 
     if (rk_out) run(rk_out, nullptr, nullptr);
     if (dens_out) run(nullptr, dens_out, nullptr);
     if (igrp_out) run(nullptr, nullptr, igrp_out);
+}
+
+// every kernel that a device array of up to RSC_MAX particles goes through from the
+// load to the outputs, but the search
+bool load_small_set_kernels()
+{
+    bool ok = kernel_loaded(k_unpack_soa) && kernel_loaded(k_gather<true>) && kernel_loaded(k_up_boxes) &&
+              kernel_loaded(k_scatter_fields);
+    const bool clusters[] = {rs_cluster_ready<uint64_t, 1, 8>(), rs_cluster_ready<uint64_t, 1, 16>(),
+                             rs_cluster_ready<uint64_t, 2, 16>()};
+    ok = ok && kernel_loaded(k_rs_cluster<uint64_t, 1, 8>) && kernel_loaded(k_rs_cluster<uint64_t, 1, 16>) &&
+         kernel_loaded(k_rs_cluster<uint64_t, 2, 16>);
+    if (!(clusters[0] && clusters[1] && clusters[2])) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        ok = ok && kernel_loaded(k_rs_hist<uint64_t>) && kernel_loaded(k_rs_pass<uint64_t, 8, uint32_t>);
+        rs_pass_ready<uint64_t, 8, uint32_t>(dev);
+    }
+    return ok;
 }
 
 }  // namespace asg

@@ -239,4 +239,10 @@ void launch_pack_staged(const float4* rec, const float* rk, int n, void* aos, cu
 void launch_scatter_fields(const int* perm, const float* rk, const float4* vel, const int* igrp,
                            int n, float* rk_out, float* dens_out, int* igrp_out, cudaStream_t s);
 
+// ---- loading ahead (the allocation-free search) ----------------------------------------
+// load the kernels that such a call can launch, whatever its particle count; false: a
+// CUDA error
+bool load_small_set_kernels();
+bool load_search_kernels();
+
 }  // namespace asg

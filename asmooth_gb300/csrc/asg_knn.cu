@@ -778,4 +778,13 @@ void launch_dens(const float4* pos, const TreeView& t, const float* t33, const i
     count_launches(2);
 }
 
+// every kernel of the search and density with leaves of 16 particles
+bool load_search_kernels()
+{
+    return kernel_loaded(k_knn_t33<4, true, 4>) && kernel_loaded(k_knn_t33<2, true, 2>) &&
+           kernel_loaded(k_knn_t33<1, true, 1>) && kernel_loaded(k_knn_ties) &&
+           kernel_loaded(k_dens_scatter<true, true>) && kernel_loaded(k_dens_scatter<true, false>) &&
+           kernel_loaded(k_dens_finish);
+}
+
 }  // namespace asg

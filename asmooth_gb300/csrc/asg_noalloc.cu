@@ -11,20 +11,21 @@
 // device buffers for the inputs and outputs.
 //
 // Costs and limits of the fixed scratch:
-//   * the array (NOALLOC_BYTES, about 10 MB) takes device memory on a GPU
+//   * the array (NOALLOC_BYTES, about 5 MB) takes device memory on a GPU
 //     from the moment the library's module is loaded there until the process
 //     exits.  With CUDA's lazy module loading (the default) that is the first
 //     call into this file on that device, not the dlopen of the library, so a
 //     caller that reserves its memory pool up front makes a preparing call
-//     (np = 0 and null pointers) on each device before the reservation;
+//     (np = 0 and null pointers) on each device before the reservation.  That call
+//     also loads the kernels of every particle count, which differ;
 //   * at most NOALLOC_MAX_N particles per call; larger inputs are rejected
 //     with ASG_ERR_NOALLOC_LIMIT;
 //   * every call on a device uses the same array and leaves the last call's
 //     contents in it, so calls that overlap on the GPU (other streams, other
 //     host threads) race and must be serialised by the caller;
 //   * the first call on each device (the preparing call, or the first search)
-//     looks up the array's device address (cudaGetSymbolAddress) and keeps it
-//     for later calls; make that first call before any stream capture.  After a
+//     looks up the array's device address (cudaGetSymbolAddress), keeps it for
+//     later calls and loads the kernels; make that first call before any stream capture.  After a
 //     cudaDeviceReset the kept address is stale: a preparing call looks it up
 //     again;
 //   * the call is synchronous: it returns when its work on the stream is done.
@@ -78,9 +79,9 @@ static NoallocLayout noalloc_layout(size_t n)
 }
 
 // About 142 bytes per particle in the arrays above plus the radix sort's scratch
-// (radix_sort_temp_bytes) and 256-byte alignment of every array: 304 bytes per
+// (radix_sort_temp_bytes) and 256-byte alignment of every array: 145 bytes per
 // particle and 64 KB cover them (the call checks the total)
-constexpr size_t NOALLOC_BYTES = 304u * (size_t)NOALLOC_MAX_N + 64u * 1024u;
+constexpr size_t NOALLOC_BYTES = 145u * (size_t)NOALLOC_MAX_N + 64u * 1024u;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
@@ -88,7 +89,7 @@ static void* g_scratch_ptr[NOALLOC_MAX_DEVICES];
 static std::mutex g_scratch_mu;
 
 // device address of the scratch on the current device, looked up once per
-// device (again when refresh is set: the preparing call)
+// device (again when refresh is set: the preparing call), when the kernels are loaded, too
 static int scratch_address(int dev, void** out, bool refresh)
 {
     if (dev < 0 || dev >= NOALLOC_MAX_DEVICES) return ASG_ERR_ARG;
@@ -96,7 +97,7 @@ static int scratch_address(int dev, void** out, bool refresh)
     if (!g_scratch_ptr[dev] || refresh) {
         void* p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-        if (e != cudaSuccess || !p) {
+        if (e != cudaSuccess || !p || !load_small_set_kernels() || !load_search_kernels()) {
             cudaGetLastError();
             return ASG_ERR_CUDA;
         }

@@ -367,7 +367,7 @@ int asg_deposit_stats(asg_ctx* ctx, long long* pairs, long long* tiles, long lon
  * Same results as asg_neighbor_search (rk = sqrtf of the 33rd neighbour d2,
  * tent weights added to dens), but inputs and outputs are the caller's device
  * arrays: d_x (np*3 floats), d_rk (np floats, written), d_dens (np floats,
- * added to).  The scratch is a fixed array inside the library (about 10 MB),
+ * added to).  The scratch is a fixed array inside the library (about 5 MB),
  * so the call makes no cudaMalloc/cudaFree.  Limits: 33 <= np <=
  * ASG_NOALLOC_MAX_PARTICLES (larger inputs return ASG_ERR_NOALLOC_LIMIT).
  * All calls on one device share that scratch: calls that overlap on the GPU
@@ -376,7 +376,8 @@ int asg_deposit_stats(asg_ctx* ctx, long long* pairs, long long* tiles, long lon
  * module on the current device, which is when the scratch takes its device
  * memory (with CUDA's default lazy loading that is the first call on the
  * device, not the loading of the library), looks up the scratch's device
- * address and returns ASG_OK.  Make it on each device before reserving the
+ * address, loads the kernels that a search of any np can launch (their first
+ * launch would, and may take device memory) and returns ASG_OK.  Make it on each device before reserving the
  * memory pool, and again after a cudaDeviceReset (the address kept from before
  * is stale then).  Without it the first search on a device does the same
  * set-up.

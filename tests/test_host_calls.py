@@ -236,3 +236,21 @@ def test_every_persistent_kernel_gets_its_attributes(fresh_fake):
         first = next(i for i, ln in enumerate(lines) if ln[:2] == ["launch", k])
         assert {ln[2] for ln in lines[:first] if ln[:2] == ["attr", k]} == {smem, carveout}
     fresh_fake.asg_destroy(ctx)
+
+
+def test_preparing_call_loads_what_a_search_launches(fresh_fake):
+    """asg_neighbor_search_noalloc: the preparing call loads the kernels of every
+    particle count (a first load later may take device memory), allocates nothing, and
+    the fixed scratch holds every count."""
+    fake = fresh_fake
+    assert fake.asg_neighbor_search_noalloc(None, 0, 0.0, 0.0, None, None, None) == 0
+    loaded = {ln[1] for ln in log(fake) if ln[0] == "load"}
+    a = np.zeros(3 * 32768, np.float32)
+    p = C.c_void_p(a.ctypes.data)
+    edges = [33, 64, 1024, 4099, 4864, 4865, 8192, 8193, 16384, 16385, 20000, 24320, 24321, 32767, 32768]
+    for n in edges + list(range(33, 32768, 487)):
+        assert fake.asg_neighbor_search_noalloc(p, n, 0.0, 1.0, p, p, None) == 0
+    lines = log(fake)
+    launched = {ln[1] for ln in lines if ln[0] == "launch"}
+    assert len(launched) > 10 and launched <= loaded
+    assert not any(ln[0] == "malloc" for ln in lines)
