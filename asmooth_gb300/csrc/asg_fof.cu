@@ -84,6 +84,7 @@ k_fof_link(const float4* __restrict__ pos, const __grid_constant__ TreeView t, f
             const long long last = (((long long)id + 1) << (5 * level)) * t.leaf - 1;
             return last > base && boxes_dist2_fast(box, c) <= bound;
         },
+        [](const TreeBox&) { return true; },  // a test of each query gains less than it costs here
         [&](int id) {
             const int first = id * t.leaf, cnt = leaf_count(t, id);
             if (!__any_sync(FM, active && first + cnt - 1 > q &&
@@ -259,7 +260,7 @@ k_mark_halos(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
         const int per = t.leaf <= 16 ? 2 : 1, width = 32 / per;
         int turn = 0;
         if (inside)
-            tree_walk_groups(t, pass, [&](int g) {
+            tree_walk_groups(t, pass, [](const TreeBox&) { return true; }, [&](int g) {
                 if (turn++ % split != share) return true;
                 const unsigned m = group_leaves(t, g, pass);
                 // a warp's load covers `per` leaves; four loads in flight

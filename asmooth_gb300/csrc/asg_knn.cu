@@ -181,7 +181,10 @@ __device__ __forceinline__ void knn_scan(unsigned warp_base, f32x2 qx, f32x2 qy,
 // bundle's box, as an integer key with the lane in its low bits, so one warp
 // minimum gives the nearest child left, and a node is done when that one lies
 // beyond the largest radius of the bundle.  Keys of the levels above wait in
-// shared memory.  A leaf is scanned if some lane's own radius reaches its box.
+// shared memory.  A node is opened and a leaf scanned if some lane's own radius reaches
+// its box: at the edge of a clump a bundle's box holds all of it, and without the test
+// at the nodes its warp looked at every leaf (3 M particles in one Gaussian clump 14.0
+// -> 1.9 ms, 16.8 M in NFW halos 10.0 -> 9.5).
 // LEAF16: leaves of 16 particles (the default), one chunk each.
 //
 // SPLIT > 1 (few bundles): the block's SPLIT warps search for the same bundle, each
@@ -336,7 +339,11 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
             for (;;) {
                 const unsigned m = __reduce_min_sync(FULL, k);
                 if (m > bound) break;
-                S.keys[L - 1][lane] = k == m ? ~0u : k;
+                k = k == m ? ~0u : k;
+                if (!__any_sync(FULL, point_box_fast(qx, qy, qz, tree_box(t, L, id * 32 + (int)(m & 31u))) <=
+                                          prune_bound(SPLIT > 1 ? limit : a[K_NN - 1])))
+                    continue;
+                S.keys[L - 1][lane] = k;
                 id = id * 32 + (int)(m & 31u);
                 --L;
                 const int c = id * 32 + lane;
@@ -532,6 +539,7 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
         }
         tree_walk(t,
             [&](const TreeBox& c, int, int) { return boxes_dist2_fast(box, c) <= reach; },
+            [&](const TreeBox& c) { return __any_sync(FULL, open && point_box_fast(xq, c) <= bound) != 0; },
             [&](int id) {
                 if (!__any_sync(FULL, open && point_box_fast(xq, tree_box(t, 0, id)) <= bound))
                     return true;
@@ -699,6 +707,8 @@ k_dens_scatter(const float4* __restrict__ pos, const __grid_constant__ TreeView 
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) reach = fmaxf(reach, __shfl_xor_sync(FULL, reach, o));
     tree_walk(t, [&](const TreeBox& c, int, int) { return boxes_dist2_fast(box, c) <= reach; },
+              // (70,000 particles in one Gaussian clump 573 -> 137 us)
+              [&](const TreeBox& c) { return __any_sync(FULL, point_box_fast(xq, c) <= bound) != 0; },
               [&](int id) {
                   if (id % parts == part) visit(id);
                   return true;

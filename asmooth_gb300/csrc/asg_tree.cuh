@@ -82,11 +82,12 @@ __device__ __forceinline__ int leaf_count(const TreeView& t, int id)
 }
 
 // Visits, in a fixed order, every group of 32 leaves (32 g ... 32 g + 31) all of whose
-// ancestors pass: pass(box, level, id) is asked by each lane for its own child,
-// group(g) is called by the whole warp (and may end the walk by returning false).
+// ancestors pass: pass(box, level, id) is asked by each lane for its own child, then
+// reach(box) by the whole warp for a child that passed, group(g) is called by the whole
+// warp (and may end the walk by returning false).
 // Lane l keeps the pending children of the node open at level l.
-template <class Pass, class Group>
-__device__ __forceinline__ void tree_walk_groups(const TreeView& t, Pass pass, Group group)
+template <class Pass, class Reach, class Group>
+__device__ __forceinline__ void tree_walk_groups(const TreeView& t, Pass pass, Reach reach, Group group)
 {
     constexpr unsigned ALL = 0xffffffffu;
     const int lane = threadIdx.x & 31, top = t.nlev - 1;
@@ -114,6 +115,7 @@ __device__ __forceinline__ void tree_walk_groups(const TreeView& t, Pass pass, G
         }
         if (lane == L) pending = m & (m - 1);
         const int id = g * 32 + __ffs(m) - 1;
+        if (!reach(tree_box(t, L, id))) continue;
         if (L == 1) {
             if (!group(id)) return;
         } else {
@@ -134,12 +136,12 @@ __device__ __forceinline__ unsigned group_leaves(const TreeView& t, int g, Pass 
     return __ballot_sync(0xffffffffu, ok);
 }
 
-// Visits, in a fixed order, every leaf all of whose ancestors pass; leaf(id) is
-// called by the whole warp and may end the walk by returning false.
-template <class Pass, class Leaf>
-__device__ __forceinline__ void tree_walk(const TreeView& t, Pass pass, Leaf leaf)
+// Visits, in a fixed order, every leaf all of whose ancestors pass and are reached;
+// leaf(id) is called by the whole warp and may end the walk by returning false.
+template <class Pass, class Reach, class Leaf>
+__device__ __forceinline__ void tree_walk(const TreeView& t, Pass pass, Reach reach, Leaf leaf)
 {
-    tree_walk_groups(t, pass, [&](int g) {
+    tree_walk_groups(t, pass, reach, [&](int g) {
         for (unsigned m = group_leaves(t, g, pass); m; m &= m - 1)
             if (!leaf(g * 32 + __ffs(m) - 1)) return false;
         return true;
