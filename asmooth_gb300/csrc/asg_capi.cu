@@ -150,7 +150,6 @@ T* P(Buf& b) { return reinterpret_cast<T*>(b.p); }
 int device_status(int bits)
 {
     if (bits & ERR_NONFINITE) return ASG_ERR_NONFINITE;
-    if (bits & ERR_STACK) return ASG_ERR_STACK;
     if (bits & ERR_FEW) return ASG_ERR_FEW;
     if (bits & ERR_ZERO_RK) return ASG_ERR_ZERO_RK;
     if (bits & ERR_TIES) return ASG_ERR_TIES;
@@ -1007,8 +1006,8 @@ int asg_run_fof(asg_ctx* ctx, float ll, int* ngroup)
     launch_fof_finish(P<float4>(ctx->pos), n, P<int>(ctx->uf), P<int>(ctx->minin), P<int>(ctx->mark),
                       ctx->s);
     exclusive_scan_u32(P<uint32_t>(ctx->mark), (size_t)n + 1, ctx->scan_tmp.p, ctx->s);
-    launch_fof_label(P<float4>(ctx->pos), n, P<int>(ctx->uf), P<int>(ctx->minin),
-                     P<uint32_t>(ctx->mark), P<int>(ctx->igrp), ctx->s);
+    launch_fof_label(n, P<int>(ctx->uf), P<int>(ctx->minin), P<uint32_t>(ctx->mark), P<int>(ctx->igrp),
+                     ctx->s);
     phase_end(ctx);
     if (int r = finish(ctx, "fof", {P<uint32_t>(ctx->mark) + n, 1})) return r;
     *ngroup = (int)ctx->host->word[0];

@@ -18,7 +18,6 @@ constexpr int LEAF_DEFAULT = 16;
 constexpr int TIE_MAX = 16;     // exact d2 ties kept per pass of k_knn_ties at the 33rd neighbour
 
 // device error bits (ctx->d_err)
-constexpr int ERR_STACK = 1;       // a traversal ran out of its storage (no kernel sets it: the tree's depth is fixed)
 constexpr int ERR_FEW = 2;         // a query found fewer than 33 particles
 constexpr int ERR_ZERO_RK = 4;     // 33rd distance is zero (>= 33 coincident particles)
 constexpr int ERR_TIES = 8;        // tie selection ran out of passes (not reached for k = 33)

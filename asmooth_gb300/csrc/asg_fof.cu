@@ -168,10 +168,9 @@ __global__ void k_fof_label(int n, const int* __restrict__ P, const int* __restr
     igrp[i] = (int)scan[minin[P[i]]] + 1;
 }
 
-void launch_fof_label(const float4* pos, int n, const int* parent, const int* minin,
-                      const uint32_t* scan, int* igrp_sorted, cudaStream_t s)
+void launch_fof_label(int n, const int* parent, const int* minin, const uint32_t* scan,
+                      int* igrp_sorted, cudaStream_t s)
 {
-    (void)pos;
     if (n <= 0) return;
     launch(k_fof_label, (n + 255) / 256, 256, 0, s, n, parent, minin, scan, igrp_sorted);
     count_launches(1);

@@ -181,8 +181,8 @@ void launch_fof_link(const float4* pos, const TreeView& t, float ll, int* parent
                      cudaStream_t s);
 void launch_fof_finish(const float4* pos, int n, int* parent, int* minin, int* mark,
                        cudaStream_t s);
-void launch_fof_label(const float4* pos, int n, const int* parent, const int* minin,
-                      const uint32_t* scan, int* igrp_sorted, cudaStream_t s);
+void launch_fof_label(int n, const int* parent, const int* minin, const uint32_t* scan,
+                      int* igrp_sorted, cudaStream_t s);
 void launch_mark_halos(const float4* pos, const TreeView& t, const float* halos, int nh,
                        float left, float right, int* igrp, long long* counts, double* mass8,
                        cudaStream_t s);

@@ -110,7 +110,6 @@ static int scratch_address(int dev, void** out, bool refresh)
 static int noalloc_status(int bits)
 {
     if (bits & ERR_NONFINITE) return ASG_ERR_NONFINITE;
-    if (bits & ERR_STACK) return ASG_ERR_STACK;
     if (bits & ERR_FEW) return ASG_ERR_FEW;
     if (bits & ERR_ZERO_RK) return ASG_ERR_ZERO_RK;
     if (bits & ERR_TIES) return ASG_ERR_TIES;

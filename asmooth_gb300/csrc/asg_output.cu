@@ -287,7 +287,3 @@ extern "C" int asg_write_mesh(const char* filename, const float* mesh, int nc, f
     ok = (std::fclose(fp) == 0) && ok;
     return ok ? ASG_OK : ASG_ERR_IO;
 }
-
-namespace asg {
-
-}  // namespace asg

@@ -48,7 +48,7 @@ enum {
     ASG_ERR_FEW = -4,         /* fewer than 33 particles can be reached by a query */
     ASG_ERR_ZERO_RK = -5,     /* 33rd neighbour distance is 0 (>= 33 coincident particles) */
     ASG_ERR_NONFINITE = -6,   /* NaN or infinite position */
-    ASG_ERR_STACK = -7,       /* tree deeper than the traversal stack */
+    ASG_ERR_STACK = -7,       /* no longer returned: the tree's depth is fixed */
     ASG_ERR_TIES = -8,        /* more than 16 particles tied exactly at the 33rd distance */
     ASG_ERR_RANGE = -9,       /* periodic deposit: kernel support wider than the mesh */
     ASG_ERR_STATE = -10,      /* call needs a previous step (e.g. deposit before search) */
@@ -343,7 +343,8 @@ long long asg_kernel_launches(asg_ctx* ctx);
  * and zeroes the accumulators; asg_phase_ms fills ms[0..ASG_NPHASES-1] with the
  * device time accumulated per phase since then. */
 #define ASG_NPHASES 10
-/* UPLOAD: the host-to-device copy of an end-to-end call's inputs; OUTPUT: from
+/* CHECK: no longer timed (the kernels check the smoothing lengths as they go).
+ * UPLOAD: the host-to-device copy of an end-to-end call's inputs; OUTPUT: from
  * the end of its last deposit until its copies to the host are done. */
 enum { ASG_PH_INDEX = 0, ASG_PH_KNN = 1, ASG_PH_TIES = 2, ASG_PH_CHECK = 3, ASG_PH_DENS = 4,
        ASG_PH_DEPOSIT = 5, ASG_PH_HALOS = 6, ASG_PH_FOF = 7, ASG_PH_UPLOAD = 8,
