@@ -1117,10 +1117,14 @@ void launch_pack_staged(const float4* rec, const float* rk, int n, void* aos, cu
 // in slices of that size (the particles of input positions [first, first + count)), so
 // that the L2 takes all stores to a sector before it goes to memory: rk and dens of
 // 18.3 M particles 728 -> 314 us (80 and 96 MB; 60 MB, two slices each, 425; both
-// fields in two slices 392).  A slice reads all its input again, so from more than
-// SCATTER_SLICES on there is one.
-constexpr long long SCATTER_L2 = 80LL << 20;
+// fields in two slices 392), of 60 M, three slices each, 6.8 -> 3.1 ms.  A slice reads
+// all its input again, so from more than SCATTER_SLICES on there is one.
+// STREAM: loads that leave the L2 to the stores, from SCATTER_STREAM of fields on (rk
+// and dens of 10 M particles 149 -> 136 us, all three 259 -> 198; rk of 5 M 34 and 39).  Without
+// slices nothing waits for perm but the stores (rk of 18 M 131 -> 110 us).
+constexpr long long SCATTER_L2 = 80LL << 20, SCATTER_STREAM = 40LL << 20;
 constexpr int SCATTER_SLICES = 5;
+template <bool SLICED, bool STREAM>
 __global__ void k_scatter_fields(const int* __restrict__ perm, const float* __restrict__ rk,
                                  const float4* __restrict__ vel, const int* __restrict__ igrp,
                                  int n, int first, int count, float* rk_out, float* dens_out, int* igrp_out)
@@ -1128,34 +1132,37 @@ __global__ void k_scatter_fields(const int* __restrict__ perm, const float* __re
     grid_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int o = __ldcs(perm + i);
-    if ((unsigned)(o - first) >= (unsigned)count) return;
-    if (rk_out) rk_out[o] = __ldcs(rk + i);
+    auto load = [](auto* p) { return STREAM ? __ldcs(p) : *p; };
+    const int o = load(perm + i);
+    if (SLICED && (unsigned)(o - first) >= (unsigned)count) return;
+    if (rk_out) rk_out[o] = load(rk + i);
     if (dens_out) dens_out[o] = __ldcs(&vel[i].w);
-    if (igrp_out) igrp_out[o] = __ldcs(igrp + i);
+    if (igrp_out) igrp_out[o] = load(igrp + i);
 }
 
 void launch_scatter_fields(const int* perm, const float* rk, const float4* vel, const int* igrp,
                            int n, float* rk_out, float* dens_out, int* igrp_out, cudaStream_t s)
 {
     if (n <= 0) return;
-    auto run = [&](float* r, float* d, int* g) {
-        const int fields = (r != nullptr) + (d != nullptr) + (g != nullptr);
-        int slices = (int)((4LL * n * fields - 1) / SCATTER_L2) + 1;
-        if (slices > SCATTER_SLICES) slices = 1;
+    const int fields = (rk_out != nullptr) + (dens_out != nullptr) + (igrp_out != nullptr);
+    const long long bytes = 4LL * n, all = bytes * fields;
+    auto run = [&](int slices, float* r, float* d, int* g) {
         const int count = (n + slices - 1) / slices;
+        auto kern = slices > 1 ? k_scatter_fields<true, true>
+                               : all > SCATTER_STREAM ? k_scatter_fields<false, true> : k_scatter_fields<false, false>;
         for (int k = 0; k < slices; ++k)
-            launch(k_scatter_fields, (n + 255) / 256, 256, 0, s, perm, rk, vel, igrp, n, k * count, count, r, d, g);
+            launch(kern, (n + 255) / 256, 256, 0, s, perm, rk, vel, igrp, n, k * count, count, r, d, g);
         count_launches(slices);
     };
-    const int fields = (rk_out != nullptr) + (dens_out != nullptr) + (igrp_out != nullptr);
-    if (4LL * n * fields <= SCATTER_L2) {
-        run(rk_out, dens_out, igrp_out);
+    if (all <= SCATTER_L2) {
+        run(1, rk_out, dens_out, igrp_out);
         return;
     }
-    if (rk_out) run(rk_out, nullptr, nullptr);
-    if (dens_out) run(nullptr, dens_out, nullptr);
-    if (igrp_out) run(nullptr, nullptr, igrp_out);
+    int slices = (int)((bytes - 1) / SCATTER_L2) + 1;
+    if (slices > SCATTER_SLICES) slices = 1;
+    if (rk_out) run(slices, rk_out, nullptr, nullptr);
+    if (dens_out) run(slices, nullptr, dens_out, nullptr);
+    if (igrp_out) run(slices, nullptr, nullptr, igrp_out);
 }
 
 // every kernel that a device array of up to RSC_MAX particles goes through from the
@@ -1163,7 +1170,7 @@ void launch_scatter_fields(const int* perm, const float* rk, const float4* vel, 
 bool load_small_set_kernels()
 {
     bool ok = kernel_loaded(k_unpack_soa) && kernel_loaded(k_gather<true>) && kernel_loaded(k_up_boxes) &&
-              kernel_loaded(k_scatter_fields);
+              kernel_loaded(k_scatter_fields<false, false>);
     const bool clusters[] = {rs_cluster_ready<uint64_t, 1, 8>(), rs_cluster_ready<uint64_t, 1, 16>(),
                              rs_cluster_ready<uint64_t, 2, 16>()};
     ok = ok && kernel_loaded(k_rs_cluster<uint64_t, 1, 8>) && kernel_loaded(k_rs_cluster<uint64_t, 1, 16>) &&
