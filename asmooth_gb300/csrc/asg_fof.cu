@@ -78,42 +78,51 @@ k_fof_link(const float4* __restrict__ pos, const __grid_constant__ TreeView t, f
     bool bad = false;
     int rq = q;  // a root, now or earlier, of the query's component
     const TreeBox box = bundle_box(t, base / t.leaf, (min(base + 32, n) - 1) / t.leaf);
-    tree_walk(t,
-        [&](const TreeBox& c, int level, int id) {
-            // only partners with a larger sorted position are linked from q
-            const long long last = (((long long)id + 1) << (5 * level)) * t.leaf - 1;
-            return last > base && boxes_dist2_fast(box, c) <= bound;
-        },
-        [](const TreeBox&) { return true; },  // a test of each query gains less than it costs here
-        [&](int id) {
-            const int first = id * t.leaf, cnt = leaf_count(t, id);
-            if (!__any_sync(FM, active && first + cnt - 1 > q &&
-                                    point_box_fast(xq, tree_box(t, 0, id)) <= bound))
-                return true;
-            float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-            int rc = -1;
-            if (lane < cnt) {
-                p = pos[first + lane];
-                rc = uf_find(P, first + lane);
+    auto pass = [&](const TreeBox& c, int level, int id) {
+        // only partners with a larger sorted position are linked from q
+        const long long last = (((long long)id + 1) << (5 * level)) * t.leaf - 1;
+        return last > base && boxes_dist2_fast(box, c) <= bound;
+    };
+    auto link = [&](int id) {
+        const int first = id * t.leaf, cnt = leaf_count(t, id);
+        if (!__any_sync(FM, active && first + cnt - 1 > q &&
+                                point_box_fast(xq, tree_box(t, 0, id)) <= bound))
+            return;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        int rc = -1;
+        if (lane < cnt) {
+            p = pos[first + lane];
+            rc = uf_find(P, first + lane);
+        }
+        rq = uf_find(P, rq);
+        const int r0 = __shfl_sync(FM, rq, 0);
+        if (__all_sync(FM, rq == r0 && (rc < 0 || rc == r0))) return;
+        __syncwarp();
+        if (lane < cnt) cand[warp][lane] = make_float4(p.x, p.y, p.z, __int_as_float(rc));
+        __syncwarp();
+        for (int j = 0; j < cnt; ++j) {
+            const int s = first + j;
+            const float4 c = cand[warp][j];
+            if (active && s > q && __float_as_int(c.w) != rq &&
+                norm2_rn(xq.x, xq.y, xq.z, c.x, c.y, c.z) <= ll2) {
+                const int r = uf_union(P, rq, __float_as_int(c.w));
+                bad |= r < 0;
+                rq = r < 0 ? rq : r;
             }
-            rq = uf_find(P, rq);
-            const int r0 = __shfl_sync(FM, rq, 0);
-            if (__all_sync(FM, rq == r0 && (rc < 0 || rc == r0))) return true;
-            __syncwarp();
-            if (lane < cnt) cand[warp][lane] = make_float4(p.x, p.y, p.z, __int_as_float(rc));
-            __syncwarp();
-            for (int j = 0; j < cnt; ++j) {
-                const int s = first + j;
-                const float4 c = cand[warp][j];
-                if (active && s > q && __float_as_int(c.w) != rq &&
-                    norm2_rn(xq.x, xq.y, xq.z, c.x, c.y, c.z) <= ll2) {
-                    const int r = uf_union(P, rq, __float_as_int(c.w));
-                    bad |= r < 0;
-                    rq = r < 0 ? rq : r;
-                }
-            }
+        }
+    };
+    // A bundle's box that reaches a whole group may hold far more than its queries do (around
+    // a clump), so such a group is tested for each query: 262,144 particles in one Gaussian
+    // clump, a linking length of a fortieth of the mean separation, 348 -> 152 us.  The
+    // same test of every node costs other sets 1 to 4%.
+    tree_walk_groups(t, pass, [](int, int) { return true; }, [&](int g) {
+        unsigned m = group_leaves(t, g, pass);
+        if (m == ~0u && t.nlev > 1 &&
+            !__any_sync(FM, active && point_box_fast(xq, tree_box(t, 1, g)) <= bound))
             return true;
-        });
+        for (; m; m &= m - 1) link(g * 32 + __ffs(m) - 1);
+        return true;
+    });
     if (bad) atomicOr(err, ERR_UF);
 }
 
@@ -259,7 +268,7 @@ k_mark_halos(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
         const int per = t.leaf <= 16 ? 2 : 1, width = 32 / per;
         int turn = 0;
         if (inside)
-            tree_walk_groups(t, pass, [](const TreeBox&) { return true; }, [&](int g) {
+            tree_walk_groups(t, pass, [](int, int) { return true; }, [&](int g) {
                 if (turn++ % split != share) return true;
                 const unsigned m = group_leaves(t, g, pass);
                 // a warp's load covers `per` leaves; four loads in flight

@@ -539,7 +539,9 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
         }
         tree_walk(t,
             [&](const TreeBox& c, int, int) { return boxes_dist2_fast(box, c) <= reach; },
-            [&](const TreeBox& c) { return __any_sync(FULL, open && point_box_fast(xq, c) <= bound) != 0; },
+            [&](int level, int id) {
+                return __any_sync(FULL, open && point_box_fast(xq, tree_box(t, level, id)) <= bound) != 0;
+            },
             [&](int id) {
                 if (!__any_sync(FULL, open && point_box_fast(xq, tree_box(t, 0, id)) <= bound))
                     return true;
@@ -708,7 +710,9 @@ k_dens_scatter(const float4* __restrict__ pos, const __grid_constant__ TreeView 
     for (int o = 16; o > 0; o >>= 1) reach = fmaxf(reach, __shfl_xor_sync(FULL, reach, o));
     tree_walk(t, [&](const TreeBox& c, int, int) { return boxes_dist2_fast(box, c) <= reach; },
               // (70,000 particles in one Gaussian clump 573 -> 137 us)
-              [&](const TreeBox& c) { return __any_sync(FULL, point_box_fast(xq, c) <= bound) != 0; },
+              [&](int level, int id) {
+                  return __any_sync(FULL, point_box_fast(xq, tree_box(t, level, id)) <= bound) != 0;
+              },
               [&](int id) {
                   if (id % parts == part) visit(id);
                   return true;

@@ -83,7 +83,7 @@ __device__ __forceinline__ int leaf_count(const TreeView& t, int id)
 
 // Visits, in a fixed order, every group of 32 leaves (32 g ... 32 g + 31) all of whose
 // ancestors pass: pass(box, level, id) is asked by each lane for its own child, then
-// reach(box) by the whole warp for a child that passed, group(g) is called by the whole
+// reach(level, id) by the whole warp for a child that passed, group(g) is called by the whole
 // warp (and may end the walk by returning false).
 // Lane l keeps the pending children of the node open at level l.
 template <class Pass, class Reach, class Group>
@@ -115,7 +115,7 @@ __device__ __forceinline__ void tree_walk_groups(const TreeView& t, Pass pass, R
         }
         if (lane == L) pending = m & (m - 1);
         const int id = g * 32 + __ffs(m) - 1;
-        if (!reach(tree_box(t, L, id))) continue;
+        if (!reach(L, id)) continue;
         if (L == 1) {
             if (!group(id)) return;
         } else {

@@ -34,3 +34,18 @@ def test_clump_and_outskirts(oracle, monkeypatch, leaf, n, sigma):
     assert np.array_equal(idx33, ie)
     _, _, d64 = oracle.dens_from_lists(x, nbr, te)
     assert np.max(np.abs(p["dens"] - d64) / d64) <= 1e-5
+
+
+@pytest.mark.parametrize("n,sigma,ll", [(20000, 0.2, 0.002), (100000, 0.5, 0.004), (100000, 0.5, 0.03)])
+def test_groups_of_clump_and_outskirts(gpu_ctx, oracle, n, sigma, ll):
+    """FOF with a linking length far below the boxes of the outer bundles, which open
+    many nodes: the same groups as the exact oracle."""
+    import pyoracle as po
+
+    rng = np.random.default_rng(n)
+    x = np.clip(50.0 + sigma * rng.standard_t(2, (n, 3)), 0.0, 99.9).astype(np.float32)
+    p = api.make_particles(x)
+    ng = gpu_ctx.group_fof(p, 0.0, 100.0, ll)
+    lab, want = oracle.group_fof(x, 0.0, 100.0, np.float32(ll), exact=True)
+    assert ng == want
+    assert np.array_equal(po.canonical_groups(p["igrp"]), po.canonical_groups(lab))
