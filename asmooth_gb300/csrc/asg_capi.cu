@@ -236,6 +236,8 @@ int finish(asg_ctx* ctx, const char* what, Words a = {})
         cudaGetLastError();
         return fail(ctx, r, std::string(what) + ": " + ctx->last);
     }
+    // fetch() may return before the events recorded ahead of it are done
+    if (!ctx->pending.empty()) CK(cudaEventSynchronize(ctx->pending.back().second.second));
     for (auto& pe : ctx->pending) {
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, pe.second.first, pe.second.second) == cudaSuccess)
@@ -2041,7 +2043,8 @@ int asg_batch_run(asg_batch* b)
             if (rs && (!r || r == ASG_ERR_STATE)) r = fail(ctx, rs, b->sub[s]->last);
         }
         float ms = 0.0f;
-        if (cudaEventElapsedTime(&ms, b->e0, b->e1) == cudaSuccess) b->last_ms = ms;
+        if (cudaEventSynchronize(b->e1) == cudaSuccess && cudaEventElapsedTime(&ms, b->e0, b->e1) == cudaSuccess)
+            b->last_ms = ms;
         if (r != ASG_ERR_STATE) return r;  // ERR_CAP: the inputs outgrew the plan
         batch_drop_graph(b);
     }

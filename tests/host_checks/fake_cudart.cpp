@@ -34,6 +34,9 @@ std::map<char*, size_t> g_blocks;
 uint32_t g_entries = 0;
 unsigned long long g_pairs[3] = {};
 int g_timed = 0, g_fastest = INT_MAX;
+bool g_spin = false;              // the device flags allow the host to poll
+cudaError_t g_last = cudaSuccess;  // what cudaGetLastError returns next
+std::map<cudaEvent_t, bool> g_done;  // events, done when something waited for them
 
 void line(const std::string& s) { g_log += s + "\n"; }
 std::string num(unsigned long long v) { return std::to_string(v); }
@@ -116,6 +119,9 @@ void fake_counts(uint32_t entries, unsigned long long pairs844, unsigned long lo
     g_pairs[1] = pairs884;
     g_pairs[2] = pairs888;
 }
+
+// contexts created from now on may poll for their results instead of waiting
+void fake_spin(int on) { g_spin = on != 0; }
 
 // of the times that are asked for, the n-th from now on is the shortest
 void fake_fastest(int n)
@@ -240,7 +246,7 @@ cudaError_t cudaGetDevice(int* d)
 }
 cudaError_t cudaGetDeviceFlags(unsigned* f)
 {
-    *f = cudaDeviceScheduleBlockingSync;
+    *f = g_spin ? cudaDeviceScheduleAuto : cudaDeviceScheduleBlockingSync;
     return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int)
@@ -248,12 +254,21 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int)
     *v = 152;
     return cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
-cudaError_t cudaPeekAtLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError()
+{
+    const cudaError_t e = g_last;
+    g_last = cudaSuccess;
+    return e;
+}
+cudaError_t cudaPeekAtLastError() { return g_last; }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return handle(s); }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t)
+{
+    for (auto& e : g_done) e.second = true;
+    return cudaSuccess;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode)
 {
@@ -268,10 +283,19 @@ cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g)
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return handle(e); }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return handle(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t)
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t)
 {
+    g_done[e] = false;
+    return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t last)
+{
+    for (auto& e : g_done) e.second |= e.first <= last;  // those recorded before it, too
+    return cudaSuccess;
+}
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t a, cudaEvent_t b)
+{
+    if (!g_done[a] || !g_done[b]) return g_last = cudaErrorNotReady;
     *ms = (float)std::abs((long long)++g_timed - g_fastest);
     return cudaSuccess;
 }

@@ -48,6 +48,7 @@ def fresh_fake(fake, tmp_path):
 def fresh(fake):
     fake.fake_counts(0, 0, 0, 0)
     fake.fake_fastest(10 ** 6)
+    fake.fake_spin(0)
     fake.fake_clear()
 
 
@@ -254,3 +255,25 @@ def test_preparing_call_loads_what_a_search_launches(fresh_fake):
     launched = {ln[1] for ln in lines if ln[0] == "launch"}
     assert len(launched) > 10 and launched <= loaded
     assert not any(ln[0] == "malloc" for ln in lines)
+
+
+def test_times_are_read_from_events_that_are_done(fake):
+    """A call that polls for its results returns when a kernel has stored them, which
+    says nothing of the events recorded before it: times are read after a wait for them,
+    and an event that is not done would leave an error for the next call."""
+    fake.fake_spin(1)
+    ctx = context(fake)
+    assert fake.asg_set_timing(ctx, 1) == 0
+    x = np.zeros((100, 3), np.float32)
+    ms = np.zeros(10)
+    for _ in range(2):
+        assert fake.asg_load_particles_device(ctx, x.ctypes.data, None, None, None, 100, 0.0, 1.0) == 0
+        assert fake.asg_run_neighbor_search(ctx) == 0
+    assert fake.asg_phase_ms(ctx, ms.ctypes.data) == 0
+    assert (ms[[0, 1, 2, 4]] > 0).all()  # index, search, ties, density
+    b = batch(fake, ctx, [3000])
+    graph_ms = C.c_double(0.0)
+    assert fake.asg_batch_run(b) == 0 and fake.asg_batch_run(b) == 0
+    assert fake.asg_batch_stats(b, C.byref(graph_ms), None, None) == 0 and graph_ms.value > 0
+    fake.asg_batch_destroy(b)
+    fake.asg_destroy(ctx)
