@@ -738,9 +738,10 @@ __global__ void k_dens_finish(const unsigned long long* __restrict__ acc,
 // 120; in Plummer spheres 20,000 87, 61, 52; 65,000 99, 79, 98; 130,000 139, 125, 169.
 // (8 warps: never better than 4.)
 constexpr int KNN_SPLIT4 = 5 * 152, KNN_SPLIT2 = 18 * 152;
-// and k_dens_scatter 8, 4 and 2 (4099 uniform particles 45, 29, 23 and 17 us with 1, 2,
-// 4 and 8; 30,000 49, 35, 27 with 1, 2, 4; 130,000 71, 66 with 1, 2, 200,000 100, 101)
-constexpr int DENS_SPLIT8 = 152, DENS_SPLIT4 = 18 * 152, DENS_SPLIT2 = 32 * 152;
+// and k_dens_scatter 8, 4 and 2 (4099 uniform particles 45, 29, 20 and 14 us with 1, 2,
+// 4 and 8; 13,840 33, 25, 16 with 2, 4, 8 (in NFW halos 74, 61, 55); 30,000 49, 33, 25,
+// 23; 50,000 35, 33, 31; 130,000 71, 66 with 1, 2, 200,000 100, 101)
+constexpr int DENS_SPLIT8 = 10 * 152, DENS_SPLIT4 = 18 * 152, DENS_SPLIT2 = 32 * 152;
 
 static int knn_blocks(int n) { return (n + KNN_WARPS * 32 - 1) / (KNN_WARPS * 32); }
 

@@ -1,8 +1,8 @@
 """GPU test of the search where a bundle's particles lie far apart around a dense
 clump, so that its box holds most of the others while each of its radii reaches
 few: the 33rd keys equal the oracle's exactly and dens is within 1e-5 of the FP64 sum
-over the oracle's lists, with 4, 2 and 1 warps per bundle, leaf lists that overflow,
-and leaves of other sizes."""
+over the oracle's lists, with 4, 2 and 1 warps per bundle (in the density 8, 4 and 2),
+leaf lists that overflow, and leaves of other sizes."""
 import os
 
 import numpy as np
@@ -16,7 +16,7 @@ NTHREADS = os.cpu_count() or 1
 
 
 @pytest.mark.parametrize("leaf", ["", "5", "32"])
-@pytest.mark.parametrize("n,sigma", [(3000, 0.5), (20000, 0.2), (60000, 0.05), (100000, 0.5)])
+@pytest.mark.parametrize("n,sigma", [(3000, 0.5), (20000, 0.2), (48640, 0.2), (48641, 0.2), (60000, 0.05), (100000, 0.5)])
 def test_clump_and_outskirts(oracle, monkeypatch, leaf, n, sigma):
     if leaf:
         monkeypatch.setenv("ASG_LEAF_SIZE", leaf)
