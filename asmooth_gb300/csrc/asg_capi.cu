@@ -276,23 +276,27 @@ int alloc_set(asg_ctx* ctx, int n)
 {
     const size_t N = (size_t)n;
     int r = 0;
-    r |= grow(ctx, ctx->rec_in, 32 * N);
-    r |= grow(ctx, ctx->rk_in, 4 * N);
-    r |= grow(ctx, ctx->keys0, 8 * N);
-    r |= grow(ctx, ctx->keys1, 8 * N);
-    r |= grow(ctx, ctx->vals0, 4 * N);
-    r |= grow(ctx, ctx->vals1, 4 * N);
-    r |= grow(ctx, ctx->sort_tmp, radix_sort_temp_bytes(n));
-    r |= grow(ctx, ctx->pos, 16 * N);
-    r |= grow(ctx, ctx->vel, 16 * N);
-    r |= grow(ctx, ctx->igrp, 4 * N);
-    r |= grow(ctx, ctx->rk, 4 * N);
-    r |= grow(ctx, ctx->t33, 4 * N);
-    r |= grow(ctx, ctx->idx33, 4 * N);
-    r |= grow(ctx, ctx->boxes, tree_box_bytes(n, ctx->leaf));
-    r |= grow(ctx, ctx->dacc, 8 * N);
-    r |= grow(ctx, ctx->dexp, 4 * N);
-    r |= grow(ctx, ctx->blist, 4 * knn_list_words(n));
+    auto need = [&](Buf& b, size_t bytes) {
+        if (b.cap < bytes) ctx->loaded = ctx->knn_done = false;  // the loaded set goes with its arrays
+        r |= grow(ctx, b, bytes);
+    };
+    need(ctx->rec_in, 32 * N);
+    need(ctx->rk_in, 4 * N);
+    need(ctx->keys0, 8 * N);
+    need(ctx->keys1, 8 * N);
+    need(ctx->vals0, 4 * N);
+    need(ctx->vals1, 4 * N);
+    need(ctx->sort_tmp, radix_sort_temp_bytes(n));
+    need(ctx->pos, 16 * N);
+    need(ctx->vel, 16 * N);
+    need(ctx->igrp, 4 * N);
+    need(ctx->rk, 4 * N);
+    need(ctx->t33, 4 * N);
+    need(ctx->idx33, 4 * N);
+    need(ctx->boxes, tree_box_bytes(n, ctx->leaf));
+    need(ctx->dacc, 8 * N);
+    need(ctx->dexp, 4 * N);
+    need(ctx->blist, 4 * knn_list_words(n));
     return r ? ASG_ERR_NOMEM : 0;
 }
 
@@ -720,6 +724,7 @@ int asg_load_periodic_cube(asg_ctx* ctx, const asg_particle* p, int np_local, fl
     if (int r = check_shell(ctx, np_local, boxsize, buffer_factor)) return r;
     CK(cudaSetDevice(ctx->device));
     ctx->loaded = false;
+    ctx->dec_n = 0;
     const ShellIn L = shell_in_layout(np_local);
     if (int r = grow(ctx, ctx->sh_in, L.total)) return r;
     if (int r = grow(ctx, ctx->aos, sizeof(asg_particle) * (size_t)np_local)) return r;
@@ -741,6 +746,7 @@ int asg_load_periodic_cube_device(asg_ctx* ctx, const float* d_x, const float* d
     if (int r = check_shell(ctx, np_local, boxsize, buffer_factor)) return r;
     CK(cudaSetDevice(ctx->device));
     ctx->loaded = false;
+    ctx->dec_n = 0;
     const ShellIn L = shell_in_layout(np_local);
     if (int r = grow(ctx, ctx->sh_in, L.total)) return r;
     unsigned char* b = P<unsigned char>(ctx->sh_in);
@@ -1109,6 +1115,8 @@ static int queue_deposit(asg_ctx* ctx, float boxsize, const int* ncs, int n_nc, 
         MeshJob& j = p.job[k];
         int nt = 1;
         for (int a = 0; a < 3; ++a) nt *= j.tiles[a] = (nc + (1 << p.shift[a]) - 1) >> p.shift[a];
+        mb.nc = 0;  // no mesh if its array cannot be had
+        mb.words = 0;
         if (int r = grow(ctx, mb.mesh, 4 * nm)) return r;
         if (int r = grow(ctx, mb.partial, 16 * (size_t)nt)) return r;
         mb.nc = nc;

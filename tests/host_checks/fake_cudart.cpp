@@ -13,6 +13,7 @@
 #include <sys/mman.h>
 
 #include <climits>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -36,6 +37,7 @@ unsigned long long g_pairs[3] = {};
 int g_timed = 0, g_fastest = INT_MAX;
 bool g_spin = false;              // the device flags allow the host to poll
 cudaError_t g_last = cudaSuccess;  // what cudaGetLastError returns next
+size_t g_largest = SIZE_MAX;       // device blocks of more bytes are refused
 std::map<cudaEvent_t, bool> g_done;  // events, done when something waited for them
 
 void line(const std::string& s) { g_log += s + "\n"; }
@@ -123,6 +125,9 @@ void fake_counts(uint32_t entries, unsigned long long pairs844, unsigned long lo
 // contexts created from now on may poll for their results instead of waiting
 void fake_spin(int on) { g_spin = on != 0; }
 
+// device memory has no room for a block of more bytes than this
+void fake_largest(size_t bytes) { g_largest = bytes; }
+
 // of the times that are asked for, the n-th from now on is the shortest
 void fake_fastest(int n)
 {
@@ -185,7 +190,7 @@ cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunch
 cudaError_t cudaMalloc(void** p, size_t bytes)
 {
     line("malloc " + num(bytes));
-    *p = block(bytes);
+    *p = bytes > g_largest ? nullptr : block(bytes);
     return *p ? cudaSuccess : cudaErrorMemoryAllocation;
 }
 cudaError_t cudaFree(void* p)

@@ -20,6 +20,7 @@ def bind(so):
         getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
     lib.fake_log.restype = C.c_char_p
     lib.fake_counts.argtypes = [C.c_uint32] + 3 * [C.c_ulonglong]
+    lib.fake_largest.argtypes = [C.c_size_t]
     lib.path = so
     return lib
 
@@ -49,6 +50,7 @@ def fresh(fake):
     fake.fake_counts(0, 0, 0, 0)
     fake.fake_fastest(10 ** 6)
     fake.fake_spin(0)
+    fake.fake_largest(2 ** 64 - 1)
     fake.fake_clear()
 
 
@@ -276,4 +278,50 @@ def test_times_are_read_from_events_that_are_done(fake):
     assert fake.asg_batch_run(b) == 0 and fake.asg_batch_run(b) == 0
     assert fake.asg_batch_stats(b, C.byref(graph_ms), None, None) == 0 and graph_ms.value > 0
     fake.asg_batch_destroy(b)
+    fake.asg_destroy(ctx)
+
+
+def test_out_of_memory_leaves_nothing_half_loaded(fake):
+    """A load that finds no memory takes the loaded set's arrays with it, a decode the
+    decoded particles', a deposit the mesh's: calls on them are refused, and no kernel
+    runs on arrays that are gone."""
+    STATE, NOMEM, ARG = -10, -3, -1
+    ctx = context(fake)
+    x = np.zeros((200_000, 3), np.float32)
+    p, out = x.ctypes.data, np.zeros(200_000, np.float32).ctypes.data
+    n_out, groups = C.c_int(0), C.c_int(0)
+    nc = np.asarray([16], np.int32)
+
+    def load(n):
+        return fake.asg_load_particles_device(ctx, p, None, None, None, n, 0.0, 1.0)
+
+    def deposit():
+        return fake.asg_run_deposit(ctx, 1.0, nc.ctypes.data, 1, -1, 0, None, 0, None)
+
+    assert load(100) == 0 and fake.asg_run_neighbor_search(ctx) == 0 and deposit() == 0
+    assert fake.asg_load_periodic_cube_device(ctx, p, None, 100, 1.0, 0.1, None, None) != NOMEM
+    assert load(100) == 0 and fake.asg_run_neighbor_search(ctx) == 0
+    for largest in (1 << 20, 5 << 20):  # no array of the larger set fits; some do
+        fake.fake_largest(largest)
+        assert load(200_000) == NOMEM
+        log(fake)
+        assert fake.asg_run_neighbor_search(ctx) == STATE and deposit() == STATE
+        assert fake.asg_get_knn(ctx, None, None) == STATE
+        assert fake.asg_run_fof(ctx, 0.5, C.byref(groups)) == STATE
+        assert fake.asg_store_fields_device(ctx, out, out, None) == STATE
+        assert not [ln for ln in log(fake) if ln[0] == "launch"]
+    assert fake.asg_load_periodic_cube_device(ctx, p, None, 200_000, 1.0, 0.1, None, None) == NOMEM
+    log(fake)
+    assert fake.asg_load_decoded_periodic(ctx, 1.0, 0.1, C.byref(n_out), None) == STATE
+    assert fake.asg_copy_decoded(ctx, p) == STATE
+    assert not [ln for ln in log(fake) if ln[0] == "launch"]
+    assert load(100) == 0
+    nc[0] = 200
+    assert deposit() == NOMEM
+    log(fake)
+    assert fake.asg_run_normalise(ctx, 0) == ARG
+    assert fake.asg_copy_mesh(ctx, 0, out) == ARG
+    assert not [ln for ln in log(fake) if ln[0] == "launch"]
+    fake.fake_largest(2 ** 64 - 1)
+    assert load(200_000) == 0 and fake.asg_run_neighbor_search(ctx) == 0
     fake.asg_destroy(ctx)
