@@ -464,7 +464,6 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
     const int* bl = blist ? blist + (size_t)(base >> 5) * (KNN_LIST + 1) : nullptr;
     const int nlist = bl && t.leaf <= 16 ? bl[0] : -1;
     if (nlist >= 0 && __popc(few) <= TIE_FEW) {
-        bool left = false;  // a query that this form cannot resolve
         for (; few; few &= few - 1) {
             const int l = __ffs(few) - 1;
             const float x = __shfl_sync(FULL, xq.x, l), y = __shfl_sync(FULL, xq.y, l), z = __shfl_sync(FULL, xq.z, l);
@@ -495,20 +494,20 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
                     }
                 }
             }
-            const int rank = K_NN - less;  // position of the 33rd key among all the ties
+            // position of the 33rd key among all the ties: at most 32, as the query itself is
+            // nearer than any T > 0 (T = 0 is reported as ERR_ZERO_RK, whatever the index)
+            const int rank = K_NN - less;
             const int found = __shfl_sync(FULL, tie, (rank - 1) & 31);
             if (rank < 1 || rank > eq) {
                 if (lane == l) {
                     atomicOr(err, ERR_FEW);
                     idx33[q] = -1;
                 }
-            } else if (rank <= 32) {
-                if (lane == l) idx33[q] = found;
-            } else {
-                left = true;
+            } else if (lane == l) {
+                idx33[q] = found;
             }
         }
-        if (!left) return;
+        return;
     }
     int nless = 0, neq = 0;
     int need = 0;          // rank of the wanted index among the ties above floor
