@@ -201,7 +201,6 @@ __device__ __forceinline__ float max3f(float a, float b, float c)
 // a point with norm2_rn <= t is never pruned (t = +inf stays +inf)
 __device__ __forceinline__ float prune_bound(float t) { return __fmul_rn(t, 1.0f + 0x1p-21f); }
 
-// double-float accumulation (Knuth two-sum): hi + lo carries ~48 bits
 // the same (hi, lo) as two_sum_acc for hi >= 0 and x >= 0: Fast2Sum on the
 // larger and the smaller operand gives the same rounded sum and the same exact
 // error, with a shorter dependency chain
@@ -214,6 +213,7 @@ __device__ __forceinline__ void two_sum_acc_nonneg(float& hi, float& lo, float x
     lo = __fadd_rn(lo, e);
 }
 
+// double-float accumulation (Knuth two-sum): hi + lo carries ~48 bits
 __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x)
 {
     const float s = __fadd_rn(hi, x);

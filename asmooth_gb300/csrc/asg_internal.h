@@ -27,7 +27,7 @@ struct TreeView {
     int nlev;                    // levels, level 0 = leaves; the top one has at most 32 boxes
     int cnt[TREE_LEVELS];        // boxes of each level: ceil(n / leaf), then ceil(below / 32)
     long long off[TREE_LEVELS];  // first box of each level in `box`
-    const float4* box;           // two float4 per box: lo.xyz hi.x | hi.yz 0 0
+    const float4* box;           // two float4 per box: lo.x hi.x lo.y hi.y | lo.z hi.z 0 0
 };
 // the tree's shape for n particles (box not set), and the bytes of its boxes
 TreeView tree_shape(int n, int leaf);

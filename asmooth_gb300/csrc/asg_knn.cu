@@ -416,7 +416,6 @@ k_knn_t33(const float4* __restrict__ pos, const __grid_constant__ TreeView t,
 // integer atomics make the total independent of the order of the leaves.
 constexpr int FIX_BITS = 40;
 
-
 // e_j with hinv_j^3 <= 2^e_j up to rounding: minus the exponent of rk^3
 __device__ __forceinline__ int dens_exponent(float rk)
 {
