@@ -49,3 +49,24 @@ def test_groups_of_clump_and_outskirts(gpu_ctx, oracle, n, sigma, ll):
     lab, want = oracle.group_fof(x, 0.0, 100.0, np.float32(ll), exact=True)
     assert ng == want
     assert np.array_equal(po.canonical_groups(p["igrp"]), po.canonical_groups(lab))
+
+
+@pytest.mark.parametrize("leaf", ["", "5", "32"])
+@pytest.mark.parametrize("n,ll", [(33, 0.5), (40000, 0.02), (150000, 0.1), (150000, 0.4)])
+def test_groups_of_a_sheet(oracle, monkeypatch, leaf, n, ll):
+    """FOF in a thin sheet across the middle of the box, which the curve leaves and
+    enters again, so that some bundles' boxes span a part of it."""
+    import pyoracle as po
+
+    if leaf:
+        monkeypatch.setenv("ASG_LEAF_SIZE", leaf)
+    rng = np.random.default_rng(n)
+    x = rng.uniform(0, 100.0, (n, 3))
+    x[:, 2] = 50.0 + 0.1 * rng.normal(size=n)
+    x = np.clip(x, 0.0, 99.99).astype(np.float32)
+    p = api.make_particles(x)
+    with api.Context(0) as ctx:
+        ng = ctx.group_fof(p, 0.0, 100.0, ll)
+    lab, want = oracle.group_fof(x, 0.0, 100.0, np.float32(ll), exact=True)
+    assert ng == want
+    assert np.array_equal(po.canonical_groups(p["igrp"]), po.canonical_groups(lab))
