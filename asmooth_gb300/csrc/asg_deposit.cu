@@ -1240,7 +1240,9 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
 // MERGE_FEW items by itself, in item order; for a tile of more, a CTA's 8 warps add
 // an eighth of the items each and the eight sums are added in order (n, c and halo
 // as double-floats throughout).  One thread per cell over all items was a chain of
-// loads: 73 us for the 36 tiles of about 36 items of a 13,840-particle set, so 14.
+// loads: 73 us for the 36 tiles of about 36 items of a 13,840-particle set, so 14.  Where
+// nearly all pairs fall into few tiles, a CTA for all cells of each was the chain: n alone
+// of 300,000 particles in one Gaussian clump 641 -> 247 us.
 // item_tot (the tensor-core deposit): the FP64 mass of every item; null: the
 // mass is summed from the merged cells.
 constexpr int MERGE_WARPS = 8;
@@ -1337,15 +1339,17 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
         }
     };
 
-    // ---- tiles of many items first, a CTA each ----
-    for (int k = blockIdx.x; k < many; k += gridDim.x) {
-        const int tile = (int)merge[total_tiles - 1 - k];
+    // ---- tiles of many items first, a CTA each, or for each 128 cells of few such tiles
+    // (not where the cells give the mass) ----
+    const int shares = item_tot && many <= (int)gridDim.x / (cells / 128) ? cells / 128 : 1;
+    for (int k = blockIdx.x; k < many * shares; k += gridDim.x) {
+        const int tile = (int)merge[total_tiles - 1 - k / shares], share = k % shares;
         const int i0 = (int)item_off[tile], i1 = (int)item_off[tile + 1];
         const int a0 = i0 + (int)((long long)(i1 - i0) * w / MERGE_WARPS);
         const int a1 = i0 + (int)((long long)(i1 - i0) * (w + 1) / MERGE_WARPS);
         const TileGeo g = tile_geo(P, tile);
         double sn = 0.0, sh = 0.0;
-        for (int c = 4 * lane; c < cells; c += 128) {
+        for (int c = 4 * lane + 128 * share; c < cells; c += 128 * shares) {
             MergeSums m;
             sum_items(a0, a1, c, m);
 #pragma unroll
@@ -1359,6 +1363,7 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
             }
             __syncthreads();  // sums is written again
         }
+        if (share) continue;
         sum_mass(a0, a1, sn, sh);
         if (lane == 0) {
             mass[0][w] = sn;
