@@ -24,7 +24,7 @@ namespace asg {
 constexpr int FOF_WARPS = 4;
 constexpr unsigned FM = 0xffffffffu;
 constexpr int UF_LIMIT = 1 << 20;
-constexpr int FOF_MANY = 16;  // leaves of a group
+constexpr int FOF_MANY = 8;  // leaves of a group
 
 __device__ __forceinline__ int uf_find(int* P, int x)
 {
@@ -114,9 +114,9 @@ k_fof_link(const float4* __restrict__ pos, const __grid_constant__ TreeView t, f
     };
     // A bundle's box that reaches much of a group may hold far more than its queries do (around
     // a clump, or where the curve leaves the set and comes back elsewhere), so such a group
-    // is tested for each query: at 16 of 32 leaves 3,000,000 particles in a sheet across the
-    // box 1000 -> 627 us, 300,000 along a line 959 -> 290, 262,144 in one Gaussian clump
-    // 348 -> 148 (all 32 leaves: the first two as without the test).  The same test of every
+    // is tested for each query: at 8 of 32 leaves 3,000,000 particles in a sheet across the
+    // box 1000 -> 623 us, 300,000 along a line 959 -> 284, 262,144 in one Gaussian clump
+    // 348 -> 134 (at 16 leaves 627, 290, 148, at 32 1000, 959, 179).  The same test of every
     // group or node, or once some leaves were in vain, costs other sets 1 to 4%.
     tree_walk_groups(t, pass, [](int, int) { return true; }, [&](int g) {
         unsigned m = group_leaves(t, g, pass);
