@@ -677,7 +677,7 @@ k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositP
                 uint32_t max_items, const uint32_t* __restrict__ item_tile,
                 const uint32_t* __restrict__ tentry, const uint32_t* __restrict__ ekeys,
                 const uint2* __restrict__ list, const uint32_t* __restrict__ first,
-                float* __restrict__ partial, int* __restrict__ counters)
+                float* __restrict__ partial, double* __restrict__ item_tot, int* __restrict__ counters)
 {
     grid_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -797,30 +797,38 @@ k_deposit_items(const float4* __restrict__ rec, const __grid_constant__ DepositP
         }
 
         // ---- write: final tile when alone, partial tile otherwise ----
+        double sn = 0.0, sh = 0.0;
         if (nseg > 1) {
             float* pt = partial + (size_t)item * TC * partial_words(P);
+            float nh = 0.f, nl = 0.f, hh = 0.f, hl = 0.f;  // the mass of the lane's cells
             for (int e = lane; e < TC; e += 32) {
                 const int slot = tile_slot(e & (TS - 1), (e >> 3) & (TS - 1), e >> 6);
                 const float4 A = S.a[slot];
                 const float4 B = S.b[slot];
+                two_sum_acc_nonneg(nh, nl, A.x);
+                nl = __fadd_rn(nl, A.y);
+                two_sum_acc_nonneg(hh, hl, B.w);
+                hl = __fadd_rn(hl, S.hl[slot]);
                 pt[e] = A.x; pt[TC + e] = A.y;
                 if (P.density_only) continue;
                 pt[2 * TC + e] = A.z; pt[3 * TC + e] = A.w;
                 pt[4 * TC + e] = B.x; pt[5 * TC + e] = B.y; pt[6 * TC + e] = B.z;
                 pt[7 * TC + e] = B.w; pt[8 * TC + e] = S.hl[slot];
             }
+            sn = (double)nh + (double)nl;
+            sh = (double)hh + (double)hl;
         } else {
-            double sn = 0.0, sh = 0.0;
             write_tile(S, P, g, sn, sh, lane);
+        }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                sn += __shfl_down_sync(FULLM, sn, o);
-                sh += __shfl_down_sync(FULLM, sh, o);
-            }
-            if (lane == 0) {
-                J.partial[2 * g.local] = sn;
-                J.partial[2 * g.local + 1] = sh;
-            }
+        for (int o = 16; o > 0; o >>= 1) {
+            sn += __shfl_down_sync(FULLM, sn, o);
+            sh += __shfl_down_sync(FULLM, sh, o);
+        }
+        if (lane == 0) {
+            double* mass = nseg > 1 ? item_tot + 2 * (size_t)item : J.partial + 2 * (size_t)g.local;
+            mass[0] = sn;
+            mass[1] = sh;
         }
         __syncwarp();  // the next item clears the tile
     }
@@ -1243,8 +1251,7 @@ k_deposit_mma(const float4* __restrict__ rec, const __grid_constant__ DepositPar
 // loads: 73 us for the 36 tiles of about 36 items of a 13,840-particle set, so 14.  Where
 // nearly all pairs fall into few tiles, a CTA for all cells of each was the chain: n alone
 // of 300,000 particles in one Gaussian clump 641 -> 247 us.
-// item_tot (the tensor-core deposit): the FP64 mass of every item; null: the
-// mass is summed from the merged cells.
+// item_tot: the FP64 mass of every item.
 constexpr int MERGE_WARPS = 8;
 static_assert(MERGE_WARPS <= 32, "one lane per warp's mass");
 
@@ -1302,7 +1309,7 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
         for (int it = a0; it < a1; ++it)
             m.add(partial + (size_t)it * cells * words + e, (size_t)cells, all);
     };
-    auto store = [&](const TileGeo& g, int e, const MergeSums& m, double& sn, double& sh) {
+    auto store = [&](const TileGeo& g, int e, const MergeSums& m) {
         const MeshJob& J = P.job[g.job];
         const size_t nc = (size_t)g.nc, nmesh = nc * nc * nc;
         const int ly = (e >> P.shift[0]) & ((1 << P.shift[1]) - 1), lz = e >> (P.shift[0] + P.shift[1]);
@@ -1312,10 +1319,6 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
             const int lx = (e & ((1 << P.shift[0]) - 1)) + i;
             if (lx >= g.E[0]) return;
             const size_t idx = ((size_t)(g.O[2] + lz) * nc + (g.O[1] + ly)) * nc + (g.O[0] + lx);
-            if (!item_tot) {
-                sn += (double)m.s[0][i] + (double)m.s[1][i];
-                sh += (double)m.s[7][i] + (double)m.s[8][i];
-            }
             J.mesh[idx] = __fadd_rn(m.s[0][i], m.s[1][i]);
             if (all) {
                 J.mesh[nmesh + idx] = __fadd_rn(m.s[7][i], m.s[8][i]);
@@ -1325,13 +1328,13 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
             }
         }
     };
-    // items [a0, a1)'s masses and the warp's cells', to lane 0
+    // the mass of items [a0, a1), to lane 0
     auto sum_mass = [&](int a0, int a1, double& sn, double& sh) {
-        if (item_tot)
-            for (int it = a0 + lane; it < a1; it += 32) {
-                sn += item_tot[2 * (size_t)it];
-                sh += item_tot[2 * (size_t)it + 1];
-            }
+        sn = sh = 0.0;
+        for (int it = a0 + lane; it < a1; it += 32) {
+            sn += item_tot[2 * (size_t)it];
+            sh += item_tot[2 * (size_t)it + 1];
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             sn += __shfl_down_sync(FULLM, sn, o);
@@ -1339,16 +1342,15 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
         }
     };
 
-    // ---- tiles of many items first, a CTA each, or for each 128 cells of few such tiles
-    // (not where the cells give the mass) ----
-    const int shares = item_tot && many <= (int)gridDim.x / (cells / 128) ? cells / 128 : 1;
+    // ---- tiles of many items first, a CTA each, or for each 128 cells of few such tiles ----
+    const int shares = many <= (int)gridDim.x / (cells / 128) ? cells / 128 : 1;
     for (int k = blockIdx.x; k < many * shares; k += gridDim.x) {
         const int tile = (int)merge[total_tiles - 1 - k / shares], share = k % shares;
         const int i0 = (int)item_off[tile], i1 = (int)item_off[tile + 1];
         const int a0 = i0 + (int)((long long)(i1 - i0) * w / MERGE_WARPS);
         const int a1 = i0 + (int)((long long)(i1 - i0) * (w + 1) / MERGE_WARPS);
         const TileGeo g = tile_geo(P, tile);
-        double sn = 0.0, sh = 0.0;
+        double sn, sh;
         for (int c = 4 * lane + 128 * share; c < cells; c += 128 * shares) {
             MergeSums m;
             sum_items(a0, a1, c, m);
@@ -1359,7 +1361,7 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
             __syncthreads();
             if (w == 0) {
                 for (int o = 1; o < MERGE_WARPS; ++o) m.add(&sums[o][0][4 * lane], 128, all);
-                store(g, c, m, sn, sh);
+                store(g, c, m);
             }
             __syncthreads();  // sums is written again
         }
@@ -1382,11 +1384,11 @@ k_merge_tiles(const __grid_constant__ DepositParams P, int total_tiles,
         const int tile = (int)merge[k];
         const int i0 = (int)item_off[tile], i1 = (int)item_off[tile + 1];
         const TileGeo g = tile_geo(P, tile);
-        double sn = 0.0, sh = 0.0;
+        double sn, sh;
         for (int c = 4 * lane; c < cells; c += 128) {
             MergeSums m;
             sum_items(i0, i1, c, m);
-            store(g, c, m, sn, sh);
+            store(g, c, m);
         }
         sum_mass(i0, i1, sn, sh);
         if (lane == 0) {
@@ -1556,9 +1558,8 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    double* item_tot = nullptr;
+    double* item_tot = deposit_item_totals(w.partial, max_items, p);
     if (p.mma) {
-        item_tot = deposit_item_totals(w.partial, max_items, p);
         auto run = [&](auto nch, auto wide) {
             constexpr int N = decltype(nch)::value;
             constexpr bool W = decltype(wide)::value;
@@ -1574,7 +1575,7 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
     } else {
         launch_persistent<k_deposit_items>(dev, sms, 32 * DEP_WARPS, DEP_WARPS * sizeof(WarpTile), s, w.rec, p,
                                            T, w.item_off, max_items, w.item_tile, w.tentry, keys, w.list,
-                                           w.first, w.partial, w.counters);
+                                           w.first, w.partial, item_tot, w.counters);
     }
     launch(k_merge_tiles, 4 * sms, 32 * MERGE_WARPS, 0, s, p, T, w.item_off, w.merge, w.counters,
                                                        w.partial, item_tot);
