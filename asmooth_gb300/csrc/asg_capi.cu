@@ -1736,8 +1736,8 @@ int batch_plan(asg_batch* b)
         asg_ctx* c = b->sub[(size_t)i % S];
         if (int r = batch_queue_item(b, c, i, nullptr)) return fail(ctx, r, c->last);
         DepositCap& cap = b->cap[(size_t)i];  // headroom for inputs that change between runs
-        cap.entries = c->dep_nentries + c->dep_nentries / 16 + 4096;
-        cap.pairs = c->dep_npairs + c->dep_npairs / 16 + 4096;
+        cap.entries = deposit_headroom(c->dep_nentries);
+        cap.pairs = deposit_headroom(c->dep_npairs);
         cap.tiles = c->dep_shape;
         max_entries = std::max(max_entries, cap.entries);
         const uint32_t items = deposit_max_items(c->dep_tiles_n, cap.pairs, c->dep_seg, false);

@@ -1582,6 +1582,9 @@ void launch_deposit_run(int n, const DepositParams& p, int total_tiles, uint32_t
     count_launches(5);
 }
 
+// (the sort numbers entries with 31 bits)
+uint32_t deposit_headroom(uint32_t n) { return (uint32_t)std::min((uint64_t)n + n / 16 + 4096, (uint64_t)INT_MAX); }
+
 // Work items that `npairs` pairs or fewer make: a partial one per tile, and as many
 // full ones as deposit_seg leaves, of 64 pairs at least.  (Room for ITEM_SHARE whatever
 // the pairs took 76 MB for the smallest deposit of six channels, 303 for n alone.)

@@ -154,6 +154,8 @@ size_t deposit_tile_bytes(int total_tiles);
 size_t deposit_entry_bytes(uint32_t entries);
 // the per-entry arrays of w inside one block of deposit_entry_bytes
 void deposit_entry_layout(void* base, uint32_t entries, DepositScratch& w);
+// the entries or pairs that a plan for n of them has room for: a sixteenth more
+uint32_t deposit_headroom(uint32_t n);
 // work items that `npairs` pairs make at most, with at most `most` pairs each
 uint32_t deposit_max_items(int total_tiles, uint32_t npairs, int most, bool n_alone);
 int deposit_default_mma();

@@ -208,6 +208,15 @@ def test_items_fit_the_room_for_them(fake, n_alone):
                         assert items <= room(tiles, planned, most, n_alone)
 
 
+def test_headroom_stays_within_the_sort(fake):
+    """A batch's plan has room for a sixteenth more entries, but no more than the sort
+    can number (a larger count would be negative there, and nothing sorted)."""
+    room = getattr(fake, "_ZN3asg16deposit_headroomEj")
+    room.restype, room.argtypes = C.c_uint32, [C.c_uint32]
+    for n in [0, 1, 1000, 10 ** 9, 2_021_157_000, 2_021_157_300, 2 ** 31 - 5000, 2 ** 31 - 1]:
+        assert room(n) == min(n + n // 16 + 4096, 2 ** 31 - 1) >= n
+
+
 def test_tuner_times_no_setting_twice(fake):
     """Leaves of 16 run the search in blocks of their own, so the warps per block are
     no setting there: 3 x 2 settings with leaves of 16, 3 x 2 x 2 with each other size,
