@@ -73,8 +73,8 @@ void exclusive_scan_u32(uint32_t* data, size_t n, void* temp, cudaStream_t s);
 // Leaves k_knn_t33 scanned, per 32-query bundle: word 0 = their count (-1 when
 // more than KNN_LIST), then the leaf numbers.  k_dens_scatter visits these
 // instead of walking the tree again, which takes long for the bundles at the edge
-// of a halo, whose lists are the longest: with room for 96 leaves k_dens_scatter
-// took 302 us on 377 k particles in NFW halos, for 128 246, 192 208, 256 206.
+// of a halo, whose lists are the longest: with room for 96 leaves the density
+// took 206 us on 377 k particles in NFW halos, for 128 211, 192 172, 256 171.
 constexpr int KNN_LIST = 192;
 inline size_t knn_list_words(int n) { return (size_t)((n + 31) / 32) * (KNN_LIST + 1); }
 // t33, rk = sqrtf(t33), idx33 = -1 (no tie at the 33rd) or -2 (ties to resolve);

@@ -170,10 +170,10 @@ __device__ __forceinline__ void knn_scan(unsigned warp_base, f32x2 qx, f32x2 qy,
 // of the true one while values wait in the queue.  The leaves scanned go to
 // blist for k_dens_scatter.
 //
-// Bound by instruction issue: 74% of issue slots busy, 18.3 K warp instructions
-// per bundle (a fifth of them the networks' min/max on the ALU pipe, 60% busy),
-// DRAM below 1%.  16.7 -> 11.0 ms on the 256^3 step (18.3 M particles) against
-// the binary radix tree with 27.7 K; 0.43 -> 0.27 ms at 377 k particles.
+// Bound by instruction issue: 74% of issue slots busy, 17.4 K warp instructions
+// per bundle of 2.5 M particles in NFW halos (a fifth of them the networks' min/max on
+// the ALU pipe, 54% busy), DRAM below 1%.  16.7 -> 10.3 ms on the 256^3 step (18.3 M
+// particles) against the binary radix tree; 0.43 -> 0.26 ms at 377 k particles.
 //
 // The walk goes up from the bundle's own leaf: the siblings of its leaves
 // first, then at every level the siblings of its ancestor.  A node is opened by
@@ -603,7 +603,7 @@ k_knn_ties(const float4* __restrict__ pos, const __grid_constant__ TreeView t, c
 // receivers and take every second query, so no lane idles; their integer sums
 // are added by a shuffle before the atomic.
 // PARTS: nparts warps share a bundle's leaves where bundles are few.
-// Bound by instruction issue (82% of slots busy, 11.3 K warp instructions per
+// Bound by instruction issue (79% of slots busy, 10.7 K warp instructions per
 // bundle, of which the distances and weights are half): 7.10 -> 6.09 ms on the
 // 256^3 step against radix-tree buckets of 22 particles on average.
 template <bool HALVES, bool PARTS>

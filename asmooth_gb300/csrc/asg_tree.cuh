@@ -9,8 +9,8 @@
 // Why 32 children and a box test against the whole bundle: a binary radix tree
 // walked with one test per query and child took about 115 dependent visits of
 // some 60 instructions per 32-query bundle on the 256^3 cube; here a bundle
-// opens about 17 nodes of some 40 instructions, and only the leaves whose box
-// reaches the bundle's largest radius (about 110, of which 49 hold work) get a
+// opens about 17 nodes of some 40 instructions, and only the nodes and leaves whose box
+// reaches the bundle's largest radius (about 110 leaves, of which 49 hold work) get a
 // test per query.
 #pragma once
 
